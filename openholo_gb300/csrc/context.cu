@@ -2,6 +2,7 @@
 #include "context.h"
 #include "fft_fast.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -89,9 +90,33 @@ oh_status scratch(oh_ctx* ctx, const char* name, size_t bytes, void** out) {
   return OH_OK;
 }
 
-bool factorize(int n, int* radix, int* nst) {
+// Cost of one stage of radix r per line element, in FP operations: its
+// butterfly plus what every stage pays (shared-memory round trip, twiddles,
+// barrier).
+static double stage_cost(int r) {
+  static const double bf[17] = {0, 0, 2, 5, 4, 7, 6, 12, 7, 9, 9, 22, 9, 26, 14, 11, 11};
+  return 14.0 + (r <= 16 ? bf[r] : 8.0 * r);
+}
+
+// Cheapest product of radices 2..16 for a 13-smooth m (memoised over divisors).
+static double cheapest(int m, std::map<int, std::pair<double, int>>& memo) {
+  if (m == 1) return 0.0;
+  auto it = memo.find(m);
+  if (it != memo.end()) return it->second.first;
+  std::pair<double, int> best{1e30, 0};
+  for (int r = 16; r >= 2; --r)
+    if (m % r == 0) {
+      const double c = stage_cost(r) + cheapest(m / r, memo);
+      if (c < best.first) best = {c, r};
+    }
+  memo[m] = best;
+  return best.first;
+}
+
+bool factorize(int n, int prec, int* radix, int* nst) {
   if (n < 1) return false;
-  // lengths with a compile-time schedule use exactly that schedule
+  // FP32 lengths with a compile-time schedule use exactly that schedule
+  if (prec == 0) {
 #define OH_SCHED_CASE(len, ...)                                   \
   if (n == len) {                                                  \
     const int rs[] = {__VA_ARGS__};                                \
@@ -99,22 +124,38 @@ bool factorize(int n, int* radix, int* nst) {
     for (int s = 0; s < *nst; ++s) radix[s] = rs[s];               \
     return true;                                                   \
   }
-  OH_FAST_SCHEDULES(OH_SCHED_CASE)
+    OH_FAST_SCHEDULES(OH_SCHED_CASE)
 #undef OH_SCHED_CASE
-  int m = n, s = 0;
-  int twos = 0;
-  while (m % 2 == 0) { m /= 2; ++twos; }
-  while (twos >= 3) { radix[s++] = 8; twos -= 3; }
-  if (twos == 2) radix[s++] = 4;
-  if (twos == 1) radix[s++] = 2;
-  while (m % 5 == 0) { radix[s++] = 5; m /= 5; }
-  while (m % 3 == 0) { radix[s++] = 3; m /= 3; }
-  for (int p = 7; m > 1; p += 2) {
-    if (p > kMaxGenericRadix) return false;
-    while (m % p == 0) { radix[s++] = p; m /= p; }
-    if (s > kMaxStages - 1) return false;
   }
-  if (s == 0) radix[s++] = 1;   // n == 1: identity
+  int m = n, s = 0;
+  for (int p = 61; p >= 17; p -= 2)       // composites never divide what is left of m
+    while (m % p == 0) {
+      bool prime = true;
+      for (int d = 3; d * d <= p; d += 2) prime = prime && p % d != 0;
+      if (!prime) break;
+      if (s > kMaxStages - 1) return false;
+      radix[s++] = p;
+      m /= p;
+    }
+  {
+    int k = m;
+    for (int p : {2, 3, 5, 7, 11, 13})
+      while (k % p == 0) k /= p;
+    if (k != 1) return false;             // a prime factor above 61
+  }
+  std::map<int, std::pair<double, int>> memo;
+  cheapest(m, memo);
+  while (m > 1) {
+    if (s > kMaxStages - 1) return false;
+    radix[s++] = memo[m].second;
+    m /= radix[s - 1];
+  }
+  if (s == 0) radix[s++] = 1;             // n == 1: identity
+  // large radices first; an odd radix last (its reads in the last stage, whole
+  // butterflies apart, spread over the banks without pads)
+  std::sort(radix, radix + s, [](int a, int b) { return a > b; });
+  for (int i = 0; i < s - 1; ++i)
+    if (radix[i] % 2 == 1 && radix[i] > 1 && radix[s - 1] % 2 == 0) std::swap(radix[i], radix[s - 1]);
   *nst = s;
   return true;
 }
@@ -142,18 +183,34 @@ oh_status get_plan(oh_ctx* ctx, int n, int prec, FFTPlan* out) {
   FFTPlan& pl = pb.plan;
   std::memset(&pl, 0, sizeof(pl));
   pl.n = n;
-  if (!factorize(n, pl.radix, &pl.nst))
+  if (!factorize(n, prec, pl.radix, &pl.nst))
     return fail(OH_ERR_UNSUPPORTED_SIZE, "FFT length " + std::to_string(n) + " has a prime factor above " + std::to_string(kMaxGenericRadix));
   if (pl.radix[0] == 1) pl.nst = 0;
-  int m = n;
+  auto divider = [](int d) { return d > 1 ? (uint32_t)(((1ull << 32) + d - 1) / d) : 0u; };
+  // pads only where they cost little shared memory (what fits without them
+  // must keep fitting)
+  const int rl = pl.nst ? pl.radix[pl.nst - 1] : 1;
+  pl.padr = rl % 2 == 0 && n <= 8192 ? rl : 0;
+  pl.mpad = divider(pl.padr);
+  pl.lens = pl.padr ? n + n / pl.padr : n;
+  int m = n, entries = 0;
   for (int s = 0; s < pl.nst; ++s) {
-    pl.q[s] = m / pl.radix[s];
-    pl.tws[s] = n / m;
-    m = pl.q[s];
+    const int q = m / pl.radix[s];
+    pl.q[s] = q;
+    pl.qs[s] = q > 1 && pl.padr ? q + q / pl.padr : q;
+    pl.mq[s] = divider(q);
+    pl.mnb[s] = divider(n / pl.radix[s]);
+    pl.two[s] = entries;
+    if (q > 1) entries += q * (pl.radix[s] - 1);
+    m = q;
   }
-  std::vector<int> perm, iperm(n);
+  std::vector<int> perm, tabs(3 * (size_t)n);      // perm, iperm, permp
   if (pl.nst == 0) { perm.assign(n, 0); } else build_perm(n, pl.radix, pl.nst, perm);
-  for (int k = 0; k < n; ++k) iperm[perm[k]] = k;
+  for (int k = 0; k < n; ++k) {
+    tabs[k] = perm[k];
+    tabs[n + perm[k]] = k;
+    tabs[2 * (size_t)n + k] = perm[k] + (pl.padr ? perm[k] / pl.padr : 0);
+  }
   // twiddles W_n^e = exp(-2 pi i e / n), evaluated in double with the angle
   // reduced to [0, pi/4] by symmetry so that both precisions get correctly
   // rounded-quality values.
@@ -179,26 +236,37 @@ oh_status get_plan(oh_ctx* ctx, int n, int prec, FFTPlan* out) {
     }
     c[e] = cs; sn[e] = -ss;   // forward twiddle exp(-i angle)
   }
-  size_t esz = prec ? sizeof(double2) : sizeof(float2);
+  // per-stage twiddles: W_{m_s}^{j f} = W_n^{j f n / m_s}
+  std::vector<int> ste;
+  ste.reserve(entries);
+  m = n;
+  for (int s = 0; s < pl.nst; ++s) {
+    const int q = pl.q[s], step = n / m;
+    if (q > 1)
+      for (int f = 1; f < pl.radix[s]; ++f)
+        for (int j = 0; j < q; ++j) ste.push_back((int)((long long)j * f * step % n));
+    m = q;
+  }
+  const size_t esz = prec ? sizeof(double2) : sizeof(float2);
   cudaError_t e1 = cudaMalloc(&pb.tw, esz * n);
-  cudaError_t e2 = cudaMalloc((void**)&pb.perm, sizeof(int) * n);
-  cudaError_t e3 = cudaMalloc((void**)&pb.iperm, sizeof(int) * n);
+  cudaError_t e2 = cudaMalloc(&pb.stw, esz * std::max(entries, 1));
+  cudaError_t e3 = cudaMalloc((void**)&pb.perm, sizeof(int) * tabs.size());
   if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
-    cudaFree(pb.tw); cudaFree(pb.perm); cudaFree(pb.iperm); cudaGetLastError();
+    cudaFree(pb.tw); cudaFree(pb.stw); cudaFree(pb.perm); cudaGetLastError();
     return fail(OH_ERR_ALLOC, "FFT plan tables");
   }
-  if (prec) {
-    std::vector<double2> t(n);
-    for (int e = 0; e < n; ++e) t[e] = make_double2(c[e], sn[e]);
-    OH_CUDA_TRY(cudaMemcpy(pb.tw, t.data(), esz * n, cudaMemcpyHostToDevice));
-  } else {
-    std::vector<float2> t(n);
-    for (int e = 0; e < n; ++e) t[e] = make_float2((float)c[e], (float)sn[e]);
-    OH_CUDA_TRY(cudaMemcpy(pb.tw, t.data(), esz * n, cudaMemcpyHostToDevice));
-  }
-  OH_CUDA_TRY(cudaMemcpy(pb.perm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  OH_CUDA_TRY(cudaMemcpy(pb.iperm, iperm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  pl.tw = pb.tw; pl.perm = pb.perm; pl.iperm = pb.iperm;
+  auto fill = [&](auto zero) -> cudaError_t {
+    typedef decltype(zero) C;
+    std::vector<C> t(n + ste.size());
+    for (int e = 0; e < n; ++e) { t[e].x = (decltype(zero.x))c[e]; t[e].y = (decltype(zero.x))sn[e]; }
+    for (size_t i = 0; i < ste.size(); ++i) t[n + i] = t[ste[i]];
+    cudaError_t e = cudaMemcpy(pb.tw, t.data(), sizeof(C) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !ste.empty()) e = cudaMemcpy(pb.stw, t.data() + n, sizeof(C) * ste.size(), cudaMemcpyHostToDevice);
+    return e;
+  };
+  OH_CUDA_TRY(prec ? fill(double2{}) : fill(float2{}));
+  OH_CUDA_TRY(cudaMemcpy(pb.perm, tabs.data(), sizeof(int) * tabs.size(), cudaMemcpyHostToDevice));
+  pl.tw = pb.tw; pl.stw = pb.stw; pl.perm = pb.perm; pl.iperm = pb.perm + n; pl.permp = pb.perm + 2 * (size_t)n;
   ctx->plans[key] = pb;
   *out = pl;
   return OH_OK;
@@ -268,7 +336,7 @@ oh_status oh_ctx_destroy(oh_ctx* ctx) {
   cudaDeviceSynchronize();
   drop_graphs(ctx);
   for (auto& kv : ctx->scratch) cudaFree(kv.second.p);
-  for (auto& kv : ctx->plans) { cudaFree(kv.second.tw); cudaFree(kv.second.perm); cudaFree(kv.second.iperm); }
+  for (auto& kv : ctx->plans) { cudaFree(kv.second.tw); cudaFree(kv.second.stw); cudaFree(kv.second.perm); }
   for (auto& m : ctx->marks) { cudaEventDestroy(m.a); cudaEventDestroy(m.b); }
   for (auto e : ctx->event_pool) cudaEventDestroy(e);
   cudaEventDestroy(ctx->last_done);

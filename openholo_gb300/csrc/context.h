@@ -44,7 +44,7 @@ struct oh_ctx {
   std::string tune_file;
   struct Buf { void* p = nullptr; size_t bytes = 0; };
   std::map<std::string, Buf> scratch;
-  struct PlanBufs { oh::FFTPlan plan; void* tw = nullptr; int* perm = nullptr; int* iperm = nullptr; };
+  struct PlanBufs { oh::FFTPlan plan; void* tw = nullptr; void* stw = nullptr; int* perm = nullptr; };
   std::map<std::pair<int, int>, PlanBufs> plans;   // key (n, precision)
   // optional per-kernel timing: events recorded around each launch on the
   // launching stream while `timing` is set
@@ -84,8 +84,9 @@ void drop_graphs(oh_ctx* ctx);
 // use.  Fails with OH_ERR_UNSUPPORTED_SIZE when n cannot be factored.
 oh_status get_plan(oh_ctx* ctx, int n, int prec, FFTPlan* out);
 
-// Radix schedule for n (empty when unsupported).
-bool factorize(int n, int* radix, int* nst);
+// Radix schedule for n in precision prec (0 = fp32, 1 = fp64); false when
+// unsupported.
+bool factorize(int n, int prec, int* radix, int* nst);
 
 // Largest dynamic shared memory a block may use on this device.
 size_t max_smem_per_block();

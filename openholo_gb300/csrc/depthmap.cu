@@ -33,110 +33,9 @@
 #include <vector>
 #include "context.h"
 #include "dm_batch.h"
-#include "dm_kernels.cuh"
+#include "dm_generic.cuh"
 
 namespace oh {
-
-template <typename R, int KMAX, int NY>
-__global__ void __launch_bounds__(512) dm_col_pass(DMArgs<R> a) {
-  typedef typename cplx_of<R>::type C;
-  extern __shared__ unsigned char smem_raw[];
-  const int W = a.W;
-  const int Py = a.Py;
-  C* buf = reinterpret_cast<C*>(smem_raw);
-  C* exw = buf + (size_t)Py * W;                  // [W]
-  R* lfxw = reinterpret_cast<R*>(exw + W);        // [W]
-  int* kyp = reinterpret_cast<int*>(lfxw + W);    // [Py] spectrum row held at storage position
-  const int s = blockIdx.x;
-  const int kx0 = s * W;
-  const int T = blockDim.x;
-  const int nel = Py * W;
-  for (int p = threadIdx.x; p < Py; p += T) {
-    int ky = a.ply.iperm[p] + a.hy; if (ky >= Py) ky -= Py;   // S[ky] = B[(ky - hy) mod Py]
-    kyp[p] = ky;
-  }
-  for (int w = threadIdx.x; w < W; w += T) lfxw[w] = a.lfx[kx0 + w];
-  C acc[KMAX];
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k) acc[k] = mk((R)0, (R)0);
-  __syncthreads();
-
-  for (int e = 0; e < a.n_entries; ++e) {
-    const int u = a.uslot_of_entry[e];
-    if (!a.slot_any[u]) continue;
-    const uint8_t* occ = a.occ + (size_t)u * a.occ_stride;
-    const C* src = a.Rbuf + ((size_t)u * a.nstrips + s) * a.pny * W;
-    for (int idx = threadIdx.x; idx < nel; idx += T) {
-      const int i = idx / W, w = idx - i * W;
-      int y = i - a.hy; if (y < 0) y += Py;
-      const int yl = y - a.oy;
-      C val = mk((R)0, (R)0);
-      if (yl >= 0 && yl < a.pny && occ[yl]) val = src[(size_t)yl * W + w];
-      buf[idx] = val;
-    }
-    if constexpr (sizeof(R) == 4) {
-      for (int w = threadIdx.x; w < W; w += T) exw[w] = a.exc[(size_t)e * a.Px + kx0 + w];
-    } else {
-      for (int w = threadIdx.x; w < W; w += T) exw[w] = a.cst[e];
-    }
-    block_fft_n<NY, -1>(buf, W, 1, W, a.ply, true);
-    const R kz = a.kzp[e];
-    const C* eyr = a.ey + (size_t)e * Py;
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) {
-      const int idx = threadIdx.x + k * T;
-      if (idx < nel) {
-        const int p = idx / W, w = idx - p * W;
-        const int ky = kyp[p];
-        const R sv = lfxw[w] + a.lfy[ky];
-        C h;
-        if constexpr (sizeof(R) == 4) {
-          // residual of k z' (1 - sqrt(1-s)) beyond the separable s/2 term:
-          // k z' s^2 / (2 (1 + sqrt(1-s))^2), |.| < a few rad
-          const R rt = sqrt((R)1 - sv);
-          const R den = (R)1 + rt;
-          const R psi = kz * sv * sv / ((R)2 * den * den);
-          float sn, cs;
-          __sincosf(psi, &sn, &cs);
-          C g = cmul(exw[w], eyr[ky]);
-          h = cmul(g, mk(cs, sn));
-        } else {
-          // direct reference formula H = exp(i k d sqrt(1 - s)), d = -z'
-          const double sval = sqrt(1.0 - (double)sv) * (-(double)kz);
-          double sn, cs;
-          sincos(sval, &sn, &cs);
-          h = cmul(exw[w], mk((R)cs, (R)sn));
-        }
-        acc[k] = cadd(acc[k], cmul(h, buf[idx]));
-      }
-    }
-    __syncthreads();
-  }
-
-  // SSB crop + move the spectrum into the inverse-transform input order:
-  // b[i] = Uc[(i - hy) mod Py]  ->  spectrum row ky goes to i = (ky + hy) mod Py
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k) {
-    const int idx = threadIdx.x + k * T;
-    if (idx < nel) {
-      const int p = idx / W, w = idx - p * W;
-      const int ky = kyp[p];
-      const int kx = kx0 + w;
-      if (a.spectrum) a.spectrum[(size_t)ky * a.Px + kx] = acc[k];
-      const bool keep = kx >= a.cx1 && kx <= a.cx2 && ky >= a.cy1 && ky <= a.cy2;
-      int i = ky + a.hy; if (i >= Py) i -= Py;
-      // each storage slot is written exactly once (ky is a permutation)
-      buf[i * W + w] = keep ? acc[k] : mk((R)0, (R)0);
-    }
-  }
-  block_fft_n<NY, 1>(buf, W, 1, W, a.ply, true);
-  for (int idx = threadIdx.x; idx < a.pny * W; idx += T) {
-    const int yl = idx / W, w = idx - yl * W;
-    int m = a.oy + yl - a.hy; if (m < 0) m += Py;   // out[y] = B[(y - hy) mod Py]
-    const C val = cmul(buf[a.ply.perm[m] * W + w], a.shy[yl]);
-    a.V[(size_t)yl * a.Px + kx0 + w] = val;
-  }
-}
 
 // ---------------------------------------------------------------------------
 // host side
@@ -213,7 +112,7 @@ static oh_status validate(const oh_depthmap_params* p) {
 // launching anything.
 // src (nullable): a complex source field [pny][pnx] (oh_c64 / oh_c128) taken
 // as the one layer, at z' = src_z, instead of the image/depth layers.
-template <typename R, int KMAX>
+template <typename R>
 static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const uint8_t* img,
                               const uint8_t* depth, const float* phase, void* fringe, void* field,
                               void* spectrum, cudaStream_t st, FrameInfo<R>* info = nullptr,
@@ -250,8 +149,8 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
     if (p->phase_mode == OH_PHASE_REFERENCE && !src) { rre = p->rand_phase_re; rim = p->rand_phase_im; }
     double cre = std::cos(k * z), cim = std::sin(k * z);
     double are = rre * cre - rim * cim, aim = rre * cim + rim * cre;
-    if (prec == 0) {
-      // fp32 path folds the constant exp(-i k z') of H into the entry constant
+    {
+      // the constant exp(-i k z') of H folded into the entry constant
       double hre = std::cos(-k * z), him = std::sin(-k * z);
       double bre = are * hre - aim * him, bim = are * him + aim * hre;
       are = bre; aim = bim;
@@ -294,7 +193,6 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   OH_TRY(get_plan(ctx, a.Py, prec, &a.ply));
 
   const size_t smax = max_smem_per_block();
-  const int T = 512;
   const int occ_stride = (a.pny + 15) & ~15;
   a.occ_stride = occ_stride;
   a.err = ctx->dev_err;
@@ -316,39 +214,37 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
         (size_t)col_layout(col_py, a.pny, 2, kColStripW, false, occ_stride, su.n_entries, col_tab).total <= smax)
       Wfast = 2;
   }
+  // Other columns and FP64 run the plan-driven passes (dm_generic.cuh) on
+  // strips of two columns (FP32, even rows) or one: either way two rows of a
+  // strip fill a 32-byte sector.  Columns too long for one block are refused.
   int W = Wfast;
   if (W == 0) {
-    for (int cand : {8, 4, 2, 1}) {
-      if (a.Px % cand) continue;
-      size_t sm = (size_t)cand * a.Py * sizeof(C) + cand * (sizeof(C) + sizeof(R)) + (size_t)a.Py * sizeof(int);
-      if (sm <= smax && cand * a.Py <= T * KMAX) { W = cand; break; }
-    }
+    if ((size_t)a.Py * (sizeof(C) + sizeof(int)) + sizeof(C) + sizeof(R) <= smax && a.Py <= (prec ? 9216 : 18432))
+      W = prec == 0 && a.Px % 2 == 0 ? 2 : 1;
   }
   if (W == 0) return fail(OH_ERR_UNSUPPORTED_SIZE, "padded column length " + std::to_string(a.Py) + " too long for the column pass");
   a.W = W; a.nstrips = a.Px / W;
-  a.lw = W == 8 ? 3 : W == 4 ? 2 : W == 2 ? 1 : 0;
+  a.lw = W == 2 ? 1 : 0;
   a.ey_perm = Wfast ? 1 : 0;
   // Render entries evenly spaced in z' with one entry constant: the fast
-  // column pass accumulates with the layer-step recurrence (the transfer
+  // column pass and the FP64 one accumulate with the layer-step recurrence (the transfer
   // function is exp(i z' Phi(fx, fy)) times that constant, so consecutive
   // entries differ by the factor exp(-i dz Phi)).  OH_DM_LAYER_STEP=0 keeps
   // the per-layer evaluation.
   a.horner = 0;
-  if (Wfast && su.n_entries >= 2) {
+  if ((Wfast || prec) && su.n_entries >= 2) {
     const char* ev = std::getenv("OH_DM_LAYER_STEP");
     const int n = su.n_entries;
     const double dz = (su.zp[n - 1] - su.zp[0]) / (n - 1);
     const double k = 2.0 * M_PI / p->lambda;
     bool even = dz != 0.0 && !(ev && std::atoi(ev) == 0);
     for (int e = 0; e < n && even; ++e) {
-      if (std::fabs(su.zp[e] - (su.zp[0] + e * dz)) * k > 1e-7) even = false;
+      // (the phase that multiplies the deviation is k g, about k / 1000)
+      if (std::fabs(su.zp[e] - (su.zp[0] + e * dz)) * k > (prec ? 1e-8 : 1e-7)) even = false;
       if (std::fabs(su.cre[e] - su.cre[0]) > 1e-12 || std::fabs(su.cim[e] - su.cim[0]) > 1e-12) even = false;
     }
     if (even) { a.horner = 1; a.dz = dz; a.kdz_pi = (float)(k * dz / M_PI); }
   }
-  bool fastx = false;
-  with_fast_n(a.Px, [&](auto nc) { fastx = decltype(nc)::value > 0; });
-  a.xs = (prec == 0 && fastx && Wfast) ? 1 : 0;
   int r0x = 0, r0y = 0;
   with_fast_n(a.Px, [&](auto nc) { if constexpr (decltype(nc)::value > 0) r0x = FastSched<decltype(nc)::value>::r0; });
   with_fast_n(a.Py, [&](auto nc) { if constexpr (decltype(nc)::value > 0) r0y = FastSched<decltype(nc)::value>::r0; });
@@ -415,13 +311,11 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
         col_p2 = a.fkeep == col_ssb_keep<NY>() && !ext_mode && (wcol == 2 ? col_pipe2<NY, 2>() : col_pipe2<NY, 1>());
     });
   }
-  const size_t smem_col =
-      Wfast ? (size_t)col_layout(col_py, a.pny, wcol, kColStripW, a.horner != 0, occ_stride, su.n_entries, col_tab,
-                                 col_p2).total
-            : (size_t)W * a.Py * sizeof(C) + W * (sizeof(C) + sizeof(R)) + (size_t)a.Py * sizeof(int);
   int row_tab = 0, row_ls = a.Px;
+  bool fastx = false;
   with_fast_n_if<sizeof(R) == 4>(a.Px, [&](auto nc) {
     if constexpr (decltype(nc)::value > 0) {
+      fastx = true;
       row_tab = FastSched<decltype(nc)::value>::tab1_entries;
       row_ls = RowPad<decltype(nc)::value>::LSMAX;
     }
@@ -430,7 +324,22 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
                                       (size_t)((a.pnx + 7) & ~7) * sizeof(int16_t)) +
                           16 * sizeof(uint32_t) + (kTwLo + (size_t)(a.Px + 63) / 64 + row_tab) * sizeof(C);
   const size_t smem_out = (size_t)a.Px * sizeof(C) + (kTwLo + (size_t)(a.Px + 63) / 64) * sizeof(C);
+  // (the plan-driven passes need less, but take the same rows)
   if (smem_row > smax || smem_out > smax) return fail(OH_ERR_UNSUPPORTED_SIZE, "padded row length " + std::to_string(a.Px) + " exceeds shared memory");
+  DMGenPlan gen{};
+  if (!fastx || !Wfast) {
+    a.spectrum = (C*)spectrum;
+    gen = dm_gen_plan<R>(a, smax);
+    if (prec && a.horner && gen.smem_col > smax) {      // no room for the step factors
+      a.horner = 0;
+      gen = dm_gen_plan<R>(a, smax);
+    }
+    if (!Wfast && gen.smem_col > smax)
+      return fail(OH_ERR_UNSUPPORTED_SIZE, "padded column length " + std::to_string(a.Py) + " too long for the column pass");
+  }
+  const size_t smem_col = Wfast ? (size_t)col_layout(col_py, a.pny, wcol, kColStripW, a.horner != 0, occ_stride,
+                                                     su.n_entries, col_tab, col_p2).total
+                                : gen.smem_col;
 
   // scratch
   void* ptr;
@@ -457,8 +366,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   size_t off = 0;
   auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
   size_t o_lut = carve(256 * sizeof(int16_t)), o_use = carve(nE * sizeof(int16_t)), o_kz = carve(nE * sizeof(R)),
-         o_cst = carve(nE * sizeof(C)), o_exc = carve(prec ? 0 : nE * a.Px * sizeof(C)),
-         o_ey = carve(prec ? 0 : nE * a.Py * sizeof(C)),
+         o_cst = carve(nE * sizeof(C)), o_exc = carve(nE * a.Px * sizeof(C)), o_ey = carve(nE * a.Py * sizeof(C)),
          o_eth = carve(a.ey_perm ? nE * a.Py * sizeof(R) : 0), o_lfx = carve(a.Px * sizeof(R)), o_lfy = carve(a.Py * sizeof(R)), o_lfyp = carve(a.Py * sizeof(R)),
          o_shy = carve(a.pny * sizeof(C)), o_shx = carve(a.pnx * sizeof(C)), o_any = carve(nU * sizeof(int)),
          o_dxh = carve(a.horner ? a.Px * sizeof(C) : 0), o_dyh = carve(a.horner ? a.Py * sizeof(C) : 0);
@@ -522,7 +430,8 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
       ctx->dm_setup_key = ks;
     }
   }
-  // the FP32 path uses the compile-time FFT schedules; FP64 the generic engine
+  // FP32 lengths with compile-time schedules run their kernels, the others and
+  // FP64 the plan-driven ones
   oh_status rs = OH_OK;
   for (int chunk = 0; chunk < nchunks; ++chunk) {
   a.slot0 = (int)(chunk * lc);
@@ -533,12 +442,17 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   a.chunk_last = chunk == nchunks - 1;
   with_fast_n_if<sizeof(R) == 4>(a.Px, [&](auto nc) {
     constexpr int NX = decltype(nc)::value;
-    cudaError_t e = cudaFuncSetAttribute(dm_row_pass<R, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
-    if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(dm_row_pass)"); return; }
     KernelTimer kt(ctx, prec ? "dm_row_pass_f64" : "dm_row_pass", st);
-    dm_row_pass<R, NX><<<(a.pny + kRowPair - 1) / kRowPair, 512, smem_row, st>>>(a);
+    cudaError_t e;
+    if constexpr (NX > 0) {
+      e = cudaFuncSetAttribute(dm_row_pass<R, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row);
+      if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(dm_row_pass)"); return; }
+      dm_row_pass<R, NX><<<(a.pny + kRowPair - 1) / kRowPair, 512, smem_row, st>>>(a);
+      e = cudaGetLastError();
+    } else {
+      e = dm_gen_row<R>(a, gen, st);
+    }
     note_launch();
-    e = cudaGetLastError();
     if (e != cudaSuccess) rs = cuda_fail(e, "dm_row_pass launch");
   });
   OH_TRY(rs);
@@ -584,20 +498,24 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   }
   }   // layer chunks
   if (!Wfast) {
-    cudaError_t e = cudaFuncSetAttribute(dm_col_pass<R, KMAX, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(dm_col_pass)");
     KernelTimer kt(ctx, prec ? "dm_col_pass_f64" : "dm_col_pass", st);
-    dm_col_pass<R, KMAX, 0><<<a.nstrips, T, smem_col, st>>>(a);
-    OH_LAUNCH_CHECK();
+    const cudaError_t e = dm_gen_col<R>(a, gen, st);
+    note_launch();
+    if (e != cudaSuccess) return cuda_fail(e, "dm_col_gen launch");
   }
   with_fast_n_if<sizeof(R) == 4>(a.Px, [&](auto nc) {
     constexpr int NX = decltype(nc)::value;
-    cudaError_t e = cudaFuncSetAttribute(dm_out_pass<R, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out);
-    if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(dm_out_pass)"); return; }
     KernelTimer kt(ctx, prec ? "dm_out_pass_f64" : "dm_out_pass", st);
-    dm_out_pass<R, NX><<<a.pny, 256, smem_out, st>>>(a);
+    cudaError_t e;
+    if constexpr (NX > 0) {
+      e = cudaFuncSetAttribute(dm_out_pass<R, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out);
+      if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(dm_out_pass)"); return; }
+      dm_out_pass<R, NX><<<a.pny, 256, smem_out, st>>>(a);
+      e = cudaGetLastError();
+    } else {
+      e = dm_gen_out<R>(a, gen, st);
+    }
     note_launch();
-    e = cudaGetLastError();
     if (e != cudaSuccess) rs = cuda_fail(e, "dm_out_pass launch");
   });
   OH_TRY(rs);
@@ -610,12 +528,12 @@ oh_status depthmap_enqueue_f32(oh_ctx* ctx, const oh_depthmap_params* p, const u
                                void* fringe, void* field, const void* src, double src_z, cudaStream_t st) {
   OH_TRY(validate(p));
   if (!fringe || (!src && (!img || !depth))) return fail(OH_ERR_INVALID_ARG, "depth-map frame: missing buffers");
-  return run_depthmap<float, 36>(ctx, p, img, depth, nullptr, fringe, field, nullptr, st, nullptr, src, src_z);
+  return run_depthmap<float>(ctx, p, img, depth, nullptr, fringe, field, nullptr, st, nullptr, src, src_z);
 }
 
 // The planning half of run_depthmap for one FP32 frame (dm_batch.h).
 oh_status depthmap_frame_info(oh_ctx* ctx, const oh_depthmap_frame& f, cudaStream_t st, FrameInfo<float>* info) {
-  return run_depthmap<float, 36>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st, info);
+  return run_depthmap<float>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st, info);
 }
 
 oh_status depthmap_validate(const oh_depthmap_params* p) { return validate(p); }
@@ -664,8 +582,8 @@ oh_status oh_depthmap_generate(oh_ctx* ctx, oh_precision prec, const oh_depthmap
   OH_TRY(validate(p));
   if (!img || !depth || !fringe_out) return fail(OH_ERR_INVALID_ARG, "img, depth and fringe_out are required");
   if (p->phase_mode == OH_PHASE_ARRAY && !phase) return fail(OH_ERR_INVALID_ARG, "OH_PHASE_ARRAY needs a phase array");
-  if (prec == OH_FP64) return run_depthmap<double, 18>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
-  return run_depthmap<float, 36>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
+  if (prec == OH_FP64) return run_depthmap<double>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
+  return run_depthmap<float>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
 }
 
 oh_status oh_depthmap_propagate_field(oh_ctx* ctx, oh_precision prec, const oh_depthmap_params* p,
@@ -678,9 +596,9 @@ oh_status oh_depthmap_propagate_field(oh_ctx* ctx, oh_precision prec, const oh_d
   if (!field_in || !fringe_out) return fail(OH_ERR_INVALID_ARG, "field_in and fringe_out are required");
   if (!std::isfinite(z)) return fail(OH_ERR_INVALID_ARG, "propagation distance must be finite");
   if (prec == OH_FP64)
-    return run_depthmap<double, 18>(ctx, p, nullptr, nullptr, nullptr, fringe_out, field_out, spectrum_out, st, nullptr,
+    return run_depthmap<double>(ctx, p, nullptr, nullptr, nullptr, fringe_out, field_out, spectrum_out, st, nullptr,
                                     field_in, z);
-  return run_depthmap<float, 36>(ctx, p, nullptr, nullptr, nullptr, fringe_out, field_out, spectrum_out, st, nullptr,
+  return run_depthmap<float>(ctx, p, nullptr, nullptr, nullptr, fringe_out, field_out, spectrum_out, st, nullptr,
                                  field_in, z);
 }
 
@@ -722,12 +640,12 @@ oh_status oh_depthmap_generate_batch(oh_ctx* ctx, oh_precision prec, const oh_de
       const oh_depthmap_frame& f = frames[i];
       if (fp64) {
         FrameInfo<double> fi;
-        OH_TRY((run_depthmap<double, 18>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
+        OH_TRY((run_depthmap<double>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
                                          sizes ? &fi : nullptr)));
         if (sizes) sizes[i] = fi.sz;
       } else {
         FrameInfo<float> fi;
-        OH_TRY((run_depthmap<float, 36>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
+        OH_TRY((run_depthmap<float>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
                                         sizes ? &fi : nullptr)));
         if (sizes) sizes[i] = fi.sz;
       }
@@ -831,8 +749,8 @@ oh_status oh_depthmap_generate_host(oh_ctx* ctx, oh_precision prec, const oh_dep
       dp = d_phase;
     }
     void* out = fringe_mapped ? fringe_mapped : d_fringe;
-    if (prec == OH_FP64) OH_TRY((run_depthmap<double, 18>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
-    else OH_TRY((run_depthmap<float, 36>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
+    if (prec == OH_FP64) OH_TRY((run_depthmap<double>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
+    else OH_TRY((run_depthmap<float>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
     if (!fringe_mapped) OH_CUDA_TRY(cudaMemcpyAsync(fringe_host, d_fringe, fsz, cudaMemcpyDeviceToHost, st));
     return OH_OK;
   };

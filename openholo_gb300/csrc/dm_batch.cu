@@ -393,7 +393,7 @@ static oh_status batch_frame_infos(oh_ctx* ctx, const oh_depthmap_frame* frames,
     const oh_depthmap_frame& f = frames[i];
     OH_TRY(depthmap_frame_info(ctx, f, st, &(*fi)[i]));
     const FrameInfo<float>& x = (*fi)[i];
-    if (batch_class(x.a.Px) < 0 || batch_class(x.a.Py) < 0 || !x.Wfast || !x.a.xs || x.nchunks != 1 ||
+    if (batch_class(x.a.Px) < 0 || batch_class(x.a.Py) < 0 || !x.Wfast || x.nchunks != 1 ||
         !batch_col_ok(x))
       *ok = false;
   }

@@ -266,10 +266,9 @@ __device__ __forceinline__ void dm_col_body(const DMArgs<float>& a, int blk) {
   load_tw_split(twlo, twhi, static_cast<const C*>(a.ply.tw), NY);
   if constexpr (kTab > 0) fill_stage_tab<NY, R1, NY / R0, -1>(tab1, static_cast<const C*>(a.ply.tw));
   if (tid < W) {
-    // strip column kx0 + w is either spectrum column kx0 + w or, when the row
-    // pass stored its output in FFT storage order, column iperm + hx
-    int kx = kx0 + tid;
-    if (a.xs) { kx = a.plx.iperm[kx0 + tid] + a.hx; if (kx >= a.Px) kx -= a.Px; }
+    // strip column kx0 + w (row FFT storage order) is spectrum column iperm + hx
+    int kx = a.plx.iperm[kx0 + tid] + a.hx;
+    if (kx >= a.Px) kx -= a.Px;
     kxw[tid] = kx;
     lfxw[tid] = a.lfx[kx];
     if (STEP) dxw[tid] = a.dxh[kx];

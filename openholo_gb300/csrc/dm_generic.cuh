@@ -1,0 +1,395 @@
+// Depth-map passes on the plan-driven FFT engine: FP64 frames, and FP32 frames
+// whose padded row or column length has no compile-time schedule.  The same
+// frame pipeline as dm_kernels.cuh / dm_col_fast.cuh (row strips, layer flags,
+// spectrum columns in the row FFT's storage order, inverses as the adjoint of
+// the forward network), with run-time lengths.
+#pragma once
+#include "dm_kernels.cuh"
+
+namespace oh {
+
+// Row pass: nr (1 or 2) image rows per block.  Per layer present in them: stage
+// 0 straight from the source pixels, the other stages in place, then the lines
+// go to the strips in storage order (W of them, so two rows fill a 32-byte
+// sector).
+template <typename R>
+__global__ void __launch_bounds__(256) dm_row_gen(DMArgs<R> a, int nr) {
+  typedef typename cplx_of<R>::type C;
+  extern __shared__ unsigned char smem_raw[];
+  const int Px = a.Px, pnx = a.pnx, T = blockDim.x;
+  const int lip = (pnx + 7) & ~7, lens = a.plx.lens;
+  C* buf = reinterpret_cast<C*>(smem_raw);              // [nr][lens]
+  C* v = buf + nr * lens;                               // [nr][pnx] source values
+  int16_t* li = reinterpret_cast<int16_t*>(v + nr * pnx);        // [nr][lip] layer slot per pixel
+  uint32_t* mask = reinterpret_cast<uint32_t*>(li + nr * lip);   // [2][8] layers present per row
+  const int r0 = blockIdx.x * nr;
+  const int nrows = min(nr, a.pny - r0);
+  int16_t* const slut = dm_row_slut();
+  for (int i = threadIdx.x; i < 16; i += T) mask[i] = 0u;
+  for (int i = threadIdx.x; i < 256; i += T) slut[i] = a.lut[i];
+  __syncthreads();
+  for (int l = 0; l < nrows; ++l)
+    for (int c = threadIdx.x; c < pnx; c += T) {
+      const size_t off = (size_t)(r0 + l) * pnx + c;
+      int u = -1;
+      C val = mk((R)0, (R)0);
+      if (a.src) {                                      // a complex source field: one layer slot
+        u = 0;
+        val = a.src[off];
+      } else {
+        const uint8_t g = a.img[off];
+        u = g > 0 ? (int)slut[a.depth[off]] : -1;
+        if (u >= 0) {
+          const R amp = (R)g / (R)255;
+          if (a.phase_mode == OH_PHASE_REFERENCE) {
+            val = mk(amp, (R)0);
+          } else {
+            R ph;
+            if (a.phase_mode == OH_PHASE_ARRAY) ph = (R)a.phase[off];
+            else ph = (R)u24_at(a.seed, off) * (R)6.283185307179586476925;
+            R sn, cs;
+            sincos_r<R>(ph, &sn, &cs);
+            val = mk(amp * cs, amp * sn);
+          }
+        }
+      }
+      if (u >= 0) {
+        // neighbours mostly share a layer: one atomic per distinct slot of the active lanes
+        const unsigned same = __match_any_sync(__activemask(), u);
+        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicOr(&mask[l * 8 + (u >> 5)], 1u << (u & 31));
+      }
+      li[l * lip + c] = (int16_t)u;
+      v[l * pnx + c] = val;
+    }
+  __syncthreads();
+  const GStage g0 = gstage_of(a.plx, 0, sizeof(C));
+  for (int u = a.slot0; u < a.slot1; ++u) {
+    const bool p0 = (mask[u >> 5] >> (u & 31)) & 1u;
+    const bool p1 = (mask[8 + (u >> 5)] >> (u & 31)) & 1u;
+    const int ur = u - a.slot0;
+    if (threadIdx.x < nrows) a.occ[(size_t)ur * a.occ_stride + r0 + threadIdx.x] = (threadIdx.x == 0 ? p0 : p1) ? 1 : 0;
+    if (!(p0 || p1)) continue;
+    if (threadIdx.x == 0) a.slot_any[u] = 1;
+    // input i of the x-shifted, zero-padded line a[i] = u[(i - hx) mod Px]
+    auto pixel = [&](int l, int i) -> C {
+      int x = i - a.hx;
+      if (x < 0) x += Px;
+      const int c = x - a.ox;
+      return (unsigned)c < (unsigned)pnx && li[l * lip + c] == u ? v[l * pnx + c] : mk((R)0, (R)0);
+    };
+    if (a.plx.nst == 0) {
+      if (threadIdx.x < nrows) buf[threadIdx.x * lens] = pixel(threadIdx.x, 0);
+    } else {
+      with_radix<false>(g0.r, [&](auto rc) {
+        constexpr int RR = decltype(rc)::value;
+        const int total = g0.nb * nrows;
+        for (int idx = threadIdx.x; idx < total; idx += T) {
+          int l, b, j;
+          gsplit(g0, idx, -1, &l, &b);
+          C* p = buf + l * lens + gbase(g0, b, &j);
+          if constexpr (RR > 0) {
+            C x[RR];
+#pragma unroll
+            for (int t = 0; t < RR; ++t) x[t] = pixel(l, j + t * g0.q);
+            gbutterfly<RR, GFWD>(g0, j, x);
+#pragma unroll
+            for (int t = 0; t < RR; ++t) p[t * g0.qs] = x[t];
+          } else {
+            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return pixel(l, j + t * g0.q); },
+                                    [&](int f, C y) { p[f * g0.qs] = y; });
+          }
+        }
+      });
+    }
+    for (int s = 1; s < a.plx.nst; ++s) {
+      __syncthreads();
+      gstage_call<GFWD, C, false>(gstage_of(a.plx, s, sizeof(C)), 0, nrows, lens, 1, -1);
+    }
+    __syncthreads();
+    C* dst = a.Rbuf + (size_t)ur * a.nstrips * a.pny * a.W;
+    const int W = a.W, lw = a.lw;
+    for (int idx = threadIdx.x; idx < nrows * Px; idx += T) {
+      const int w = idx & (W - 1), t = idx >> lw;
+      const int l = nrows == 2 ? (t & 1) : 0, s = nrows == 2 ? (t >> 1) : t;
+      dst[((size_t)s * a.pny + r0 + l) * W + w] = buf[l * lens + pl_at(a.plx, (s << lw) + w)];
+    }
+    __syncthreads();
+  }
+}
+
+// exp(2 pi i t): table of 128 directions and a short polynomial on the rest
+// (|x| <= pi / 128: the dropped terms are below 2e-15).  An FP64 sine and
+// cosine by the general routine takes three to four times as many FP64
+// instructions, of which this part issues one per 64 FP32 ones.
+__device__ __forceinline__ double2 cis_turns(double t, const double2* tab) {
+  const double big = 6755399441055744.0;                // 1.5 2^52: adding it rounds to an integer
+  const double v = t * 128.0;
+  const double n = v + big;
+  const double x = (v - (n - big)) * 0.049087385212340519350978802863742;      // 2 pi / 128
+  const double2 d = tab[__double2loint(n) & 127];
+  const double x2 = x * x;
+  const double s = fma(x * x2, fma(x2, 1.0 / 120.0, -1.0 / 6.0), x);
+  const double c = fma(x2, fma(x2, fma(x2, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
+  return make_double2(fma(d.x, c, -d.y * s), fma(d.x, s, d.y * c));
+}
+
+// Shared memory of the column pass after the lines: kept rows' positions,
+// active entries, and in FP64 the direction table and (evenly spaced layers)
+// the step factors.
+template <typename R>
+inline size_t dm_col_gen_smem(int lens, int lwb, int nrow, int n_entries, bool horner) {
+  size_t o = (size_t)lens << lwb;
+  if (sizeof(R) == 8) o += 128 + (horner ? (size_t)nrow << lwb : 0);
+  o *= 2 * sizeof(R);
+  return o + (((size_t)nrow * 2 + 15) & ~(size_t)15) + (size_t)n_entries * 2 + 16;
+}
+
+// Column pass: 1 << lwb spectrum columns (storage positions) per block for the
+// whole frame.  Per active layer: stage 0 straight from the strips (absent and
+// padded rows are zeros), the other stages in place, then every thread adds
+// H(e) times its samples into registers.  Only the spectrum rows [row0, row0 +
+// nrow) that reach the crop are kept.  Transfer function: the entry's separable
+// tables times exp(i k z' g), g = s^2 / (2 (1 + sqrt(1 - s))^2) held per sample;
+// FP64 with evenly spaced layers accumulates acc = acc D + x instead (see
+// dm_col_fast.cuh), D in shared memory.
+//
+// What bounds it: instruction issue in FP32 (FFT butterflies plus about 20
+// instructions per kept sample and layer), the FP64 pipe in FP64.
+template <typename R, int KMAX, int T, int MINB>
+__global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int row0, int nrow) {
+  typedef typename cplx_of<R>::type C;
+  constexpr bool F64 = sizeof(R) == 8;
+  constexpr bool KEEPG = KMAX <= 16;                    // g per sample in registers
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ int s_nact;
+  const int W = 1 << lwb, Py = a.Py, pny = a.pny, lens = a.ply.lens, tid = threadIdx.x;
+  const bool step = F64 && a.horner;
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  C* tab = buf + ((size_t)lens << lwb);
+  C* dst = tab + (F64 ? 128 : 0);
+  uint16_t* pos = reinterpret_cast<uint16_t*>(dst + (step ? (size_t)nrow << lwb : 0));
+  int16_t* list = reinterpret_cast<int16_t*>(pos + ((nrow + 7) & ~7));
+  const int w = tid & (W - 1), p = (blockIdx.x << lwb) + w;
+  const bool valid = p < a.Px;
+  int kx = 0;
+  if (valid) { kx = a.plx.iperm[p] + a.hx; if (kx >= a.Px) kx -= a.Px; }
+  const int nk = nrow << lwb;
+  for (int i = tid; i < nrow; i += T) {
+    int k = row0 + i - a.hy;                            // S[ky] = B[(ky - hy) mod Py]
+    if (k < 0) k += Py;
+    pos[i] = (uint16_t)a.ply.permp[k];
+  }
+  if (tid < 32) {
+    int n = 0;
+    for (int base = 0; base < a.n_entries; base += 32) {
+      const int e = base + tid;
+      const bool act = e < a.n_entries && a.slot_any[a.uslot_of_entry[e]] != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, act);
+      if (act) list[n + __popc(m & ((1u << tid) - 1u))] = (int16_t)e;
+      n += __popc(m);
+    }
+    if (tid == 0) s_nact = n;
+  }
+  if constexpr (F64) {
+    for (int i = tid; i < 128; i += T) { double s, c; sincospi(i * (1.0 / 64.0), &s, &c); tab[i] = mk(c, s); }
+  }
+  auto resid = [&](int k) -> R {
+    const int i = (tid + k * T) >> lwb;
+    const R sv = a.lfx[kx] + a.lfy[row0 + i];
+    const R den = (R)1 + sqrt((R)1 - sv);
+    return sv * sv / ((R)2 * den * den);
+  };
+  C acc[KMAX];
+  R g[KEEPG ? KMAX : 1];
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k) {
+    acc[k] = mk((R)0, (R)0);
+    if constexpr (KEEPG) g[k] = tid + k * T < nk ? resid(k) : (R)0;
+  }
+  __syncthreads();
+  const int nact = s_nact;
+  auto gof = [&](int k) -> R { if constexpr (KEEPG) return g[k]; else return resid(k); };
+  // exp(i kz g) of sample k
+  auto residual = [&](R kz, int k) -> C {
+    if constexpr (F64) return cis_turns(kz * 0.15915494309189533576888376337251 * gof(k), tab);
+    else { float sn, cs; __sincosf(kz * gof(k), &sn, &cs); return mk(cs, sn); }
+  };
+  if constexpr (F64) {
+    if (step) {
+      // D = H(z' - dz) / H(z') per kept sample
+      const R kdz = (R)(-a.k * a.dz);
+#pragma unroll
+      for (int k = 0; k < KMAX; ++k) {
+        const int idx = tid + k * T;
+        if (idx < nk) {
+          int ky = row0 + (idx >> lwb) - a.hy;
+          if (ky < 0) ky += Py;
+          dst[idx] = cmul(cmul(a.dxh[kx], a.dyh[a.ply.perm[ky]]), residual(kdz, k));
+        }
+      }
+    }
+  }
+  const GStage g0 = gstage_of(a.ply, 0, sizeof(C));
+  for (int q = 0; q < nact; ++q) {
+    const int e = list[q], u = a.uslot_of_entry[e];
+    const uint8_t* occ = a.occ + (size_t)u * a.occ_stride;
+    const C* src = a.Rbuf + ((size_t)u * a.nstrips + (p >> a.lw)) * pny * a.W + (p & (a.W - 1));
+    // input i of the y-shifted, zero-padded column
+    auto sample = [&](int i) -> C {
+      int y = i - a.hy;
+      if (y < 0) y += Py;
+      y -= a.oy;
+      return valid && (unsigned)y < (unsigned)pny && __ldg(occ + y) ? src[y << a.lw] : mk((R)0, (R)0);
+    };
+    if (a.ply.nst == 0) {
+      if (tid < W) buf[tid] = sample(0);
+    } else {
+      with_radix<false>(g0.r, [&](auto rc) {
+        constexpr int RR = decltype(rc)::value;
+        const int total = g0.nb << lwb;
+        for (int idx = tid; idx < total; idx += T) {
+          int j;
+          C* d = buf + (gbase(g0, idx >> lwb, &j) << lwb) + w;
+          const int st = g0.qs << lwb;
+          if constexpr (RR > 0) {
+            C x[RR];
+#pragma unroll
+            for (int t = 0; t < RR; ++t) x[t] = sample(j + t * g0.q);
+            gbutterfly<RR, GFWD>(g0, j, x);
+#pragma unroll
+            for (int t = 0; t < RR; ++t) d[t * st] = x[t];
+          } else {
+            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return sample(j + t * g0.q); },
+                                    [&](int f, C y) { d[f * st] = y; });
+          }
+        }
+      });
+    }
+    for (int s = 1; s < a.ply.nst; ++s) {
+      __syncthreads();
+      const GStage gs = gstage_of(a.ply, s, sizeof(C));
+      with_radix<false>(gs.r, [&](auto rc) {
+        gstage_loop<decltype(rc)::value, GFWD, C>(gs, buf, W, 1, W, lwb);
+      });
+    }
+    __syncthreads();
+    if (F64 && step) {
+      const int gap = q > 0 ? e - list[q - 1] : 0;      // levels without pixels: one more factor each
+#pragma unroll
+      for (int k = 0; k < KMAX; ++k) {
+        const int idx = tid + k * T;
+        if (idx < nk) {
+          const C x = buf[((int)pos[idx >> lwb] << lwb) + w];
+          if (gap) {
+            const C d = dst[idx];
+            for (int r = 1; r < gap; ++r) acc[k] = cmul(acc[k], d);
+            acc[k] = mk(fma(acc[k].x, d.x, fma(-acc[k].y, d.y, x.x)), fma(acc[k].x, d.y, fma(acc[k].y, d.x, x.y)));
+          } else {
+            acc[k] = x;
+          }
+        }
+      }
+    } else if (valid) {
+      const R kz = a.kzp[e];
+      const C ex = a.exc[(size_t)e * a.Px + kx];
+      const C* ey = a.ey + (size_t)e * Py + row0;
+#pragma unroll
+      for (int k = 0; k < KMAX; ++k) {
+        const int idx = tid + k * T;
+        if (idx < nk) {
+          const C h = cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k));
+          const C x = buf[((int)pos[idx >> lwb] << lwb) + w];
+          acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
+          acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (F64 && step && nact > 0 && valid) {
+    // the recurrence ends with the last active entry's transfer function
+    const int e = list[nact - 1];
+    const R kz = a.kzp[e];
+    const C ex = a.exc[(size_t)e * a.Px + kx];
+    const C* ey = a.ey + (size_t)e * Py + row0;
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) {
+      const int idx = tid + k * T;
+      if (idx < nk) acc[k] = cmul(acc[k], cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k)));
+    }
+  }
+
+  // SSB crop, inverse y-FFT as the adjoint network, output rows.  The inverse
+  // line b[i] = Uc[(i - hy) mod Py] wants spectrum row ky at i = (ky + hy) mod Py,
+  // i.e. in storage order at permp[i].
+  for (int i = tid; i < lens << lwb; i += T) buf[i] = mk((R)0, (R)0);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k) {
+    const int idx = tid + k * T;
+    if (idx < nk && valid) {
+      const int ky = row0 + (idx >> lwb);
+      if (a.spectrum) a.spectrum[(size_t)ky * a.Px + kx] = acc[k];
+      if (kx >= a.cx1 && kx <= a.cx2 && ky >= a.cy1 && ky <= a.cy2) {
+        int i = ky + a.hy;
+        if (i >= Py) i -= Py;
+        buf[(a.ply.permp[i] << lwb) + w] = acc[k];
+      }
+    }
+  }
+  block_fft<GADJ, C, false>(0, W, 1, W, a.ply, lwb);
+  for (int idx = tid; idx < pny << lwb; idx += T) {
+    const int yl = idx >> lwb;
+    int m = a.oy + yl - a.hy;
+    if (m < 0) m += Py;
+    if (valid) a.V[(size_t)yl * a.Px + p] = cmul(buf[(pl_at(a.ply, m) << lwb) + w], a.shy[yl]);
+  }
+}
+
+// Output pass: one row per block.  V column p holds spectrum column kx =
+// (iperm[p] + hx) mod Px, which the inverse line wants at j = (kx + hx) mod Px
+// (the same storage position for even Px).
+template <typename R>
+__global__ void __launch_bounds__(256) dm_out_gen(DMArgs<R> a) {
+  typedef typename cplx_of<R>::type C;
+  extern __shared__ unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  const int yl = blockIdx.x, Px = a.Px;
+  const C* row = a.V + (size_t)yl * Px;
+  const bool even = 2 * a.hx == Px;
+  for (int p = threadIdx.x; p < Px; p += blockDim.x) {
+    int at;
+    if (even) {
+      at = pl_at(a.plx, p);
+    } else {
+      int j = a.plx.iperm[p] + 2 * a.hx;
+      if (j >= Px) j -= Px;
+      at = a.plx.permp[j];
+    }
+    buf[at] = row[p];
+  }
+  block_fft<GADJ, C, false>(0, 1, 0, 1, a.plx, -1);
+  for (int c = threadIdx.x; c < a.pnx; c += blockDim.x) {
+    int m = a.ox + c - a.hx;
+    if (m < 0) m += Px;
+    C h = buf[pl_at(a.plx, m)];
+    if (a.sig_x != 0) h = cmul(h, a.shx[c]);
+    a.fringe[(size_t)yl * a.pnx + c] = h.x;
+    if (a.field) a.field[(size_t)yl * a.pnx + c] = h;
+  }
+}
+
+// How a frame runs these passes (dm_generic.cuh's launches).
+struct DMGenPlan {
+  int nr;                 // image rows per row-pass block
+  int lwb;                // log2 columns per column-pass block
+  int row0, nrow;         // spectrum rows kept
+  bool wide;              // the column pass's many-samples variant
+  size_t smem_row, smem_col, smem_out;
+};
+template <typename R> DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax);
+template <typename R> cudaError_t dm_gen_row(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st);
+template <typename R> cudaError_t dm_gen_col(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st);
+template <typename R> cudaError_t dm_gen_out(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st);
+
+}  // namespace oh

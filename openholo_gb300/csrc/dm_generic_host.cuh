@@ -1,0 +1,93 @@
+// Host side of dm_generic.cuh, instantiated once per precision
+// (dm_generic_f32.cu, dm_generic_f64.cu).
+#pragma once
+#include <algorithm>
+#include "dm_generic.cuh"
+
+namespace oh {
+
+// Samples per thread and threads per block of the column pass: few enough that
+// the accumulators (and g) stay in registers with two blocks per SM; the wide
+// variant takes what is longer.
+template <typename R> struct DMGenCfg {
+  static constexpr int K = sizeof(R) == 8 ? 10 : 16, T = sizeof(R) == 8 ? 128 : 256, MINB = sizeof(R) == 8 ? 3 : 2;
+  static constexpr int KW = 40, TW = sizeof(R) == 8 ? 256 : 512;
+};
+
+template <typename R>
+DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax) {
+  typedef DMGenCfg<R> CF;
+  const size_t esz = 2 * sizeof(R);
+  DMGenPlan g{};
+  auto row = [&](int nr) {
+    return (size_t)nr * ((size_t)a.plx.lens * esz + (size_t)a.pnx * esz + (size_t)((a.pnx + 7) & ~7) * 2) + 64;
+  };
+  // two rows per block fill whole sectors of the strips; one where two would
+  // leave fewer than three blocks per SM or the SMs short of blocks
+  const int sms = sm_count();
+  g.nr = row(2) <= (size_t)72 * 1024 && a.pny >= 4 * sms ? 2 : 1;
+  g.smem_row = row(g.nr);
+  // spectrum rows that reach the crop (all of them when the spectrum is asked for)
+  g.row0 = a.spectrum ? 0 : a.cy1;
+  g.nrow = a.spectrum ? a.Py : a.cy2 - a.cy1 + 1;
+  const bool horner = a.horner != 0;
+  // the most columns per block (their loads and stores share sectors) that keep
+  // the narrow variant, three blocks of shared memory per SM and four blocks
+  // per SM of work
+  g.lwb = -1;
+  for (int lw = sizeof(R) == 8 ? 1 : 2; lw >= 0; --lw) {
+    const size_t sm = dm_col_gen_smem<R>(a.ply.lens, lw, g.nrow, a.n_entries, horner);
+    if ((g.nrow << lw) <= CF::K * CF::T && sm <= (lw ? (size_t)72 * 1024 : smax) &&
+        (lw == 0 || (a.Px >> lw) >= 4 * sms)) {
+      g.lwb = lw;
+      break;
+    }
+  }
+  g.wide = g.lwb < 0;
+  if (g.wide) g.lwb = 0;
+  g.smem_col = dm_col_gen_smem<R>(a.ply.lens, g.lwb, g.nrow, a.n_entries, horner);
+  g.smem_out = (size_t)a.plx.lens * esz;
+  return g;
+}
+
+template <typename K>
+static cudaError_t dm_gen_allow(K kern, size_t smem) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+template <typename R>
+cudaError_t dm_gen_row(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
+  cudaError_t e = dm_gen_allow(dm_row_gen<R>, g.smem_row);
+  if (e != cudaSuccess) return e;
+  dm_row_gen<R><<<(a.pny + g.nr - 1) / g.nr, 256, g.smem_row, st>>>(a, g.nr);
+  return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t dm_gen_col(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
+  typedef DMGenCfg<R> CF;
+  const int blocks = (a.Px + (1 << g.lwb) - 1) >> g.lwb;
+  auto launch = [&](auto kern, int threads) {
+    cudaError_t e = dm_gen_allow(kern, g.smem_col);
+    if (e != cudaSuccess) return e;
+    kern<<<blocks, threads, g.smem_col, st>>>(a, g.lwb, g.row0, g.nrow);
+    return cudaGetLastError();
+  };
+  return g.wide ? launch(dm_col_gen<R, CF::KW, CF::TW, 1>, CF::TW) : launch(dm_col_gen<R, CF::K, CF::T, CF::MINB>, CF::T);
+}
+
+template <typename R>
+cudaError_t dm_gen_out(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
+  cudaError_t e = dm_gen_allow(dm_out_gen<R>, g.smem_out);
+  if (e != cudaSuccess) return e;
+  dm_out_gen<R><<<a.pny, 256, g.smem_out, st>>>(a);
+  return cudaGetLastError();
+}
+
+#define OH_DM_GENERIC(R)                                                               \
+  template DMGenPlan dm_gen_plan<R>(const DMArgs<R>&, size_t);                          \
+  template cudaError_t dm_gen_row<R>(const DMArgs<R>&, const DMGenPlan&, cudaStream_t); \
+  template cudaError_t dm_gen_col<R>(const DMArgs<R>&, const DMGenPlan&, cudaStream_t); \
+  template cudaError_t dm_gen_out<R>(const DMArgs<R>&, const DMGenPlan&, cudaStream_t);
+
+}  // namespace oh

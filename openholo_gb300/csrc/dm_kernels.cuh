@@ -41,9 +41,9 @@ struct DMArgs {
   int16_t* uslot_of_entry;
   R* kzp;                // k*z' per entry
   C* cst;                // per-entry constant
-  C* exc;                // [entries][Px] cst*exp(i alpha fx^2)   (fp32 path)
+  C* exc;                // [entries][Px] cst*exp(i alpha fx^2)
   R* eth;                // [entries][Py] phase alpha fy^2 reduced to [-pi, pi], y storage order (fast passes)
-  C* ey;                 // [entries][Py] exp(i alpha fy^2)       (fp32 path)
+  C* ey;                 // [entries][Py] exp(i alpha fy^2)
   R* lfx;                // [Px] (lambda fx)^2
   R* lfy;                // [Py] (lambda fy)^2
   R* lfyp;               // [Py] (lambda fy)^2 in FFT storage order (fast column pass)
@@ -52,14 +52,13 @@ struct DMArgs {
   C* shx;                // [pnx] x shift phase
   int* slot_any;         // [uslots]
   uint8_t* occ;          // [uslots][pny]
-  C* Rbuf;               // [uslots][nstrips][pny][W]
-  C* V;                  // [pny][Px]
+  C* Rbuf;               // [uslots][nstrips][pny][W], columns in the row FFT's storage order
+  C* V;                  // [pny][Px], columns in the same order
   R* fringe;             // [pny][pnx]
   C* field;              // [pny][pnx] or null
   C* spectrum;           // [Py][Px] or null
   int sig_x, sig_y;
   int occ_stride;        // bytes per layer row of occ (multiple of 16)
-  int xs;                // 1: R and V columns are in the row FFT's storage order (fast passes), 0: kx order
   int hzx, hzy;          // 1: 2x padding with a radix-16 first stage (stage-0 inputs 4..11 are zero)
   int* err;              // device error word (bounded waits that ran out)
   const int* stall_flag; // error-path test hook: wait on this never-set flag before the first layer
@@ -124,7 +123,7 @@ __device__ __forceinline__ void dm_setup_body(const DMArgs<R>& a, const DMSetup&
     double lp = a.lambda * fyp;
     a.lfyp[y] = (R)(lp * lp);
   }
-  if constexpr (sizeof(R) == 4) {
+  {
     // separable paraxial factors exp(i pi lambda z' f^2), reduced in double
     for (int idx = tid; idx < s.n_entries * a.Px; idx += nthr) {
       int e = idx / a.Px, x = idx - e * a.Px;
@@ -314,7 +313,8 @@ __device__ __forceinline__ void dm_row_body(const DMArgs<R>& a, int blk) {
   const int Px = a.Px, pnx = a.pnx;
   const int lip = (pnx + 7) & ~7;                       // keeps 16-byte alignment
   typedef RowPad<NX> RP;
-  const int lsmax = NX > 0 ? RP::LSMAX : Px;
+  static_assert(NX > 0, "other lengths run dm_row_gen");
+  constexpr int lsmax = RP::LSMAX;
   C* buf = reinterpret_cast<C*>(smem_raw);              // [2][lsmax]
   C* v = buf + 2 * lsmax;                               // [2][pnx] source values
   int16_t* li = reinterpret_cast<int16_t*>(v + 2 * pnx);   // [2][lip] layer slot per pixel
@@ -325,14 +325,12 @@ __device__ __forceinline__ void dm_row_body(const DMArgs<R>& a, int blk) {
   const int r0 = blk * kRowPair;
   const int nrows = min(kRowPair, a.pny - r0);
   // fused last stage + strip store, in the padded layout
-  const bool fused = RP::fusable && a.W == 2 && a.xs && nrows == 2;
+  const bool fused = RP::fusable && a.W == 2 && nrows == 2;
   for (int i = threadIdx.x; i < 16; i += NT) mask[i] = 0u;
   int16_t* const slut = dm_row_slut();                  // depth byte -> layer slot
   for (int i = threadIdx.x; i < 256; i += NT) slut[i] = a.lut[i];
-  if constexpr (NX > 0) {
-    load_tw_split(twlo, twhi, static_cast<const C*>(a.plx.tw), NX);
-    fill_stage_tab<NX, FastSched<NX>::r1, NX / FastSched<NX>::r0, -1>(tab1, static_cast<const C*>(a.plx.tw));
-  }
+  load_tw_split(twlo, twhi, static_cast<const C*>(a.plx.tw), NX);
+  fill_stage_tab<NX, FastSched<NX>::r1, NX / FastSched<NX>::r0, -1>(tab1, static_cast<const C*>(a.plx.tw));
   __syncthreads();
   // the image and depth bytes of up to kSetupPix pixels per thread are loaded
   // before any is used, so their latency is paid once
@@ -413,120 +411,107 @@ __device__ __forceinline__ void dm_row_body(const DMArgs<R>& a, int blk) {
     }
     if (!(p0 || p1)) continue;
     if (threadIdx.x == 0) a.slot_any[u] = 1;
-    if constexpr (NX > 0) {
-      // stage 0 straight from the source rows: inputs j + t*Q0 of each
-      // x-shifted, zero-padded line a[j] = u[(j - hx) mod Px]
-      constexpr int R0 = FastSched<NX>::r0;
-      constexpr int Q0 = NX / R0;
-      const TwSplit<C> tw{twlo, twhi};
-      const int ls = fused ? RP::LS : Px, bs = fused ? RP::BS : Q0;
-      for (int idx = threadIdx.x; idx < kRowPair * Q0; idx += NT) {
-        const int l = idx / Q0, j = idx - l * Q0;
-        const int16_t* lil = li + l * lip;
-        const C* vl = v + l * pnx;
-        C x[R0];
-        if (R0 == 16 && a.hzx) {
-          // 2x padding: inputs t = 4..11 fall in the zero columns; with
-          // hx = NX/2 and ox = NX/4 the image column of input t is
-          // j + (t + 4) Q0 (t < 4) or j + (t - 12) Q0 (t >= 12)
+    // stage 0 straight from the source rows: inputs j + t*Q0 of each
+    // x-shifted, zero-padded line a[j] = u[(j - hx) mod Px]
+    constexpr int R0 = FastSched<NX>::r0;
+    constexpr int Q0 = NX / R0;
+    const TwSplit<C> tw{twlo, twhi};
+    const int ls = fused ? RP::LS : Px, bs = fused ? RP::BS : Q0;
+    for (int idx = threadIdx.x; idx < kRowPair * Q0; idx += NT) {
+      const int l = idx / Q0, j = idx - l * Q0;
+      const int16_t* lil = li + l * lip;
+      const C* vl = v + l * pnx;
+      C x[R0];
+      if (R0 == 16 && a.hzx) {
+        // 2x padding: inputs t = 4..11 fall in the zero columns; with
+        // hx = NX/2 and ox = NX/4 the image column of input t is
+        // j + (t + 4) Q0 (t < 4) or j + (t - 12) Q0 (t >= 12)
 #pragma unroll
-          for (int t = 0; t < R0; ++t) {
-            if (t >= 4 && t < 12) { x[t] = mk((R)0, (R)0); continue; }
-            const int c = j + (t < 4 ? t + 4 : t - 12) * Q0;
-            x[t] = lil[c] == u ? vl[c] : mk((R)0, (R)0);
-          }
-          dft16_halfzero<-1>(x);
-        } else {
-#pragma unroll
-          for (int t = 0; t < R0; ++t) {
-            int xx = j + t * Q0 - a.hx;
-            if (xx < 0) xx += NX;
-            const int c = xx - a.ox;
-            C val = mk((R)0, (R)0);
-            if (c >= 0 && c < pnx && lil[c] == u) val = vl[c];
-            x[t] = val;
-          }
-          DFT<R0, -1, C>::run(x);
+        for (int t = 0; t < R0; ++t) {
+          if (t >= 4 && t < 12) { x[t] = mk((R)0, (R)0); continue; }
+          const int c = j + (t < 4 ? t + 4 : t - 12) * Q0;
+          x[t] = lil[c] == u ? vl[c] : mk((R)0, (R)0);
         }
-        if (j) {
-          C wp[R0];
-          twiddle_powers<R0, -1>(tw, j, wp);
+        dft16_halfzero<-1>(x);
+      } else {
 #pragma unroll
-          for (int f = 1; f < R0; ++f) x[f] = cmul(x[f], wp[f]);
+        for (int t = 0; t < R0; ++t) {
+          int xx = j + t * Q0 - a.hx;
+          if (xx < 0) xx += NX;
+          const int c = xx - a.ox;
+          C val = mk((R)0, (R)0);
+          if (c >= 0 && c < pnx && lil[c] == u) val = vl[c];
+          x[t] = val;
         }
-        C* bl = buf + l * ls + (fused && RP::JG > 0 ? j / (RP::JG > 0 ? RP::JG : 1) : 0);
-#pragma unroll
-        for (int f = 0; f < R0; ++f) bl[j + f * bs] = x[f];
+        DFT<R0, -1, C>::run(x);
       }
-      if constexpr (RP::fusable) {
-        if (fused) {
-          // middle stage, then the last stage (no twiddles) straight from
-          // registers into the strips: thread pair (2b, 2b+1) = rows r0, r0+1
-          // of butterfly b; each writes 16 bytes (storage positions p, p+1 of
-          // its row) of the same 32-byte strip sector
-          constexpr int RL = FastSched<NX>::rlast;
-          __syncthreads();
-          fstage_tab<NX, FastSched<NX>::r1, NX / FastSched<NX>::r0, -1, C, RP::BS, RP::RLP>(buf, kRowPair, RP::LS, 1,
-                                                                                           tab1, false);
-          __syncthreads();
+      if (j) {
+        C wp[R0];
+        twiddle_powers<R0, -1>(tw, j, wp);
 #pragma unroll
-          for (int vi = 0; vi < 512 / NT; ++vi) {
-            const int vt = threadIdx.x + vi * NT;
-            const int b = vt >> 1, l = vt & 1;
-            C x[RL];
-            const C* src = buf + l * RP::LS + (b / RP::BPB) * RP::BS + (b % RP::BPB) * RP::RLP;
+        for (int f = 1; f < R0; ++f) x[f] = cmul(x[f], wp[f]);
+      }
+      C* bl = buf + l * ls + (fused && RP::JG > 0 ? j / (RP::JG > 0 ? RP::JG : 1) : 0);
 #pragma unroll
-            for (int t = 0; t < RL; ++t) x[t] = src[t];
-            DFT<RL, -1, C>::run(x);
-            float4* d4 = reinterpret_cast<float4*>(a.Rbuf + (size_t)ur * a.nstrips * a.pny * 2);
-            const size_t rowoff = (size_t)r0 + l;
-            if constexpr (RL % 2 == 0) {
+      for (int f = 0; f < R0; ++f) bl[j + f * bs] = x[f];
+    }
+    if constexpr (RP::fusable) {
+      if (fused) {
+        // middle stage, then the last stage (no twiddles) straight from
+        // registers into the strips: thread pair (2b, 2b+1) = rows r0, r0+1
+        // of butterfly b; each writes 16 bytes (storage positions p, p+1 of
+        // its row) of the same 32-byte strip sector
+        constexpr int RL = FastSched<NX>::rlast;
+        __syncthreads();
+        fstage_tab<NX, FastSched<NX>::r1, NX / FastSched<NX>::r0, -1, C, RP::BS, RP::RLP>(buf, kRowPair, RP::LS, 1,
+                                                                                         tab1, false);
+        __syncthreads();
 #pragma unroll
-              for (int f = 0; f < RL; f += 2) {
+        for (int vi = 0; vi < 512 / NT; ++vi) {
+          const int vt = threadIdx.x + vi * NT;
+          const int b = vt >> 1, l = vt & 1;
+          C x[RL];
+          const C* src = buf + l * RP::LS + (b / RP::BPB) * RP::BS + (b % RP::BPB) * RP::RLP;
+#pragma unroll
+          for (int t = 0; t < RL; ++t) x[t] = src[t];
+          DFT<RL, -1, C>::run(x);
+          float4* d4 = reinterpret_cast<float4*>(a.Rbuf + (size_t)ur * a.nstrips * a.pny * 2);
+          const size_t rowoff = (size_t)r0 + l;
+          if constexpr (RL % 2 == 0) {
+#pragma unroll
+            for (int f = 0; f < RL; f += 2) {
+              const int s2 = (b * RL + f) >> 1;
+              d4[(size_t)s2 * a.pny + rowoff] = make_float4(x[f].x, x[f].y, x[f + 1].x, x[f + 1].y);
+            }
+          } else {
+            // odd RL: even b also writes (its last, b+1's first), from lane + 2
+            const C nxt0 = make_float2(__shfl_down_sync(0xffffffffu, x[0].x, 2),
+                                       __shfl_down_sync(0xffffffffu, x[0].y, 2));
+            const int f0 = b & 1;                     // first paired output
+#pragma unroll
+            for (int f = 0; f + 1 < RL; ++f) {
+              if (((f - f0) & 1) == 0 && f >= f0) {
                 const int s2 = (b * RL + f) >> 1;
                 d4[(size_t)s2 * a.pny + rowoff] = make_float4(x[f].x, x[f].y, x[f + 1].x, x[f + 1].y);
               }
-            } else {
-              // odd RL: even b also writes (its last, b+1's first), from lane + 2
-              const C nxt0 = make_float2(__shfl_down_sync(0xffffffffu, x[0].x, 2),
-                                         __shfl_down_sync(0xffffffffu, x[0].y, 2));
-              const int f0 = b & 1;                     // first paired output
-#pragma unroll
-              for (int f = 0; f + 1 < RL; ++f) {
-                if (((f - f0) & 1) == 0 && f >= f0) {
-                  const int s2 = (b * RL + f) >> 1;
-                  d4[(size_t)s2 * a.pny + rowoff] = make_float4(x[f].x, x[f].y, x[f + 1].x, x[f + 1].y);
-                }
-              }
-              if (f0 == 0) {
-                const int s2 = (b * RL + RL - 1) >> 1;
-                d4[(size_t)s2 * a.pny + rowoff] = make_float4(x[RL - 1].x, x[RL - 1].y, nxt0.x, nxt0.y);
-              }
+            }
+            if (f0 == 0) {
+              const int s2 = (b * RL + RL - 1) >> 1;
+              d4[(size_t)s2 * a.pny + rowoff] = make_float4(x[RL - 1].x, x[RL - 1].y, nxt0.x, nxt0.y);
             }
           }
-          __syncthreads();
-          continue;
         }
+        __syncthreads();
+        continue;
       }
-      FastSched<NX>::template run_rest_tab<-1>(buf, kRowPair, Px, 1, tab1, tw, false);
-      __syncthreads();
-    } else {
-      // shifted, zero-padded source lines: a[j] = u[(j - hx) mod Px]
-      for (int idx = threadIdx.x; idx < kRowPair * Px; idx += NT) {
-        const int l = idx / Px, j = idx - l * Px;
-        int x = j - a.hx; if (x < 0) x += Px;
-        const int c = x - a.ox;
-        C val = mk((R)0, (R)0);
-        if (c >= 0 && c < pnx && li[l * lip + c] == u) val = v[l * pnx + c];
-        buf[idx] = val;
-      }
-      block_fft<-1>(buf, kRowPair, Px, 1, a.plx, false);
     }
-    // store: strip s holds rows r0, r0+1 contiguously -> 2*W values per strip
-    // (W is a power of two: index split with shifts)
+    FastSched<NX>::template run_rest_tab<-1>(buf, kRowPair, Px, 1, tab1, tw, false);
+    __syncthreads();
+    // store in FFT storage order: strip s holds rows r0, r0+1 contiguously ->
+    // 2*W values per strip (W is a power of two: index split with shifts)
     C* dst = a.Rbuf + (size_t)ur * a.nstrips * a.pny * a.W;
     const int W = a.W, lw = a.lw;
-    if (sizeof(R) == 4 && W == 2 && nrows == 2 && a.xs) {
+    if (W == 2 && nrows == 2) {
       // FP32, strips of two columns, FFT storage order: a thread pair moves
       // one strip's 2 x 2 block (32 contiguous bytes, one full sector), one
       // row each, with 16-byte accesses
@@ -545,14 +530,7 @@ __device__ __forceinline__ void dm_row_body(const DMArgs<R>& a, int blk) {
       const int l = nrows == 2 ? (t & 1) : 0;
       const int s = nrows == 2 ? (t >> 1) : t;
       const int col = (s << lw) + w;                     // strip column
-      C val;
-      if (a.xs) {
-        val = buf[l * Px + col];                         // FFT storage order
-      } else {
-        int m = col - a.hx; if (m < 0) m += Px;          // S[kx] = A[(kx - hx) mod Px]
-        val = buf[l * Px + a.plx.perm[m]];
-      }
-      dst[((size_t)s * a.pny + r0 + l) * W + w] = val;
+      dst[((size_t)s * a.pny + r0 + l) * W + w] = buf[l * Px + col];
     }
     __syncthreads();
   }
@@ -572,52 +550,17 @@ __device__ __forceinline__ void dm_out_body(const DMArgs<R>& a, int yl) {
   C* twlo = buf + a.Px;
   C* twhi = twlo + kTwLo;
   const C* row = a.V + (size_t)yl * a.Px;
-  if constexpr (NX > 0) load_tw_split(twlo, twhi, static_cast<const C*>(a.plx.tw), NX);
-  if constexpr (NX > 0) {
-    if (a.xs) {
-      // V column p holds spectrum column kx = (iperm[p] + hx) mod Px, whose
-      // place in the inverse line is (kx + hx) mod Px = iperm[p]: the row is
-      // in the x-FFT's storage order, the input order of the adjoint network
-      // (output in natural order)
-      for (int p = threadIdx.x; p < NX; p += blockDim.x) buf[p] = row[p];
-      FastSched<NX>::run_adj(buf, 1, NX, 1, TwSplit<C>{twlo, twhi}, false);
-      __syncthreads();
-      for (int c = threadIdx.x; c < a.pnx; c += blockDim.x) {
-        int m = a.ox + c - a.hx; if (m < 0) m += NX;
-        C h = buf[m];
-        if (a.sig_x != 0) h = cmul(h, a.shx[c]);
-        a.fringe[(size_t)yl * a.pnx + c] = h.x;
-        if (a.field) a.field[(size_t)yl * a.pnx + c] = h;
-      }
-      return;
-    }
-  }
-  if (a.xs) {
-    // V column p holds spectrum column kx = (iperm[p] + hx) mod Px; the
-    // inverse line wants it at j = (kx + hx) mod Px
-    for (int p = threadIdx.x; p < a.Px; p += blockDim.x) {
-      int kx = a.plx.iperm[p] + a.hx; if (kx >= a.Px) kx -= a.Px;
-      int j = kx + a.hx; if (j >= a.Px) j -= a.Px;
-      buf[j] = row[p];
-    }
-  } else {
-    for (int j = threadIdx.x; j < a.Px; j += blockDim.x) {
-      int kx = j - a.hx; if (kx < 0) kx += a.Px;
-      buf[j] = row[kx];
-    }
-  }
-  if constexpr (NX > 0) {
-    FastSched<NX>::template run_t<1>(buf, 1, a.Px, 1, TwSplit<C>{twlo, twhi}, false);
-    __syncthreads();
-  } else {
-    block_fft<1>(buf, 1, a.Px, 1, a.plx, false);
-  }
+  load_tw_split(twlo, twhi, static_cast<const C*>(a.plx.tw), NX);
+  // V column p holds spectrum column kx = (iperm[p] + hx) mod Px, whose place
+  // in the inverse line is (kx + hx) mod Px = iperm[p]: the row is in the
+  // x-FFT's storage order, the input order of the adjoint network (output in
+  // natural order)
+  for (int p = threadIdx.x; p < NX; p += blockDim.x) buf[p] = row[p];
+  FastSched<NX>::run_adj(buf, 1, NX, 1, TwSplit<C>{twlo, twhi}, false);
+  __syncthreads();
   for (int c = threadIdx.x; c < a.pnx; c += blockDim.x) {
-    int m = a.ox + c - a.hx; if (m < 0) m += a.Px;
-    int pm;
-    if constexpr (NX > 0) pm = FastSched<NX>::perm(m);
-    else pm = a.plx.perm[m];
-    C h = buf[pm];
+    int m = a.ox + c - a.hx; if (m < 0) m += NX;
+    C h = buf[m];
     if (a.sig_x != 0) h = cmul(h, a.shx[c]);
     a.fringe[(size_t)yl * a.pnx + c] = h.x;
     if (a.field) a.field[(size_t)yl * a.pnx + c] = h;

@@ -1,5 +1,5 @@
-// Generic 2-D / batched 1-D complex FFT built on the shared-memory engine
-// (fft_core.cuh).  The 2-D transform is a row pass (each block owns whole
+// Generic 2-D / batched 1-D complex FFT built on the shared-memory engines
+// (fft_fast.cuh, fft_generic.cuh).  The 2-D transform is a row pass (each block owns whole
 // rows) followed by a column pass (each block owns a strip of W adjacent
 // columns, so global loads/stores are W*sizeof(complex)-byte segments).
 //
@@ -13,6 +13,26 @@
 
 namespace oh {
 
+// Storage of a line: N > 0 runs the compile-time schedule on the plain layout
+// (X[k] at perm[k]), N = 0 the plan's engine on its padded layout.
+template <int N> __device__ __forceinline__ int line_at(const FFTPlan& pl, int p) {
+  if constexpr (N > 0) return p;
+  else return pl_at(pl, p);
+}
+template <int N> __device__ __forceinline__ int line_out(const FFTPlan& pl, int k) {
+  if constexpr (N > 0) return pl.perm[k];
+  else return pl.permp[k];
+}
+template <int N, int SGN, typename C>
+__device__ __forceinline__ void line_fft(C* buf, int nl, int ls, int es, const FFTPlan& pl, int lw) {
+  if constexpr (N > 0) {
+    FastSched<N>::template run<SGN>(buf, nl, ls, es, static_cast<const C*>(pl.tw), lw >= 0);
+    __syncthreads();
+  } else {
+    block_fft<SGN < 0 ? GFWD : GINV, C>(0, nl, ls, es, pl, lw);
+  }
+}
+
 template <typename R, int SGN, int N>
 __global__ void __launch_bounds__(256) fft_rows_kernel(const typename cplx_of<R>::type* __restrict__ in,
                                                        typename cplx_of<R>::type* __restrict__ out,
@@ -23,52 +43,64 @@ __global__ void __launch_bounds__(256) fft_rows_kernel(const typename cplx_of<R>
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int row0 = blockIdx.x * rpb;
   const int nrows = min(rpb, ny - row0);
+  const int ls = N > 0 ? nx : pl.lens;
   const int hx = shift ? nx / 2 : 0;
-  for (int idx = threadIdx.x; idx < nrows * nx; idx += blockDim.x) {
-    int l = idx / nx, j = idx - l * nx;
-    int src = j - hx; if (src < 0) src += nx;
-    buf[l * nx + j] = in[(size_t)(row0 + l) * nx + src];
+  for (int l = 0; l < nrows; ++l) {
+    const C* src = in + (size_t)(row0 + l) * nx;
+    for (int j = threadIdx.x; j < nx; j += blockDim.x) {
+      int i = j - hx; if (i < 0) i += nx;
+      buf[l * ls + line_at<N>(pl, j)] = src[i];
+    }
   }
-  block_fft_n<N, SGN>(buf, nrows, nx, 1, pl, false);
-  for (int idx = threadIdx.x; idx < nrows * nx; idx += blockDim.x) {
-    int l = idx / nx, k = idx - l * nx;
-    int m = k - hx; if (m < 0) m += nx;     // out[k] = A[(k - hx) mod nx]
-    C v = buf[l * nx + pl.perm[m]];
-    out[(size_t)(row0 + l) * nx + k] = cscale(v, scale);
+  line_fft<N, SGN>(buf, nrows, ls, 1, pl, -1);
+  for (int l = 0; l < nrows; ++l) {
+    C* dst = out + (size_t)(row0 + l) * nx;
+    for (int k = threadIdx.x; k < nx; k += blockDim.x) {
+      int m = k - hx; if (m < 0) m += nx;     // out[k] = A[(k - hx) mod nx]
+      dst[k] = cscale(buf[l * ls + line_out<N>(pl, m)], scale);
+    }
   }
 }
 
-// Column pass over strips of W columns.  aux (nullable) receives the
+// Column pass over strips of W = 1 << lw columns.  aux (nullable) receives the
 // unshifted transform FFT2(shift(in)) as cudaFFT leaves it in its input
 // buffer (HologramKernel.cu:207-210).
 template <typename R, int SGN, int N>
 __global__ void __launch_bounds__(512) fft_cols_kernel(typename cplx_of<R>::type* data,
                                                        typename cplx_of<R>::type* aux,
-                                                       int nx, int ny, int W, int shift, R scale,
+                                                       int nx, int ny, int lw, int shift, R scale,
                                                        FFTPlan pl) {
   typedef typename cplx_of<R>::type C;
   extern __shared__ unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
+  const int W = 1 << lw;
   const int x0 = blockIdx.x * W;
   const int hy = shift ? ny / 2 : 0;
   const int hx = shift ? nx / 2 : 0;
   for (int idx = threadIdx.x; idx < ny * W; idx += blockDim.x) {
-    int i = idx / W, w = idx - i * W;
+    const int i = idx >> lw, w = idx & (W - 1);
     int src = i - hy; if (src < 0) src += ny;
-    buf[idx] = data[(size_t)src * nx + x0 + w];
+    buf[line_at<N>(pl, i) * W + w] = data[(size_t)src * nx + x0 + w];
   }
-  block_fft_n<N, SGN>(buf, W, 1, W, pl, true);
+  line_fft<N, SGN>(buf, W, 1, W, pl, lw);
   for (int idx = threadIdx.x; idx < ny * W; idx += blockDim.x) {
-    int k = idx / W, w = idx - k * W;
+    const int k = idx >> lw, w = idx & (W - 1);
     int m = k - hy; if (m < 0) m += ny;
-    C v = buf[pl.perm[m] * W + w];
-    data[(size_t)k * nx + x0 + w] = cscale(v, scale);
+    data[(size_t)k * nx + x0 + w] = cscale(buf[line_out<N>(pl, m) * W + w], scale);
     if (aux) {
-      C u = buf[pl.perm[k] * W + w];
       int xu = x0 + w - hx; if (xu < 0) xu += nx;
-      aux[(size_t)k * nx + xu] = u;
+      aux[(size_t)k * nx + xu] = buf[line_out<N>(pl, k) * W + w];
     }
   }
+}
+
+static int log2_of(int w) { return w == 8 ? 3 : w == 4 ? 2 : w == 2 ? 1 : 0; }
+
+// Rows per block of a row pass: the most of 1, 2, 4, 8 that 48 KB hold.
+static int rows_per_block(int nx, int lens, size_t esz) {
+  int rpb = 1;
+  while (rpb < 8 && (size_t)(rpb * 2) * lens * esz <= 48 * 1024 && rpb * 2 * nx <= 4096) rpb *= 2;
+  return rpb;
 }
 
 template <typename R>
@@ -80,14 +112,12 @@ static oh_status launch_fft2d(oh_ctx* ctx, int nx, int ny, const void* in, void*
   OH_TRY(get_plan(ctx, nx, prec, &px));
   OH_TRY(get_plan(ctx, ny, prec, &py));
   const size_t smax = max_smem_per_block();
-  // rows
-  int rpb = 1;
-  while (rpb < 8 && (size_t)(rpb * 2) * nx * sizeof(C) <= 48 * 1024 && rpb * 2 * nx <= 4096) rpb *= 2;
-  size_t srow = (size_t)rpb * nx * sizeof(C);
+  const int rpb = rows_per_block(nx, px.lens, sizeof(C));
+  size_t srow = (size_t)rpb * px.lens * sizeof(C);
   if (srow > smax) return fail(OH_ERR_UNSUPPORTED_SIZE, "row length " + std::to_string(nx) + " exceeds shared memory");
-  int W = pick_strip_width(nx, ny, sizeof(C), smax);
+  int W = pick_strip_width(nx, py.lens, sizeof(C), smax);
   if (W == 0) return fail(OH_ERR_UNSUPPORTED_SIZE, "column length " + std::to_string(ny) + " exceeds shared memory");
-  size_t scol = (size_t)W * ny * sizeof(C);
+  size_t scol = (size_t)W * py.lens * sizeof(C);
   R scale = normalize ? (R)(1.0 / ((double)nx * (double)ny)) : (R)1;
   const C* cin = static_cast<const C*>(in);
   C* cout_ = static_cast<C*>(out);
@@ -111,7 +141,7 @@ static oh_status launch_fft2d(oh_ctx* ctx, int nx, int ny, const void* in, void*
       cudaError_t e = cudaFuncSetAttribute(fft_cols_kernel<R, SG, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol);
       if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(fft_cols)"); return; }
       KernelTimer kt(ctx, "fft_cols", st);
-      fft_cols_kernel<R, SG, NY><<<nx / W, 512, scol, st>>>(cout_, static_cast<C*>(aux), nx, ny, W, shift, scale, py);
+      fft_cols_kernel<R, SG, NY><<<nx / W, 512, scol, st>>>(cout_, static_cast<C*>(aux), nx, ny, log2_of(W), shift, scale, py);
       note_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) rs = cuda_fail(e, "fft_cols launch");
     });
@@ -128,9 +158,8 @@ static oh_status launch_fft_rows(oh_ctx* ctx, int nx, int ny, const void* in, vo
   const int prec = sizeof(R) == 8 ? 1 : 0;
   FFTPlan px;
   OH_TRY(get_plan(ctx, nx, prec, &px));
-  int rpb = 1;
-  while (rpb < 8 && (size_t)(rpb * 2) * nx * sizeof(C) <= 48 * 1024 && rpb * 2 * nx <= 4096) rpb *= 2;
-  size_t srow = (size_t)rpb * nx * sizeof(C);
+  const int rpb = rows_per_block(nx, px.lens, sizeof(C));
+  size_t srow = (size_t)rpb * px.lens * sizeof(C);
   if (srow > max_smem_per_block()) return fail(OH_ERR_UNSUPPORTED_SIZE, "row length exceeds shared memory");
   R scale = normalize ? (R)(1.0 / (double)nx) : (R)1;
   if (direction < 0) {
@@ -157,16 +186,16 @@ static oh_status launch_fft_cols(oh_ctx* ctx, int nx, int ny, void* data, int di
   const int prec = sizeof(R) == 8 ? 1 : 0;
   FFTPlan py;
   OH_TRY(get_plan(ctx, ny, prec, &py));
-  const int W = pick_strip_width(nx, ny, sizeof(C), max_smem_per_block());
+  const int W = pick_strip_width(nx, py.lens, sizeof(C), max_smem_per_block());
   if (W == 0) return fail(OH_ERR_UNSUPPORTED_SIZE, "column length " + std::to_string(ny) + " exceeds shared memory");
-  const size_t scol = (size_t)W * ny * sizeof(C);
+  const size_t scol = (size_t)W * py.lens * sizeof(C);
   const R scale = normalize ? (R)(1.0 / (double)ny) : (R)1;
   if (direction < 0) {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_cols_kernel<R, -1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol));
-    fft_cols_kernel<R, -1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, W, 0, scale, py);
+    fft_cols_kernel<R, -1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
   } else {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_cols_kernel<R, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol));
-    fft_cols_kernel<R, 1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, W, 0, scale, py);
+    fft_cols_kernel<R, 1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
   }
   OH_LAUNCH_CHECK();
   return OH_OK;
@@ -202,7 +231,7 @@ extern "C" {
 
 int oh_fft_supported(int n, oh_precision prec) {
   int radix[kMaxStages], nst;
-  if (n < 1 || !factorize(n, radix, &nst)) return 0;
+  if (n < 1 || !factorize(n, prec == OH_FP64 ? 1 : 0, radix, &nst)) return 0;
   size_t esz = prec == OH_FP64 ? sizeof(double2) : sizeof(float2);
   return (size_t)n * esz <= max_smem_per_block() ? 1 : 0;
 }

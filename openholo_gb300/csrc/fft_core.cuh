@@ -1,7 +1,6 @@
 // Block-level mixed-radix FFT on data resident in shared memory.
 //
-// A length-n line (n = r0*r1*...*r_{S-1}, radices 2,3,4,5,8 and any other
-// prime through a generic O(r^2) butterfly) is transformed in place with the
+// A length-n line (n = r0*r1*...*r_{S-1}) is transformed in place with the
 // decimation-in-frequency (Sande-Tukey) recursion:
 //   stage s works on blocks of m_s = r_s*q_s elements; for j < q_s it takes
 //   x[j + t*q_s], t < r_s, forms the r_s-point DFT y_f, multiplies y_f by
@@ -20,19 +19,38 @@
 
 namespace oh {
 
-constexpr int kMaxStages = 24;
+constexpr int kMaxStages = 16;
 constexpr int kMaxGenericRadix = 64;
 
+// A plan's line is stored with one pad element after every padr elements when
+// its last radix is even (padr = that radix; the last stage would otherwise
+// crowd its reads onto few shared-memory banks), else without pads (padr = 0).
+// padr divides every stage's block and stride, so all stages keep fixed
+// strides.  The compile-time engine (fft_fast.cuh) has layouts of its own.
 struct FFTPlan {
   int n;
   int nst;
+  int lens;               // stored length of a line: n, or n + n / padr
+  int padr;
+  uint32_t mpad;          // divider of padr (see fdiv)
   int radix[kMaxStages];
   int q[kMaxStages];      // stride inside a block at stage s
-  int tws[kMaxStages];    // twiddle index step n/m_s
+  int qs[kMaxStages];     // the stored stride
+  int two[kMaxStages];    // first entry of stage s in stw
+  uint32_t mq[kMaxStages];    // dividers of q and of n / radix
+  uint32_t mnb[kMaxStages];
   const void* tw;         // n complex twiddles W_n^e (precision of the kernel)
+  const void* stw;        // per stage with q > 1: W_{m_s}^{j f} at [f - 1][j], 1 <= f < radix, j < q
   const int* perm;        // perm[k]: position of X[k] after the last stage
   const int* iperm;       // iperm[pos]: frequency k stored at pos
+  const int* permp;       // perm in stored positions
 };
+
+// i / d for i < 2^18, d < 2^15 with m = ceil(2^32 / d) (0 stands for d = 1)
+__device__ __forceinline__ int fdiv(int i, uint32_t m) { return m ? (int)__umulhi((uint32_t)i, m) : i; }
+
+// stored position of line element p
+__device__ __forceinline__ int pl_at(const FFTPlan& pl, int p) { return pl.padr ? p + fdiv(p, pl.mpad) : p; }
 
 // ---- small DFT kernels (forward SGN=-1, inverse SGN=+1) -------------------
 
@@ -103,103 +121,6 @@ __device__ __forceinline__ C twiddle(const C* tw, int e) {
   C w = tw[e];
   if (SGN > 0) w.y = -w.y;
   return w;
-}
-
-// One DIF stage over `nl` lines.  col_major selects the thread mapping:
-// true -> line index fastest (interleaved column strips), false -> butterfly
-// index fastest (contiguous rows).
-template <int SGN, typename C>
-__device__ __forceinline__ void fft_stage(C* buf, int nl, int ls, int es, int n,
-                                          int r, int q, int tws, const C* tw,
-                                          bool line_fastest) {
-  const int nb = n / r;            // butterflies per line
-  const int total = nb * nl;
-  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    int line, b;
-    if (line_fastest) { line = idx % nl; b = idx / nl; }
-    else { b = idx % nb; line = idx / nb; }
-    const int blk = b / q, j = b - blk * q;
-    const int base = line * ls + (blk * r * q + j) * es;
-    const int st = q * es;
-    switch (r) {
-      case 2: {
-        C a = buf[base], c = buf[base + st];
-        dft2<SGN>(a, c);
-        if (j) c = cmul(c, twiddle<SGN>(tw, j * tws));
-        buf[base] = a; buf[base + st] = c;
-      } break;
-      case 3: {
-        C a = buf[base], c = buf[base + st], d = buf[base + 2 * st];
-        dft3<SGN>(a, c, d);
-        if (j) { c = cmul(c, twiddle<SGN>(tw, j * tws)); d = cmul(d, twiddle<SGN>(tw, 2 * j * tws)); }
-        buf[base] = a; buf[base + st] = c; buf[base + 2 * st] = d;
-      } break;
-      case 4: {
-        C x0 = buf[base], x1 = buf[base + st], x2 = buf[base + 2 * st], x3 = buf[base + 3 * st];
-        dft4<SGN>(x0, x1, x2, x3);
-        if (j) {
-          const int e = j * tws;
-          x1 = cmul(x1, twiddle<SGN>(tw, e));
-          x2 = cmul(x2, twiddle<SGN>(tw, 2 * e));
-          x3 = cmul(x3, twiddle<SGN>(tw, 3 * e));
-        }
-        buf[base] = x0; buf[base + st] = x1; buf[base + 2 * st] = x2; buf[base + 3 * st] = x3;
-      } break;
-      case 5: {
-        C x0 = buf[base], x1 = buf[base + st], x2 = buf[base + 2 * st], x3 = buf[base + 3 * st], x4 = buf[base + 4 * st];
-        dft5<SGN>(x0, x1, x2, x3, x4);
-        if (j) {
-          const int e = j * tws;
-          x1 = cmul(x1, twiddle<SGN>(tw, e));
-          x2 = cmul(x2, twiddle<SGN>(tw, 2 * e));
-          x3 = cmul(x3, twiddle<SGN>(tw, 3 * e));
-          x4 = cmul(x4, twiddle<SGN>(tw, 4 * e));
-        }
-        buf[base] = x0; buf[base + st] = x1; buf[base + 2 * st] = x2; buf[base + 3 * st] = x3; buf[base + 4 * st] = x4;
-      } break;
-      case 8: {
-        C x[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) x[t] = buf[base + t * st];
-        dft8<SGN>(x);
-        if (j) {
-          const int e = j * tws;
-#pragma unroll
-          for (int t = 1; t < 8; ++t) x[t] = cmul(x[t], twiddle<SGN>(tw, t * e));
-        }
-#pragma unroll
-        for (int t = 0; t < 8; ++t) buf[base + t * st] = x[t];
-      } break;
-      default: {
-        // generic odd radix: y_f = sum_t x_t w_r^{t f}, w_r^m = W_n^{m n / r}
-        C x[kMaxGenericRadix];
-        for (int t = 0; t < r; ++t) x[t] = buf[base + t * st];
-        const int step = n / r;
-        for (int f = 0; f < r; ++f) {
-          C acc = x[0];
-          int m = 0;
-          for (int t = 1; t < r; ++t) {
-            m += f; if (m >= r) m -= r;
-            acc = cadd(acc, cmul(x[t], twiddle<SGN>(tw, m * step)));
-          }
-          if (j && f) acc = cmul(acc, twiddle<SGN>(tw, f * j * tws));
-          buf[base + f * st] = acc;
-        }
-      } break;
-    }
-  }
-}
-
-// Full in-place transform of nl lines; ends with __syncthreads().
-template <int SGN, typename C>
-__device__ void block_fft(C* buf, int nl, int ls, int es, const FFTPlan& pl,
-                          bool line_fastest) {
-  const C* tw = static_cast<const C*>(pl.tw);
-  for (int s = 0; s < pl.nst; ++s) {
-    __syncthreads();
-    fft_stage<SGN>(buf, nl, ls, es, pl.n, pl.radix[s], pl.q[s], pl.tws[s], tw, line_fastest);
-  }
-  __syncthreads();
 }
 
 }  // namespace oh

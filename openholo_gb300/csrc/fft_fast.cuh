@@ -524,16 +524,4 @@ template <int N> struct FastSched { static constexpr bool ok = false; };
 OH_FAST_SCHEDULES(OH_DEFINE_SCHED)
 #undef OH_DEFINE_SCHED
 
-// In-place transform of nl lines with the compile-time schedule for N when
-// N > 0, else the generic engine; ends with __syncthreads().
-template <int N, int SGN, typename C>
-__device__ __forceinline__ void block_fft_n(C* buf, int nl, int ls, int es, const FFTPlan& pl, bool line_fastest) {
-  if constexpr (N > 0) {
-    FastSched<N>::template run<SGN>(buf, nl, ls, es, static_cast<const C*>(pl.tw), line_fastest);
-    __syncthreads();
-  } else {
-    block_fft<SGN>(buf, nl, ls, es, pl, line_fastest);
-  }
-}
-
 }  // namespace oh

@@ -2,7 +2,7 @@
 #pragma once
 #include <type_traits>
 #include "context.h"
-#include "fft_fast.cuh"
+#include "fft_generic.cuh"
 
 namespace oh {
 
