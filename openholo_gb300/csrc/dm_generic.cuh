@@ -8,18 +8,21 @@
 
 namespace oh {
 
-// Row pass: nr (1 or 2) image rows per block.  Per layer present in them: stage
-// 0 straight from the source pixels, the other stages in place, then the lines
-// go to the strips in storage order (W of them, so two rows fill a 32-byte
-// sector).
+// Row pass: nr (1 or 2) image rows per block.  The layers present in them are
+// taken G at a time (short lines alone leave most threads idle): stage 0
+// straight from the source pixels, the other stages in place, then the lines go
+// to the strips in storage order (two columns per strip in FP32: two rows fill
+// a 32-byte sector).
 template <typename R>
-__global__ void __launch_bounds__(256) dm_row_gen(DMArgs<R> a, int nr) {
+__global__ void __launch_bounds__(256, 2) dm_row_gen(DMArgs<R> a, int nr, int G) {
   typedef typename cplx_of<R>::type C;
   extern __shared__ unsigned char smem_raw[];
   const int Px = a.Px, pnx = a.pnx, T = blockDim.x;
   const int lip = (pnx + 7) & ~7, lens = a.plx.lens;
-  C* buf = reinterpret_cast<C*>(smem_raw);              // [nr][lens]
-  C* v = buf + nr * lens;                               // [nr][pnx] source values
+  __shared__ int16_t present[kMaxEntries];
+  __shared__ int s_np;
+  C* buf = reinterpret_cast<C*>(smem_raw);              // [G][nr][lens]
+  C* v = buf + G * nr * lens;                           // [nr][pnx] source values
   int16_t* li = reinterpret_cast<int16_t*>(v + nr * pnx);        // [nr][lip] layer slot per pixel
   uint32_t* mask = reinterpret_cast<uint32_t*>(li + nr * lip);   // [2][8] layers present per row
   const int r0 = blockIdx.x * nr;
@@ -62,40 +65,59 @@ __global__ void __launch_bounds__(256) dm_row_gen(DMArgs<R> a, int nr) {
       v[l * pnx + c] = val;
     }
   __syncthreads();
+  // the slots present in the block's rows, their flags per row
+  auto has = [&](int l, int u) { return (mask[l * 8 + (u >> 5)] >> (u & 31)) & 1u; };
+  if (threadIdx.x < 32) {
+    int n = 0;
+    for (int base = a.slot0; base < a.slot1; base += 32) {
+      const int u = base + threadIdx.x;
+      const bool p = u < a.slot1 && (has(0, u) || has(1, u));
+      const unsigned m = __ballot_sync(0xffffffffu, p);
+      if (p) {
+        present[n + __popc(m & ((1u << threadIdx.x) - 1u))] = (int16_t)u;
+        a.slot_any[u] = 1;
+      }
+      n += __popc(m);
+    }
+    if (threadIdx.x == 0) s_np = n;
+  }
+  for (int i = threadIdx.x; i < nrows * (a.slot1 - a.slot0); i += T) {
+    const int l = nrows == 2 ? i & 1 : 0, ur = nrows == 2 ? i >> 1 : i;
+    a.occ[(size_t)ur * a.occ_stride + r0 + l] = has(l, a.slot0 + ur) ? 1 : 0;
+  }
+  __syncthreads();
   const GStage g0 = gstage_of(a.plx, 0, sizeof(C));
-  for (int u = a.slot0; u < a.slot1; ++u) {
-    const bool p0 = (mask[u >> 5] >> (u & 31)) & 1u;
-    const bool p1 = (mask[8 + (u >> 5)] >> (u & 31)) & 1u;
-    const int ur = u - a.slot0;
-    if (threadIdx.x < nrows) a.occ[(size_t)ur * a.occ_stride + r0 + threadIdx.x] = (threadIdx.x == 0 ? p0 : p1) ? 1 : 0;
-    if (!(p0 || p1)) continue;
-    if (threadIdx.x == 0) a.slot_any[u] = 1;
+  const int np = s_np, W = a.W, lw = a.lw;
+  for (int q = 0; q < np; q += G) {
+    const int nq = min(G, np - q), ng = nq * nrows;      // line k: slot q + k / nrows, row k % nrows
+    auto slot_of = [&](int k) { return (int)present[q + (nrows == 2 ? k >> 1 : k)]; };
     // input i of the x-shifted, zero-padded line a[i] = u[(i - hx) mod Px]
-    auto pixel = [&](int l, int i) -> C {
+    auto pixel = [&](int l, int u, int i) -> C {
       int x = i - a.hx;
       if (x < 0) x += Px;
       const int c = x - a.ox;
       return (unsigned)c < (unsigned)pnx && li[l * lip + c] == u ? v[l * pnx + c] : mk((R)0, (R)0);
     };
     if (a.plx.nst == 0) {
-      if (threadIdx.x < nrows) buf[threadIdx.x * lens] = pixel(threadIdx.x, 0);
+      if (threadIdx.x < ng) buf[threadIdx.x * lens] = pixel(nrows == 2 ? threadIdx.x & 1 : 0, slot_of(threadIdx.x), 0);
     } else {
       with_radix<false>(g0.r, [&](auto rc) {
         constexpr int RR = decltype(rc)::value;
-        const int total = g0.nb * nrows;
+        const int total = g0.nb * ng;
         for (int idx = threadIdx.x; idx < total; idx += T) {
-          int l, b, j;
-          gsplit(g0, idx, -1, &l, &b);
-          C* p = buf + l * lens + gbase(g0, b, &j);
+          int off, b, j;
+          const int k = gsplit(g0, idx, ng, lens, 0, &off, &b);
+          const int l = nrows == 2 ? k & 1 : 0, u = slot_of(k);
+          C* p = buf + off + gbase(g0, b, &j);
           if constexpr (RR > 0) {
             C x[RR];
 #pragma unroll
-            for (int t = 0; t < RR; ++t) x[t] = pixel(l, j + t * g0.q);
+            for (int t = 0; t < RR; ++t) x[t] = pixel(l, u, j + t * g0.q);
             gbutterfly<RR, GFWD>(g0, j, x);
 #pragma unroll
             for (int t = 0; t < RR; ++t) p[t * g0.qs] = x[t];
           } else {
-            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return pixel(l, j + t * g0.q); },
+            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return pixel(l, u, j + t * g0.q); },
                                     [&](int f, C y) { p[f * g0.qs] = y; });
           }
         }
@@ -103,15 +125,17 @@ __global__ void __launch_bounds__(256) dm_row_gen(DMArgs<R> a, int nr) {
     }
     for (int s = 1; s < a.plx.nst; ++s) {
       __syncthreads();
-      gstage_call<GFWD, C, false>(gstage_of(a.plx, s, sizeof(C)), 0, nrows, lens, 1, -1);
+      gstage_call<GFWD, C, false>(gstage_of(a.plx, s, sizeof(C)), 0, ng, lens, 0);
     }
     __syncthreads();
-    C* dst = a.Rbuf + (size_t)ur * a.nstrips * a.pny * a.W;
-    const int W = a.W, lw = a.lw;
-    for (int idx = threadIdx.x; idx < nrows * Px; idx += T) {
-      const int w = idx & (W - 1), t = idx >> lw;
-      const int l = nrows == 2 ? (t & 1) : 0, s = nrows == 2 ? (t >> 1) : t;
-      dst[((size_t)s * a.pny + r0 + l) * W + w] = buf[l * lens + pl_at(a.plx, (s << lw) + w)];
+    for (int k = 0; k < nq; ++k) {
+      C* dst = a.Rbuf + (size_t)(present[q + k] - a.slot0) * a.nstrips * a.pny * W;
+      const C* line = buf + k * nrows * lens;
+      for (int idx = threadIdx.x; idx < nrows * Px; idx += T) {
+        const int w = idx & (W - 1), t = idx >> lw;
+        const int l = nrows == 2 ? (t & 1) : 0, s = nrows == 2 ? (t >> 1) : t;
+        dst[((size_t)s * a.pny + r0 + l) * W + w] = line[l * lens + pl_at(a.plx, (s << lw) + w)];
+      }
     }
     __syncthreads();
   }
@@ -137,17 +161,18 @@ __device__ __forceinline__ double2 cis_turns(double t, const double2* tab) {
 // active entries, and in FP64 the direction table and (evenly spaced layers)
 // the step factors.
 template <typename R>
-inline size_t dm_col_gen_smem(int lens, int lwb, int nrow, int n_entries, bool horner) {
-  size_t o = (size_t)lens << lwb;
+inline size_t dm_col_gen_smem(int lens, int lwb, int G, int nrow, int n_entries, bool horner) {
+  size_t o = (size_t)G * lens << lwb;
   if (sizeof(R) == 8) o += 128 + (horner ? (size_t)nrow << lwb : 0);
   o *= 2 * sizeof(R);
   return o + (((size_t)nrow * 2 + 15) & ~(size_t)15) + (size_t)n_entries * 2 + 16;
 }
 
 // Column pass: 1 << lwb spectrum columns (storage positions) per block for the
-// whole frame.  Per active layer: stage 0 straight from the strips (absent and
-// padded rows are zeros), the other stages in place, then every thread adds
-// H(e) times its samples into registers.  Only the spectrum rows [row0, row0 +
+// whole frame.  The active layers are taken G at a time (short columns alone
+// leave most threads idle): stage 0 straight from the strips (absent and padded
+// rows are zeros), the other stages in place, then every thread adds H(e) times
+// its samples into registers.  Only the spectrum rows [row0, row0 +
 // nrow) that reach the crop are kept.  Transfer function: the entry's separable
 // tables times exp(i k z' g), g = s^2 / (2 (1 + sqrt(1 - s))^2) held per sample;
 // FP64 with evenly spaced layers accumulates acc = acc D + x instead (see
@@ -156,7 +181,7 @@ inline size_t dm_col_gen_smem(int lens, int lwb, int nrow, int n_entries, bool h
 // What bounds it: instruction issue in FP32 (FFT butterflies plus about 20
 // instructions per kept sample and layer), the FP64 pipe in FP64.
 template <typename R, int KMAX, int T, int MINB>
-__global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int row0, int nrow) {
+__global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int G, int row0, int nrow) {
   typedef typename cplx_of<R>::type C;
   constexpr bool F64 = sizeof(R) == 8;
   constexpr bool KEEPG = KMAX <= 16;                    // g per sample in registers
@@ -165,7 +190,8 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
   const int W = 1 << lwb, Py = a.Py, pny = a.pny, lens = a.ply.lens, tid = threadIdx.x;
   const bool step = F64 && a.horner;
   C* buf = reinterpret_cast<C*>(smem_raw);
-  C* tab = buf + ((size_t)lens << lwb);
+  const int gs = lens << lwb;                           // a layer's lines
+  C* tab = buf + (size_t)G * gs;
   C* dst = tab + (F64 ? 128 : 0);
   uint16_t* pos = reinterpret_cast<uint16_t*>(dst + (step ? (size_t)nrow << lwb : 0));
   int16_t* list = reinterpret_cast<int16_t*>(pos + ((nrow + 7) & ~7));
@@ -230,36 +256,41 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
     }
   }
   const GStage g0 = gstage_of(a.ply, 0, sizeof(C));
-  for (int q = 0; q < nact; ++q) {
-    const int e = list[q], u = a.uslot_of_entry[e];
-    const uint8_t* occ = a.occ + (size_t)u * a.occ_stride;
-    const C* src = a.Rbuf + ((size_t)u * a.nstrips + (p >> a.lw)) * pny * a.W + (p & (a.W - 1));
-    // input i of the y-shifted, zero-padded column
-    auto sample = [&](int i) -> C {
+  for (int q = 0; q < nact; q += G) {
+    const int ng = min(G, nact - q);
+    // input i of the y-shifted, zero-padded column of entry list[q + k]
+    auto sample = [&](const C* src, const uint8_t* occ, int i) -> C {
       int y = i - a.hy;
       if (y < 0) y += Py;
       y -= a.oy;
       return valid && (unsigned)y < (unsigned)pny && __ldg(occ + y) ? src[y << a.lw] : mk((R)0, (R)0);
     };
+    auto column = [&](int u) { return a.Rbuf + ((size_t)u * a.nstrips + (p >> a.lw)) * pny * a.W + (p & (a.W - 1)); };
     if (a.ply.nst == 0) {
-      if (tid < W) buf[tid] = sample(0);
+      for (int k = tid >> lwb; k < ng; k += T >> lwb) {
+        const int u = a.uslot_of_entry[list[q + k]];
+        buf[k * gs + w] = sample(column(u), a.occ + (size_t)u * a.occ_stride, 0);
+      }
     } else {
       with_radix<false>(g0.r, [&](auto rc) {
         constexpr int RR = decltype(rc)::value;
-        const int total = g0.nb << lwb;
+        const int total = (g0.nb * ng) << lwb, st = g0.qs << lwb;
         for (int idx = tid; idx < total; idx += T) {
-          int j;
-          C* d = buf + (gbase(g0, idx >> lwb, &j) << lwb) + w;
-          const int st = g0.qs << lwb;
+          int off, b, j;
+          const int k = gsplit(g0, idx, ng, gs, lwb, &off, &b);
+          const int u = a.uslot_of_entry[list[q + k]];
+          const uint8_t* occ = a.occ + (size_t)u * a.occ_stride;
+          const C* src = column(u);
+          C* d = buf + off + (gbase(g0, b, &j) << lwb);
           if constexpr (RR > 0) {
             C x[RR];
 #pragma unroll
-            for (int t = 0; t < RR; ++t) x[t] = sample(j + t * g0.q);
+            for (int t = 0; t < RR; ++t) x[t] = sample(src, occ, j + t * g0.q);
             gbutterfly<RR, GFWD>(g0, j, x);
 #pragma unroll
             for (int t = 0; t < RR; ++t) d[t * st] = x[t];
           } else {
-            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return sample(j + t * g0.q); },
+            gbutterfly_any<GFWD, C>(g0, j, [&](int t) { return sample(src, occ, j + t * g0.q); },
                                     [&](int f, C y) { d[f * st] = y; });
           }
         }
@@ -267,40 +298,44 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
     }
     for (int s = 1; s < a.ply.nst; ++s) {
       __syncthreads();
-      const GStage gs = gstage_of(a.ply, s, sizeof(C));
-      with_radix<false>(gs.r, [&](auto rc) {
-        gstage_loop<decltype(rc)::value, GFWD, C>(gs, buf, W, 1, W, lwb);
+      const GStage gs1 = gstage_of(a.ply, s, sizeof(C));
+      with_radix<false>(gs1.r, [&](auto rc) {
+        gstage_loop<decltype(rc)::value, GFWD, C>(gs1, buf, ng, gs, lwb);
       });
     }
     __syncthreads();
-    if (F64 && step) {
-      const int gap = q > 0 ? e - list[q - 1] : 0;      // levels without pixels: one more factor each
+    for (int k0 = 0; k0 < ng; ++k0) {
+      const int e = list[q + k0];
+      const C* line = buf + k0 * gs + w;
+      if (F64 && step) {
+        const int gap = q + k0 > 0 ? e - list[q + k0 - 1] : 0;      // levels without pixels: one more factor each
 #pragma unroll
-      for (int k = 0; k < KMAX; ++k) {
-        const int idx = tid + k * T;
-        if (idx < nk) {
-          const C x = buf[((int)pos[idx >> lwb] << lwb) + w];
-          if (gap) {
-            const C d = dst[idx];
-            for (int r = 1; r < gap; ++r) acc[k] = cmul(acc[k], d);
-            acc[k] = mk(fma(acc[k].x, d.x, fma(-acc[k].y, d.y, x.x)), fma(acc[k].x, d.y, fma(acc[k].y, d.x, x.y)));
-          } else {
-            acc[k] = x;
+        for (int k = 0; k < KMAX; ++k) {
+          const int idx = tid + k * T;
+          if (idx < nk) {
+            const C x = line[(int)pos[idx >> lwb] << lwb];
+            if (gap) {
+              const C d = dst[idx];
+              for (int r = 1; r < gap; ++r) acc[k] = cmul(acc[k], d);
+              acc[k] = mk(fma(acc[k].x, d.x, fma(-acc[k].y, d.y, x.x)), fma(acc[k].x, d.y, fma(acc[k].y, d.x, x.y)));
+            } else {
+              acc[k] = x;
+            }
           }
         }
-      }
-    } else if (valid) {
-      const R kz = a.kzp[e];
-      const C ex = a.exc[(size_t)e * a.Px + kx];
-      const C* ey = a.ey + (size_t)e * Py + row0;
+      } else if (valid) {
+        const R kz = a.kzp[e];
+        const C ex = a.exc[(size_t)e * a.Px + kx];
+        const C* ey = a.ey + (size_t)e * Py + row0;
 #pragma unroll
-      for (int k = 0; k < KMAX; ++k) {
-        const int idx = tid + k * T;
-        if (idx < nk) {
-          const C h = cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k));
-          const C x = buf[((int)pos[idx >> lwb] << lwb) + w];
-          acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
-          acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
+        for (int k = 0; k < KMAX; ++k) {
+          const int idx = tid + k * T;
+          if (idx < nk) {
+            const C h = cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k));
+            const C x = line[(int)pos[idx >> lwb] << lwb];
+            acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
+            acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
+          }
         }
       }
     }
@@ -337,7 +372,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
       }
     }
   }
-  block_fft<GADJ, C, false>(0, W, 1, W, a.ply, lwb);
+  block_fft<GADJ, C, false>(0, 1, 0, lwb, a.ply);
   for (int idx = tid; idx < pny << lwb; idx += T) {
     const int yl = idx >> lwb;
     int m = a.oy + yl - a.hy;
@@ -368,7 +403,7 @@ __global__ void __launch_bounds__(256) dm_out_gen(DMArgs<R> a) {
     }
     buf[at] = row[p];
   }
-  block_fft<GADJ, C, false>(0, 1, 0, 1, a.plx, -1);
+  block_fft<GADJ, C, false>(0, 1, 0, 0, a.plx);
   for (int c = threadIdx.x; c < a.pnx; c += blockDim.x) {
     int m = a.ox + c - a.hx;
     if (m < 0) m += Px;
@@ -381,8 +416,8 @@ __global__ void __launch_bounds__(256) dm_out_gen(DMArgs<R> a) {
 
 // How a frame runs these passes (dm_generic.cuh's launches).
 struct DMGenPlan {
-  int nr;                 // image rows per row-pass block
-  int lwb;                // log2 columns per column-pass block
+  int nr, gr;             // image rows per row-pass block, layers taken at a time
+  int lwb, gc;            // log2 columns per column-pass block, layers taken at a time
   int row0, nrow;         // spectrum rows kept
   bool wide;              // the column pass's many-samples variant
   size_t smem_row, smem_col, smem_out;

@@ -7,10 +7,10 @@
 namespace oh {
 
 // Samples per thread and threads per block of the column pass: few enough that
-// the accumulators (and g) stay in registers with two blocks per SM; the wide
+// the accumulators (and g) stay in registers with three blocks per SM; the wide
 // variant takes what is longer.
 template <typename R> struct DMGenCfg {
-  static constexpr int K = sizeof(R) == 8 ? 10 : 16, T = sizeof(R) == 8 ? 128 : 256, MINB = sizeof(R) == 8 ? 3 : 2;
+  static constexpr int K = sizeof(R) == 8 ? 10 : 8, T = sizeof(R) == 8 ? 128 : 256, MINB = 3;
   static constexpr int KW = 40, TW = sizeof(R) == 8 ? 256 : 512;
 };
 
@@ -19,14 +19,23 @@ DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax) {
   typedef DMGenCfg<R> CF;
   const size_t esz = 2 * sizeof(R);
   DMGenPlan g{};
-  auto row = [&](int nr) {
-    return (size_t)nr * ((size_t)a.plx.lens * esz + (size_t)a.pnx * esz + (size_t)((a.pnx + 7) & ~7) * 2) + 64;
+  const size_t budget = (size_t)72 * 1024;              // three blocks per SM
+  const int sms = sm_count();
+  // layers taken at a time: enough lines for two butterflies per thread in the
+  // first stage, while they fit
+  auto groups = [&](const FFTPlan& pl, int lines, int threads, int most) {
+    const int per = std::max(1, pl.nst ? pl.n / pl.radix[0] : 1) * lines;
+    return std::max(1, std::min({16, most, 2 * threads / per}));
+  };
+  auto row = [&](int nr, int G) {
+    return (size_t)nr * ((size_t)G * a.plx.lens * esz + (size_t)a.pnx * esz + (size_t)((a.pnx + 7) & ~7) * 2) + 64;
   };
   // two rows per block fill whole sectors of the strips; one where two would
   // leave fewer than three blocks per SM or the SMs short of blocks
-  const int sms = sm_count();
-  g.nr = row(2) <= (size_t)72 * 1024 && a.pny >= 4 * sms ? 2 : 1;
-  g.smem_row = row(g.nr);
+  g.nr = row(2, 1) <= budget && a.pny >= 4 * sms ? 2 : 1;
+  g.gr = groups(a.plx, g.nr, 256, a.slot1 - a.slot0);
+  while (g.gr > 1 && row(g.nr, g.gr) > budget) --g.gr;
+  g.smem_row = row(g.nr, g.gr);
   // spectrum rows that reach the crop (all of them when the spectrum is asked for)
   g.row0 = a.spectrum ? 0 : a.cy1;
   g.nrow = a.spectrum ? a.Py : a.cy2 - a.cy1 + 1;
@@ -35,9 +44,9 @@ DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax) {
   // the narrow variant, three blocks of shared memory per SM and four blocks
   // per SM of work
   g.lwb = -1;
-  for (int lw = sizeof(R) == 8 ? 1 : 2; lw >= 0; --lw) {
-    const size_t sm = dm_col_gen_smem<R>(a.ply.lens, lw, g.nrow, a.n_entries, horner);
-    if ((g.nrow << lw) <= CF::K * CF::T && sm <= (lw ? (size_t)72 * 1024 : smax) &&
+  for (int lw = 1; lw >= 0; --lw) {
+    const size_t sm = dm_col_gen_smem<R>(a.ply.lens, lw, 1, g.nrow, a.n_entries, horner);
+    if ((g.nrow << lw) <= CF::K * CF::T && sm <= (lw ? budget : smax) &&
         (lw == 0 || (a.Px >> lw) >= 4 * sms)) {
       g.lwb = lw;
       break;
@@ -45,7 +54,9 @@ DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax) {
   }
   g.wide = g.lwb < 0;
   if (g.wide) g.lwb = 0;
-  g.smem_col = dm_col_gen_smem<R>(a.ply.lens, g.lwb, g.nrow, a.n_entries, horner);
+  g.gc = groups(a.ply, 1 << g.lwb, g.wide ? CF::TW : CF::T, a.n_entries);
+  while (g.gc > 1 && dm_col_gen_smem<R>(a.ply.lens, g.lwb, g.gc, g.nrow, a.n_entries, horner) > budget) --g.gc;
+  g.smem_col = dm_col_gen_smem<R>(a.ply.lens, g.lwb, g.gc, g.nrow, a.n_entries, horner);
   g.smem_out = (size_t)a.plx.lens * esz;
   return g;
 }
@@ -59,7 +70,7 @@ template <typename R>
 cudaError_t dm_gen_row(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
   cudaError_t e = dm_gen_allow(dm_row_gen<R>, g.smem_row);
   if (e != cudaSuccess) return e;
-  dm_row_gen<R><<<(a.pny + g.nr - 1) / g.nr, 256, g.smem_row, st>>>(a, g.nr);
+  dm_row_gen<R><<<(a.pny + g.nr - 1) / g.nr, 256, g.smem_row, st>>>(a, g.nr, g.gr);
   return cudaGetLastError();
 }
 
@@ -70,7 +81,7 @@ cudaError_t dm_gen_col(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) 
   auto launch = [&](auto kern, int threads) {
     cudaError_t e = dm_gen_allow(kern, g.smem_col);
     if (e != cudaSuccess) return e;
-    kern<<<blocks, threads, g.smem_col, st>>>(a, g.lwb, g.row0, g.nrow);
+    kern<<<blocks, threads, g.smem_col, st>>>(a, g.lwb, g.gc, g.row0, g.nrow);
     return cudaGetLastError();
   };
   return g.wide ? launch(dm_col_gen<R, CF::KW, CF::TW, 1>, CF::TW) : launch(dm_col_gen<R, CF::K, CF::T, CF::MINB>, CF::T);

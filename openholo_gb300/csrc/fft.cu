@@ -29,12 +29,12 @@ __device__ __forceinline__ void line_fft(C* buf, int nl, int ls, int es, const F
     FastSched<N>::template run<SGN>(buf, nl, ls, es, static_cast<const C*>(pl.tw), lw >= 0);
     __syncthreads();
   } else {
-    block_fft<SGN < 0 ? GFWD : GINV, C>(0, nl, ls, es, pl, lw);
+    block_fft<SGN < 0 ? GFWD : GINV, C>(0, lw < 0 ? nl : 1, ls, lw < 0 ? 0 : lw, pl);
   }
 }
 
 template <typename R, int SGN, int N>
-__global__ void __launch_bounds__(256) fft_rows_kernel(const typename cplx_of<R>::type* __restrict__ in,
+__global__ void __launch_bounds__(256, N > 0 ? 1 : sizeof(R) == 8 ? 2 : 3) fft_rows_kernel(const typename cplx_of<R>::type* __restrict__ in,
                                                        typename cplx_of<R>::type* __restrict__ out,
                                                        int nx, int ny, int rpb, int shift, R scale,
                                                        FFTPlan pl) {

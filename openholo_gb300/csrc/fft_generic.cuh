@@ -124,12 +124,16 @@ __device__ __forceinline__ GStage gstage_of(const FFTPlan& pl, int s, size_t esz
   return g;
 }
 
-// Butterfly index idx of nl lines -> line, butterfly b; lw >= 0: nl = 1 << lw
-// interleaved lines (line fastest), lw < 0: contiguous lines (butterfly
-// fastest).
-__device__ __forceinline__ void gsplit(const GStage& g, int idx, int lw, int* line, int* b) {
-  if (lw >= 0) { *line = idx & ((1 << lw) - 1); *b = idx >> lw; }
-  else { *line = fdiv(idx, g.mnb); *b = idx - *line * g.nb; }
+// Lines come as ng groups of 1 << lw interleaved lines, group k's element at
+// stored position p of line w at k * ls + (p << lw) + w (lw = 0: contiguous
+// lines ls apart).  Butterfly index idx -> offset of its line, butterfly b:
+// line within the group fastest, then the butterfly, then the group.
+__device__ __forceinline__ int gsplit(const GStage& g, int idx, int ng, int ls, int lw, int* off, int* b) {
+  const int r = idx >> lw;
+  const int k = ng > 1 ? fdiv(r, g.mnb) : 0;
+  *b = r - k * g.nb;
+  *off = k * ls + (idx & ((1 << lw) - 1));
+  return k;
 }
 
 // Stored position of input 0 of butterfly b and its offset j.
@@ -187,15 +191,14 @@ __device__ __forceinline__ void gbutterfly_any(const GStage& g, int j, G get, P 
   }
 }
 
-// One in-place stage over nl lines, line l's element at stored position p at
-// buf[l * ls + p * es].
+// One in-place stage.
 template <int R, int MODE, typename C>
-__device__ __forceinline__ void gstage_loop(const GStage& g, C* buf, int nl, int ls, int es, int lw) {
-  const int total = g.nb * nl, st = g.qs * es;
+__device__ __forceinline__ void gstage_loop(const GStage& g, C* buf, int ng, int ls, int lw) {
+  const int total = (g.nb * ng) << lw, st = g.qs << lw;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    int line, b, j;
-    gsplit(g, idx, lw, &line, &b);
-    C* p = buf + line * ls + gbase(g, b, &j) * es;
+    int off, b, j;
+    gsplit(g, idx, ng, ls, lw, &off, &b);
+    C* p = buf + off + (gbase(g, b, &j) << lw);
     if constexpr (R > 0) {
       C x[R];
 #pragma unroll
@@ -209,24 +212,24 @@ __device__ __forceinline__ void gstage_loop(const GStage& g, C* buf, int nl, int
   }
 }
 
-// The same as a call: one copy of the seventeen radices per translation unit.
-// off is the lines' byte offset in the kernel's dynamic shared memory (so that
-// the accesses stay shared-memory ones).
+// The same as a call: one copy of the radices per kernel.  off is the lines'
+// byte offset in the kernel's dynamic shared memory (so that the accesses stay
+// shared-memory ones).
 template <int MODE, typename C, bool WIDE>
-__device__ __noinline__ void gstage_call(GStage g, int off, int nl, int ls, int es, int lw) {
+__device__ __noinline__ void gstage_call(GStage g, int off, int ng, int ls, int lw) {
   extern __shared__ unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw + off);
-  with_radix<WIDE>(g.r, [&](auto rc) { gstage_loop<decltype(rc)::value, MODE, C>(g, buf, nl, ls, es, lw); });
+  with_radix<WIDE>(g.r, [&](auto rc) { gstage_loop<decltype(rc)::value, MODE, C>(g, buf, ng, ls, lw); });
 }
 
-// Full in-place transform of nl lines at byte offset off of the dynamic shared
+// Full in-place transform of the lines at byte offset off of the dynamic shared
 // memory; a barrier before every stage and after the last.  WIDE: see
 // with_radix (lengths with a compile-time schedule may pass through here).
 template <int MODE, typename C, bool WIDE = sizeof(C) == 8>
-__device__ __forceinline__ void block_fft(int off, int nl, int ls, int es, const FFTPlan& pl, int lw) {
+__device__ __forceinline__ void block_fft(int off, int ng, int ls, int lw, const FFTPlan& pl) {
   for (int i = 0; i < pl.nst; ++i) {
     __syncthreads();
-    gstage_call<MODE, C, WIDE>(gstage_of(pl, MODE == GADJ ? pl.nst - 1 - i : i, sizeof(C)), off, nl, ls, es, lw);
+    gstage_call<MODE, C, WIDE>(gstage_of(pl, MODE == GADJ ? pl.nst - 1 - i : i, sizeof(C)), off, ng, ls, lw);
   }
   __syncthreads();
 }
