@@ -14,7 +14,7 @@ template <typename R> __device__ __forceinline__ R ratan2(R y, R x);
 template <> __device__ __forceinline__ float ratan2<float>(float y, float x) { return atan2f(y, x); }
 template <> __device__ __forceinline__ double ratan2<double>(double y, double x) { return atan2(y, x); }
 
-enum RedOp { RED_MAX_ABS = 0, RED_MINMAX_REAL = 1, RED_MAX_NI = 2, RED_MAX_PHASE = 3, RED_MINMAX_SSB = 4 };
+enum RedOp { RED_MAX_ABS = 0, RED_MINMAX_REAL = 1, RED_MAX_NI = 2 };
 
 // Block partial reductions: out[2*b] = min, out[2*b+1] = max of the mapped value.
 template <typename R>
@@ -26,9 +26,7 @@ __global__ void __launch_bounds__(256) reduce_partial(const void* __restrict__ i
   auto take = [&](C c) {
     R v;
     if (op == RED_MAX_ABS) v = hypot(c.x, c.y);
-    else if (op == RED_MAX_NI) { R re = c.x + ref; v = re * re + c.y * c.y; }
-    else if (op == RED_MAX_PHASE) v = ratan2<R>(c.y, c.x) + (R)3.14159265358979323846;
-    else v = c.x;   // RED_MINMAX_SSB: real part
+    else { R re = c.x + ref; v = re * re + c.y * c.y; }   // RED_MAX_NI
     mn = v < mn ? v : mn;
     mx = v > mx ? v : mx;
   };
@@ -149,13 +147,6 @@ __global__ void __launch_bounds__(256) encode_map(int kind, int nx, int ny, cons
         R* row = o + r * (size_t)(2 * nx);
         row[2 * c] = ph + del; row[2 * c + 1] = ph - del;
       } break;
-      case OH_ENC_PHASE_ONLY_U8: {
-        const R ph = ratan2<R>(u.y, u.x) + pi;
-        R v = (R)255 * ph / red1[1];
-        // MATLAB uint8(): round half away from zero, saturate
-        v = v < 0 ? 0 : (v > 255 ? 255 : v);
-        static_cast<uint8_t*>(out)[i] = (uint8_t)floor(v + (R)0.5);
-      } break;
       default: break;
     }
   };
@@ -172,27 +163,258 @@ __global__ void __launch_bounds__(256) encode_map(int kind, int nx, int ny, cons
   for (; i < n; i += stride) emit(i, U[i]);
 }
 
-// SSB: zero half of the centred spectrum (fn_encoding.m:33-41).
+// ---- SSB (fn_encoding.m:33-41) ----------------------------------------------
+// Real part of the inverse transform of the centred spectrum with one half
+// zeroed, scaled to min..max.  The mask depends on one axis only, so the
+// transforms along the other axis undo each other and are left out: one kernel
+// per row (LEFT, RIGHT) or column strip (TOP, BOTTOM) does the forward
+// transform, the mask and the inverse (the adjoint network, from storage order),
+// and the block's minimum and maximum; the scaling kernel finishes the
+// reduction.  Both transforms shift by floor(n/2) on both sides, as the 2-D
+// transform does: over an odd length n the round trip moves the samples by
+// one and multiplies sample m of the inverse by exp(-2 pi i m / n), the same
+// along the axis left out.
+//
+// 1920x1080 FP32: two 2-D transforms, mask, reduction and scaling took 118 us;
+// bound now by latency (one wave of blocks, 17 MB in, 8 MB out).
+template <typename R> __device__ __forceinline__ bool is_nan(R v) { return v != v; }
+
+// minimum and maximum of the block's values; a NaN among them makes both NaN
+// (the whole image was NaN when a transform along either axis met one)
 template <typename R>
-__global__ void ssb_mask(int kind, int nx, int ny, typename cplx_of<R>::type* A) {
-  const size_t n = (size_t)nx * ny;
-  const int hx = nx / 2, hy = ny / 2;   // MATLAB floor(N/2), 1-based -> 0-based start hx-1
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / nx), c = (int)(i - (size_t)r * nx);
-    bool zero = false;
-    if (kind == OH_ENC_SSB_LEFT) zero = c >= hx - 1;
-    else if (kind == OH_ENC_SSB_RIGHT) zero = c <= hx - 1;
-    else if (kind == OH_ENC_SSB_TOP) zero = r >= hy - 1;
-    else if (kind == OH_ENC_SSB_BOTTOM) zero = r <= hy - 1;
-    if (zero) { A[i].x = 0; A[i].y = 0; }
+__device__ __forceinline__ void block_minmax(R mn, R mx, R* out) {
+  __shared__ R smn[32], smx[32];
+  auto lo = [](R a, R b) { return a < b || is_nan(a) ? a : b; };
+  auto hi = [](R a, R b) { return a > b || is_nan(a) ? a : b; };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mn = lo(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    mx = hi(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  const int nw = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) { smn[threadIdx.x >> 5] = mn; smx[threadIdx.x >> 5] = mx; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < nw; ++i) { mn = lo(mn, smn[i]); mx = hi(mx, smx[i]); }
+    out[0] = mn;
+    out[1] = mx;
+  }
+}
+
+// The masked axis has length n, the other length m: COLS ? strips of 1 << lw
+// columns : 1 << lw rows per block.
+template <typename R, bool COLS>
+__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 3) ssb_lines(int kind, const typename cplx_of<R>::type* __restrict__ in,
+                                                 R* __restrict__ out, R* __restrict__ part, int n, int m, int lw,
+                                                 FFTPlan pl, const void* __restrict__ tw_other) {
+  typedef typename cplx_of<R>::type C;
+  extern __shared__ unsigned char smem_raw[];
+  C* buf = reinterpret_cast<C*>(smem_raw);
+  const int L = 1 << lw, l0 = blockIdx.x << lw, nl = min(L, m - l0);
+  const int h = n / 2, ho = m / 2, lens = pl.lens;
+  const bool odd = n & 1, odd_o = m & 1;
+  // element i of line l: rows contiguous in shared memory, strips interleaved
+  auto at = [&](int l, int p) { return COLS ? (p << lw) + l : l * lens + p; };
+  auto line = [&](int l) { int s = l0 + l - 2 * ho; if (s < 0) s += m; return s; };   // the line read for line l
+  if constexpr (COLS) {
+    for (int idx = threadIdx.x; idx < n << lw; idx += blockDim.x) {
+      const int l = idx & (L - 1), i = idx >> lw;
+      int src = i - h; if (src < 0) src += n;
+      buf[at(l, pl_at(pl, i))] = l < nl ? in[(size_t)src * m + line(l)] : mk((R)0, (R)0);
+    }
+  } else {
+    for (int l = 0; l < nl; ++l) {
+      const C* row = in + (size_t)line(l) * n;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        int src = i - h; if (src < 0) src += n;
+        buf[at(l, pl_at(pl, i))] = row[src];
+      }
+    }
+  }
+  block_fft<GFWD, C>(0, COLS ? 1 : nl, lens, COLS ? lw : 0, pl);
+  // centred index c of the frequency at position p; MATLAB's floor(n/2), 1-based
+  const bool upper = kind == OH_ENC_SSB_LEFT || kind == OH_ENC_SSB_TOP;
+  for (int p = threadIdx.x; p < n; p += blockDim.x) {
+    int c = pl.iperm[p] + h; if (c >= n) c -= n;
+    if (upper ? c >= h - 1 : c <= h - 1)
+      for (int l = 0; l < nl; ++l) buf[at(l, pl_at(pl, p))] = mk((R)0, (R)0);
+  }
+  block_fft<GADJ, C>(0, COLS ? 1 : nl, lens, COLS ? lw : 0, pl);
+  const C* tw = static_cast<const C*>(pl.tw);
+  const C* two = static_cast<const C*>(tw_other);
+  const R scale = (R)(1.0 / (double)n);
+  R mn = (R)INFINITY, mx = -(R)INFINITY;
+  auto emit = [&](int l, int k) {
+    int i = k - h; if (i < 0) i += n;
+    C v = buf[at(l, pl_at(pl, i))];
+    if (odd) v = cmul(v, tw[i]);
+    if (odd_o) { int o = l0 + l - ho; if (o < 0) o += m; v = cmul(v, two[o]); }
+    const R r = v.x * scale;
+    out[COLS ? (size_t)k * m + l0 + l : (size_t)(l0 + l) * n + k] = r;
+    mn = r < mn || is_nan(r) ? r : mn;
+    mx = r > mx || is_nan(r) ? r : mx;
+  };
+  if constexpr (COLS) {
+    for (int idx = threadIdx.x; idx < n << lw; idx += blockDim.x)
+      if ((idx & (L - 1)) < nl) emit(idx & (L - 1), idx >> lw);
+  } else {
+    for (int l = 0; l < nl; ++l)
+      for (int k = threadIdx.x; k < n; k += blockDim.x) emit(l, k);
+  }
+  block_minmax(mn, mx, part + 2 * blockIdx.x);
+}
+
+// out = (out - min) / (max - min), the extremes of np block partials
+template <typename R>
+__global__ void __launch_bounds__(256) ssb_finish(size_t n, const R* __restrict__ part, int np, const R* in, R* out) {
+  __shared__ R ext[2];
+  R mn = (R)INFINITY, mx = -(R)INFINITY;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) {
+    const R a = part[2 * i], b = part[2 * i + 1];
+    mn = a < mn || is_nan(a) ? a : mn;
+    mx = b > mx || is_nan(b) ? b : mx;
+  }
+  block_minmax(mn, mx, ext);
+  __syncthreads();
+  const R lo = ext[0], rng = ext[1] - ext[0];
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    R v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = in[i + q * stride];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[i + q * stride] = (v[q] - lo) / rng;
+  }
+  for (; i < n; i += stride) out[i] = (in[i] - lo) / rng;
+}
+
+template <typename R>
+static oh_status run_ssb(oh_ctx* ctx, int kind, int nx, int ny, const void* field, void* out, cudaStream_t st) {
+  typedef typename cplx_of<R>::type C;
+  const int prec = sizeof(R) == 8 ? 1 : 0;
+  FFTPlan px, py;
+  OH_TRY(get_plan(ctx, nx, prec, &px));
+  OH_TRY(get_plan(ctx, ny, prec, &py));
+  const size_t smax = max_smem_per_block();
+  if ((size_t)px.lens * sizeof(C) > smax || (size_t)py.lens * sizeof(C) > smax)
+    return fail(OH_ERR_UNSUPPORTED_SIZE, "SSB: a side's line exceeds shared memory");
+  const bool cols = kind == OH_ENC_SSB_TOP || kind == OH_ENC_SSB_BOTTOM;
+  const FFTPlan& pl = cols ? py : px;
+  const int n = cols ? ny : nx, m = cols ? nx : ny;
+  // lines per block: up to 8 (columns: whole sectors) within 48 KB while the
+  // SMs still get two blocks each
+  int lw = 0;
+  while (lw < 3 && ((size_t)pl.lens * sizeof(C) << (lw + 1)) <= 48 * 1024 && (m >> (lw + 1)) >= 2 * oh::sm_count()) ++lw;
+  const int blocks = (m + (1 << lw) - 1) >> lw;
+  const size_t smem = (size_t)pl.lens * sizeof(C) << lw;
+  const size_t total = (size_t)nx * ny;
+  void* ptr;
+  OH_TRY(scratch(ctx, "enc.red1", sizeof(R) * 2 * blocks, &ptr));
+  // an output over the field itself waits in scratch until every line is read
+  R* real = (R*)out;
+  const char *f0 = (const char*)field, *o0 = (const char*)out;
+  if (o0 < f0 + total * sizeof(C) && f0 < o0 + total * sizeof(R)) {
+    void* tmp;
+    OH_TRY(scratch(ctx, "enc.ssb", total * sizeof(R), &tmp));
+    real = (R*)tmp;
+  }
+  auto kern = cols ? ssb_lines<R, true> : ssb_lines<R, false>;
+  OH_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  {
+    KernelTimer kt(ctx, "ssb_lines", st);
+    kern<<<blocks, 256, smem, st>>>(kind, (const C*)field, real, (R*)ptr, n, m, lw, pl, cols ? px.tw : py.tw);
+    OH_LAUNCH_CHECK();
+  }
+  KernelTimer kt(ctx, "ssb_finish", st);
+  ssb_finish<R><<<(int)std::min<size_t>((total + 1023) / 1024, oh::sm_count() * 16), 256, 0, st>>>(total, (const R*)ptr, blocks, real, (R*)out);
+  OH_LAUNCH_CHECK();
+  return OH_OK;
+}
+
+// ---- phase-only uint8 (Hologram_WRP.m:57-60) -----------------------------------
+// Pass 1 writes angle + pi to scratch and every block's maximum, pass 2
+// finishes the maximum and scales to bytes: one arc tangent per pixel (two
+// before, one per pass) and two launches instead of three.
+template <typename R>
+__global__ void __launch_bounds__(256) phase_pass(const typename cplx_of<R>::type* __restrict__ U, size_t n,
+                                                  R* __restrict__ ph, R* __restrict__ part) {
+  typedef typename cplx_of<R>::type C;
+  __shared__ R smx[8];
+  R mx = -(R)INFINITY;
+  auto take = [&](size_t i, C c) {
+    const R v = ratan2<R>(c.y, c.x) + (R)3.14159265358979323846;
+    ph[i] = v;
+    mx = v > mx ? v : mx;
+  };
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    C c[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] = U[i + q * stride];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) take(i + q * stride, c[q]);
+  }
+  for (; i < n; i += stride) take(i, U[i]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) smx[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < 8; ++q) mx = max(mx, smx[q]);
+    part[blockIdx.x] = mx;
   }
 }
 
 template <typename R>
-__global__ void ssb_finish(size_t n, const typename cplx_of<R>::type* A, const R* red, R* out) {
-  const R mn = red[0], rng = red[1] - red[0];
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    out[i] = (A[i].x - mn) / rng;
+__global__ void __launch_bounds__(256) phase_u8(const R* __restrict__ ph, size_t n, const R* __restrict__ part, int np,
+                                                uint8_t* __restrict__ out) {
+  __shared__ R smx[8];
+  R mx = -(R)INFINITY;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) mx = max(mx, part[i]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) smx[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = smx[0];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) mx = max(mx, smx[q]);
+  auto byte = [&](R p) {
+    R v = (R)255 * p / mx;
+    // MATLAB uint8(): round half away from zero, saturate
+    v = v < 0 ? 0 : (v > 255 ? 255 : v);
+    return (uint8_t)floor(v + (R)0.5);
+  };
+  // four pixels per thread and store where the output is aligned
+  const size_t stride = (size_t)gridDim.x * blockDim.x, first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t n4 = reinterpret_cast<uintptr_t>(out) % 4 == 0 ? n / 4 : 0;
+  for (size_t i = first; i < n4; i += stride) {
+    R p[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) p[q] = ph[4 * i + q];
+    reinterpret_cast<uchar4*>(out)[i] = make_uchar4(byte(p[0]), byte(p[1]), byte(p[2]), byte(p[3]));
+  }
+  for (size_t i = 4 * n4 + first; i < n; i += stride) out[i] = byte(ph[i]);
+}
+
+template <typename R>
+static oh_status run_phase_u8(oh_ctx* ctx, size_t n, const void* field, void* out, cudaStream_t st) {
+  typedef typename cplx_of<R>::type C;
+  const int np = (int)std::min<size_t>((n + 255) / 256, oh::sm_count() * 6);
+  void* ptr;
+  OH_TRY(scratch(ctx, "enc.phase", n * sizeof(R) + sizeof(R) * np, &ptr));
+  R* ph = (R*)ptr;
+  R* part = ph + n;
+  {
+    KernelTimer kt(ctx, "phase_pass", st);
+    phase_pass<R><<<np, 256, 0, st>>>((const C*)field, n, ph, part);
+    OH_LAUNCH_CHECK();
+  }
+  KernelTimer kt(ctx, "phase_u8", st);
+  phase_u8<R><<<(int)std::min<size_t>((n + 1023) / 1024, oh::sm_count() * 16), 256, 0, st>>>(ph, n, part, np, (uint8_t*)out);
+  OH_LAUNCH_CHECK();
+  return OH_OK;
 }
 
 template <typename R>
@@ -220,27 +442,14 @@ static oh_status run_encode(oh_ctx* ctx, int kind, int nx, int ny, const void* f
   const int grid = (int)std::min<size_t>((n + 255) / 256, oh::sm_count() * 16);
   R* red1 = nullptr;
   R* red2 = nullptr;
-  if (kind >= OH_ENC_SSB_LEFT && kind <= OH_ENC_SSB_BOTTOM) {
-    void* ptr;
-    OH_TRY(scratch(ctx, "enc.ssb", n * sizeof(C), &ptr));
-    C* A = (C*)ptr;
-    const int prec = sizeof(R) == 8 ? 1 : 0;
-    OH_TRY(fft2d_enqueue(ctx, prec, nx, ny, field, A, nullptr, -1, 1, 0, st));
-    ssb_mask<R><<<grid, 256, 0, st>>>(kind, nx, ny, A);
-    OH_LAUNCH_CHECK();
-    OH_TRY(fft2d_enqueue(ctx, prec, nx, ny, A, A, nullptr, 1, 1, 1, st));
-    OH_TRY(reduce<R>(ctx, A, n, RED_MINMAX_SSB, (const R*)nullptr, &red1, st, "enc.red1"));
-    ssb_finish<R><<<grid, 256, 0, st>>>(n, A, red1, (R*)out);
-    OH_LAUNCH_CHECK();
-    return OH_OK;
-  }
+  if (kind >= OH_ENC_SSB_LEFT && kind <= OH_ENC_SSB_BOTTOM) return run_ssb<R>(ctx, kind, nx, ny, field, out, st);
+  if (kind == OH_ENC_PHASE_ONLY_U8) return run_phase_u8<R>(ctx, n, field, out, st);
   if (kind == OH_ENC_NUM_INTERFERENCE || kind == OH_ENC_BURCKHARDT || kind == OH_ENC_TWO_PHASE)
     OH_TRY(reduce<R>(ctx, field, n, RED_MAX_ABS, (const R*)nullptr, &red1, st, "enc.red1"));
   if (kind == OH_ENC_NUM_INTERFERENCE) {
     // max |U + max|U||^2, the reference value read on the device
     OH_TRY(reduce<R>(ctx, field, n, RED_MAX_NI, red1, &red2, st, "enc.red2"));
   }
-  if (kind == OH_ENC_PHASE_ONLY_U8) OH_TRY(reduce<R>(ctx, field, n, RED_MAX_PHASE, (const R*)nullptr, &red1, st, "enc.red1"));
   KernelTimer kt(ctx, "encode_map", st);
   encode_map<R><<<grid, 256, 0, st>>>(kind, nx, ny, (const C*)field, red1, red2, out);
   OH_LAUNCH_CHECK();
