@@ -1,0 +1,541 @@
+// Point-cloud hologram (exact distances) as a contraction on the tensor cores.
+//
+// Over a plane region of 128 rows x 64 columns around (Xc, Yc), with r0 the
+// distance from a point to the region's centre, u, v the offsets from it and
+//   p = (2 dx u + u^2) / r0^2,  q = (2 dy v + v^2) / r0^2,
+// the distance is r = r0 sqrt(1 + p + q), and
+//   sqrt(1 + p + q) = sqrt(1 + p) + sqrt(1 + q) - 1 - P Q / 4 + O(p^2 q^2 / 10),
+//   P = 2 (1 - 1 / sqrt(1 + p)),  Q = 2 (1 - 1 / sqrt(1 + q))
+// (the terms linear in p or in q are exact).  So the phase k r is separable up
+// to the cross term chi = -(k r0 / 4) P Q, a few hundredths of a radian, and
+//   exp(i k r) = sum_n [E(v) Qh^n] [E(u) (i kq P)^n / n!],  chi = kq P Qh,
+// four terms (n < 4) in all: W[y][x] = sum over points and n of L_n[y] R_n[x], a
+// complex matrix product with K = 4 per point.  Embedded in reals (K column 2k,
+// 2k+1 = Re, Im of term k; B rows 2x, 2x+1 give Re, Im of column x) it is a
+// product C = A B^T with M = 128, N = 128 and K = 8 per point.
+//
+// Operands (amplitudes scaled by a power of two to at most one) are split into
+// a multiple of 2^-8 and an FP16 remainder (absolute error 2^-21).  The tensor
+// core truncates each FP32 accumulation (a plain FP16 high/low split in one
+// accumulator lost 2e-5 over 700 points that way), so the products of the
+// multiples of 2^-8 have an accumulator of their own, in which sums up to 256
+// are exact, and the three products with a remainder, 2^-8 of that, another.
+//
+// pc_tc_prep decides in FP64 per point whether the dropped terms stay below
+// 1e-6 rad at the worst corner of the plane; other points (near or strongly
+// off-axis scenes) go to a list that the caller sums directly.
+//
+// One CTA per region and split of the points, 320 threads, two CTAs per SM: warp
+// 9 forms the per-region records of 32 points at a time (FP64 phases reduced to
+// 32-bit fractions of a turn), warps 0-7 build the operands of four points (K =
+// 32) per stage straight into shared memory in the 64-byte-swizzled layout a TMA
+// load would give, warp 8 issues tcgen05.mma, warps 4-7 read the accumulators.  Splits write partial planes that pc_tc_sum adds in order, so the
+// result does not depend on timing.  Waits are bounded: on timeout the CTA sets
+// the device error word and writes nothing.
+//
+// What bounds it: the operand producers (53 % of the issue slots) and shared
+// memory (63 %: their stores and the tensor core's operand reads).  16 producer
+// warps in two groups were slower (0.79 against 0.73 ms: spills and spinning
+// waits).
+#include <cuda_fp16.h>
+#include <algorithm>
+#include <cmath>
+#include "pc_tc.cuh"
+#include "tc_common.cuh"
+
+namespace oh {
+
+namespace {
+
+using namespace pctc;
+using tc::su32;
+
+constexpr int kBK = 8 * kPts;                          // K per stage
+constexpr int kStages = 2;
+constexpr int kTile = 128 * kBK * 2;                   // 8 KB: 128 rows x 32 FP16
+constexpr int kStageBytes = 4 * kTile;                 // Ahi, Alo, Bhi, Blo
+constexpr int kAccCols = 128, kTmemCols = 2 * kAccCols;   // exact products, products with remainders
+constexpr int kProducers = 8, kThreads = 32 * (kProducers + 2);
+constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // FP16 in, FP32 out
+
+// One point as a region sees it: phase in turns = frac(t0 + cy m) + rest(m) along
+// the rows (m = row - 64), the same with cx along the columns (m = column - 32,
+// no t0).
+struct alignas(16) PcRec {
+  int t0, cx, cy;
+  float amp;
+  float c0, ax, bx, ay;            // r0 / lambda; p = m (ax + bx m), q = m (ay + by m)
+  float by, iqs, kq, pad;          // 1 / max |Q|; cross factor kq (rad)
+};
+
+struct PcTcArgs {
+  PCGeom g;
+  const PcPt* pts;
+  const int* list;                 // fast points, unless every point is fast
+  Counts* cnt;
+  int n, regions_x, splits;
+  float2* part;                    // [splits][ny][nx]
+  int* err;
+};
+
+// Per point: FP64 position, and whether the separable form holds over the whole
+// plane: every dropped term below 1e-6 rad at the plane's worst corner (see the
+// head of this file), fp64: near 1e-10 rad there.
+__global__ void pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int fp64, PcPt* __restrict__ pts,
+                           Counts* __restrict__ cnt) {
+  unsigned amax = 0u;
+  int slow = 0;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const float4 p = in[j];
+    PcPt o;
+    o.x = (double)p.x * g.sx; o.y = (double)p.y * g.sy; o.z = (double)p.z * g.sz + g.off;
+    o.a = p.w;
+    const double az = fabs(o.z);
+    const float U = (float)(0.5 * kCols * g.px), V = (float)(0.5 * kRows * g.py), zf = (float)az, kf = (float)g.k;
+    // |p| r0^2 = |(dx + u)^2 - dx^2| over the plane's pixels: with D the farthest
+    // pixel, a region that ends at the edge gives 2 D U - U^2, one that runs past
+    // it 2 D U + U^2 at most
+    const float DX = (float)(g.hlx + fabs(o.x)), DY = (float)(g.hly + fabs(o.y));
+    const float eu = g.nx % kCols ? U : -U, ev = g.ny % kRows ? V : -V;
+    const float iz = 1.f / zf, iz2 = iz * iz;
+    const float pm = fminf((2.f * DX + eu) * U * iz2, U * iz + U * U * iz2);
+    const float qm = fminf((2.f * DY + ev) * V * iz2, V * iz + V * V * iz2);
+    const float r0 = sqrtf((DX + U) * (DX + U) + (DY + V) * (DY + V) + zf * zf);
+    const float chi = 0.25f * kf * r0 * pm * qm, m = fmaxf(pm, qm);
+    const float turns = kf * r0 * 0.15915494f;
+    // separable form: rank-four remainder, p^2 q^2 term, series ends (phase of
+    // one axis, P and Q), and the float part of the axis phases below 4 turns
+    bool ok = m < 0.01f && chi * chi * chi * chi < 24e-6f && 0.1f * kf * r0 * pm * pm * qm * qm < 2e-7f &&
+                    0.0273f * m * m * m * m * m * turns < 3e-8f && chi * 0.55f * m * m * m < 2e-7f &&
+                    turns * 0.5f * fmaxf(U, V) * fmaxf(U, V) * iz2 < 4.f && fminf(U, V) * fminf(U, V) * iz2 > 1e-25f && fabsf(p.w) < 1e30f &&
+                    fabs(o.x) < 1e3 && fabs(o.y) < 1e3 && az < 1e3;
+    if (fp64) {
+      // rank-six remainder; terms past p^2 q^2; the axis series' m^7 term
+      const float c3 = chi * chi * chi, t = fmaxf(U, V) * iz, t3 = t * t * t;
+      ok = ok && c3 * c3 < 720.f * 1.2e-10f && kf * r0 * (pm * qm) * (pm * qm) * (pm + qm) < 1e-10f &&
+           turns * t3 * t3 * t < 3e-11f;
+    }
+    o.fast = ok ? 1 : 0;
+    if (ok) amax = max(amax, __float_as_uint(fabsf(p.w)));
+    else ++slow;
+    pts[j] = o;
+  }
+  amax = __reduce_max_sync(0xffffffffu, amax);
+  slow = __reduce_add_sync(0xffffffffu, slow);
+  if ((threadIdx.x & 31) == 0) {
+    if (amax) atomicMax(&cnt->amax, amax);
+    if (slow) atomicAdd(&cnt->slow, slow);
+  }
+}
+
+// One block: the fast points' indices and the slow points in input order.  With
+// no slow point the index list stays unwritten (and unread).
+__global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ in, const PcPt* __restrict__ pts, int n,
+                                                    int* __restrict__ list, float4* __restrict__ slow,
+                                                    Counts* __restrict__ cnt) {
+  __shared__ int wsum[32];
+  if (cnt->slow == 0) {
+    if (threadIdx.x == 0) cnt->fast = n;
+    return;
+  }
+  int before = 0;                                     // fast points of earlier rounds
+  for (int base = 0; base < n; base += 1024) {
+    const int j = base + threadIdx.x;
+    const bool in_range = j < n;
+    const bool f = in_range && pts[j].fast;
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = __popc(m);
+    __syncthreads();
+    int pre = before, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < (int)(threadIdx.x >> 5)) pre += wsum[w];
+      all += wsum[w];
+    }
+    pre += __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+    if (f) list[pre] = j;
+    else if (in_range) slow[j - pre] = in[j];
+    before += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) cnt->fast = before;
+}
+
+__device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const int* abort) {
+  const long long t0 = clock64();
+  while (!tc::mb_try(b, parity)) {
+    if (*((volatile const int*)abort) || clock64() - t0 > kWaitCycles) return false;
+  }
+  return true;
+}
+__device__ __forceinline__ void arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
+}
+
+// Byte offset of 16-byte chunk c of row r in a [128][32] FP16 tile with 64-byte swizzle.
+__device__ __forceinline__ int sw_off(int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); }
+
+__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+// Multiples of 2^-8 nearest (a, b), |a|, |b| <= 1 (adding 6 in FP16 rounds to
+// them), and FP16 remainders.
+__device__ __forceinline__ void split2(float a, float b, uint32_t* hi, uint32_t* lo) {
+  const __half2 six = __floats2half2_rn(6.f, 6.f);
+  const __half2 h = __hsub2(__hadd2(__floats2half2_rn(a, b), six), six);
+  const float2 f = __half22float2(h);
+  *hi = h2u(h);
+  *lo = h2u(__floats2half2_rn(a - f.x, b - f.y));
+}
+
+// turns -> (cos, sin)
+__device__ __forceinline__ void cis(float t, float* c, float* s) {
+  t = 6.28318530717958647692f * (t - rintf(t));
+  *c = __cosf(t);
+  *s = __sinf(t);
+}
+__device__ __forceinline__ float axis_rest(float c0, float w, float bm2) {
+  // (r0 / lambda) (sqrt(1 + w) - 1) without its linear term
+  return c0 * fmaf(0.5f, bm2, w * w * fmaf(w, fmaf(w, -0.0390625f, 0.0625f), -0.125f));
+}
+__device__ __forceinline__ float cross_arg(float w) { return w * fmaf(w, fmaf(w, 0.625f, -0.75f), 1.f); }
+
+__global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
+  extern __shared__ unsigned char smem_dyn[];
+  __shared__ PcRec recs[2][kBatch];
+  const uint32_t raw = su32(smem_dyn);
+  unsigned char* base = smem_dyn + (((raw + 1023u) & ~1023u) - raw);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);
+  uint64_t* full = bars;                  // [kStages], one arrival per producer warp
+  uint64_t* empty = bars + kStages;       // [kStages], tcgen05.commit
+  uint64_t* done = bars + 2 * kStages;
+  uint64_t* rfull = done + 1;             // [2], the record warp's
+  uint64_t* rempty = done + 3;            // [2], one arrival per producer warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 5);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int X0 = (blockIdx.x % a.regions_x) * kCols, Y0 = (blockIdx.x / a.regions_x) * kRows;
+  const int nx = a.g.nx, ny = a.g.ny;
+  const int nfast = a.cnt->fast;
+  const bool identity = a.cnt->slow == 0;
+  const int nbatch = (nfast + kBatch - 1) / kBatch;
+  const int b0 = (int)((long long)blockIdx.y * nbatch / a.splits), b1 = (int)((long long)(blockIdx.y + 1) * nbatch / a.splits);
+  const int first = b0 * kBatch, last = min(b1 * kBatch, nfast);
+  const int nst = (last - first + kPts - 1) / kPts;
+  float2* part = a.part + (size_t)blockIdx.y * nx * ny;
+  if (nfast == 0) return;                 // pc_tc_sum reads no partial plane then
+  if (nst <= 0) {
+    for (int i = threadIdx.x; i < kRows * kCols; i += kThreads) {
+      const int r = Y0 + i / kCols, c = X0 + i % kCols;
+      if (r < ny && c < nx) part[(size_t)r * nx + c] = make_float2(0.f, 0.f);
+    }
+    return;
+  }
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) { tc::mb_init(&full[s], kProducers); tc::mb_init(&empty[s], 1); }
+    tc::mb_init(done, 1);
+    for (int s = 0; s < 2; ++s) { tc::mb_init(&rfull[s], 1); tc::mb_init(&rempty[s], kProducers); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tc::tmem_alloc(tmem_slot, kTmemCols);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp < kProducers) {
+    // point slot j of the stage, A rows rb and rb + 64, B column rb
+    const int j = threadIdx.x & 3, rb = threadIdx.x >> 2;
+    const int offA0 = sw_off(rb, j), offA1 = sw_off(rb + 64, j);
+    // the two B rows of a column, in an order that spreads a quarter-warp over the banks
+    const int par = rb & 1;
+    const int offB0 = sw_off(2 * rb + par, j), offB1 = sw_off(2 * rb + 1 - par, j);
+    constexpr int kPer = kBatch / kPts;                // stages per record batch
+    for (int it = 0; it < nst; ++it) {
+      const int s = it % kStages, batch = it / kPer, rs = batch & 1;
+      bool ok = true;
+      if (lane == 0) {
+        if (it % kPer == 0) ok = wait_live(&rfull[rs], (uint32_t)((batch >> 1) & 1), abort_flag);
+        ok = ok && wait_live(&empty[s], (uint32_t)(((it / kStages) & 1) ^ 1), abort_flag);
+        if (!ok) atomicExch(abort_flag, 1);
+      }
+      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
+      __syncwarp();                       // the record warp's writes, seen by lane 0's wait
+      const PcRec q = recs[rs][(it % kPer) * kPts + j];
+      unsigned char* sAh = base + s * kStageBytes;
+      unsigned char* sAl = sAh + kTile;
+      unsigned char* sBh = sAh + 2 * kTile;
+      unsigned char* sBl = sAh + 3 * kTile;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = rb - 64 + 64 * h;
+        const float mf = (float)m;
+        const float bm = q.by * mf, w = mf * (q.ay + bm);
+        float c, sn;
+        cis((float)(int)((unsigned)q.t0 + (unsigned)q.cy * (unsigned)m) * 2.3283064365386963e-10f + axis_rest(q.c0, w, bm * mf), &c, &sn);
+        const float Qh = cross_arg(w) * q.iqs;
+        float re = q.amp * c, im = q.amp * sn;
+        uint4 hi, lo;
+        split2(re, im, &hi.x, &lo.x);
+        re *= Qh; im *= Qh;
+        split2(re, im, &hi.y, &lo.y);
+        re *= Qh; im *= Qh;
+        split2(re, im, &hi.z, &lo.z);
+        re *= Qh; im *= Qh;
+        split2(re, im, &hi.w, &lo.w);
+        const int off = h ? offA1 : offA0;
+        *reinterpret_cast<uint4*>(sAh + off) = hi;
+        *reinterpret_cast<uint4*>(sAl + off) = lo;
+      }
+      {
+        const int m = rb - 32;
+        const float mf = (float)m;
+        const float bm = q.bx * mf, w = mf * (q.ax + bm);
+        float c, sn;
+        cis((float)(int)((unsigned)q.cx * (unsigned)m) * 2.3283064365386963e-10f + axis_rest(q.c0, w, bm * mf), &c, &sn);
+        const float x = q.kq * cross_arg(w);
+        const float x2 = 0.5f * x * x, x3 = x * x2 * 0.33333333333f;
+        // R_n = (c + i s) (i x)^n / n!
+        uint4 hi, lo;
+        split2(c, sn, &hi.x, &lo.x);
+        split2(-x * sn, x * c, &hi.y, &lo.y);
+        split2(-x2 * c, -x2 * sn, &hi.z, &lo.z);
+        split2(x3 * sn, -x3 * c, &hi.w, &lo.w);
+        // row 2x takes (Re, -Im) of each term, row 2x + 1 (Im, Re)
+        const uint32_t neg = 0x80000000u;
+        const uint4 h0 = make_uint4(hi.x ^ neg, hi.y ^ neg, hi.z ^ neg, hi.w ^ neg);
+        const uint4 l0 = make_uint4(lo.x ^ neg, lo.y ^ neg, lo.z ^ neg, lo.w ^ neg);
+        const uint4 h1 = make_uint4(__byte_perm(hi.x, 0, 0x1032), __byte_perm(hi.y, 0, 0x1032),
+                                    __byte_perm(hi.z, 0, 0x1032), __byte_perm(hi.w, 0, 0x1032));
+        const uint4 l1 = make_uint4(__byte_perm(lo.x, 0, 0x1032), __byte_perm(lo.y, 0, 0x1032),
+                                    __byte_perm(lo.z, 0, 0x1032), __byte_perm(lo.w, 0, 0x1032));
+        *reinterpret_cast<uint4*>(sBh + offB0) = par ? h1 : h0;
+        *reinterpret_cast<uint4*>(sBl + offB0) = par ? l1 : l0;
+        *reinterpret_cast<uint4*>(sBh + offB1) = par ? h0 : h1;
+        *reinterpret_cast<uint4*>(sBl + offB1) = par ? l0 : l1;
+      }
+      // generic-proxy writes -> visible to the tensor core's async proxy
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        arrive(&full[s]);
+        if (it % kPer == kPer - 1) arrive(&rempty[rs]);
+      }
+    }
+  } else if (warp == kProducers) {
+    if (lane == 0) {
+      for (int it = 0; it < nst; ++it) {
+        const int s = it % kStages;
+        if (!wait_live(&full[s], (uint32_t)((it / kStages) & 1), abort_flag)) {
+          atomicExch(abort_flag, 1);
+          break;
+        }
+        tc::fence_after();
+        unsigned char* st0 = base + s * kStageBytes;
+        const uint64_t ah = tc::desc_sw64(su32(st0), 16, 512), al = tc::desc_sw64(su32(st0 + kTile), 16, 512);
+        const uint64_t bh = tc::desc_sw64(su32(st0 + 2 * kTile), 16, 512), bl = tc::desc_sw64(su32(st0 + 3 * kTile), 16, 512);
+#pragma unroll
+        for (int kk = 0; kk < kBK / 16; ++kk) {
+          const uint64_t adv = (uint64_t)((kk * 32) >> 4);
+          tc::umma_bf16(tmem, ah + adv, bh + adv, kIdesc, (it | kk) ? 1u : 0u);
+          tc::umma_bf16(tmem + kAccCols, ah + adv, bl + adv, kIdesc, (it | kk) ? 1u : 0u);
+          tc::umma_bf16(tmem + kAccCols, al + adv, bh + adv, kIdesc, 1u);
+          tc::umma_bf16(tmem + kAccCols, al + adv, bl + adv, kIdesc, 1u);
+        }
+        tc::umma_commit(&empty[s]);
+      }
+      tc::umma_commit(done);              // arrives when every MMA issued above has completed
+    }
+  } else {
+    // record warp: lane k forms point k of each batch
+    const double il = a.g.k * 0.15915494309189533576888376337251;      // 1 / lambda
+    const double Xc = ((double)(X0 + kCols / 2) + 0.5) * a.g.px - a.g.hlx;
+    const double Yc = a.g.hly - ((double)(Y0 + kRows / 2) + 0.5) * a.g.py;
+    const double ref = Xc * a.g.stx + Yc * a.g.sty;
+    float unscale;
+    const float scale = amp_scale(a.cnt->amax, &unscale);
+    auto frac32 = [](double t) { return (int)__double2ll_rn((t - rint(t)) * 4294967296.0); };
+    const int batches = b1 - b0;
+    for (int b = 0; b < batches; ++b) {
+      const int rs = b & 1;
+      bool ok = true;
+      if (lane == 0) {
+        ok = wait_live(&rempty[rs], (uint32_t)(((b >> 1) & 1) ^ 1), abort_flag);
+        if (!ok) atomicExch(abort_flag, 1);
+      }
+      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
+      const int k = first + b * kBatch + lane;
+      PcRec r{};
+      if (k < last) {
+        const PcPt p = a.pts[identity ? k : a.list[k]];
+        const double dx = Xc - p.x, dy = Yc - p.y;
+        const double r2 = fma(dx, dx, fma(dy, dy, p.z * p.z));
+        const double ri = rsqrt(r2), r0 = r2 * ri;
+        const double sx = dx * ri, sy = dy * ri;
+        r.t0 = frac32((r0 - ref) * il);
+        r.cx = frac32((sx - a.g.stx) * a.g.px * il);
+        r.cy = frac32((a.g.sty - sy) * a.g.py * il);
+        const float rif = (float)ri, pxr = (float)a.g.px * rif, pyr = (float)a.g.py * rif;
+        r.amp = p.a * scale;
+        r.c0 = (float)(r0 * il);
+        r.ax = 2.f * (float)sx * pxr; r.bx = pxr * pxr;
+        r.ay = -2.f * (float)sy * pyr; r.by = pyr * pyr;
+        const float qs = fabsf(r.ay) * (kRows / 2) + r.by * (kRows / 2) * (kRows / 2);
+        r.iqs = 1.f / qs;
+        r.kq = -1.57079632679f * r.c0 * qs;
+      }
+      recs[rs][lane] = r;
+      __syncwarp();
+      if (lane == 0) arrive(&rfull[rs]);
+    }
+  }
+  // epilogue: warps 4-7 own TMEM lanes 32 (warp - 4) .. + 31 = region rows
+  __syncwarp();
+  const bool epi = warp >= 4 && warp < 8;
+  bool ok_done = true;
+  if (epi) ok_done = tc::mb_wait(done, 0, kWaitCycles);
+  tc::fence_after();
+  const bool good = __syncthreads_and(ok_done && !*((volatile int*)abort_flag));
+  if (good && epi) {
+    const int Y = Y0 + 32 * (warp - 4) + lane;
+#pragma unroll 1
+    for (int c = 0; c < 2 * kCols / 32; ++c) {
+      uint32_t v[32], lo[32];
+      const uint32_t at = tmem + ((uint32_t)(32 * (warp - 4)) << 16) + (uint32_t)(c * 32);
+      tc::tmem_ld32(at, v);
+      tc::tmem_ld32(at + kAccCols, lo);
+#pragma unroll
+      for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(lo[q]));
+      if (Y < ny) {
+        float2* dst = part + (size_t)Y * nx + X0 + 16 * c;
+        if (nx % 2 == 0) {
+#pragma unroll
+          for (int q = 0; q < 16; q += 2)
+            if (X0 + 16 * c + q < nx)
+              *reinterpret_cast<uint4*>(dst + q) = make_uint4(v[2 * q], v[2 * q + 1], v[2 * q + 2], v[2 * q + 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (X0 + 16 * c + q < nx) dst[q] = make_float2(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
+        }
+      }
+    }
+  } else if (!good && threadIdx.x == 0) {
+    atomicOr(a.err, 8);
+    atomicOr(&a.cnt->aborted, 1);
+    tc::mb_wait(done, 0, kWaitCycles);    // the MMAs must have finished reading shared memory and TMEM
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after();
+    tc::tmem_dealloc(tmem, kTmemCols);
+  }
+}
+
+// The splits' partial planes added in order, unscaled, into the outputs.  After
+// a timeout nothing is written.
+__global__ void __launch_bounds__(256) pc_tc_sum(const float2* __restrict__ part, int splits, size_t n,
+                                                 const Counts* __restrict__ cnt,
+                                                 float2* __restrict__ field, float* __restrict__ fringe, int accumulate) {
+  if (cnt->aborted) return;
+  const bool none = cnt->fast == 0;
+  float unscale;
+  amp_scale(cnt->amax, &unscale);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    float2 v = make_float2(0.f, 0.f);
+    if (!none)
+      for (int s = 0; s < splits; ++s) v = cadd(v, part[(size_t)s * n + i]);
+    v = cscale(v, unscale);
+    if (field) field[i] = accumulate ? cadd(field[i], v) : v;
+    if (fringe) fringe[i] += v.x;
+  }
+}
+
+}  // namespace
+
+namespace pctc {
+
+static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+size_t sorted_bytes(int n) {
+  return 256 + align256((size_t)n * sizeof(PcPt)) + align256((size_t)n * sizeof(int)) + align256((size_t)n * sizeof(float4));
+}
+
+oh_status sort_points(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, bool fp64, void* base, Sorted* out,
+                      cudaStream_t st) {
+  char* p = static_cast<char*>(base);
+  out->cnt = (Counts*)p;
+  p += 256;
+  out->pts = (PcPt*)p;
+  p += align256((size_t)n * sizeof(PcPt));
+  out->list = (int*)p;
+  p += align256((size_t)n * sizeof(int));
+  out->slow = (float4*)p;
+  OH_CUDA_TRY(cudaMemsetAsync(out->cnt, 0, sizeof(Counts), st));
+  KernelTimer kt(ctx, "pc_tc_prep", st);
+  pc_tc_prep<<<std::min((n + 127) / 128, sm_count() * 8), 128, 0, st>>>(g, pts, n, fp64 ? 1 : 0, out->pts, out->cnt);
+  OH_LAUNCH_CHECK();
+  pc_tc_split<<<1, 1024, 0, st>>>(pts, out->pts, n, out->list, out->slow, out->cnt);
+  OH_LAUNCH_CHECK();
+  return OH_OK;
+}
+
+int point_splits(int regions, int n, int slots, int batches) {
+  int splits = 1;
+  double best = 0.0;
+  for (int s = 1; s <= 8 && (s == 1 || n / (kBatch * s) >= batches); ++s) {
+    const double waves = (double)regions * s / slots, fill = waves / std::ceil(waves);
+    if (fill > best + 1e-9) { best = fill; splits = s; }
+    if (best >= 0.95) break;
+  }
+  return splits;
+}
+
+}  // namespace pctc
+
+bool pc_tc_wants(const PCGeom& g, int n, bool fp64) {
+  // FP32: the direct kernels take about 0.24 us per point (a block's serial
+  // chain) or 1.1e-6 us per term, whichever sum is due; below 60 us they beat the
+  // six launches and part-filled regions here (640x480 x 100 points: 57 us
+  // direct, 54 us here; 1024x1024 x 200: 247 and 78; 128x128 x 1000: 250 and 66).
+  const double terms = (double)n * g.nx * g.ny;
+  if (fp64 ? 7.0 * n + 7.3e-5 * terms < 150.0 : 0.24 * n + 1.1e-6 * terms < 60.0) return false;
+  int dev = 0, major = 0, minor = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const long long regions = (long long)((g.nx + kCols - 1) / kCols) * ((g.ny + kRows - 1) / kRows);
+  return major == 10 && minor == 3 && regions < (1 << 24);
+}
+
+oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, float2* field, float* fringe,
+                        bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st) {
+  const int rx = (g.nx + kCols - 1) / kCols, ry = (g.ny + kRows - 1) / kRows, regions = rx * ry;
+  const int splits = point_splits(regions, n, 2 * sm_count(), 4);
+  const size_t plane = (size_t)g.nx * g.ny, o_part = sorted_bytes(n);
+  void* ptr;
+  OH_TRY(scratch(ctx, "pc.tc", o_part + plane * splits * sizeof(float2), &ptr));
+  float2* part = (float2*)((char*)ptr + o_part);
+  Sorted s;
+  OH_TRY(sort_points(ctx, g, pts, n, false, ptr, &s, st));
+  const int smem = kStages * kStageBytes + 1024 + 256;
+  OH_CUDA_TRY(cudaFuncSetAttribute(pc_tc_regions, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  PcTcArgs a{g, s.pts, s.list, s.cnt, n, rx, splits, part, ctx->dev_err};
+  {
+    KernelTimer kt(ctx, "pc_tc_regions", st);
+    pc_tc_regions<<<dim3(regions, splits), kThreads, smem, st>>>(a);
+    OH_LAUNCH_CHECK();
+  }
+  KernelTimer kt(ctx, "pc_tc_sum", st);
+  pc_tc_sum<<<(int)std::min<size_t>((plane + 255) / 256, (size_t)sm_count() * 16), 256, 0, st>>>(
+      part, splits, plane, s.cnt, field, fringe, accumulate ? 1 : 0);
+  OH_LAUNCH_CHECK();
+  *slow = s.slow;
+  *slow_n = &s.cnt->slow;
+  return OH_OK;
+}
+
+}  // namespace oh
