@@ -80,7 +80,7 @@ struct PcTcArgs {
 
 // Per point: FP64 position, and whether the separable form holds over the whole
 // plane: every dropped term below 1e-6 rad at the plane's worst corner (see the
-// head of this file), fp64: near 1e-10 rad there.
+// head of this file), fp64: near 1e-10 rad there (see pc_tc64.cu).
 __global__ void pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int fp64, PcPt* __restrict__ pts,
                            Counts* __restrict__ cnt) {
   unsigned amax = 0u;
@@ -499,6 +499,9 @@ bool pc_tc_wants(const PCGeom& g, int n, bool fp64) {
   // chain) or 1.1e-6 us per term, whichever sum is due; below 60 us they beat the
   // six launches and part-filled regions here (640x480 x 100 points: 57 us
   // direct, 54 us here; 1024x1024 x 200: 247 and 78; 128x128 x 1000: 250 and 66).
+  // FP64: directly 3 to 7 us per point (a block's serial chain) or 73 ps per term
+  // (the FP64 pipe); here 55 us at least (100x100 x 30 points: 90 us directly, 57
+  // us here; 300x300 x 30: 262 and 61).
   const double terms = (double)n * g.nx * g.ny;
   if (fp64 ? 7.0 * n + 7.3e-5 * terms < 150.0 : 0.24 * n + 1.1e-6 * terms < 60.0) return false;
   int dev = 0, major = 0, minor = 0;

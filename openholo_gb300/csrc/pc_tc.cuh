@@ -1,5 +1,5 @@
 // Point-cloud sums on the tensor cores: what pointcloud.cu needs of them, and
-// their parts.
+// what the FP32 (pc_tc.cu) and FP64 (pc_tc64.cu) forms share.
 #pragma once
 #include "context.h"
 
@@ -18,9 +18,11 @@ bool pc_tc_wants(const PCGeom& g, int n, bool fp64);
 // regions (see pc_tc.cu) into field / fringe (field is added to when accumulate,
 // else overwritten; fringe is always added to).  The other points are left in
 // slow[0, *slow_n) (device) for the caller; the order within both groups is the
-// input's.
+// input's.  FP64: field double2, fringe double.
 oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, float2* field, float* fringe,
                         bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st);
+oh_status pc_tc64_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, double2* field, double* fringe,
+                          bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st);
 
 namespace pctc {
 
