@@ -1,6 +1,7 @@
 // Context, scratch arena, FFT plan cache and error plumbing.
 #include "context.h"
 #include "fft_fast.cuh"
+#include "two_float.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -258,13 +259,13 @@ oh_status get_plan(oh_ctx* ctx, int n, int prec, FFTPlan* out) {
   auto fill = [&](auto zero) -> cudaError_t {
     typedef decltype(zero) C;
     std::vector<C> t(n + ste.size());
-    for (int e = 0; e < n; ++e) { t[e].x = (decltype(zero.x))c[e]; t[e].y = (decltype(zero.x))sn[e]; }
+    for (int e = 0; e < n; ++e) t[e] = mk((decltype(zero.x))c[e], (decltype(zero.x))sn[e]);
     for (size_t i = 0; i < ste.size(); ++i) t[n + i] = t[ste[i]];
     cudaError_t e = cudaMemcpy(pb.tw, t.data(), sizeof(C) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !ste.empty()) e = cudaMemcpy(pb.stw, t.data() + n, sizeof(C) * ste.size(), cudaMemcpyHostToDevice);
     return e;
   };
-  OH_CUDA_TRY(prec ? fill(double2{}) : fill(float2{}));
+  OH_CUDA_TRY(prec == 2 ? fill(ffc{}) : prec == 1 ? fill(double2{}) : fill(float2{}));
   OH_CUDA_TRY(cudaMemcpy(pb.perm, tabs.data(), sizeof(int) * tabs.size(), cudaMemcpyHostToDevice));
   pl.tw = pb.tw; pl.stw = pb.stw; pl.perm = pb.perm; pl.iperm = pb.perm + n; pl.permp = pb.perm + 2 * (size_t)n;
   ctx->plans[key] = pb;

@@ -45,7 +45,7 @@ struct oh_ctx {
   struct Buf { void* p = nullptr; size_t bytes = 0; };
   std::map<std::string, Buf> scratch;
   struct PlanBufs { oh::FFTPlan plan; void* tw = nullptr; void* stw = nullptr; int* perm = nullptr; };
-  std::map<std::pair<int, int>, PlanBufs> plans;   // key (n, precision)
+  std::map<std::pair<int, int>, PlanBufs> plans;   // key (n, precision of get_plan)
   // optional per-kernel timing: events recorded around each launch on the
   // launching stream while `timing` is set
   bool timing = false;
@@ -80,8 +80,8 @@ oh_status scratch(oh_ctx* ctx, const char* name, size_t bytes, void** out);
 // Destroys every captured graph (they hold scratch addresses).
 void drop_graphs(oh_ctx* ctx);
 
-// Plan for length n in precision prec (0 = fp32, 1 = fp64); built on first
-// use.  Fails with OH_ERR_UNSUPPORTED_SIZE when n cannot be factored.
+// Plan for length n in precision prec (0 = fp32, 1 = fp64, 2 = two-float); built
+// on first use.  Fails with OH_ERR_UNSUPPORTED_SIZE when n cannot be factored.
 oh_status get_plan(oh_ctx* ctx, int n, int prec, FFTPlan* out);
 
 // Radix schedule for n in precision prec (0 = fp32, 1 = fp64); false when

@@ -118,7 +118,10 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
                               void* spectrum, cudaStream_t st, FrameInfo<R>* info = nullptr,
                               const void* src = nullptr, double src_z = 0.0) {
   typedef typename cplx_of<R>::type C;
-  const int prec = sizeof(R) == 8 ? 1 : 0;
+  typedef typename DMArgs<R>::O O;
+  typedef typename DMArgs<R>::OC OC;
+  const int prec = sizeof(R) == 8 ? 1 : 0;              // (two-float frames are FP64 ones)
+  const int plan_prec = std::is_same<R, ff>::value ? 2 : prec;
   Levels L;
   OH_TRY(compute_levels(p, &L));
   int nd = p->num_of_depth;
@@ -189,8 +192,8 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
     else { int cropx = a.Px / 2; cropx1 = cropx - cropx / 2; cropx2 = cropx1 + cropx - 1; }
     a.cx1 = cropx1 - 1; a.cx2 = cropx2 - 1; a.cy1 = cropy1 - 1; a.cy2 = cropy2 - 1;
   }
-  OH_TRY(get_plan(ctx, a.Px, prec, &a.plx));
-  OH_TRY(get_plan(ctx, a.Py, prec, &a.ply));
+  OH_TRY(get_plan(ctx, a.Px, plan_prec, &a.plx));
+  OH_TRY(get_plan(ctx, a.Py, plan_prec, &a.ply));
 
   const size_t smax = max_smem_per_block();
   const int occ_stride = (a.pny + 15) & ~15;
@@ -328,7 +331,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   if (smem_row > smax || smem_out > smax) return fail(OH_ERR_UNSUPPORTED_SIZE, "padded row length " + std::to_string(a.Px) + " exceeds shared memory");
   DMGenPlan gen{};
   if (!fastx || !Wfast) {
-    a.spectrum = (C*)spectrum;
+    a.spectrum = (OC*)spectrum;
     gen = dm_gen_plan<R>(a, smax);
     if (prec && a.horner && gen.smem_col > smax) {      // no room for the step factors
       a.horner = 0;
@@ -380,7 +383,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
     b.slot_any = (int*)at(o_any);
     b.dxh = a.horner ? (C*)at(o_dxh) : nullptr;
     b.dyh = a.horner ? (C*)at(o_dyh) : nullptr;
-    b.fringe = (R*)fringe; b.field = (C*)field; b.spectrum = (C*)spectrum;
+    b.fringe = (O*)fringe; b.field = (OC*)field; b.spectrum = (OC*)spectrum;
     info->a = b;
     info->su = su;
     info->Wfast = Wfast; info->wcol = wcol; info->nchunks = nchunks;
@@ -400,7 +403,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   a.slot_any = (int*)(base + o_any);
   a.dxh = a.horner ? (C*)(base + o_dxh) : nullptr;
   a.dyh = a.horner ? (C*)(base + o_dyh) : nullptr;
-  a.fringe = (R*)fringe; a.field = (C*)field; a.spectrum = (C*)spectrum;
+  a.fringe = (O*)fringe; a.field = (OC*)field; a.spectrum = (OC*)spectrum;
 
   {
     // the tables depend only on the parameters: rebuild them when those (or
@@ -415,7 +418,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
     } key;
     std::memset(&key, 0, sizeof(key));
     key.su = su;
-    key.prec = prec; key.pnx = a.pnx; key.pny = a.pny; key.Px = a.Px; key.Py = a.Py;
+    key.prec = plan_prec; key.pnx = a.pnx; key.pny = a.pny; key.Px = a.Px; key.Py = a.Py;
     key.sig_x = a.sig_x; key.sig_y = a.sig_y; key.ey_perm = a.ey_perm; key.horner = a.horner;
     key.src_mode = src ? 1 : 0;
     key.ppx = a.ppx; key.ppy = a.ppy; key.lambda = a.lambda;
@@ -522,6 +525,45 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   return OH_OK;
 }
 
+// FP64 frames compute in two-float arithmetic (2^-47 per operation) where the
+// propagation phase k z' reaches 1e5 radians: evaluated whole it rounds by 1e-11 in
+// FP64.  1920 x 1080, 32 layers, k z' = 6e6: 3.4 ms and 7e-14 from the exact frame
+// against 10.8 ms for the same passes in FP64 and, phases evaluated whole, 48 ms and
+// 3e-10.  Shorter ranges, values that two floats do not span (the random phase's
+// constant) and residual phases beyond a thousand turns keep the FP64 kernels.
+static bool two_float_ok(const oh_depthmap_params* p) {
+  const double c = std::max(std::fabs(p->rand_phase_re), std::fabs(p->rand_phase_im));
+  if (p->phase_mode == OH_PHASE_REFERENCE && !(c == 0.0 || (c > 1e-12 && c < 1e12))) return false;
+  const double sx = p->lambda / (2.0 * p->ppx), sy = p->lambda / (2.0 * p->ppy), s = sx * sx + sy * sy;
+  if (!(s < 1.0)) return false;
+  Levels L;
+  if (compute_levels(p, &L) != OH_OK) return false;
+  double z = 0.0;
+  for (double v : L.ztrans) z = std::max(z, std::fabs(v));
+  z /= p->lambda;
+  return 6.2831853 * z >= 1e5 && z * s * s < 1000.0;
+}
+static oh_status run_depthmap64(oh_ctx* ctx, const oh_depthmap_params* p, const uint8_t* img, const uint8_t* depth,
+                                const float* phase, void* fringe, void* field, void* spectrum, cudaStream_t st,
+                                DMScratch* sizes = nullptr) {
+  // (both kinds' plans, so that a capture after a frame of either kind finds them)
+  FFTPlan pl;
+  for (int prec = 1; prec <= 2; ++prec) {
+    OH_TRY(get_plan(ctx, p->pad * p->pnx, prec, &pl));
+    OH_TRY(get_plan(ctx, p->pad * p->pny, prec, &pl));
+  }
+  if (two_float_ok(p)) {
+    FrameInfo<ff> fi;
+    const oh_status r = run_depthmap<ff>(ctx, p, img, depth, phase, fringe, field, spectrum, st, sizes ? &fi : nullptr);
+    if (r == OH_OK && sizes) *sizes = fi.sz;
+    if (r != OH_ERR_UNSUPPORTED_SIZE) return r;         // (its tables take 2 KB more shared memory)
+  }
+  FrameInfo<double> fi;
+  OH_TRY(run_depthmap<double>(ctx, p, img, depth, phase, fringe, field, spectrum, st, sizes ? &fi : nullptr));
+  if (sizes) *sizes = fi.sz;
+  return OH_OK;
+}
+
 // One FP32 frame with the caller holding the context (the surrogate's two
 // uses: image/depth layers, or one complex source field at src_z).
 oh_status depthmap_enqueue_f32(oh_ctx* ctx, const oh_depthmap_params* p, const uint8_t* img, const uint8_t* depth,
@@ -582,7 +624,7 @@ oh_status oh_depthmap_generate(oh_ctx* ctx, oh_precision prec, const oh_depthmap
   OH_TRY(validate(p));
   if (!img || !depth || !fringe_out) return fail(OH_ERR_INVALID_ARG, "img, depth and fringe_out are required");
   if (p->phase_mode == OH_PHASE_ARRAY && !phase) return fail(OH_ERR_INVALID_ARG, "OH_PHASE_ARRAY needs a phase array");
-  if (prec == OH_FP64) return run_depthmap<double>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
+  if (prec == OH_FP64) return run_depthmap64(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
   return run_depthmap<float>(ctx, p, img, depth, phase, fringe_out, field_out, spectrum_out, st);
 }
 
@@ -639,10 +681,8 @@ oh_status oh_depthmap_generate_batch(oh_ctx* ctx, oh_precision prec, const oh_de
     for (int i = 0; i < n; ++i) {
       const oh_depthmap_frame& f = frames[i];
       if (fp64) {
-        FrameInfo<double> fi;
-        OH_TRY((run_depthmap<double>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
-                                         sizes ? &fi : nullptr)));
-        if (sizes) sizes[i] = fi.sz;
+        OH_TRY(run_depthmap64(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
+                              sizes ? &sizes[i] : nullptr));
       } else {
         FrameInfo<float> fi;
         OH_TRY((run_depthmap<float>(ctx, &f.params, f.img, f.depth, f.phase, f.fringe, f.field, nullptr, st,
@@ -749,7 +789,7 @@ oh_status oh_depthmap_generate_host(oh_ctx* ctx, oh_precision prec, const oh_dep
       dp = d_phase;
     }
     void* out = fringe_mapped ? fringe_mapped : d_fringe;
-    if (prec == OH_FP64) OH_TRY((run_depthmap<double>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
+    if (prec == OH_FP64) OH_TRY(run_depthmap64(ctx, p, di, dd, dp, out, nullptr, nullptr, st));
     else OH_TRY((run_depthmap<float>(ctx, p, di, dd, dp, out, nullptr, nullptr, st)));
     if (!fringe_mapped) OH_CUDA_TRY(cudaMemcpyAsync(fringe_host, d_fringe, fsz, cudaMemcpyDeviceToHost, st));
     return OH_OK;

@@ -1,5 +1,6 @@
-// Depth-map passes on the plan-driven FFT engine: FP64 frames, and FP32 frames
-// whose padded row or column length has no compile-time schedule.  The same
+// Depth-map passes on the plan-driven FFT engine: FP64 frames (computed in
+// two-float arithmetic, or in FP64 where a frame's range asks for it), and FP32
+// frames whose padded row or column length has no compile-time schedule.  The same
 // frame pipeline as dm_kernels.cuh / dm_col_fast.cuh (row strips, layer flags,
 // spectrum columns in the row FFT's storage order, inverses as the adjoint of
 // the forward network), with run-time lengths.
@@ -7,6 +8,28 @@
 #include "dm_kernels.cuh"
 
 namespace oh {
+
+// Amplitude of an image byte and exp(i phase) of a pixel per compute type; tab: the
+// two-float directions (see ff_cis).
+__device__ __forceinline__ void amp_of(uint8_t g, float* v) { *v = (float)g / 255.f; }
+__device__ __forceinline__ void amp_of(uint8_t g, double* v) { *v = (double)g / 255.0; }
+__device__ __forceinline__ void amp_of(uint8_t g, ff* v) { *v = ff((double)g / 255.0); }
+template <typename R>
+__device__ __forceinline__ typename cplx_of<R>::type phase_of(float radians, float turns, bool seeded, const float4* tab) {
+  if constexpr (std::is_same<R, ff>::value) {
+    if (!seeded && !(fabsf(radians) <= 16.f)) {           // turns to 2^-47 of a few
+      double sn, cs;
+      sincos((double)radians, &sn, &cs);
+      return mk(ff(cs), ff(sn));
+    }
+    return ff_cis(seeded ? ff(turns) : ff_mulf(ff(0.15915494309189533576888376337251), radians), tab);
+  } else {
+    const R ph = seeded ? (R)turns * (R)6.283185307179586476925 : (R)radians;
+    R sn, cs;
+    sincos_r<R>(ph, &sn, &cs);
+    return mk(cs, sn);
+  }
+}
 
 // Row pass: nr (1 or 2) image rows per block.  The layers present in them are
 // taken G at a time (short lines alone leave most threads idle): stage 0
@@ -28,6 +51,12 @@ __global__ void __launch_bounds__(256, 2) dm_row_gen(DMArgs<R> a, int nr, int G)
   const int r0 = blockIdx.x * nr;
   const int nrows = min(nr, a.pny - r0);
   int16_t* const slut = dm_row_slut();
+  const float4* tab = nullptr;
+  if constexpr (std::is_same<R, ff>::value) {
+    __shared__ float4 dirs[256];
+    if (a.phase_mode != OH_PHASE_REFERENCE) ff_directions(dirs, threadIdx.x, T);
+    tab = dirs;
+  }
   for (int i = threadIdx.x; i < 16; i += T) mask[i] = 0u;
   for (int i = threadIdx.x; i < 256; i += T) slut[i] = a.lut[i];
   __syncthreads();
@@ -43,16 +72,14 @@ __global__ void __launch_bounds__(256, 2) dm_row_gen(DMArgs<R> a, int nr, int G)
         const uint8_t g = a.img[off];
         u = g > 0 ? (int)slut[a.depth[off]] : -1;
         if (u >= 0) {
-          const R amp = (R)g / (R)255;
+          R amp;
+          amp_of(g, &amp);
           if (a.phase_mode == OH_PHASE_REFERENCE) {
             val = mk(amp, (R)0);
           } else {
-            R ph;
-            if (a.phase_mode == OH_PHASE_ARRAY) ph = (R)a.phase[off];
-            else ph = (R)u24_at(a.seed, off) * (R)6.283185307179586476925;
-            R sn, cs;
-            sincos_r<R>(ph, &sn, &cs);
-            val = mk(amp * cs, amp * sn);
+            const bool seeded = a.phase_mode == OH_PHASE_SEEDED;
+            const C e = phase_of<R>(seeded ? 0.f : a.phase[off], seeded ? u24_at(a.seed, off) : 0.f, seeded, tab);
+            val = mk(amp * e.x, amp * e.y);
           }
         }
       }
@@ -157,13 +184,17 @@ __device__ __forceinline__ double2 cis_turns(double t, const double2* tab) {
   return make_double2(fma(d.x, c, -d.y * s), fma(d.x, s, d.y * c));
 }
 
+// Directions of the column pass's sine/cosine table (FP64 cis_turns, two-float
+// ff_cis).
+template <typename R> constexpr int kDirs = sizeof(R) == 4 ? 0 : std::is_same<R, ff>::value ? 256 : 128;
+
 // Shared memory of the column pass after the lines: kept rows' positions,
 // active entries, and in FP64 the direction table and (evenly spaced layers)
 // the step factors.
 template <typename R>
 inline size_t dm_col_gen_smem(int lens, int lwb, int G, int nrow, int n_entries, bool horner) {
   size_t o = (size_t)G * lens << lwb;
-  if (sizeof(R) == 8) o += 128 + (horner ? (size_t)nrow << lwb : 0);
+  if (sizeof(R) == 8) o += kDirs<R> + (horner ? (size_t)nrow << lwb : 0);
   o *= 2 * sizeof(R);
   return o + (((size_t)nrow * 2 + 15) & ~(size_t)15) + (size_t)n_entries * 2 + 16;
 }
@@ -175,11 +206,12 @@ inline size_t dm_col_gen_smem(int lens, int lwb, int G, int nrow, int n_entries,
 // its samples into registers.  Only the spectrum rows [row0, row0 +
 // nrow) that reach the crop are kept.  Transfer function: the entry's separable
 // tables times exp(i k z' g), g = s^2 / (2 (1 + sqrt(1 - s))^2) held per sample;
-// FP64 with evenly spaced layers accumulates acc = acc D + x instead (see
-// dm_col_fast.cuh), D in shared memory.
+// FP64 and two-float frames with evenly spaced layers accumulate acc = acc D + x
+// instead (see dm_col_fast.cuh), D in shared memory.
 //
 // What bounds it: instruction issue in FP32 (FFT butterflies plus about 20
-// instructions per kept sample and layer), the FP64 pipe in FP64.
+// instructions per kept sample and layer) and two-float (about 300 a sample in
+// the FFT), the FP64 pipe in FP64.
 template <typename R, int KMAX, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int G, int row0, int nrow) {
   typedef typename cplx_of<R>::type C;
@@ -192,7 +224,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int gs = lens << lwb;                           // a layer's lines
   C* tab = buf + (size_t)G * gs;
-  C* dst = tab + (F64 ? 128 : 0);
+  C* dst = tab + kDirs<R>;
   uint16_t* pos = reinterpret_cast<uint16_t*>(dst + (step ? (size_t)nrow << lwb : 0));
   int16_t* list = reinterpret_cast<int16_t*>(pos + ((nrow + 7) & ~7));
   const int w = tid & (W - 1), p = (blockIdx.x << lwb) + w;
@@ -216,14 +248,22 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
     }
     if (tid == 0) s_nact = n;
   }
-  if constexpr (F64) {
+  if constexpr (std::is_same<R, ff>::value) {
+    ff_directions(reinterpret_cast<float4*>(tab), tid, T);
+  } else if constexpr (F64) {
     for (int i = tid; i < 128; i += T) { double s, c; sincospi(i * (1.0 / 64.0), &s, &c); tab[i] = mk(c, s); }
   }
   auto resid = [&](int k) -> R {
     const int i = (tid + k * T) >> lwb;
-    const R sv = a.lfx[kx] + a.lfy[row0 + i];
-    const R den = (R)1 + sqrt((R)1 - sv);
-    return sv * sv / ((R)2 * den * den);
+    if constexpr (F64) {                                // g / 2 pi
+      const double sv = (double)a.lfx[kx] + (double)a.lfy[row0 + i];
+      const double den = 1.0 + sqrt(1.0 - sv);
+      return (R)(sv * sv / (12.566370614359172953850573533118 * den * den));
+    } else {
+      const R sv = a.lfx[kx] + a.lfy[row0 + i];
+      const R den = (R)1 + sqrt((R)1 - sv);
+      return sv * sv / ((R)2 * den * den);
+    }
   };
   C acc[KMAX];
   R g[KEEPG ? KMAX : 1];
@@ -237,7 +277,8 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
   auto gof = [&](int k) -> R { if constexpr (KEEPG) return g[k]; else return resid(k); };
   // exp(i kz g) of sample k
   auto residual = [&](R kz, int k) -> C {
-    if constexpr (F64) return cis_turns(kz * 0.15915494309189533576888376337251 * gof(k), tab);
+    if constexpr (std::is_same<R, ff>::value) return ff_cis(kz * gof(k), reinterpret_cast<const float4*>(tab));
+    else if constexpr (F64) return cis_turns(kz * gof(k), tab);
     else { float sn, cs; __sincosf(kz * gof(k), &sn, &cs); return mk(cs, sn); }
   };
   if constexpr (F64) {
@@ -331,7 +372,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
         for (int k = 0; k < KMAX; ++k) {
           const int idx = tid + k * T;
           if (idx < nk) {
-            const C h = cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k));
+            const C h = cmul(cmul(ex, ldg_c(ey + (idx >> lwb))), residual(kz, k));
             const C x = line[(int)pos[idx >> lwb] << lwb];
             acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
             acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
@@ -350,7 +391,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
 #pragma unroll
     for (int k = 0; k < KMAX; ++k) {
       const int idx = tid + k * T;
-      if (idx < nk) acc[k] = cmul(acc[k], cmul(cmul(ex, __ldg(ey + (idx >> lwb))), residual(kz, k)));
+      if (idx < nk) acc[k] = cmul(acc[k], cmul(cmul(ex, ldg_c(ey + (idx >> lwb))), residual(kz, k)));
     }
   }
 
@@ -364,7 +405,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
     const int idx = tid + k * T;
     if (idx < nk && valid) {
       const int ky = row0 + (idx >> lwb);
-      if (a.spectrum) a.spectrum[(size_t)ky * a.Px + kx] = acc[k];
+      if (a.spectrum) a.spectrum[(size_t)ky * a.Px + kx] = mk(to_out(acc[k].x), to_out(acc[k].y));
       if (kx >= a.cx1 && kx <= a.cx2 && ky >= a.cy1 && ky <= a.cy2) {
         int i = ky + a.hy;
         if (i >= Py) i -= Py;
@@ -409,8 +450,8 @@ __global__ void __launch_bounds__(256) dm_out_gen(DMArgs<R> a) {
     if (m < 0) m += Px;
     C h = buf[pl_at(a.plx, m)];
     if (a.sig_x != 0) h = cmul(h, a.shx[c]);
-    a.fringe[(size_t)yl * a.pnx + c] = h.x;
-    if (a.field) a.field[(size_t)yl * a.pnx + c] = h;
+    a.fringe[(size_t)yl * a.pnx + c] = to_out(h.x);
+    if (a.field) a.field[(size_t)yl * a.pnx + c] = mk(to_out(h.x), to_out(h.y));
   }
 }
 

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include "context.h"
 #include "fft_kernels.cuh"
+#include "two_float.cuh"
 
 namespace oh {
 
@@ -23,9 +24,18 @@ struct DMSetup {
   int16_t lut[256];                  // depth byte -> unique slot (-1: none)
 };
 
+// The type a frame's outputs have: the compute type, double for two-float frames.
+template <typename R> struct out_of { typedef R type; };
+template <> struct out_of<ff> { typedef double type; };
+__device__ __forceinline__ float to_out(float v) { return v; }
+__device__ __forceinline__ double to_out(double v) { return v; }
+__device__ __forceinline__ double to_out(ff v) { return (double)v; }
+
 template <typename R>
 struct DMArgs {
   typedef typename cplx_of<R>::type C;
+  typedef typename out_of<R>::type O;
+  typedef typename cplx_of<O>::type OC;
   int pnx, pny, Px, Py, ox, oy, hx, hy;
   int W, lw, nstrips, n_entries, n_uslots;     // lw = log2(W)
   int cx1, cx2, cy1, cy2;            // SSB crop window on the (padded) spectrum
@@ -54,9 +64,9 @@ struct DMArgs {
   uint8_t* occ;          // [uslots][pny]
   C* Rbuf;               // [uslots][nstrips][pny][W], columns in the row FFT's storage order
   C* V;                  // [pny][Px], columns in the same order
-  R* fringe;             // [pny][pnx]
-  C* field;              // [pny][pnx] or null
-  C* spectrum;           // [Py][Px] or null
+  O* fringe;             // [pny][pnx]
+  OC* field;             // [pny][pnx] or null
+  OC* spectrum;          // [Py][Px] or null
   int sig_x, sig_y;
   int occ_stride;        // bytes per layer row of occ (multiple of 16)
   int hzx, hzy;          // 1: 2x padding with a radix-16 first stage (stage-0 inputs 4..11 are zero)

@@ -106,8 +106,8 @@ __device__ __forceinline__ void dft8(C* x) {
   dft4<SGN>(o0, o1, o2, o3);
   // w8^k for k = 1,2,3 (forward e^{-i pi k/4})
   C w1, w3;
-  w1.x = h; w1.y = (R)SGN * h;
-  w3.x = -h; w3.y = (R)SGN * h;
+  w1.x = h; w1.y = SGN < 0 ? -h : h;
+  w3.x = -h; w3.y = SGN < 0 ? -h : h;
   o1 = cmul(o1, w1);
   o3 = cmul(o3, w3);
   x[0] = cadd(e0, o0); x[4] = csub(e0, o0);

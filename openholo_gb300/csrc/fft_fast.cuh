@@ -76,8 +76,8 @@ __device__ __forceinline__ C wmul(C a, int m) {
     // and a difference, then one real scale
     const R h = (R)0.70710678118654752440;
     C u;
-    if (m == 2) { u.x = a.x - (R)SGN * a.y; u.y = a.y + (R)SGN * a.x; return cscale(u, h); }
-    u.x = a.x + (R)SGN * a.y; u.y = a.y - (R)SGN * a.x;
+    if (m == 2) { u.x = SGN < 0 ? a.x + a.y : a.x - a.y; u.y = SGN < 0 ? a.y - a.x : a.y + a.x; return cscale(u, h); }
+    u.x = SGN < 0 ? a.x - a.y : a.x + a.y; u.y = SGN < 0 ? a.y + a.x : a.y - a.x;
     return cscale(u, -h);
   }
   R c, s;
@@ -91,7 +91,7 @@ __device__ __forceinline__ C wmul(C a, int m) {
   } else {
     c = (R)w9c(m); s = (R)w9s(m);
   }
-  C w; w.x = c; w.y = (R)SGN * s;
+  C w; w.x = c; w.y = SGN < 0 ? -s : s;
   return cmul(a, w);
 }
 

@@ -13,6 +13,7 @@
 #pragma once
 #include <type_traits>
 #include "fft_fast.cuh"
+#include "two_float.cuh"
 
 namespace oh {
 
@@ -68,6 +69,12 @@ template <int SGN, typename C> struct DFT<13, SGN, C> {
 template <int SGN, typename C> struct DFT<14, SGN, C> {
   __device__ __forceinline__ static void run(C* x) { dft_pfa<2, 7, SGN>(x); }
 };
+
+template <typename C> __device__ __forceinline__ C ldg_c(const C* p) { return __ldg(p); }
+__device__ __forceinline__ ffc ldg_c(const ffc* p) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  return mk(ff(v.x, v.y), ff(v.z, v.w));
+}
 
 // Calls f(std::integral_constant<int, r>) for the straight-line radices and
 // f(std::integral_constant<int, 0>) for any other.
@@ -152,7 +159,7 @@ __device__ __forceinline__ void gbutterfly(const GStage& g, int j, C* x) {
   if constexpr (MODE == GADJ) {
     if (j) {
 #pragma unroll
-      for (int f = 1; f < R; ++f) x[f] = cmulc(x[f], __ldg(tw + (f - 1) * g.q));
+      for (int f = 1; f < R; ++f) x[f] = cmulc(x[f], ldg_c(tw + (f - 1) * g.q));
     }
     DFT<R, 1, C>::run(x);
   } else {
@@ -160,7 +167,7 @@ __device__ __forceinline__ void gbutterfly(const GStage& g, int j, C* x) {
     if (j) {
 #pragma unroll
       for (int f = 1; f < R; ++f) {
-        const C w = __ldg(tw + (f - 1) * g.q);
+        const C w = ldg_c(tw + (f - 1) * g.q);
         x[f] = MODE == GFWD ? cmul(x[f], w) : cmulc(x[f], w);
       }
     }

@@ -1,52 +1,10 @@
-// Two-float arithmetic (a value as the unevaluated sum h + l of two FP32
-// numbers, about 48 bits) and the per-axis factors of the FP64 point-cloud sum
-// in it.  FP64 runs at 1/64 of the FP32 rate on this part, so error-free FP32
-// transforms (Dekker, Knuth; products by FMA) are several times faster.
-// Everything is written with explicitly rounded operations: a contraction to
-// FMA would break the error terms.  The functions also run on the host.
+// The per-axis factors of the FP64 point-cloud sum in two-float arithmetic.  The
+// functions also run on the host.
 #pragma once
-#include <cmath>
-#include <cstdint>
-#include <cstring>
 #include <cuda_bf16.h>
-#include <cuda_runtime.h>
+#include "two_float.cuh"
 
 namespace oh {
-
-#if defined(__CUDA_ARCH__)
-#define OH_FADD(a, b) __fadd_rn(a, b)
-#define OH_FSUB(a, b) __fsub_rn(a, b)
-#define OH_FMUL(a, b) __fmul_rn(a, b)
-#define OH_FFMA(a, b, c) __fmaf_rn(a, b, c)
-#else
-#define OH_FADD(a, b) ((float)((a) + (b)))
-#define OH_FSUB(a, b) ((float)((a) - (b)))
-#define OH_FMUL(a, b) ((float)((a) * (b)))
-#define OH_FFMA(a, b, c) std::fma((float)(a), (float)(b), (float)(c))
-#endif
-#define OH_HD __host__ __device__ __forceinline__
-
-struct ff { float h, l; };
-
-OH_HD ff ff_quick(float a, float b) {            // |a| >= |b| or a = 0
-  const float s = OH_FADD(a, b);
-  return {s, OH_FSUB(b, OH_FSUB(s, a))};
-}
-OH_HD ff ff_sum(float a, float b) {
-  const float s = OH_FADD(a, b), t = OH_FSUB(s, a);
-  return {s, OH_FADD(OH_FSUB(a, OH_FSUB(s, t)), OH_FSUB(b, t))};
-}
-// (products are not renormalised: l may reach a few units in h's last place)
-OH_HD ff ff_mul(ff a, ff b) {
-  const float p = OH_FMUL(a.h, b.h);
-  return {p, OH_FFMA(a.l, b.h, OH_FFMA(a.h, b.l, OH_FFMA(a.h, b.h, -p)))};
-}
-OH_HD ff ff_mulf(ff a, float b) {
-  const float p = OH_FMUL(a.h, b);
-  return {p, OH_FFMA(a.l, b, OH_FFMA(a.h, b, -p))};
-}
-OH_HD ff ff_neg(ff a) { return {-a.h, -a.l}; }
-OH_HD ff ff_of(double v) { const float h = (float)v; return {h, (float)(v - (double)h)}; }
 
 // One axis of a point as a plane region sees it: the phase in turns at offset m
 // from the region's centre is t0 + m (c1 + m (c2 + m (c3 + m c4))) mod 1 in 64-bit
@@ -59,12 +17,9 @@ struct AxisRec {
   ff a, b;
 };
 
-struct ffc { ff re, im; };
-
-// exp(2 pi i t / 2^64): the nearest of 256 directions (tab[i] = cos h, cos l, sin
-// h, sin l of 2 pi i / 256) times a short series on the rest; extra: a further
-// phase in turns, below 1e-6.
-OH_HD ffc ff_cis(uint64_t t, float extra, const float4* tab) {
+// exp(2 pi i t / 2^64); extra: a further phase in turns, below 1e-6; tab: see
+// ff_rotate.
+OH_HD ffc ff_cis64(uint64_t t, float extra, const float4* tab) {
   const uint64_t r = t + (1ull << 55);
   const int idx = (int)(r >> 56);
   const int64_t f = (int64_t)(t - ((uint64_t)idx << 56));         // [-2^55, 2^55)
@@ -76,39 +31,14 @@ OH_HD ffc ff_cis(uint64_t t, float extra, const float4* tab) {
   const float cb = 3.4061215800304e-19f;                         // 2 pi 2^-64
   const float p = OH_FMUL(A, ch);
   const float q = OH_FFMA(A, cl, OH_FFMA(A, ch, -p));
-  const ff x{p, OH_FFMA(6.28318530717958647692f, extra, OH_FFMA(B, cb, q))};
-  const float x2 = OH_FMUL(x.h, x.h);
-  const float x2l = OH_FFMA(OH_FMUL(2.f, x.h), x.l, OH_FFMA(x.h, x.h, -x2));
-  // sin x = x - x^3 (1 / 6 - x^2 / 120), cos x - 1 = -x^2 / 2 + x^4 (1 / 24 - x^2 / 720), |x| <= pi / 256
-  const ff s{x.h, OH_FFMA(OH_FMUL(-x.h, x2), OH_FFMA(x2, -0.0083333333f, 0.16666667f), x.l)};
-  const float ch1 = -0.5f * x2;
-  const float cl1 = OH_FFMA(-0.5f, x2l, OH_FMUL(OH_FMUL(x2, x2), OH_FFMA(x2, -0.0013888889f, 0.041666668f)));
-  const float4 T = tab[idx & 255];
-  ffc o;
-  {
-    const float p1 = OH_FMUL(T.x, ch1), p2 = OH_FMUL(T.z, s.h);
-    const float e1 = OH_FFMA(T.y, ch1, OH_FFMA(T.x, cl1, OH_FFMA(T.x, ch1, -p1)));
-    const float e2 = OH_FFMA(T.w, s.h, OH_FFMA(T.z, s.l, OH_FFMA(T.z, s.h, -p2)));
-    const ff d = ff_sum(p1, -p2);
-    const ff g = ff_sum(T.x, d.h);
-    o.re = ff_quick(g.h, OH_FADD(g.l, OH_FADD(T.y, OH_FADD(d.l, OH_FSUB(e1, e2)))));
-  }
-  {
-    const float p1 = OH_FMUL(T.z, ch1), p2 = OH_FMUL(T.x, s.h);
-    const float e1 = OH_FFMA(T.w, ch1, OH_FFMA(T.z, cl1, OH_FFMA(T.z, ch1, -p1)));
-    const float e2 = OH_FFMA(T.y, s.h, OH_FFMA(T.x, s.l, OH_FFMA(T.x, s.h, -p2)));
-    const ff d = ff_sum(p1, p2);
-    const ff g = ff_sum(T.z, d.h);
-    o.im = ff_quick(g.h, OH_FADD(g.l, OH_FADD(T.w, OH_FADD(d.l, OH_FADD(e1, e2)))));
-  }
-  return o;
+  return ff_rotate({p, OH_FFMA(6.28318530717958647692f, extra, OH_FFMA(B, cb, q))}, tab[idx & 255]);
 }
 
 OH_HD ffc axis_cis(const AxisRec& r, int m, const float4* tab) {
   const uint64_t um = (uint64_t)(int64_t)m;
   const uint64_t t = r.t0 + um * (r.c1 + um * (r.c2 + um * (r.c3 + um * r.c4)));
   const float mf = (float)m, m2 = mf * mf;
-  return ff_cis(t, OH_FMUL(OH_FMUL(m2, OH_FMUL(m2, mf)), OH_FFMA(r.c6, mf, r.c5)), tab);
+  return ff_cis64(t, OH_FMUL(OH_FMUL(m2, OH_FMUL(m2, mf)), OH_FFMA(r.c6, mf, r.c5)), tab);
 }
 
 // w (1 - 3/4 w + 5/8 w^2 - 35/64 w^3) / Qs, w / Qs = m (a + b m)

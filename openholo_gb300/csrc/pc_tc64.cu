@@ -10,7 +10,7 @@
 // Axis phases are 64-bit fractions of a turn (a quartic in the pixel offset in
 // exact integer arithmetic, its coefficients from FP64 once per point and
 // region), their sines and cosines and the factors two-float numbers
-// (pc_ff.cuh, about 1e-13).
+// (pc_ff.cuh, about 2e-13).
 //
 // The products run on BF16 operands without rounding error: terms 0, 1 are
 // split into multiples of 2^-8, 2^-16 and 2^-24 of at most 256 steps each and two
@@ -175,12 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = threadIdx.x; i < 256; i += kThreads) {
-    double s, c;
-    sincospi(i * (1.0 / 128.0), &s, &c);
-    const ff fc = ff_of(c), fs = ff_of(s);
-    tab[i] = make_float4(fc.h, fc.l, fs.h, fs.l);
-  }
+  ff_directions(tab, threadIdx.x, kThreads);
   if (warp == 1) tc::tmem_alloc(tmem_slot, kTmemCols);
   tc::fence_before();
   __syncthreads();
@@ -239,8 +234,8 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       const AxisRec ax{r.t0, r.c1, r.c2, r.c3, r.c4, r.c5, r.c6, r.a, r.b};
       const ffc E = axis_cis(ax, m, tab);
       const ff Q = axis_cross(ax, m, r.qs);
-      ff re = ff_mulf(E.re, r.amp), im = ff_mulf(E.im, r.amp);
-      const ff r1 = ff_mul(re, Q), i1 = ff_mul(im, Q);
+      ff re = ff_mulf(E.x, r.amp), im = ff_mulf(E.y, r.amp);
+      const ff r1 = re * Q, i1 = im * Q;
       {
         float a0[5], a1[5], b0_[5], b1_[5];
         ff_slices<true>(re, a0);
@@ -250,8 +245,8 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) put(A + k * kTile, off0, pack(a0[k], a1[k]), pack(b0_[k], b1_[k]));
       }
-      re = ff_mul(r1, Q);
-      im = ff_mul(i1, Q);
+      re = r1 * Q;
+      im = i1 * Q;
       const float r3 = re.h * Q.h, i3 = im.h * Q.h;
       {
         float a0[5], a1[5], b0_[5], b1_[5];
@@ -298,12 +293,12 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       const RecB& r = recB[rs][(it % kPer) * kPts + j];
       const AxisRec ax{0ull, r.c1, r.c2, r.c3, r.c4, r.c5, r.c6, r.a, r.b};
       const ffc E = axis_cis(ax, m, tab);
-      const ff ch = ff_mul(r.kq, axis_cross(ax, m, 1.f));
-      const ff R1r = ff_mul(ff_neg(E.im), ch), R1i = ff_mul(E.re, ch);            // i chi E
+      const ff ch = r.kq * axis_cross(ax, m, 1.f);
+      const ff R1r = -E.y * ch, R1i = E.x * ch;            // i chi E
       {
         float a0[5], a1[5], b0_[5], b1_[5];
-        ff_slices<true>(E.re, a0);
-        ff_slices<true>(E.im, a1);
+        ff_slices<true>(E.x, a0);
+        ff_slices<true>(E.y, a1);
         ff_slices<true>(R1r, b0_);
         ff_slices<true>(R1i, b1_);
 #pragma unroll
@@ -311,23 +306,23 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       }
       // (-chi^2 / 2 + i mu) E,  (-i chi^3 / 6 - chi mu) E,  chi^4 / 24 E,  i chi^5 / 120 E
       const ff hc{0.5f * ch.h, 0.5f * ch.l};
-      ff R2r = ff_mul(ff_neg(R1i), hc), R2i = ff_mul(R1r, hc);
+      ff R2r = -R1i * hc, R2i = R1r * hc;
       const float c2 = ch.h * ch.h, c3 = c2 * ch.h, mu = r.cmu * c2;
-      R2r.l = OH_FFMA(-mu, E.im.h, R2r.l);
-      R2i.l = OH_FFMA(mu, E.re.h, R2i.l);
+      R2r.l = OH_FFMA(-mu, E.y.h, R2r.l);
+      R2i.l = OH_FFMA(mu, E.x.h, R2i.l);
       const float k3 = c3 * 0.16666667f, m3 = -c3 * r.cmu;
       {
         float a0[5], a1[5], b0_[5], b1_[5];
         ff_slices<false>(R2r, a0);
         ff_slices<false>(R2i, a1);
-        ff_slices<false>(ff{E.re.h * m3 + E.im.h * k3, 0.f}, b0_);
-        ff_slices<false>(ff{E.im.h * m3 - E.re.h * k3, 0.f}, b1_);
+        ff_slices<false>(ff{E.x.h * m3 + E.y.h * k3, 0.f}, b0_);
+        ff_slices<false>(ff{E.y.h * m3 - E.x.h * k3, 0.f}, b1_);
 #pragma unroll
         for (int k = 1; k < 5; ++k) put2(B + k * kTile, p0, p1, a0[k], a1[k], b0_[k], b1_[k]);
       }
       {
         const float k4 = c2 * c2 * 0.041666668f, k5 = c3 * c2 * 0.0083333333f;
-        const float r4 = E.re.h * k4, i4 = E.im.h * k4, r5 = -E.im.h * k5, i5 = E.re.h * k5;
+        const float r4 = E.x.h * k4, i4 = E.y.h * k4, r5 = -E.y.h * k5, i5 = E.x.h * k5;
         const float r4h = bf16_round(r4), i4h = bf16_round(i4), r5h = bf16_round(r5), i5h = bf16_round(i5);
         put2(B, p0, p1, r4h, i4h, r5h, i5h);
         put2(B + 5 * kTile, o0, o1, r4 - r4h, i4 - i4h, r5 - r5h, i5 - i5h);
@@ -413,12 +408,12 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
         const float qm = (float)(fabs(ay) * (kRows / 2) + by * (kRows / 2) * (kRows / 2));
         const int ex = (__float_as_int(qm) >> 23) - 126;
         const double qs = __hiloint2double((1023 + ex) << 20, 0), iqs = __hiloint2double((1023 - ex) << 20, 0);
-        ra.a = ff_of(ay * iqs); ra.b = ff_of(by * iqs);
+        ra.a = ff(ay * iqs); ra.b = ff(by * iqs);
         ra.qs = (float)qs;
         ra.amp = p.a * scale;
-        rb.a = ff_of(2.0 * sx * tx); rb.b = ff_of(tx * tx);
+        rb.a = ff(2.0 * sx * tx); rb.b = ff(tx * tx);
         const double kr = 6.283185307179586476925286766559 * C;
-        rb.kq = ff_of(-0.25 * kr * qs);
+        rb.kq = ff(-0.25 * kr * qs);
         rb.cmu = -1.5f / (float)kr;
       }
       recA[rs][lane] = ra;
