@@ -163,13 +163,18 @@ __device__ __forceinline__ void wrp_point(const WRPGeom& g, const double* xyz, i
 
 // Two binnings share one count / start / list layout: 64 x 64 tiles for the
 // direct tile kernels (bins [0, nd)) and, for points the tensor-core form
-// takes (series == 2 and use_tc), 64-column x 128-row regions (bins
-// [nd, nd + regions)).
-constexpr int kTcW = 64, kTcH = 128;
+// takes (series == 2 and use_tc), 128 x 128 regions (bins [nd, nd + regions)).
+// Windows of up to half a region bin by their centre: cells of step = 128 - 2 w
+// pixels, whose points' windows all lie inside the region that starts w before
+// the cell's first pixel, so a point has one bin; the regions overlap.  Wider
+// windows bin by every region of a partition of the plane that they touch.
+constexpr int kTcR = 128;
 
 struct WrpBins {
   int tiles_x, nd;          // direct tiles across, direct bin count
   int regions_x;            // tensor regions across
+  int step;                 // pixels from one region to the next
+  int off;                  // region r starts at pixel r step - off (0: partition)
   int use_tc;
 };
 
@@ -186,9 +191,13 @@ __device__ __forceinline__ bool wrp_bin_range(int c, int w, int n, int size, int
 template <class F>
 __device__ __forceinline__ void wrp_for_bins(const WRPGeom& g, const WrpBins& b, const WrpPt& q, F f) {
   const bool tc = b.use_tc && q.series == 2;
-  const int bw = tc ? kTcW : kWrpTile, bh = tc ? kTcH : kWrpTile;
+  const int size = tc ? kTcR : kWrpTile;
   int x0, x1, y0, y1;
-  if (!wrp_bin_range(q.tx, q.w, g.nx, bw, &x0, &x1) || !wrp_bin_range(q.ty, q.w, g.ny, bh, &y0, &y1)) return;
+  if (!wrp_bin_range(q.tx, q.w, g.nx, size, &x0, &x1) || !wrp_bin_range(q.ty, q.w, g.ny, size, &y0, &y1)) return;
+  if (tc && b.off) {
+    f(b.nd + (q.ty + q.w) / b.step * b.regions_x + (q.tx + q.w) / b.step);
+    return;
+  }
   for (int ty = y0; ty <= y1; ++ty)
     for (int tx = x0; tx <= x1; ++tx) f(tc ? b.nd + ty * b.regions_x + tx : ty * b.tiles_x + tx);
 }
@@ -433,32 +442,38 @@ __global__ void __launch_bounds__(256) wrp_tile_f32(WRPGeom g, const WrpPt* __re
 }
 
 // ---- tensor-core form of the fixed-window sum (series == 2 points) ---------
-// Over a 128-row x 64-column plane region, the separable windows make the sum
+// Over a 128 x 128 plane region, the separable windows make the sum
 //   W[y][x] = sum_p L0_p[y] R0_p[x] + L1_p[y] R1_p[x],
 //   L0 = a0 e^{2 pi i (base_t + f(uy))} A(uy),  L1 = uy L0,
 //   R0 = e^{2 pi i f(ux)} A(ux),                R1 = i kappa ux R0
 // (zero outside each window) a complex matrix product with K = 2 per point.
 // Embedded in reals as in the point-sum GEMM (K column 2k / 2k+1 = Re / Im of
-// term k; B rows 2x / 2x+1 give Re / Im of column x), C = A B^T is the
-// region's complex64 sum, M = 128, N = 128, K = 4 per point.  BF16 high and
+// term k; B rows x / 128 + x give Re / Im of column x), C = A B^T is the
+// region's complex64 sum, M = 128, N = 256, K = 4 per point.  BF16 high and
 // low parts, three products (Ahi Bhi + Ahi Blo + Alo Bhi), FP32 in TMEM.
 //
 // One CTA per region, 288 threads.  Warps 0-7 write the operands of 8 points
 // (K = 32) per stage straight into shared memory, in the layout a TMA load
-// with 64-byte swizzle would give, then arrive on the stage's full barrier:
-// thread t takes point slot t & 7, A rows (t >> 3) + 32 m (m < 4) and B
-// columns (t >> 3) + 32 m (m < 2), so its swizzled offsets are fixed.  Warp 8
-// issues tcgen05.mma (M 128, N 128, K 16) and releases stages with
-// tcgen05.commit; warps 4-7 read the accumulator (tcgen05.ld) and add the
-// region into the plane.  Waits are bounded: on timeout the CTA sets the
-// device error word, skips the add, waits for its MMAs and frees TMEM.
+// with 64-byte swizzle would give, then arrive on the stage's full barrier.  A
+// warp takes a pair of point slots, alternating between them over its lanes:
+// 16 rows from each window's first on (modulo the region), so that only window
+// pixels are evaluated, the rest of the rows get zeros, and the 8-byte stores of
+// the pair fill the banks wherever the two windows start.  Warp 8 issues
+// tcgen05.mma (M 128, N 256, K 16) and releases stages with tcgen05.commit;
+// warps 0-7 read the accumulator (tcgen05.ld) and add it to the plane through
+// shared memory with vector reductions (neighbouring regions overlap).  Waits are
+// bounded: on timeout the CTA sets the device error word, skips the add, waits
+// for its MMAs and frees TMEM.
+//
+// What bounds it: the operand builders' issue slots, then the MMAs (about 100
+// clocks per point) and shared memory.
 namespace tcw {
 
-constexpr int kRows = kTcH, kCols = kTcW;             // region
 constexpr int kBK = 32, kPts = kBK / 4, kStages = 2;
 constexpr int kTile = 128 * kBK * 2;                   // 8 KB: 128 rows x 32 BF16
-constexpr int kStageBytes = 4 * kTile;                 // Ahi, Alo, Bhi, Blo
-constexpr int kTmemCols = 128;
+constexpr int kStageBytes = 6 * kTile;                 // Ahi, Alo, Bhi, Blo (B: 256 rows)
+constexpr int kTmemCols = 256;
+constexpr int kEpiRow = 32 * 8 + 16;                   // 32 pixels of a row, padded
 constexpr int kProducerWarps = 8, kThreads = 32 * kProducerWarps + 32;   // + the MMA warp
 constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
 constexpr long long kWaitCycles = 2000000000LL;
@@ -496,8 +511,8 @@ __device__ __forceinline__ uint64_t sw_desc(uint32_t saddr) {
   d |= (uint64_t)4 << 61;
   return d;
 }
-// kind::f16, D FP32, A and B BF16, K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) |
+// kind::f16, D FP32, A and B BF16, K-major, N = 256, M = 128
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
                             ((uint32_t)(128 >> 4) << 24);
 __device__ __forceinline__ void umma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accum) {
   asm volatile(
@@ -521,25 +536,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Byte offset of point slot j (4 BF16 = 8 bytes) in row r of a [128][32] BF16
+// Byte offset of point slot j (4 BF16 = 8 bytes) in row r of a [rows][32] BF16
 // tile with 64-byte swizzle: 16-byte chunk c of the row lands at c ^ ((r >> 1) & 3).
 __device__ __forceinline__ int sw_off(int r, int j) {
   return r * 64 + (((j >> 1) ^ ((r >> 1) & 3)) << 4) + ((j & 1) << 3);
-}
-
-// BF16 high / low parts of four values, written as 8 bytes each
-__device__ __forceinline__ void put4(unsigned char* hi, unsigned char* lo, int off, float a, float b, float c,
-                                     float d) {
-  const __nv_bfloat162 h0 = __floats2bfloat162_rn(a, b), h1 = __floats2bfloat162_rn(c, d);
-  const __nv_bfloat162 l0 = __floats2bfloat162_rn(a - __low2float(h0), b - __high2float(h0));
-  const __nv_bfloat162 l1 = __floats2bfloat162_rn(c - __low2float(h1), d - __high2float(h1));
-  uint2 vh, vl;
-  vh.x = *reinterpret_cast<const uint32_t*>(&h0);
-  vh.y = *reinterpret_cast<const uint32_t*>(&h1);
-  vl.x = *reinterpret_cast<const uint32_t*>(&l0);
-  vl.y = *reinterpret_cast<const uint32_t*>(&l1);
-  *reinterpret_cast<uint2*>(hi + off) = vh;
-  *reinterpret_cast<uint2*>(lo + off) = vl;
 }
 
 __device__ __forceinline__ float frac_turns(float f) { return f - rintf(f); }
@@ -596,9 +596,9 @@ __device__ __forceinline__ Rec load_rec(const WrpPt* __restrict__ pts, const int
 
 }  // namespace tcw
 
-__global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpPt* __restrict__ pts,
+__global__ void __launch_bounds__(tcw::kThreads, 2) wrp_tc(WRPGeom g, const WrpPt* __restrict__ pts,
                                                            const int* __restrict__ start,
-                                                           const int* __restrict__ list, int regions_x,
+                                                           const int* __restrict__ list, WrpBins bins,
                                                            float2* __restrict__ wrp, int* err) {
   using namespace tcw;
   extern __shared__ unsigned char smem_raw[];
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpP
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int region = blockIdx.x;
-  const int X0 = (region % regions_x) * kCols, Y0 = (region / regions_x) * kRows;
+  const int X0 = (region % bins.regions_x) * bins.step - bins.off, Y0 = (region / bins.regions_x) * bins.step - bins.off;
   const int b = start[region], e = start[region + 1];
   if (b == e) return;                    // uniform: no window reaches this region
   const int npts = e - b;
@@ -637,20 +637,10 @@ __global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpP
   const uint32_t tmem = *tmem_slot;
 
   if (warp < kProducerWarps) {
-    // producers: point slot j, A rows rb + 32 m, B columns rb + 32 m; the
-    // record of this stage's point sits in registers, the next stage's is
-    // loaded while this stage is built
-    const int pt = threadIdx.x;
-    const int j = pt & (kPts - 1), rb = pt >> 3;
-    int offA[4], YA[4], offB0[2], offB1[2], XB[2];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) { offA[m] = sw_off(rb + 32 * m, j); YA[m] = Y0 + rb + 32 * m; }
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      offB0[m] = sw_off(2 * (rb + 32 * m), j);
-      offB1[m] = sw_off(2 * (rb + 32 * m) + 1, j);
-      XB[m] = X0 + rb + 32 * m;
-    }
+    // producers: the record of this stage's point sits in registers, the next
+    // stage's is loaded while this stage is built
+    const int j = 2 * (warp & 3) + (lane & 1);           // point slot
+    const int i0 = 16 * (warp >> 2) + (lane >> 1);       // rows i0 + 32 m from the window's first on
     // two-level prefetch: the list entry two stages ahead, the record of the
     // next stage (its address known a stage in advance), so the dependent
     // list -> record loads are not on one stage's critical path
@@ -669,41 +659,58 @@ __global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpP
       unsigned char* sAh = base + s * kStageBytes;
       unsigned char* sAl = sAh + kTile;
       unsigned char* sBh = sAh + 2 * kTile;
-      unsigned char* sBl = sAh + 3 * kTile;
+      unsigned char* sBl = sAh + 4 * kTile;
       const Rec qn = load_rec_at(pts, idx_next);
       idx_next = list_at(list, b + (it + 2) * kPts + j, e);
-      // A: branch-free, rows outside the window (or the plane) get amplitude 0
+      const unsigned ww = 2 * q.w;
+      const int ys0 = q.ty - q.w - Y0, xs0 = q.tx - q.w - X0;
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        const int wy = YA[m] - q.ty;
-        const bool in = YA[m] < g.ny && (unsigned)(wy + q.w) < (unsigned)(2 * q.w);
-        const float ys = (float)wy * q.sx, uy = ys * ys;
-        const float f = frac_turns(fmaf(uy, fmaf(uy, fmaf(uy, q.c3, q.c2), q.c1), q.base_t));
-        float sn, cs;
-        __sincosf(6.28318530717958647692f * f, &sn, &cs);
-        const float amp = in ? q.a0c * fmaf(uy, fmaf(uy, q.beta, q.alpha), 1.f) : 0.f;
-        const float v0 = amp * cs, v1 = amp * sn;
-        put4(sAh, sAl, offA[m], v0, v1, uy * v0, uy * v1);
+        const int r = (ys0 + i0 + 32 * m) & 127;
+        const int off = sw_off(r, j);
+        const int wy = Y0 + r - q.ty;
+        if ((unsigned)(wy + q.w) < ww) {
+          const float ys = (float)wy * q.sx, uy = ys * ys;
+          const float f = frac_turns(fmaf(uy, fmaf(uy, fmaf(uy, q.c3, q.c2), q.c1), q.base_t));
+          float sn, cs;
+          __sincosf(6.28318530717958647692f * f, &sn, &cs);
+          const float amp = q.a0c * fmaf(uy, fmaf(uy, q.beta, q.alpha), 1.f);
+          const float v0 = amp * cs, v1 = amp * sn;
+          const Split4 v = split4(v0, v1, uy * v0, uy * v1);
+          *reinterpret_cast<uint2*>(sAh + off) = make_uint2(v.h01, v.h23);
+          *reinterpret_cast<uint2*>(sAl + off) = make_uint2(v.l01, v.l23);
+        } else {
+          *reinterpret_cast<uint2*>(sAh + off) = make_uint2(0u, 0u);
+          *reinterpret_cast<uint2*>(sAl + off) = make_uint2(0u, 0u);
+        }
       }
-      // B: R1 = i kappa ux R0; row 2x: (R0x, -R0y, R1x, -R1y), row 2x+1:
+      // B: R1 = i kappa ux R0; row x: (R0x, -R0y, R1x, -R1y), row 128 + x:
       // (R0y, R0x, R1y, R1x), from one split by swapping halves and flipping signs
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int wx = XB[m] - q.tx;
-        const bool in = XB[m] < g.nx && (unsigned)(wx + q.w) < (unsigned)(2 * q.w);
-        const float xs = (float)wx * q.sx, ux = xs * xs;
-        const float f = frac_turns(ux * fmaf(ux, fmaf(ux, q.c3, q.c2), q.c1));
-        float sn, cs;
-        __sincosf(6.28318530717958647692f * f, &sn, &cs);
-        const float amp = in ? fmaf(ux, fmaf(ux, q.beta, q.alpha), 1.f) : 0.f;
-        const float r0x = amp * cs, r0y = amp * sn;
-        const float kx = q.kappa * ux;
-        const Split4 v = split4(r0x, r0y, -kx * r0y, kx * r0x);
-        const uint32_t neg_hi = 0x80000000u;               // sign of the second BF16 of a pair
-        *reinterpret_cast<uint2*>(sBh + offB0[m]) = make_uint2(v.h01 ^ neg_hi, v.h23 ^ neg_hi);
-        *reinterpret_cast<uint2*>(sBl + offB0[m]) = make_uint2(v.l01 ^ neg_hi, v.l23 ^ neg_hi);
-        *reinterpret_cast<uint2*>(sBh + offB1[m]) = make_uint2(__byte_perm(v.h01, 0, 0x1032), __byte_perm(v.h23, 0, 0x1032));
-        *reinterpret_cast<uint2*>(sBl + offB1[m]) = make_uint2(__byte_perm(v.l01, 0, 0x1032), __byte_perm(v.l23, 0, 0x1032));
+      for (int m = 0; m < 4; ++m) {
+        const int r = (xs0 + i0 + 32 * m) & 127;
+        const int off = sw_off(r, j);
+        const int wx = X0 + r - q.tx;
+        uint2 h0 = make_uint2(0u, 0u), l0 = h0, h1 = h0, l1 = h0;
+        if ((unsigned)(wx + q.w) < ww) {
+          const float xs = (float)wx * q.sx, ux = xs * xs;
+          const float f = frac_turns(ux * fmaf(ux, fmaf(ux, q.c3, q.c2), q.c1));
+          float sn, cs;
+          __sincosf(6.28318530717958647692f * f, &sn, &cs);
+          const float amp = fmaf(ux, fmaf(ux, q.beta, q.alpha), 1.f);
+          const float r0x = amp * cs, r0y = amp * sn;
+          const float kx = q.kappa * ux;
+          const Split4 v = split4(r0x, r0y, -kx * r0y, kx * r0x);
+          const uint32_t neg_hi = 0x80000000u;             // sign of the second BF16 of a pair
+          h0 = make_uint2(v.h01 ^ neg_hi, v.h23 ^ neg_hi);
+          l0 = make_uint2(v.l01 ^ neg_hi, v.l23 ^ neg_hi);
+          h1 = make_uint2(__byte_perm(v.h01, 0, 0x1032), __byte_perm(v.h23, 0, 0x1032));
+          l1 = make_uint2(__byte_perm(v.l01, 0, 0x1032), __byte_perm(v.l23, 0, 0x1032));
+        }
+        *reinterpret_cast<uint2*>(sBh + off) = h0;
+        *reinterpret_cast<uint2*>(sBl + off) = l0;
+        *reinterpret_cast<uint2*>(sBh + kTile + off) = h1;
+        *reinterpret_cast<uint2*>(sBl + kTile + off) = l1;
       }
       // generic-proxy writes -> visible to the tensor core's async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -723,7 +730,7 @@ __global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpP
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       unsigned char* st0 = base + s * kStageBytes;
       const uint64_t ah = sw_desc(su32(st0)), al = sw_desc(su32(st0 + kTile));
-      const uint64_t bh = sw_desc(su32(st0 + 2 * kTile)), bl = sw_desc(su32(st0 + 3 * kTile));
+      const uint64_t bh = sw_desc(su32(st0 + 2 * kTile)), bl = sw_desc(su32(st0 + 4 * kTile));
 #pragma unroll
       for (int kk = 0; kk < kBK / 16; ++kk) {
         const uint64_t adv = (uint64_t)((kk * 32) >> 4);
@@ -735,32 +742,48 @@ __global__ void __launch_bounds__(tcw::kThreads, 3) wrp_tc(WRPGeom g, const WrpP
     }
     umma_commit(done);                   // arrives when every MMA issued above has completed
   }
-  // epilogue: warps 4-7 own TMEM lanes 32 (warp - 4) .. + 31 = region rows
+  // epilogue: warp w reads TMEM lanes (region rows) 32 (w % 4) .. + 31, pixels
+  // 64 (w / 4) .. + 63 in two halves, turned by way of its shared memory into rows
   __syncwarp();
-  const bool epi = warp >= 4 && warp < 8;
+  const bool epi = warp < kProducerWarps;
   bool ok_done = true;
   if (epi) ok_done = mb_wait(done, 0);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const bool good = __syncthreads_and(ok_done && !*((volatile int*)abort_flag));
   if (good && epi) {
-    const int r = 32 * (warp - 4) + lane;
-    const int Y = Y0 + r;
+    unsigned char* rows = base + warp * 32 * kEpiRow;
+    const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const bool wide = ((reinterpret_cast<uintptr_t>(wrp) | ((uintptr_t)g.nx * sizeof(float2))) & 15) == 0;
 #pragma unroll 1
-    for (int c = 0; c < 2 * kCols / 32; ++c) {
-      uint32_t v[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * (warp - 4)) << 16) + (uint32_t)(c * 32), v);
-      if (Y < g.ny) {
-        float2* dst = wrp + (size_t)Y * g.nx + X0 + 16 * c;
+    for (int c = 0; c < 2; ++c) {
+      const int x0 = 64 * (warp >> 2) + 32 * c;
+      uint32_t re[32], im[32];
+      tmem_ld32(taddr + (uint32_t)x0, re);
+      tmem_ld32(taddr + (uint32_t)(128 + x0), im);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          if (X0 + 16 * c + q < g.nx) {
-            float2 o = dst[q];
-            o.x += __uint_as_float(v[2 * q]);
-            o.y += __uint_as_float(v[2 * q + 1]);
-            dst[q] = o;
-          }
+      for (int q = 0; q < 16; ++q)
+        *reinterpret_cast<uint4*>(rows + lane * kEpiRow + 16 * q) =
+            make_uint4(re[2 * q], im[2 * q], re[2 * q + 1], im[2 * q + 1]);
+      __syncwarp();
+      // two rows per instruction, two pixels per lane
+      const int X = X0 + x0 + 2 * (lane & 15);
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int r = 2 * i + (lane >> 4), Y = Y0 + 32 * (warp & 3) + r;
+        const float4 v = *reinterpret_cast<const float4*>(rows + r * kEpiRow + 16 * (lane & 15));
+        if (Y < 0 || Y >= g.ny) continue;
+        float2* dst = wrp + (size_t)Y * g.nx + X;
+        if (wide && X >= 0 && X + 1 < g.nx) {              // X is even
+          if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f)
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y),
+                         "f"(v.z), "f"(v.w)
+                         : "memory");
+        } else {
+          if (X >= 0 && X < g.nx) { atomicAdd(&dst[0].x, v.x); atomicAdd(&dst[0].y, v.y); }
+          if (X + 1 >= 0 && X + 1 < g.nx) { atomicAdd(&dst[1].x, v.z); atomicAdd(&dst[1].y, v.w); }
         }
       }
+      __syncwarp();
     }
   } else if (!good && threadIdx.x == 0) {
     atomicOr(err, 4);
@@ -862,13 +885,14 @@ oh_status oh_wrp_accumulate(oh_ctx* ctx, oh_precision prec, const oh_wrp_params*
   if (n_points == 0) return OH_OK;
   WRPGeom g{p->nx, p->ny, p->pitch, p->lambda, p->z_wrp, p->window};
   const int tiles_x = (p->nx + kWrpTile - 1) / kWrpTile, tiles_y = (p->ny + kWrpTile - 1) / kWrpTile;
-  const int regions_x = (p->nx + kTcW - 1) / kTcW, regions_y = (p->ny + kTcH - 1) / kTcH;
+  const bool centred = p->window <= kTcR / 4;           // windows of at most half a region: one bin per point
+  const int step = centred ? kTcR - 2 * p->window : kTcR, off = centred ? 2 * p->window : 0;
+  const int regions_x = (p->nx + off - 1) / step + 1, regions_y = (p->ny + off - 1) / step + 1;
   // bins a window touches per axis: direct tiles, tensor regions
   const int span = p->window > 0 ? (2 * p->window + kWrpTile - 1) / kWrpTile + 1 : 0;
-  const int span_rx = p->window > 0 ? (2 * p->window + kTcW - 1) / kTcW + 1 : 0;
-  const int span_ry = p->window > 0 ? (2 * p->window + kTcH - 1) / kTcH + 1 : 0;
+  const int span_r = p->window > 0 && !centred ? (2 * p->window + kTcR - 1) / kTcR + 1 : 1;
   const size_t cap_d = (size_t)std::min(span, tiles_x) * std::min(span, tiles_y);
-  const size_t cap_t = (size_t)std::min(span_rx, regions_x) * std::min(span_ry, regions_y);
+  const size_t cap_t = (size_t)std::min(span_r, regions_x) * std::min(span_r, regions_y);
   const size_t cap = (size_t)n_points * std::max(cap_d, cap_t);
   if (p->window > 0 && p->window < (1 << 28) && cap < (size_t)INT32_MAX) {
     // fixed windows: binned, tiled accumulation; in FP32 the separable points
@@ -897,7 +921,7 @@ oh_status oh_wrp_accumulate(oh_ctx* ctx, oh_precision prec, const oh_wrp_params*
     int* start = (int*)(base + off_start);
     int* cur = (int*)(base + off_cur);
     int* list = (int*)(base + off_list);
-    const WrpBins bins{tiles_x, ntiles, regions_x, use_tc ? 1 : 0};
+    const WrpBins bins{tiles_x, ntiles, regions_x, step, off, use_tc ? 1 : 0};
     if (use_tc)
       OH_CUDA_TRY(cudaFuncSetAttribute(wrp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tcw::kSmemBytes));
     KernelTimer kt(ctx, "wrp_accumulate", st);
@@ -911,7 +935,7 @@ oh_status oh_wrp_accumulate(oh_ctx* ctx, oh_precision prec, const oh_wrp_params*
     OH_LAUNCH_CHECK();
     if (use_tc) {
       KernelTimer kt2(ctx, "wrp_tc", st);
-      wrp_tc<<<nregions, tcw::kThreads, tcw::kSmemBytes, st>>>(g, pts, start + ntiles, list, regions_x,
+      wrp_tc<<<nregions, tcw::kThreads, tcw::kSmemBytes, st>>>(g, pts, start + ntiles, list, bins,
                                                               (float2*)wrp, ctx->dev_err);
       OH_LAUNCH_CHECK();
     }
