@@ -9,10 +9,7 @@
 //   GEMM with M = 128 pixels (a bx x by patch), N = BN output channels,
 //   K = taps x cin in 32-channel steps.  The A tile of a K step is one TMA
 //   load of the 4-D activation map at the tap's offset: out-of-range pixels
-//   read as zero, which is the convolution's zero padding.  When a tile is
-//   128 pixels of one image row, one 136-pixel load of the row at dy (from
-//   x - 1) serves all three dx taps: their A operands start 0, 1 and 2 pixel
-//   rows into it, so each K step of 32 channels loads a third of the input.  s = +1 is the
+//   read as zero, which is the convolution's zero padding.  s = +1 is the
 //   forward convolution; s = -1 with the transposed weight matrix
 //   Wt[ci][tap*cout + co] is the gradient with respect to the input (dgrad).
 //   Epilogue: + bias, ReLU, multiplication by (mask > 0) (the ReLU derivative
@@ -56,23 +53,54 @@ __device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const in
 
 constexpr int pow2_at_least(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
 
-template <int BN, bool HALO = false> struct FwdCfg {
-  // HALO: one 136-pixel row box per (dy, 32 channels) serves the three dx
-  // taps, whose A operands start 0, 1 and 2 pixel rows into it
-  static constexpr int kABox = HALO ? 136 * 64 : 128 * 64;
-  static constexpr int kA = (kABox + 1023) / 1024 * 1024;
-  static constexpr int kBBox = BN * 64;                // BN rows x 32 K
-  static constexpr int kBStride = (kBBox + 1023) / 1024 * 1024;
-  static constexpr int kTapsPerStage = HALO ? 3 : 1;
-  static constexpr int kB = kTapsPerStage * kBStride;
+template <int BN> struct FwdCfg {
+  static constexpr int kA = 128 * 64;                  // 128 pixels x 32 channels
+  static constexpr int kB = BN * 64;                   // BN rows x 32 K
   static constexpr int kStage = kA + kB;
-  static constexpr int kStagesRaw = (BN <= 64 ? 80 : 200) * 1024 / kStage;
-  static constexpr int kStages = HALO ? (kStagesRaw < 2 ? 2 : kStagesRaw > 6 ? 6 : kStagesRaw) : (BN >= 192 ? 5 : 6);
+  static constexpr int kStages = BN >= 192 ? 5 : 6;
   static constexpr int kTmemBuf = pow2_at_least(BN);  // columns of one accumulator
   static constexpr int kTmem = 2 * kTmemBuf;          // two accumulators: MMA and epilogue overlap
   static constexpr int kThreads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
   static constexpr int kSmem = kStages * kStage + 1024 + 256;
 };
+
+// 32 output channels cb.. of pixel pix from the accumulator's columns r: bias,
+// ReLU, mask, BF16 store.
+__device__ __forceinline__ void conv_store32(const ConvArgs& a, const uint32_t* r, const float* bias, size_t pix,
+                                             int cb) {
+  float v[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+#pragma unroll
+  for (int e = 0; e < 32; ++e) v[e] += bias[e];
+  if (a.relu) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = fmaxf(v[e], 0.f);
+  }
+  if (a.mask) {
+    const uint4* mp = reinterpret_cast<const uint4*>(a.mask + pix * a.mask_cs + cb);
+#pragma unroll
+    for (int g4 = 0; g4 < 4; ++g4) {
+      const uint4 mv = __ldg(mp + g4);
+      const __nv_bfloat162* mb = reinterpret_cast<const __nv_bfloat162*>(&mv);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(mb[e]);
+        if (!(f.x > 0.f)) v[g4 * 8 + 2 * e] = 0.f;
+        if (!(f.y > 0.f)) v[g4 * 8 + 2 * e + 1] = 0.f;
+      }
+    }
+  }
+  uint4* op = reinterpret_cast<uint4*>(a.out + pix * a.out_cs + cb);
+#pragma unroll
+  for (int g4 = 0; g4 < 4; ++g4) {
+    uint4 o;
+    __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ob[e] = __floats2bfloat162_rn(v[g4 * 8 + 2 * e], v[g4 * 8 + 2 * e + 1]);
+    op[g4] = o;
+  }
+}
 
 // Persistent CTAs: CTA i takes pixel tiles i, i + gridDim.x, ... of output
 // channel tile blockIdx.y.  The TMA producer streams the K steps of all its
@@ -80,11 +108,11 @@ template <int BN, bool HALO = false> struct FwdCfg {
 // TMEM buffer j & 1 and commits it to the epilogue warps, which drain it
 // (bias, ReLU, mask, BF16 store) while the next tile accumulates in the
 // other buffer.
-template <int BN, bool HALO>
-__global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const __grid_constant__ CUtensorMap mX,
-                                                                          const __grid_constant__ CUtensorMap mW,
-                                                                          ConvArgs a) {
-  typedef FwdCfg<BN, HALO> Cfg;
+template <int BN>
+__global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid_constant__ CUtensorMap mX,
+                                                                    const __grid_constant__ CUtensorMap mW,
+                                                                    ConvArgs a) {
+  typedef FwdCfg<BN> Cfg;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = tc::su32(smem_raw);
   unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -103,7 +131,7 @@ __global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const 
   const int ntl = blockIdx.x < tiles ? (int)((tiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
   const int co0 = blockIdx.y * BN;
   const int cchunks = a.cin >> 5;
-  const int nk = (HALO ? 3 : a.taps) * cchunks;
+  const int nk = a.taps * cchunks;
   const long long nsteps = (long long)ntl * nk;
 
   if (threadIdx.x == 0) {
@@ -146,25 +174,12 @@ __global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const 
             break;
           }
           unsigned char* st = base + s * Cfg::kStage;
-          if constexpr (HALO) {
-            // row y0 + dy' from x0 - 1: the dx' = -1, 0, +1 taps start 0, 1, 2 rows in
-            const int dyi = it / cchunks, cc = it - dyi * cchunks;
-            const int dyp = dyi - 1;
-            tc::mb_expect_tx(&full[s], (uint32_t)(Cfg::kABox + 3 * Cfg::kBBox));
-            tc::tma_load_4d(st, &mX, cc * 32, x0 - 1, y0 + dyp, img, &full[s]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              const int tap = 3 * (1 + a.sign * dyp) + (1 + a.sign * (j - 1));
-              tc::tma_load_2d(st + Cfg::kA + j * Cfg::kBStride, &mW, tap * a.cin + cc * 32, co0, &full[s]);
-            }
-          } else {
-            const int tap = it / cchunks, cc = it - tap * cchunks;
-            int dx = 0, dy = 0;
-            if (a.taps == 9) { dx = (tap % 3 - 1) * a.sign; dy = (tap / 3 - 1) * a.sign; }
-            tc::mb_expect_tx(&full[s], (uint32_t)Cfg::kStage);
-            tc::tma_load_4d(st, &mX, cc * 32, x0 + dx, y0 + dy, img, &full[s]);
-            tc::tma_load_2d(st + Cfg::kA, &mW, tap * a.cin + cc * 32, co0, &full[s]);
-          }
+          const int tap = it / cchunks, cc = it - tap * cchunks;
+          int dx = 0, dy = 0;
+          if (a.taps == 9) { dx = (tap % 3 - 1) * a.sign; dy = (tap / 3 - 1) * a.sign; }
+          tc::mb_expect_tx(&full[s], (uint32_t)Cfg::kStage);
+          tc::tma_load_4d(st, &mX, cc * 32, x0 + dx, y0 + dy, img, &full[s]);
+          tc::tma_load_2d(st + Cfg::kA, &mW, tap * a.cin + cc * 32, co0, &full[s]);
         }
       }
       if (g >= 0) *issued = (int)nsteps;
@@ -196,19 +211,11 @@ __global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const 
           }
           tc::fence_after();
           const uint32_t sa = tc::su32(base + s * Cfg::kStage);
+          const uint64_t da = tc::desc_sw64(sa, 16, 512), db = tc::desc_sw64(sa + Cfg::kA, 16, 512);
 #pragma unroll
-          for (int j = 0; j < Cfg::kTapsPerStage; ++j) {
-            // HALO: tap dx' = j - 1 starts j pixel rows (64 bytes each) into the
-            // row box; the swizzle follows the absolute shared-memory address,
-            // which the TMA write and the MMA read share, so the start address
-            // simply moves (matrix base offset 0)
-            const uint64_t da = tc::desc_sw64(sa + (HALO ? j * 64 : 0), 16, 512);
-            const uint64_t db = tc::desc_sw64(sa + Cfg::kA + j * Cfg::kBStride, 16, 512);
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-              const uint64_t adv = (uint64_t)((kk * 32) >> 4);      // 16 BF16 = 32 bytes along K
-              tc::umma_bf16(acc, da + adv, db + adv, idesc, (it | j | kk) ? 1u : 0u);
-            }
+          for (int kk = 0; kk < 2; ++kk) {
+            const uint64_t adv = (uint64_t)((kk * 32) >> 4);        // 16 BF16 = 32 bytes along K
+            tc::umma_bf16(acc, da + adv, db + adv, idesc, (it | kk) ? 1u : 0u);
           }
           tc::umma_commit(&empty[s]);
         }
@@ -239,38 +246,7 @@ __global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const 
         tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * Cfg::kTmemBuf + c * 32), r);
         const int cb = co0 + c * 32;
         if (!inside || cb >= a.cout) continue;
-        float v[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) v[e] += sbias[c * 32 + e];
-        if (a.relu) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = fmaxf(v[e], 0.f);
-        }
-        if (a.mask) {
-          const uint4* mp = reinterpret_cast<const uint4*>(a.mask + pix * a.mask_cs + cb);
-#pragma unroll
-          for (int g4 = 0; g4 < 4; ++g4) {
-            const uint4 mv = __ldg(mp + g4);
-            const __nv_bfloat162* mb = reinterpret_cast<const __nv_bfloat162*>(&mv);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 f = __bfloat1622float2(mb[e]);
-              if (!(f.x > 0.f)) v[g4 * 8 + 2 * e] = 0.f;
-              if (!(f.y > 0.f)) v[g4 * 8 + 2 * e + 1] = 0.f;
-            }
-          }
-        }
-        uint4* op = reinterpret_cast<uint4*>(a.out + pix * a.out_cs + cb);
-#pragma unroll
-        for (int g4 = 0; g4 < 4; ++g4) {
-          uint4 o;
-          __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) ob[e] = __floats2bfloat162_rn(v[g4 * 8 + 2 * e], v[g4 * 8 + 2 * e + 1]);
-          op[g4] = o;
-        }
+        conv_store32(a, r, sbias + c * 32, pix, cb);
       }
       tc::fence_before();
       __syncwarp();
@@ -292,6 +268,314 @@ __global__ void __launch_bounds__(FwdCfg<BN, HALO>::kThreads) conv_fwd_tc(const 
   if (warp == 1) {
     tc::fence_after();
     tc::tmem_dealloc(tmem, Cfg::kTmem);
+  }
+}
+
+// 3x3 over whole 128-pixel rows: a tile is 128 pixels of `rows` consecutive output
+// rows (an accumulator each).  The weights of a (dy, 32 channels) step are loaded
+// once for the tile's rows; a row's 136-pixel box of input row y + dy (from x - 1)
+// serves the three dx taps (A operands that start 0, 1 and 2 pixels into it).  An
+// output sums over dy, then channels, then dx, whatever the tile.
+//
+// What bounds it: an MMA of N channels takes max(N / 2, 32 + N / 4) clocks (the
+// tensor rate; its operands from shared memory at 128 bytes a clock), but one warp
+// that waits for a box, issues six and commits needs about 90 to 120 for each, and
+// one that waits for a slot and loads a box about 500.  So up to four warps load
+// boxes, a fifth the weights, and up to four issue, each for its own output rows.
+// 4 x 512 x 512 pixels, 192 -> 64 channels: 188 us (470 with one warp each), where
+// the MMAs take 150 to 180 at the clocks of such a load.
+//
+// A barrier's parity tells its last two phases apart only to a warp that waits for
+// every one of them: loader w fills issuer w's own slots, and every issuer waits
+// for every weight step.
+//
+// Warps 0-4 TMA, warps 5-8 MMA, warps 9-16 epilogue; one CTA per SM takes tiles
+// blockIdx.x, + gridDim.x, ... of channel tile blockIdx.y.
+struct RowsCfg {
+  int rows, nbuf;                      // output rows per tile (1, 2 or a multiple of 4), accumulator sets (2: MMAs
+                                       // and epilogue overlap)
+  int na;                              // box slots, a multiple of the issuers
+  uint32_t tmem_cols;
+};
+constexpr int kRowsA = 136 * 64, kRowsAStride = (kRowsA + 1023) / 1024 * 1024;
+constexpr int kRowsLoaders = 4, kRowsIssuers = 4, kRowsEpiWarps = 8;
+constexpr int kRowsIssue0 = kRowsLoaders + 1, kRowsEpi0 = kRowsIssue0 + kRowsIssuers;       // first warp of each role
+constexpr int kRowsThreads = 32 * (kRowsEpi0 + kRowsEpiWarps);
+constexpr int kRowsA_Slots = 16, kRowsB_Slots = 3;
+constexpr int kRowsFixed = 1024 + kRowsEpiWarps * 2048 + (2 * kRowsA_Slots + 2 * kRowsB_Slots + 8) * 8 +
+                           (kRowsA_Slots + kRowsB_Slots) * 4 + 64;
+
+template <int BN>
+__global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_constant__ CUtensorMap mX,
+                                                                 const __grid_constant__ CUtensorMap mW, ConvArgs a,
+                                                                 RowsCfg rc) {
+  constexpr int kTap = BN * 64, kB = 3 * kTap;
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t raw = tc::su32(smem_raw);
+  unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  unsigned char* sB = base + (size_t)rc.na * kRowsAStride;
+  unsigned char* sE = sB + kRowsB_Slots * kB;           // 2 KB per epilogue warp
+  uint64_t* fullA = reinterpret_cast<uint64_t*>(sE + kRowsEpiWarps * 2048);
+  uint64_t* emptyA = fullA + kRowsA_Slots;
+  uint64_t* fullB = emptyA + kRowsA_Slots;
+  uint64_t* emptyB = fullB + kRowsB_Slots;
+  uint64_t* tfull = emptyB + kRowsB_Slots;             // [2] accumulators ready (MMA commit)
+  uint64_t* tempty = tfull + 2;                        // [2] accumulators drained (epilogue warps)
+  uint64_t* done = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+  int* usesA = abort_flag + 1;                         // loads issued per slot
+  int* usesB = usesA + kRowsA_Slots;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  const int tiles_r = (a.h + rc.rows - 1) / rc.rows;
+  const long long tiles = (long long)a.n * tiles_r * a.tiles_x;
+  const int ntl = blockIdx.x < tiles ? (int)((tiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+  const int co0 = blockIdx.y * BN;
+  const int cchunks = a.cin >> 5;
+  const int ni = min(rc.rows, kRowsIssuers);           // issuing warps (1, 2 or 4): row r belongs to the r % ni-th
+  const int own = rc.na / ni;                          // box slots per issuer
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < rc.na; ++s) { tc::mb_init(&fullA[s], 1); tc::mb_init(&emptyA[s], 1); }
+    for (int s = 0; s < kRowsB_Slots; ++s) { tc::mb_init(&fullB[s], 1); tc::mb_init(&emptyB[s], ni); }
+    for (int b = 0; b < 2; ++b) { tc::mb_init(&tfull[b], ni); tc::mb_init(&tempty[b], kRowsEpiWarps); }
+    tc::mb_init(done, ni);
+    *abort_flag = 0;
+    for (int i = 0; i < kRowsA_Slots + kRowsB_Slots; ++i) usesA[i] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __shared__ float sbias[BN];
+  for (int c = threadIdx.x; c < BN; c += blockDim.x)
+    sbias[c] = (a.bias && co0 + c < a.cout) ? a.bias[co0 + c] : 0.f;
+  if (warp == kRowsIssue0) tc::tmem_alloc(tmem_slot, rc.tmem_cols);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  // tile j of this CTA: image, first pixel, first row, rows inside the image
+  auto tile_origin = [&](int j, int* img, int* x0, int* y0) -> int {
+    uint32_t t = blockIdx.x + (uint32_t)j * gridDim.x;         // (tiles < 2^31)
+    const uint32_t u = t / (uint32_t)a.tiles_x;
+    *x0 = (int)(t - u * (uint32_t)a.tiles_x) * 128;
+    *img = (int)(u / (uint32_t)tiles_r);
+    *y0 = (int)(u - (uint32_t)*img * (uint32_t)tiles_r) * rc.rows;
+    return min(rc.rows, a.h - *y0);
+  };
+  // a ring position: slot and the parity of its current use
+  struct Ring {
+    int s, n;
+    uint32_t ph;
+    __device__ __forceinline__ void next() { if (++s == n) { s = 0; ph ^= 1u; } }
+  };
+
+  // waits with the whole warp (converged control flow: a ring's addresses and the
+  // descriptors stay in uniform registers)
+  auto wait_warp = [&](uint64_t* bar, uint32_t ph) -> bool {
+    return __all_sync(0xffffffffu, tc::mb_try(bar, ph)) || __all_sync(0xffffffffu, wait_live(bar, ph, abort_flag));
+  };
+
+  if (warp <= kRowsLoaders) {
+    const bool el = tc::elect_one();
+    Ring ra{0, own, 0}, rb{0, kRowsB_Slots, 0};
+    auto load_b = [&](int dyi, int cc) -> bool {
+      if (!wait_warp(&emptyB[rb.s], rb.ph ^ 1u)) return false;
+      if (el) {
+        unsigned char* st = sB + (size_t)rb.s * kB;
+        usesB[rb.s] += 1;
+        tc::mb_expect_tx(&fullB[rb.s], (uint32_t)kB);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int tap = 3 * (1 + a.sign * (dyi - 1)) + (1 + a.sign * (j - 1));
+          tc::tma_load_2d(st + j * kTap, &mW, tap * a.cin + cc * 32, co0, &fullB[rb.s]);
+        }
+      }
+      return true;
+    };
+    auto load_a = [&](int slot, int cc, int x0, int y, int img) -> bool {
+      if (!wait_warp(&emptyA[slot], ra.ph ^ 1u)) return false;
+      if (el) {
+        usesA[slot] += 1;
+        tc::mb_expect_tx(&fullA[slot], (uint32_t)kRowsA);
+        tc::tma_load_4d(base + (size_t)slot * kRowsAStride, &mX, cc * 32, x0 - 1, y, img, &fullA[slot]);
+      }
+      return true;
+    };
+    bool ok = true;
+    for (int j = 0; j < ntl && ok; ++j) {
+      int img, x0, y0;
+      const int nr = tile_origin(j, &img, &x0, &y0);
+      for (int dyi = 0; dyi < 3 && ok; ++dyi)
+        for (int cc = 0; cc < cchunks && ok; ++cc) {
+          if (warp == kRowsLoaders) {
+            ok = load_b(dyi, cc);
+            rb.next();
+          } else if (warp < ni) {
+            for (int r = warp; r < nr && ok; r += ni) {
+              ok = load_a(warp * own + ra.s, cc, x0, y0 + r + dyi - 1, img);
+              ra.next();
+            }
+          }
+        }
+    }
+    if (!ok && lane == 0) atomicExch(abort_flag, 1);
+  } else if (warp < kRowsIssue0 + ni) {
+    constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
+    const int w = warp - kRowsIssue0;
+    const bool el = tc::elect_one();
+    Ring ra{0, own, 0}, rb{0, kRowsB_Slots, 0};
+    bool ok = true;
+    if (a.stall_flag) ok = __all_sync(0xffffffffu, stall_on_unset_flag(a.stall_flag, a.stall_cycles));
+    // the three dx taps of one box into one output row's accumulator; the swizzle
+    // follows the absolute shared-memory address, which the TMA write and the MMA
+    // read share, so a tap's start address simply moves by whole pixels
+    auto taps = [&](uint32_t acc, uint32_t sa, uint32_t sb, bool first) {
+      const uint64_t da = tc::desc_sw64(sa, 16, 512), db = tc::desc_sw64(sb, 16, 512);
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk)                          // 16 BF16 = 32 bytes along K
+          if (el)
+            tc::umma_bf16(acc, da + (uint64_t)((j * 64 + kk * 32) >> 4), db + (uint64_t)((j * kTap + kk * 32) >> 4),
+                          idesc, (j | kk) ? 1u : first ? 0u : 1u);
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (el) tc::umma_commit(bar);
+    };
+    auto wait_full = [&](uint64_t* bar, uint32_t ph) -> bool {
+      if (!wait_warp(bar, ph)) return false;
+      tc::fence_after();
+      return true;
+    };
+    const uint32_t sA = tc::su32(base), sBb = tc::su32(sB);
+    for (int j = 0; j < ntl && ok; ++j) {
+      const int b = rc.nbuf == 2 ? j & 1 : 0;
+      const int use = rc.nbuf == 2 ? j >> 1 : j;
+      if (!(ok = wait_full(&tempty[b], (uint32_t)((use & 1) ^ 1)))) break;
+      const uint32_t acc = tmem + (uint32_t)(b * rc.rows * BN);
+      int img, x0, y0;
+      const int nr = tile_origin(j, &img, &x0, &y0);
+      for (int dyi = 0; dyi < 3 && ok; ++dyi)
+        for (int cc = 0; cc < cchunks && ok; ++cc) {
+          if (!(ok = wait_full(&fullB[rb.s], rb.ph))) break;
+          for (int r = w; r < nr; r += ni) {
+            const int slot = w * own + ra.s;
+            if (!(ok = wait_full(&fullA[slot], ra.ph))) break;
+            taps(acc + (uint32_t)(r * BN), sA + (uint32_t)slot * kRowsAStride, sBb + (uint32_t)rb.s * kB,
+                 dyi == 0 && cc == 0);
+            commit(&emptyA[slot]);
+            ra.next();
+          }
+          commit(&emptyB[rb.s]);
+          rb.next();
+        }
+      if (ok) commit(&tfull[b]);
+    }
+    if (!ok && lane == 0) atomicExch(abort_flag, 1);
+    commit(done);                                        // arrives when every MMA issued above has completed
+  } else if (warp >= kRowsEpi0) {
+    // epilogue: TMEM lane quarter (warp % 4) = pixels 32 (warp % 4) .. + 31 of each
+    // row; two warps per quarter share the rows' 32-channel blocks.  A block goes by
+    // way of shared memory (64 bytes a pixel, chunks swizzled), so that four lanes
+    // store a pixel's 64 bytes and read its mask; the mask's loads run a block ahead.
+    const int q = warp & 3, half = (warp - kRowsEpi0) >> 2;
+    unsigned char* stage = sE + (warp - kRowsEpi0) * 2048;
+    const int pc = lane & 3, pr = lane >> 2;
+    for (int j = 0; j < ntl; ++j) {
+      const int b = rc.nbuf == 2 ? j & 1 : 0;
+      const int use = rc.nbuf == 2 ? j >> 1 : j;
+      int img, x0, y0;
+      const int nr = tile_origin(j, &img, &x0, &y0);
+      const int nblk = nr * (BN / 32), xq = x0 + 32 * q + pr;
+      const size_t row0 = ((size_t)img * a.h + y0) * a.w;
+      auto load_mask = [&](int k, uint4* mv) {
+        if (!a.mask || k >= nblk) return;
+        const __nv_bfloat16* mp = a.mask + (row0 + (size_t)(k / (BN / 32)) * a.w + xq) * a.mask_cs + co0 +
+                                  k % (BN / 32) * 32 + 8 * pc;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (xq + 8 * i < a.w) mv[i] = __ldg(reinterpret_cast<const uint4*>(mp + (size_t)(8 * i) * a.mask_cs));
+      };
+      if (a.mask && j + 1 < ntl) {                       // the next tile's mask into L2
+        int img1, x1, y1;
+        const int nblk1 = tile_origin(j + 1, &img1, &x1, &y1) * (BN / 32);
+        const int xp = x1 + 32 * q + pr;
+        const __nv_bfloat16* mp = a.mask + (((size_t)img1 * a.h + y1) * a.w + xp) * a.mask_cs + co0 + 8 * pc;
+        for (int k = half; k < nblk1; k += 2)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (!(pc & 1) && xp + 8 * i < a.w)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                  mp + ((size_t)(k / (BN / 32)) * a.w + 8 * i) * a.mask_cs + k % (BN / 32) * 32));
+      }
+      uint4 mv[4], mn[4];
+      load_mask(half, mv);
+      bool ok = true;
+      if (lane == 0) ok = wait_live(&tfull[b], (uint32_t)(use & 1), abort_flag);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) break;
+      tc::fence_after();
+#pragma unroll 1
+      for (int k = half; k < nblk; k += 2) {
+        const int r = k / (BN / 32), c = k % (BN / 32);
+        load_mask(k + 2, mn);
+        uint32_t v[32];
+        tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((b * rc.rows + r) * BN + c * 32), v);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 o;
+          __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int n = g * 8 + 2 * e;
+            float f0 = __uint_as_float(v[n]) + sbias[c * 32 + n], f1 = __uint_as_float(v[n + 1]) + sbias[c * 32 + n + 1];
+            if (a.relu) { f0 = fmaxf(f0, 0.f); f1 = fmaxf(f1, 0.f); }
+            ob[e] = __floats2bfloat162_rn(f0, f1);
+          }
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4)) = o;
+        }
+        __syncwarp();
+        __nv_bfloat16* op = a.out + (row0 + (size_t)r * a.w + xq) * a.out_cs + co0 + c * 32 + 8 * pc;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int p = 8 * i + pr;
+          uint4 o = *reinterpret_cast<const uint4*>(stage + p * 64 + ((pc ^ ((p >> 1) & 3)) << 4));
+          if (a.mask) {
+            const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
+            const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mv[i]);
+            uint32_t* o2 = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o2[e] &= __hgt2_mask(m2[e], z);
+            mv[i] = mn[i];
+          }
+          if (xq + 8 * i < a.w) *reinterpret_cast<uint4*>(op + (size_t)(8 * i) * a.out_cs) = o;
+        }
+        __syncwarp();
+      }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::su32(&tempty[b])) : "memory");
+    }
+  }
+  __syncwarp();
+  // every MMA issued has completed before TMEM is freed; copies issued but
+  // not consumed land before the CTA exits
+  if (threadIdx.x == 0) tc::mb_wait(done, 0, kWaitCycles);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (*((volatile int*)abort_flag)) atomicOr(a.err, 2);
+    // (each slot's last use; the earlier ones were consumed)
+    for (int i = 0; i < rc.na; ++i)
+      if (usesA[i]) tc::mb_wait(&fullA[i], (uint32_t)((usesA[i] - 1) & 1), kWaitCycles);
+    for (int i = 0; i < kRowsB_Slots; ++i)
+      if (usesB[i]) tc::mb_wait(&fullB[i], (uint32_t)((usesB[i] - 1) & 1), kWaitCycles);
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == kRowsIssue0) {
+    tc::fence_after();
+    tc::tmem_dealloc(tmem, rc.tmem_cols);
   }
 }
 
@@ -608,10 +892,10 @@ bool patch_shape(int w, int pixels, int* bx, int* by) {
   return true;
 }
 
-template <int BN, bool HALO>
+template <int BN>
 oh_status launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArgs& a, long long tiles, cudaStream_t st) {
-  typedef FwdCfg<BN, HALO> Cfg;
-  OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_tc<BN, HALO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  typedef FwdCfg<BN> Cfg;
+  OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   // persistent grid: the CTAs that fit on an SM by shared memory and tensor
   // memory (512 columns), at most four, times the SMs, spread over the
   // output-channel tiles
@@ -620,7 +904,59 @@ oh_status launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArg
   const int ctiles = (a.cout + BN - 1) / BN;
   const long long want = std::max(1LL, (long long)sm_count() * per_sm / ctiles);
   const int gx = (int)std::min(tiles, want);
-  conv_fwd_tc<BN, HALO><<<dim3(gx, ctiles), Cfg::kThreads, Cfg::kSmem, st>>>(mX, mW, a);
+  conv_fwd_tc<BN><<<dim3(gx, ctiles), Cfg::kThreads, Cfg::kSmem, st>>>(mX, mW, a);
+  OH_LAUNCH_CHECK();
+  return OH_OK;
+}
+
+// The row kernel's channel tile and rows per tile for a layer: the least estimated
+// clocks of a CTA, from the MMAs' clocks (see conv_fwd_rows; 120 from one issuer), 40
+// bytes a clock of loads, and 1000 clocks per warp and block of the epilogue.
+// Measured, 4 x 512 x 512 pixels, 192 -> 64 channels: 188 us with tiles of 4 rows and
+// two accumulator sets, 211 with 8 rows and one, 288 with 2 rows; 64 -> 192: 242 us
+// with channel tiles of 96 and 2 rows, 257 with 64 and 4, 284 with 192 and 2.
+struct RowsPlan {
+  RowsCfg c;
+  int bn, smem;
+};
+RowsPlan rows_plan(const ConvArgs& a) {
+  RowsPlan best{};
+  double best_t = 0.0;
+  const double cchunks = a.cin / 32;
+  const int budget = 226 * 1024 - kRowsFixed;            // (1 KB for the biases)
+  for (int bn : {32, 64, 96, 128, 192, 256}) {
+    if (a.cout % bn) continue;
+    const int step = 3 * bn * 64;                        // weights of one (dy, 32 channels)
+    const int gx = std::max(1, sm_count() / (a.cout / bn));
+    for (int rows = 1; rows <= 16 && rows * bn <= 512; rows *= 2) {
+      const long long tiles = (long long)a.n * ((a.h + rows - 1) / rows) * a.tiles_x;
+      const double waves = (double)((tiles + gx - 1) / gx);
+      const int ni = std::min(rows, kRowsIssuers), nbuf = 2 * rows * bn <= 512 ? 2 : 1;
+      const int na = std::min(kRowsA_Slots, (budget - kRowsB_Slots * step) / kRowsAStride) / ni * ni;
+      if (na < std::max(ni, 4)) continue;
+      const double mma = std::max({bn / 2.0, 32.0 + bn / 4.0, 120.0 / ni});
+      const double epi = (rows * (bn / 32) + 1) / 2 * 1000.0;
+      const double calc = cchunks * std::max(rows * 18.0 * mma, 3.0 * (rows * kRowsA + step) / 40.0);
+      const double t = waves * ((nbuf == 2 ? std::max(calc, epi) : calc + epi) + 300.0) + (nbuf == 2 ? epi : 0.0);
+      if (best.bn == 0 || t < best_t) {
+        best_t = t;
+        best.bn = bn;
+        best.smem = na * kRowsAStride + kRowsB_Slots * step + kRowsFixed;
+        best.c = RowsCfg{rows, nbuf, na, (uint32_t)pow2_at_least(nbuf * rows * bn)};
+      }
+    }
+  }
+  return best;
+}
+
+template <int BN>
+oh_status launch_rows(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArgs& a, const RowsPlan& p,
+                      cudaStream_t st) {
+  OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_rows<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+  const int ctiles = a.cout / BN;
+  const long long tiles = (long long)a.n * ((a.h + p.c.rows - 1) / p.c.rows) * a.tiles_x;
+  const int gx = (int)std::min(tiles, (long long)std::max(1, sm_count() / ctiles));
+  conv_fwd_rows<BN><<<dim3(gx, ctiles), kRowsThreads, p.smem, st>>>(mX, mW, a, p.c);
   OH_LAUNCH_CHECK();
   return OH_OK;
 }
@@ -669,6 +1005,23 @@ oh_status conv_enqueue(oh_ctx* ctx, const ConvDesc& d, cudaStream_t st, const ch
   if (ctx->stall_mask & kStallConvolution) { a.stall_flag = ctx->dev_err + 1; a.stall_cycles = ctx->stall_cycles; }
   const long long tiles = (long long)a.tiles_x * a.tiles_y * d.n;
   if (tiles > 0x7fffffffLL) return fail(OH_ERR_UNSUPPORTED_SIZE, "convolution: too many pixel tiles");
+  CUtensorMap mX, mW;
+  // 3x3 over whole 128-pixel rows
+  const char* hv = std::getenv("OH_CONV_HALO");
+  if (d.taps == 9 && a.by == 1 && a.bx == 128 && !(hv && std::atoi(hv) == 0)) {
+    const RowsPlan p = rows_plan(a);
+    OH_TRY(tc::map_act4d(&mX, d.x, d.cin, d.x_cs, d.w, d.h, d.n, 136, 1));
+    OH_TRY(tc::map_mat2d(&mW, d.w_mat, d.taps * d.cin, d.cout, p.bn));
+    KernelTimer kt(ctx, timer_name, st);
+    switch (p.bn) {
+      case 32: return launch_rows<32>(mX, mW, a, p, st);
+      case 64: return launch_rows<64>(mX, mW, a, p, st);
+      case 96: return launch_rows<96>(mX, mW, a, p, st);
+      case 128: return launch_rows<128>(mX, mW, a, p, st);
+      case 192: return launch_rows<192>(mX, mW, a, p, st);
+      default: return launch_rows<256>(mX, mW, a, p, st);
+    }
+  }
   // output-channel tile: all of cout up to 256 (384 as two halves), else the
   // largest of 256, 192, 128, 96, 64, 32 that divides it; halved while the
   // pixel tiles alone cannot fill two CTAs per SM
@@ -677,20 +1030,16 @@ oh_status conv_enqueue(oh_ctx* ctx, const ConvDesc& d, cudaStream_t st, const ch
     if (d.cout % c == 0) { bn = c; break; }
   while ((bn == 256 || bn == 128 || bn == 64 || bn == 192) && tiles * ((d.cout + bn - 1) / bn) < 2LL * sm_count())
     bn /= 2;
-  // 3x3 over whole 128-pixel rows: one halo row box per (dy, 32 channels)
-  const char* hv = std::getenv("OH_CONV_HALO");
-  const bool halo = d.taps == 9 && a.by == 1 && a.bx == 128 && !(hv && std::atoi(hv) == 0);
-  CUtensorMap mX, mW;
-  OH_TRY(tc::map_act4d(&mX, d.x, d.cin, d.x_cs, d.w, d.h, d.n, halo ? 136 : a.bx, a.by));
+  OH_TRY(tc::map_act4d(&mX, d.x, d.cin, d.x_cs, d.w, d.h, d.n, a.bx, a.by));
   OH_TRY(tc::map_mat2d(&mW, d.w_mat, d.taps * d.cin, d.cout, bn));
   KernelTimer kt(ctx, timer_name, st);
   switch (bn) {
-    case 32: return halo ? launch_fwd<32, true>(mX, mW, a, tiles, st) : launch_fwd<32, false>(mX, mW, a, tiles, st);
-    case 64: return halo ? launch_fwd<64, true>(mX, mW, a, tiles, st) : launch_fwd<64, false>(mX, mW, a, tiles, st);
-    case 96: return halo ? launch_fwd<96, true>(mX, mW, a, tiles, st) : launch_fwd<96, false>(mX, mW, a, tiles, st);
-    case 128: return halo ? launch_fwd<128, true>(mX, mW, a, tiles, st) : launch_fwd<128, false>(mX, mW, a, tiles, st);
-    case 192: return halo ? launch_fwd<192, true>(mX, mW, a, tiles, st) : launch_fwd<192, false>(mX, mW, a, tiles, st);
-    default: return halo ? launch_fwd<256, true>(mX, mW, a, tiles, st) : launch_fwd<256, false>(mX, mW, a, tiles, st);
+    case 32: return launch_fwd<32>(mX, mW, a, tiles, st);
+    case 64: return launch_fwd<64>(mX, mW, a, tiles, st);
+    case 96: return launch_fwd<96>(mX, mW, a, tiles, st);
+    case 128: return launch_fwd<128>(mX, mW, a, tiles, st);
+    case 192: return launch_fwd<192>(mX, mW, a, tiles, st);
+    default: return launch_fwd<256>(mX, mW, a, tiles, st);
   }
 }
 
