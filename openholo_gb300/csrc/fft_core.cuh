@@ -19,7 +19,9 @@
 
 namespace oh {
 
-constexpr int kMaxStages = 16;
+// (a line in shared memory needs at most six: 5^6; the batch kernel keeps two plans
+// per frame in shared memory)
+constexpr int kMaxStages = 8;
 constexpr int kMaxGenericRadix = 64;
 
 // A plan's line is stored with one pad element after every padr elements when
