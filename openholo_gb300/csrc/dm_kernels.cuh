@@ -320,10 +320,11 @@ __device__ __forceinline__ void dm_row_body(const DMArgs<R>& a, int blk) {
   typedef typename cplx_of<R>::type C;
   static_assert(512 % NT == 0, "row pass: 512 thread slots over NT threads");
   extern __shared__ unsigned char smem_raw[];
-  const int Px = a.Px, pnx = a.pnx;
+  static_assert(NX > 0, "other lengths run dm_row_gen");
+  constexpr int Px = NX;
+  const int pnx = a.pnx;
   const int lip = (pnx + 7) & ~7;                       // keeps 16-byte alignment
   typedef RowPad<NX> RP;
-  static_assert(NX > 0, "other lengths run dm_row_gen");
   constexpr int lsmax = RP::LSMAX;
   C* buf = reinterpret_cast<C*>(smem_raw);              // [2][lsmax]
   C* v = buf + 2 * lsmax;                               // [2][pnx] source values
