@@ -21,9 +21,9 @@
 //   64-pixel steps; both operands are MN-major (channels contiguous), K split
 //   across CTAs, partial sums added with vector reductions.
 //
-// Roles (128 threads): thread 0 issues TMA loads into a ring of stages,
-// thread 32 issues tcgen05.mma and releases stages with tcgen05.commit, all
-// four warps read the accumulator (warp w owns TMEM lanes 32w..32w+31).  Every
+// Roles: one or more warps issue TMA loads into a ring of stages, one or more
+// issue tcgen05.mma and release stages with tcgen05.commit, four or eight read the
+// accumulators (warp w TMEM lanes 32 (w % 4) .. + 31).  Every
 // mbarrier wait gives up after about one second of SM clock: the CTA then
 // sets the device error word, lets its copies and MMAs land, frees TMEM and
 // returns.  Pipeline waits (a stage's copies, a stage's release) also give
@@ -51,16 +51,28 @@ __device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const in
   return true;
 }
 
+// Waits for the copies of each stage's last use, which two loaders arrive on
+// (uses[2][n]: loads issued): after an abort one may be a use ahead of the other,
+// whose arrival is made up here.
+__device__ __forceinline__ void land_pairs(uint64_t* full, const int* uses, int n) {
+  for (int i = 0; i < n; ++i) {
+    const int u = uses[i], v = uses[n + i];
+    if (u != v) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::su32(&full[i])) : "memory");
+    if (max(u, v)) tc::mb_wait(&full[i], (uint32_t)((max(u, v) - 1) & 1), kWaitCycles);
+  }
+}
+
 constexpr int pow2_at_least(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
 
 template <int BN> struct FwdCfg {
   static constexpr int kA = 128 * 64;                  // 128 pixels x 32 channels
   static constexpr int kB = BN * 64;                   // BN rows x 32 K
-  static constexpr int kStage = kA + kB;
-  static constexpr int kStages = BN >= 192 ? 5 : 6;
+  static constexpr int kSteps = 3;                     // K steps per stage: a wait and a commit per six MMAs
+  static constexpr int kStage = kSteps * (kA + kB);
+  static constexpr int kStages = BN <= 64 ? 3 : BN == 96 ? 5 : BN == 128 ? 4 : 3;
   static constexpr int kTmemBuf = pow2_at_least(BN);  // columns of one accumulator
   static constexpr int kTmem = 2 * kTmemBuf;          // two accumulators: MMA and epilogue overlap
-  static constexpr int kThreads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+  static constexpr int kThreads = 224;                // warps 0, 1 TMA, warp 2 MMA, warps 3-6 epilogue
   static constexpr int kSmem = kStages * kStage + 1024 + 256;
 };
 
@@ -103,11 +115,15 @@ __device__ __forceinline__ void conv_store32(const ConvArgs& a, const uint32_t* 
 }
 
 // Persistent CTAs: CTA i takes pixel tiles i, i + gridDim.x, ... of output
-// channel tile blockIdx.y.  The TMA producer streams the K steps of all its
-// tiles through one ring of stages; the MMA issuer accumulates tile j into
-// TMEM buffer j & 1 and commits it to the epilogue warps, which drain it
-// (bias, ReLU, mask, BF16 store) while the next tile accumulates in the
-// other buffer.
+// channel tile blockIdx.y.  Two loading warps stream the K steps of all its
+// tiles (one the pixels, one the weights) through one ring of stages; the MMA
+// issuer accumulates tile j into TMEM buffer j & 1 and commits it to the epilogue
+// warps, which drain it (bias, ReLU, mask, BF16 store) while the next tile
+// accumulates in the other buffer.
+//
+// What bounds it: the layers that come here are narrow (less than 128 pixels),
+// often one tile per CTA, and its K steps run in series: about 350 clocks for each
+// when every step had its own wait and commit.
 template <int BN>
 __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid_constant__ CUtensorMap mX,
                                                                     const __grid_constant__ CUtensorMap mW,
@@ -123,8 +139,7 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
   uint64_t* done = tempty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
-  int* issued = abort_flag + 1;
-  int* consumed = abort_flag + 2;
+  int* uses = abort_flag + 1;                          // [2][kStages] loads issued per stage: pixels, weights
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   const long long tiles = (long long)a.n * a.tiles_y * a.tiles_x;
@@ -132,100 +147,100 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
   const int co0 = blockIdx.y * BN;
   const int cchunks = a.cin >> 5;
   const int nk = a.taps * cchunks;
-  const long long nsteps = (long long)ntl * nk;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < Cfg::kStages; ++s) { tc::mb_init(&full[s], 1); tc::mb_init(&empty[s], 1); }
+    for (int s = 0; s < Cfg::kStages; ++s) {
+      tc::mb_init(&full[s], 2); tc::mb_init(&empty[s], 1);
+      uses[s] = uses[Cfg::kStages + s] = 0;
+    }
     for (int b = 0; b < 2; ++b) { tc::mb_init(&tfull[b], 1); tc::mb_init(&tempty[b], 4); }
     tc::mb_init(done, 1);
-    *abort_flag = 0; *issued = 0; *consumed = 0;
+    *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __shared__ float sbias[BN];               // this CTA's output-channel biases (0 without bias)
   for (int c = threadIdx.x; c < BN; c += blockDim.x)
     sbias[c] = (a.bias && co0 + c < a.cout) ? a.bias[co0 + c] : 0.f;
-  if (warp == 1) tc::tmem_alloc(tmem_slot, Cfg::kTmem);
+  if (warp == 2) tc::tmem_alloc(tmem_slot, Cfg::kTmem);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
 
   auto tile_origin = [&](int j, int* img, int* x0, int* y0) {
-    long long t = blockIdx.x + (long long)j * gridDim.x;
-    const int tx = (int)(t % a.tiles_x); t /= a.tiles_x;
-    const int ty = (int)(t % a.tiles_y);
-    *img = (int)(t / a.tiles_y);
-    *x0 = tx * a.bx; *y0 = ty * a.by;
+    uint32_t t = blockIdx.x + (uint32_t)j * gridDim.x;         // (tiles < 2^31)
+    const uint32_t u = t / (uint32_t)a.tiles_x;
+    *x0 = (int)(t - u * (uint32_t)a.tiles_x) * a.bx;
+    *img = (int)(u / (uint32_t)a.tiles_y);
+    *y0 = (int)(u - (uint32_t)*img * (uint32_t)a.tiles_y) * a.by;
+  };
+  // (whole warps wait, so that addresses and descriptors stay in uniform registers)
+  auto wait_warp = [&](uint64_t* bar, uint32_t ph) -> bool {
+    return __all_sync(0xffffffffu, tc::mb_try(bar, ph)) || __all_sync(0xffffffffu, wait_live(bar, ph, abort_flag));
   };
 
-  if (warp == 0) {
-    if (lane == 0) {
-      long long g = 0;
-      for (int j = 0; j < ntl && g >= 0; ++j) {
+  if (warp < 3) {
+    const bool el = tc::elect_one();
+    bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
+    auto next = [&]() { if (++s == Cfg::kStages) { s = 0; ph ^= 1u; } };
+    if (warp < 2) {
+      for (int j = 0; j < ntl && ok; ++j) {
         int img, x0, y0;
         tile_origin(j, &img, &x0, &y0);
-        for (int it = 0; it < nk; ++it, ++g) {
-          const int s = (int)(g % Cfg::kStages);
-          const uint32_t ph = (uint32_t)((g / Cfg::kStages) & 1);
-          if (!wait_live(&empty[s], ph ^ 1u, abort_flag) || *((volatile int*)abort_flag)) {
-            atomicExch(abort_flag, 1);
-            *issued = (int)g;
-            g = -1;
-            break;
+        int tap = 0, cc = 0;
+        for (int it = 0; it < nk && ok; it += Cfg::kSteps) {
+          if (!(ok = wait_warp(&empty[s], ph ^ 1u))) break;
+          const int m = min(Cfg::kSteps, nk - it);
+          unsigned char* st = base + s * Cfg::kStage + (warp ? Cfg::kSteps * Cfg::kA : 0);
+          if (el) {
+            uses[warp * Cfg::kStages + s] += 1;
+            tc::mb_expect_tx(&full[s], (uint32_t)(m * (warp ? Cfg::kB : Cfg::kA)));
           }
-          unsigned char* st = base + s * Cfg::kStage;
-          const int tap = it / cchunks, cc = it - tap * cchunks;
-          int dx = 0, dy = 0;
-          if (a.taps == 9) { dx = (tap % 3 - 1) * a.sign; dy = (tap / 3 - 1) * a.sign; }
-          tc::mb_expect_tx(&full[s], (uint32_t)Cfg::kStage);
-          tc::tma_load_4d(st, &mX, cc * 32, x0 + dx, y0 + dy, img, &full[s]);
-          tc::tma_load_2d(st + Cfg::kA, &mW, tap * a.cin + cc * 32, co0, &full[s]);
+          for (int i = 0; i < m; ++i) {
+            int dx = 0, dy = 0;
+            if (a.taps == 9) { dx = (tap % 3 - 1) * a.sign; dy = (tap / 3 - 1) * a.sign; }
+            if (el) {
+              if (warp == 0) tc::tma_load_4d(st + i * Cfg::kA, &mX, cc * 32, x0 + dx, y0 + dy, img, &full[s]);
+              else tc::tma_load_2d(st + i * Cfg::kB, &mW, tap * a.cin + cc * 32, co0, &full[s]);
+            }
+            if (++cc == cchunks) { cc = 0; ++tap; }
+          }
+          next();
         }
       }
-      if (g >= 0) *issued = (int)nsteps;
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    } else {
       constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
-      long long g = 0;
-      bool stop = false;
-      if (a.stall_flag && !stall_on_unset_flag(a.stall_flag, a.stall_cycles)) {
-        atomicExch(abort_flag, 1);
-        stop = true;
-      }
-      for (int j = 0; j < ntl && !stop; ++j) {
+      if (a.stall_flag) ok = __all_sync(0xffffffffu, stall_on_unset_flag(a.stall_flag, a.stall_cycles));
+      const uint32_t sbase = tc::su32(base);
+      for (int j = 0; j < ntl && ok; ++j) {
         const int b = j & 1;
-        if (!wait_live(&tempty[b], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag)) {
-          atomicExch(abort_flag, 1);
-          break;
-        }
+        if (!(ok = wait_warp(&tempty[b], (uint32_t)(((j >> 1) & 1) ^ 1)))) break;
         tc::fence_after();
         const uint32_t acc = tmem + (uint32_t)(b * Cfg::kTmemBuf);
-        for (int it = 0; it < nk; ++it, ++g) {
-          const int s = (int)(g % Cfg::kStages);
-          const uint32_t ph = (uint32_t)((g / Cfg::kStages) & 1);
-          if (!wait_live(&full[s], ph, abort_flag) || *((volatile int*)abort_flag)) {
-            atomicExch(abort_flag, 1);
-            stop = true;
-            break;
-          }
+        for (int it = 0; it < nk; it += Cfg::kSteps) {
+          if (!(ok = wait_warp(&full[s], ph))) break;
           tc::fence_after();
-          const uint32_t sa = tc::su32(base + s * Cfg::kStage);
-          const uint64_t da = tc::desc_sw64(sa, 16, 512), db = tc::desc_sw64(sa + Cfg::kA, 16, 512);
+          const uint32_t sa = sbase + (uint32_t)(s * Cfg::kStage);
+          const uint64_t da = tc::desc_sw64(sa, 16, 512), db = tc::desc_sw64(sa + Cfg::kSteps * Cfg::kA, 16, 512);
 #pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {
-            const uint64_t adv = (uint64_t)((kk * 32) >> 4);        // 16 BF16 = 32 bytes along K
-            tc::umma_bf16(acc, da + adv, db + adv, idesc, (it | kk) ? 1u : 0u);
-          }
-          tc::umma_commit(&empty[s]);
+          for (int i = 0; i < Cfg::kSteps; ++i)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)                      // 16 BF16 = 32 bytes along K
+              if (el && it + i < nk)
+                tc::umma_bf16(acc, da + (uint64_t)((i * Cfg::kA + kk * 32) >> 4),
+                              db + (uint64_t)((i * Cfg::kB + kk * 32) >> 4), idesc, (it | i | kk) ? 1u : 0u);
+          if (el) tc::umma_commit(&empty[s]);
+          next();
         }
-        if (!stop) tc::umma_commit(&tfull[b]);
+        if (ok && el) tc::umma_commit(&tfull[b]);
       }
-      *consumed = (int)g;
-      tc::umma_commit(done);                             // arrives when every MMA issued above has completed
+      if (el) tc::umma_commit(done);                       // arrives when every MMA issued above has completed
     }
+    if (!ok && lane == 0) atomicExch(abort_flag, 1);
   } else {
-    // epilogue warps 2-5: TMEM lane quarter (warp % 4) = pixels 32 (warp % 4) .. + 31 of the tile
+    // epilogue warps: TMEM lane quarter (warp % 4) = pixels 32 (warp % 4) .. + 31 of the tile
     const int q = warp & 3;
     const int m = q * 32 + lane;
     for (int j = 0; j < ntl; ++j) {
@@ -260,12 +275,11 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
   __syncthreads();
   if (threadIdx.x == 0) {
     if (*((volatile int*)abort_flag)) atomicOr(a.err, 2);
-    for (int g = *consumed; g < *issued; ++g)
-      tc::mb_wait(&full[g % Cfg::kStages], (uint32_t)((g / Cfg::kStages) & 1), kWaitCycles);
+    land_pairs(full, uses, Cfg::kStages);
   }
   tc::fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 2) {
     tc::fence_after();
     tc::tmem_dealloc(tmem, Cfg::kTmem);
   }
@@ -727,6 +741,12 @@ __global__ void __launch_bounds__(kConvThreads) conv_wgrad_tc(const __grid_const
 // M group g (rows 32 g .. 32 g + 31) is the box shifted by g pixels, i.e.
 // the taps dx = g - 1 for g < 3 (group 3 is computed and dropped).  One
 // accumulator per dy shares the dZ tile.
+//
+// What bounds it: an MMA takes 48 clocks at 64 channels, one warp that waits and
+// issues about 120, so a warp issues for each dy (1-3); warps 0 and 4 load the X
+// boxes and the dZ tile.
+constexpr int kWgHThreads = 160;
+
 template <int BN> struct WgHCfg {
   static constexpr int kABox = 72 * 64;
   static constexpr int kAStride = (kABox + 1023) / 1024 * 1024;
@@ -743,7 +763,7 @@ template <int BN> struct WgHCfg {
 };
 
 template <int BN>
-__global__ void __launch_bounds__(kConvThreads) conv_wgrad_halo(const __grid_constant__ CUtensorMap mX,
+__global__ void __launch_bounds__(kWgHThreads) conv_wgrad_halo(const __grid_constant__ CUtensorMap mX,
                                                                 const __grid_constant__ CUtensorMap mD, WgArgs a) {
   typedef WgHCfg<BN> Cfg;
   extern __shared__ unsigned char smem_raw[];
@@ -754,8 +774,7 @@ __global__ void __launch_bounds__(kConvThreads) conv_wgrad_halo(const __grid_con
   uint64_t* done = empty + Cfg::kStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
-  int* issued = abort_flag + 1;
-  int* consumed = abort_flag + 2;
+  int* uses = abort_flag + 1;                           // [2][kStages] loads issued per stage: X, dZ
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   const int cchunks = a.cin >> 5;
@@ -768,9 +787,12 @@ __global__ void __launch_bounds__(kConvThreads) conv_wgrad_halo(const __grid_con
   const int nk = kb1 - kb0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < Cfg::kStages; ++s) { tc::mb_init(&full[s], 1); tc::mb_init(&empty[s], 1); }
-    tc::mb_init(done, 1);
-    *abort_flag = 0; *issued = 0; *consumed = 0;
+    for (int s = 0; s < Cfg::kStages; ++s) {
+      tc::mb_init(&full[s], 2); tc::mb_init(&empty[s], ndy);
+      uses[s] = uses[Cfg::kStages + s] = 0;
+    }
+    tc::mb_init(done, ndy);
+    *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tc::tmem_alloc(tmem_slot, Cfg::kTmem);
@@ -779,60 +801,59 @@ __global__ void __launch_bounds__(kConvThreads) conv_wgrad_halo(const __grid_con
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (threadIdx.x == 0) {
-    int it = 0;
-    for (; it < nk; ++it) {
-      const int s = it % Cfg::kStages;
-      const uint32_t ph = (uint32_t)((it / Cfg::kStages) & 1);
-      if (!wait_live(&empty[s], ph ^ 1u, abort_flag) || *((volatile int*)abort_flag)) {
-        atomicExch(abort_flag, 1);
-        break;
-      }
-      int kb = kb0 + it;
-      const int tx = kb % a.tiles_x; kb /= a.tiles_x;
-      const int ty = kb % a.tiles_y;
-      const int img = kb / a.tiles_y;
-      const int x0 = tx * a.bx, y0 = ty * a.by;
+  auto wait_warp = [&](uint64_t* bar, uint32_t ph) -> bool {
+    return __all_sync(0xffffffffu, tc::mb_try(bar, ph)) || __all_sync(0xffffffffu, wait_live(bar, ph, abort_flag));
+  };
+  const bool el = tc::elect_one();
+  bool ok = true;
+  int s = 0;
+  uint32_t ph = 0;
+  if (warp == 0 || warp == 4) {
+    int kb = kb0;
+    int tx = kb % a.tiles_x; kb /= a.tiles_x;
+    int ty = kb % a.tiles_y, img = kb / a.tiles_y;
+    for (int it = 0; it < nk; ++it) {
+      if (!(ok = wait_warp(&empty[s], ph ^ 1u))) break;
       unsigned char* st = base + s * Cfg::kStage;
-      tc::mb_expect_tx(&full[s], (uint32_t)(ndy * Cfg::kABox + Cfg::kB));
-      for (int d = 0; d < ndy; ++d)
-        tc::tma_load_4d(st + d * Cfg::kAStride, &mX, cc * 32, x0 - 1, y0 + (dy0 + d - 1), img, &full[s]);
+      if (el) {
+        uses[(warp >> 2) * Cfg::kStages + s] += 1;
+        if (warp == 0) {
+          tc::mb_expect_tx(&full[s], (uint32_t)(ndy * Cfg::kABox));
+          for (int d = 0; d < ndy; ++d)
+            tc::tma_load_4d(st + d * Cfg::kAStride, &mX, cc * 32, tx * 64 - 1, ty + (dy0 + d - 1), img, &full[s]);
+        } else {
+          tc::mb_expect_tx(&full[s], (uint32_t)Cfg::kB);
 #pragma unroll
-      for (int j = 0; j < BN / 32; ++j)
-        tc::tma_load_4d(st + Cfg::kA + j * Cfg::kBBox, &mD, j * 32, x0, y0, img, &full[s]);
-    }
-    *issued = it;
-  } else if (threadIdx.x == 32) {
-    constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 1, 1);
-    int it = 0;
-    bool stalled = false;
-    if (a.stall_flag && !stall_on_unset_flag(a.stall_flag, a.stall_cycles)) {
-      atomicExch(abort_flag, 1);
-      stalled = true;
-    }
-    for (; it < nk && !stalled; ++it) {
-      const int s = it % Cfg::kStages;
-      const uint32_t ph = (uint32_t)((it / Cfg::kStages) & 1);
-      if (!wait_live(&full[s], ph, abort_flag) || *((volatile int*)abort_flag)) {
-        atomicExch(abort_flag, 1);
-        break;
-      }
-      tc::fence_after();
-      const uint32_t sa = tc::su32(base + s * Cfg::kStage);
-      for (int d = 0; d < ndy; ++d) {
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          // 16 pixels = two 8-row K groups, 1024 bytes; M groups one pixel row apart
-          const uint64_t da = tc::desc_sw64(sa + d * Cfg::kAStride + kk * 1024, 64, 512);
-          const uint64_t db = tc::desc_sw64(sa + Cfg::kA + kk * 1024, Cfg::kBBox, 512);
-          tc::umma_bf16(tmem + (uint32_t)(d * Cfg::kTmemBuf), da, db, idesc, (it | kk) ? 1u : 0u);
+          for (int j = 0; j < BN / 32; ++j)
+            tc::tma_load_4d(st + Cfg::kA + j * Cfg::kBBox, &mD, j * 32, tx * 64, ty, img, &full[s]);
         }
       }
-      tc::umma_commit(&empty[s]);
+      if (++tx == a.tiles_x) { tx = 0; if (++ty == a.tiles_y) { ty = 0; ++img; } }
+      if (++s == Cfg::kStages) { s = 0; ph ^= 1u; }
     }
-    *consumed = it;
-    tc::umma_commit(done);
+  } else if (warp <= ndy) {
+    constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 1, 1);
+    const int d = warp - 1;
+    if (a.stall_flag) ok = __all_sync(0xffffffffu, stall_on_unset_flag(a.stall_flag, a.stall_cycles));
+    const uint32_t sbase = tc::su32(base);
+    for (int it = 0; it < nk && ok; ++it) {
+      if (!(ok = wait_warp(&full[s], ph))) break;
+      tc::fence_after();
+      const uint32_t sa = sbase + (uint32_t)(s * Cfg::kStage);
+      // 16 pixels = two 8-row K groups, 1024 bytes; M groups one pixel row apart
+      const uint64_t da = tc::desc_sw64(sa + d * Cfg::kAStride, 64, 512);
+      const uint64_t db = tc::desc_sw64(sa + Cfg::kA, Cfg::kBBox, 512);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+        if (el)
+          tc::umma_bf16(tmem + (uint32_t)(d * Cfg::kTmemBuf), da + (uint64_t)(kk * 64), db + (uint64_t)(kk * 64), idesc,
+                        (it | kk) ? 1u : 0u);
+      if (el) tc::umma_commit(&empty[s]);
+      if (++s == Cfg::kStages) { s = 0; ph ^= 1u; }
+    }
+    if (el) tc::umma_commit(done);
   }
+  if (!ok && lane == 0) atomicExch(abort_flag, 1);
   __syncwarp();
   const bool ok_done = tc::mb_wait(done, 0, kWaitCycles);
   tc::fence_after();
@@ -858,8 +879,7 @@ __global__ void __launch_bounds__(kConvThreads) conv_wgrad_halo(const __grid_con
     atomicOr(a.err, 2);
   }
   if (threadIdx.x == 0) {
-    for (int it = *consumed; it < *issued; ++it)
-      tc::mb_wait(&full[it % Cfg::kStages], (uint32_t)((it / Cfg::kStages) & 1), kWaitCycles);
+    land_pairs(full, uses, Cfg::kStages);
   }
   tc::fence_before();
   __syncthreads();
@@ -878,7 +898,7 @@ oh_status launch_wgrad_halo(const CUtensorMap& mX, const CUtensorMap& mD, const 
   long long splits = std::max(1LL, (4LL * sm_count() + gx - 1) / gx);
   splits = std::min(splits, std::max(1LL, kb_total / 16));
   splits = std::min(splits, 65535LL);
-  conv_wgrad_halo<BN><<<dim3(gx, (int)splits), kConvThreads, Cfg::kSmem, st>>>(mX, mD, a);
+  conv_wgrad_halo<BN><<<dim3(gx, (int)splits), kWgHThreads, Cfg::kSmem, st>>>(mX, mD, a);
   OH_LAUNCH_CHECK();
   return OH_OK;
 }
