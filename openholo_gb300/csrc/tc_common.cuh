@@ -53,6 +53,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "l"(map), "r"(c0), "r"(c1), "r"(su32(bar))
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          su32(dst)),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(su32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                             uint64_t* bar) {
   asm volatile(
@@ -168,6 +175,22 @@ inline oh_status map_mat2d(CUtensorMap* m, const void* ptr, int k, int rows, int
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(OH_ERR_CUDA, "cuTensorMapEncodeTiled (matrix) failed (" + std::to_string((int)r) + ")");
+  return OH_OK;
+}
+
+// BF16 matrix [rows][taps * k] (k contiguous per tap): box {32, box_rows, box_taps},
+// 64-byte swizzle, so that a load brings box_taps tiles of box_rows rows.
+inline oh_status map_taps3d(CUtensorMap* m, const void* ptr, int k, int rows, int taps, int box_rows, int box_taps) {
+  EncodeTiledFn fn;
+  OH_TRY(encode_tiled_fn(&fn));
+  const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)rows, (cuuint64_t)taps};
+  const cuuint64_t strides[2] = {(cuuint64_t)k * taps * 2, (cuuint64_t)k * 2};
+  const cuuint32_t box[3] = {32, (cuuint32_t)box_rows, (cuuint32_t)box_taps};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(OH_ERR_CUDA, "cuTensorMapEncodeTiled (weights) failed (" + std::to_string((int)r) + ")");
   return OH_OK;
 }
 

@@ -274,8 +274,10 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
   if (threadIdx.x == 0) tc::mb_wait(done, 0, kWaitCycles);
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (*((volatile int*)abort_flag)) atomicOr(a.err, 2);
-    land_pairs(full, uses, Cfg::kStages);
+    if (*((volatile int*)abort_flag)) {
+      atomicOr(a.err, 2);
+      land_pairs(full, uses, Cfg::kStages);
+    }
   }
   tc::fence_before();
   __syncthreads();
@@ -295,9 +297,9 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
 // tensor rate; its operands from shared memory at 128 bytes a clock), but one warp
 // that waits for a box, issues six and commits needs about 90 to 120 for each, and
 // one that waits for a slot and loads a box about 500.  So up to four warps load
-// boxes, a fifth the weights, and up to four issue, each for its own output rows.
-// 4 x 512 x 512 pixels, 192 -> 64 channels: 188 us (470 with one warp each), where
-// the MMAs take 150 to 180 at the clocks of such a load.
+// boxes, a fifth the weights (three taps in one load), and up to four issue, each
+// for its own output rows.  4 x 512 x 512 pixels, 192 -> 64 channels: 188 us (470
+// with one warp each), where the MMAs take 150 to 180 at the clocks of such a load.
 //
 // A barrier's parity tells its last two phases apart only to a warp that waits for
 // every one of them: loader w fills issuer w's own slots, and every issuer waits
@@ -308,14 +310,14 @@ __global__ void __launch_bounds__(FwdCfg<BN>::kThreads) conv_fwd_tc(const __grid
 struct RowsCfg {
   int rows, nbuf;                      // output rows per tile (1, 2 or a multiple of 4), accumulator sets (2: MMAs
                                        // and epilogue overlap)
-  int na;                              // box slots, a multiple of the issuers
+  int na, nb;                          // slots: boxes (a multiple of the issuers), weight steps
   uint32_t tmem_cols;
 };
 constexpr int kRowsA = 136 * 64, kRowsAStride = (kRowsA + 1023) / 1024 * 1024;
 constexpr int kRowsLoaders = 4, kRowsIssuers = 4, kRowsEpiWarps = 8;
 constexpr int kRowsIssue0 = kRowsLoaders + 1, kRowsEpi0 = kRowsIssue0 + kRowsIssuers;       // first warp of each role
 constexpr int kRowsThreads = 32 * (kRowsEpi0 + kRowsEpiWarps);
-constexpr int kRowsA_Slots = 16, kRowsB_Slots = 3;
+constexpr int kRowsA_Slots = 32, kRowsB_Slots = 16;     // at most
 constexpr int kRowsFixed = 1024 + kRowsEpiWarps * 2048 + (2 * kRowsA_Slots + 2 * kRowsB_Slots + 8) * 8 +
                            (kRowsA_Slots + kRowsB_Slots) * 4 + 64;
 
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
   const uint32_t raw = tc::su32(smem_raw);
   unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   unsigned char* sB = base + (size_t)rc.na * kRowsAStride;
-  unsigned char* sE = sB + kRowsB_Slots * kB;           // 2 KB per epilogue warp
+  unsigned char* sE = sB + (size_t)rc.nb * kB;           // 2 KB per epilogue warp
   uint64_t* fullA = reinterpret_cast<uint64_t*>(sE + kRowsEpiWarps * 2048);
   uint64_t* emptyA = fullA + kRowsA_Slots;
   uint64_t* fullB = emptyA + kRowsA_Slots;
@@ -350,13 +352,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
   const int ni = min(rc.rows, kRowsIssuers);           // issuing warps (1, 2 or 4): row r belongs to the r % ni-th
   const int own = rc.na / ni;                          // box slots per issuer
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < rc.na; ++s) { tc::mb_init(&fullA[s], 1); tc::mb_init(&emptyA[s], 1); }
-    for (int s = 0; s < kRowsB_Slots; ++s) { tc::mb_init(&fullB[s], 1); tc::mb_init(&emptyB[s], ni); }
-    for (int b = 0; b < 2; ++b) { tc::mb_init(&tfull[b], ni); tc::mb_init(&tempty[b], kRowsEpiWarps); }
-    tc::mb_init(done, ni);
-    *abort_flag = 0;
-    for (int i = 0; i < kRowsA_Slots + kRowsB_Slots; ++i) usesA[i] = 0;
+  {
+    // (one barrier per thread: in turn they took 1.3 us)
+    const int i = threadIdx.x;
+    if (i < rc.na) { tc::mb_init(&fullA[i], 1); tc::mb_init(&emptyA[i], 1); usesA[i] = 0; }
+    if (i < rc.nb) { tc::mb_init(&fullB[i], 1); tc::mb_init(&emptyB[i], ni); usesB[i] = 0; }
+    if (i < 2) { tc::mb_init(&tfull[i], ni); tc::mb_init(&tempty[i], kRowsEpiWarps); }
+    if (i == 0) { tc::mb_init(done, ni); *abort_flag = 0; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __shared__ float sbias[BN];
@@ -392,18 +394,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
 
   if (warp <= kRowsLoaders) {
     const bool el = tc::elect_one();
-    Ring ra{0, own, 0}, rb{0, kRowsB_Slots, 0};
+    Ring ra{0, own, 0}, rb{0, rc.nb, 0};
     auto load_b = [&](int dyi, int cc) -> bool {
       if (!wait_warp(&emptyB[rb.s], rb.ph ^ 1u)) return false;
       if (el) {
         unsigned char* st = sB + (size_t)rb.s * kB;
         usesB[rb.s] += 1;
         tc::mb_expect_tx(&fullB[rb.s], (uint32_t)kB);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int tap = 3 * (1 + a.sign * (dyi - 1)) + (1 + a.sign * (j - 1));
-          tc::tma_load_2d(st + j * kTap, &mW, tap * a.cin + cc * 32, co0, &fullB[rb.s]);
-        }
+        // the three taps of input row dy = dyi - 1 (mirrored for the input gradient)
+        tc::tma_load_3d(st, &mW, cc * 32, co0, 3 * (1 + a.sign * (dyi - 1)), &fullB[rb.s]);
       }
       return true;
     };
@@ -438,7 +437,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
     constexpr uint32_t idesc = tc::idesc_bf16(128, BN, 0, 0);
     const int w = warp - kRowsIssue0;
     const bool el = tc::elect_one();
-    Ring ra{0, own, 0}, rb{0, kRowsB_Slots, 0};
+    Ring ra{0, own, 0}, rb{0, rc.nb, 0};
     bool ok = true;
     if (a.stall_flag) ok = __all_sync(0xffffffffu, stall_on_unset_flag(a.stall_flag, a.stall_cycles));
     // the three dx taps of one box into one output row's accumulator; the swizzle
@@ -451,8 +450,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk)                          // 16 BF16 = 32 bytes along K
           if (el)
-            tc::umma_bf16(acc, da + (uint64_t)((j * 64 + kk * 32) >> 4), db + (uint64_t)((j * kTap + kk * 32) >> 4),
-                          idesc, (j | kk) ? 1u : first ? 0u : 1u);
+            tc::umma_bf16(acc, da + (uint64_t)((j * 64 + kk * 32) >> 4),
+                          db + (uint64_t)(((a.sign > 0 ? j : 2 - j) * kTap + kk * 32) >> 4), idesc,
+                          (j | kk) ? 1u : first ? 0u : 1u);
     };
     auto commit = [&](uint64_t* bar) {
       if (el) tc::umma_commit(bar);
@@ -577,12 +577,12 @@ __global__ void __launch_bounds__(kRowsThreads, 1) conv_fwd_rows(const __grid_co
   // not consumed land before the CTA exits
   if (threadIdx.x == 0) tc::mb_wait(done, 0, kWaitCycles);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (*((volatile int*)abort_flag)) atomicOr(a.err, 2);
+  if (threadIdx.x == 0 && *((volatile int*)abort_flag)) {
+    atomicOr(a.err, 2);
     // (each slot's last use; the earlier ones were consumed)
     for (int i = 0; i < rc.na; ++i)
       if (usesA[i]) tc::mb_wait(&fullA[i], (uint32_t)((usesA[i] - 1) & 1), kWaitCycles);
-    for (int i = 0; i < kRowsB_Slots; ++i)
+    for (int i = 0; i < rc.nb; ++i)
       if (usesB[i]) tc::mb_wait(&fullB[i], (uint32_t)((usesB[i] - 1) & 1), kWaitCycles);
   }
   tc::fence_before();
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(kWgHThreads) conv_wgrad_halo(const __grid_cons
     atomicOr(a.err, 2);
   }
   if (threadIdx.x == 0) {
-    land_pairs(full, uses, Cfg::kStages);
+    if (*((volatile int*)abort_flag)) land_pairs(full, uses, Cfg::kStages);
   }
   tc::fence_before();
   __syncthreads();
@@ -931,7 +931,8 @@ oh_status launch_fwd(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArg
 
 // The row kernel's channel tile and rows per tile for a layer: the least estimated
 // clocks of a CTA, from the MMAs' clocks (see conv_fwd_rows; 120 from one issuer), 40
-// bytes a clock of loads, and 1000 clocks per warp and block of the epilogue.
+// bytes a clock of loads, 2000 clocks of latency over the steps in flight, and 1000
+// clocks per warp and block of the epilogue.
 // Measured, 4 x 512 x 512 pixels, 192 -> 64 channels: 188 us with tiles of 4 rows and
 // two accumulator sets, 211 with 8 rows and one, 288 with 2 rows; 64 -> 192: 242 us
 // with channel tiles of 96 and 2 rows, 257 with 64 and 4, 284 with 192 and 2.
@@ -952,17 +953,19 @@ RowsPlan rows_plan(const ConvArgs& a) {
       const long long tiles = (long long)a.n * ((a.h + rows - 1) / rows) * a.tiles_x;
       const double waves = (double)((tiles + gx - 1) / gx);
       const int ni = std::min(rows, kRowsIssuers), nbuf = 2 * rows * bn <= 512 ? 2 : 1;
-      const int na = std::min(kRowsA_Slots, (budget - kRowsB_Slots * step) / kRowsAStride) / ni * ni;
+      // as many steps in flight of both kinds as fit
+      const int nb = std::min(kRowsB_Slots, std::max(3, budget / (rows * kRowsAStride + step)));
+      const int na = std::min(kRowsA_Slots, (budget - nb * step) / kRowsAStride) / ni * ni;
       if (na < std::max(ni, 4)) continue;
       const double mma = std::max({bn / 2.0, 32.0 + bn / 4.0, 120.0 / ni});
       const double epi = (rows * (bn / 32) + 1) / 2 * 1000.0;
-      const double calc = cchunks * std::max(rows * 18.0 * mma, 3.0 * (rows * kRowsA + step) / 40.0);
+      const double calc = 3.0 * cchunks * std::max({rows * 6.0 * mma, (rows * kRowsA + step) / 40.0, 2000.0 / nb, 2000.0 * rows / na});
       const double t = waves * ((nbuf == 2 ? std::max(calc, epi) : calc + epi) + 300.0) + (nbuf == 2 ? epi : 0.0);
       if (best.bn == 0 || t < best_t) {
         best_t = t;
         best.bn = bn;
-        best.smem = na * kRowsAStride + kRowsB_Slots * step + kRowsFixed;
-        best.c = RowsCfg{rows, nbuf, na, (uint32_t)pow2_at_least(nbuf * rows * bn)};
+        best.smem = na * kRowsAStride + nb * step + kRowsFixed;
+        best.c = RowsCfg{rows, nbuf, na, nb, (uint32_t)pow2_at_least(nbuf * rows * bn)};
       }
     }
   }
@@ -1031,7 +1034,7 @@ oh_status conv_enqueue(oh_ctx* ctx, const ConvDesc& d, cudaStream_t st, const ch
   if (d.taps == 9 && a.by == 1 && a.bx == 128 && !(hv && std::atoi(hv) == 0)) {
     const RowsPlan p = rows_plan(a);
     OH_TRY(tc::map_act4d(&mX, d.x, d.cin, d.x_cs, d.w, d.h, d.n, 136, 1));
-    OH_TRY(tc::map_mat2d(&mW, d.w_mat, d.taps * d.cin, d.cout, p.bn));
+    OH_TRY(tc::map_taps3d(&mW, d.w_mat, d.cin, d.cout, d.taps, p.bn, 3));
     KernelTimer kt(ctx, timer_name, st);
     switch (p.bn) {
       case 32: return launch_rows<32>(mX, mW, a, p, st);
