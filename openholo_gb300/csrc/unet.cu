@@ -63,38 +63,35 @@ __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162f
 // channel 3 = depth_lut[depth byte], channels 4-31 zero.
 __global__ void unet_pack_input(const uint8_t* __restrict__ rgbd, const float* __restrict__ lut, long long npix,
                                 __nv_bfloat16* __restrict__ out) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
-    const uchar4 v = reinterpret_cast<const uchar4*>(rgbd)[p];
-    uint4 o[4];
-    __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(o);
-    ob[0] = __floats2bfloat162_rn(v.x * (1.f / 255.f), v.y * (1.f / 255.f));
-    ob[1] = __floats2bfloat162_rn(v.z * (1.f / 255.f), lut[v.w]);
-#pragma unroll
-    for (int i = 2; i < 16; ++i) ob[i] = __floats2bfloat162_rn(0.f, 0.f);
-    uint4* dst = reinterpret_cast<uint4*>(out + p * kInPad);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] = o[i];
+  // a thread per 8 channels: whole lines per store (a thread per pixel, its four
+  // stores 64 bytes apart, took 22.8 us at 1024 x 1024)
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 4 * npix; i += (long long)gridDim.x * blockDim.x) {
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if ((i & 3) == 0) {
+      const uchar4 v = reinterpret_cast<const uchar4*>(rgbd)[i >> 2];
+      __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+      ob[0] = __floats2bfloat162_rn(v.x * (1.f / 255.f), v.y * (1.f / 255.f));
+      ob[1] = __floats2bfloat162_rn(v.z * (1.f / 255.f), lut[v.w]);
+    }
+    reinterpret_cast<uint4*>(out)[i] = o;
   }
 }
 
 // 2x2 average pooling: dst[n][y][x][c] = mean of src[n][2y+a][2x+b][c]
-// (c < C, eight channels per thread).
-__global__ void unet_pool(const __nv_bfloat16* __restrict__ src, int src_cs, int C, int H, int W, int n,
+// (c < C, eight channels per thread; blocks along a row, rows of all frames down).
+__global__ void unet_pool(const __nv_bfloat16* __restrict__ src, int src_cs, uint32_t c8, int w, int rows,
                           __nv_bfloat16* __restrict__ dst, int dst_cs) {
-  const int h = H / 2, w = W / 2, c8 = C / 8;
-  const long long total = (long long)n * h * w * c8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    long long p = i / c8;
-    const int x = (int)(p % w); p /= w;
-    const int y = (int)(p % h);
-    const int b = (int)(p / h);
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c8 * w) return;
+  const uint32_t x = i / c8, c = (i - x * c8) * 8;
+  for (int y = blockIdx.y; y < rows; y += gridDim.y) {         // y: frame n's row is n h + row, 2 y its first source row
+    const __nv_bfloat16* s0 = src + ((size_t)(2 * y) * (2 * w) + 2 * x) * src_cs + c;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
     for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
       for (int dx = 0; dx < 2; ++dx) {
-        const uint4 v = *reinterpret_cast<const uint4*>(src + (((size_t)b * H + 2 * y + dy) * W + 2 * x + dx) * src_cs + c);
+        const uint4 v = *reinterpret_cast<const uint4*>(s0 + ((size_t)dy * (2 * w) + dx) * src_cs);
         const __nv_bfloat162* vb = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -107,24 +104,26 @@ __global__ void unet_pool(const __nv_bfloat16* __restrict__ src, int src_cs, int
     __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
     for (int e = 0; e < 4; ++e) ob[e] = __floats2bfloat162_rn(0.25f * acc[2 * e], 0.25f * acc[2 * e + 1]);
-    *reinterpret_cast<uint4*>(dst + (((size_t)b * h + y) * w + x) * dst_cs + c) = o;
+    *reinterpret_cast<uint4*>(dst + ((size_t)y * w + x) * dst_cs + c) = o;
   }
 }
 
 // nearest 2x upsampling into channels [off, off + C) of dst:
-// dst[n][Y][X][off + c] = src[n][Y/2][X/2][c], src h x w, dst 2h x 2w.
-__global__ void unet_up(const __nv_bfloat16* __restrict__ src, int src_cs, int C, int h, int w, int n,
+// dst[n][Y][X][off + c] = src[n][Y/2][X/2][c], src h x w, dst 2h x 2w; a thread
+// reads eight channels once and writes them four times (57 us for the three levels at
+// 1024 x 1024; a thread per output, with 64-bit index divisions, 92).
+__global__ void unet_up(const __nv_bfloat16* __restrict__ src, int src_cs, uint32_t c8, int w, int rows,
                         __nv_bfloat16* __restrict__ dst, int dst_cs, int off) {
-  const int H = 2 * h, W = 2 * w, c8 = C / 8;
-  const long long total = (long long)n * H * W * c8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % c8) * 8;
-    long long p = i / c8;
-    const int X = (int)(p % W); p /= W;
-    const int Y = (int)(p % H);
-    const int b = (int)(p / H);
-    const uint4 v = *reinterpret_cast<const uint4*>(src + (((size_t)b * h + Y / 2) * w + X / 2) * src_cs + c);
-    *reinterpret_cast<uint4*>(dst + (((size_t)b * H + Y) * W + X) * dst_cs + off + c) = v;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c8 * w) return;
+  const uint32_t x = i / c8, c = (i - x * c8) * 8;
+  for (int y = blockIdx.y; y < rows; y += gridDim.y) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src + ((size_t)y * w + x) * src_cs + c);
+    __nv_bfloat16* d = dst + ((size_t)(2 * y) * (2 * w) + 2 * x) * dst_cs + off + c;
+#pragma unroll
+    for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+      for (int dx = 0; dx < 2; ++dx) *reinterpret_cast<uint4*>(d + ((size_t)dy * (2 * w) + dx) * dst_cs) = v;
   }
 }
 
@@ -237,25 +236,58 @@ __global__ void __launch_bounds__(256) unet_bias_grad(const __nv_bfloat16* __res
 }
 
 // 1x1 head (32 -> 2 channels, FP32 weights): pred[p][k] = b[k] + sum_c W[k][c] x[p][c].
-// Inference: out[p] = scale * pred[p] (float2).  Training (target != null):
-// loss += sum (pred - target/scale)^2 / count, dpred = 2 (pred - t) / count,
-// head gradients (dW[k][c] = sum dpred[k] x[c], db[k] = sum dpred[k]) and the
-// gradient of x times its ReLU mask, dx[p][c] = sum_k dpred[k] W[k][c] (x > 0).
+// unet_head_out: out[p] = scale * pred[p] (float2), the block's pixels by way of
+// shared memory (16-byte chunks swizzled), so that loads fill lines.
+// unet_head (training): loss += sum (pred - target/scale)^2 / count, dpred =
+// 2 (pred - t) / count, head gradients (dW[k][c] = sum dpred[k] x[c], db[k] = sum
+// dpred[k]) and the gradient of x times its ReLU mask, dx[p][c] = sum_k dpred[k]
+// W[k][c] (x > 0).
 constexpr int kHeadThreads = 256;
+__global__ void __launch_bounds__(kHeadThreads) unet_head_out(const __nv_bfloat16* __restrict__ x, long long npix,
+                                                              const float* __restrict__ Wb, float scale,
+                                                              float2* __restrict__ out) {
+  __shared__ float w[2 * 32 + 2];
+  __shared__ uint4 px[4 * kHeadThreads];
+  for (int i = threadIdx.x; i < 66; i += blockDim.x) w[i] = Wb[i];
+  for (long long p0 = (long long)blockIdx.x * kHeadThreads; p0 < npix; p0 += (long long)gridDim.x * kHeadThreads) {
+    __syncthreads();
+    const uint4* xp = reinterpret_cast<const uint4*>(x + p0 * 32);
+    const long long left = 4 * (npix - p0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = threadIdx.x + k * kHeadThreads;
+      if (i < left) px[(i & ~3) | ((i ^ (i >> 3)) & 3)] = xp[i];
+    }
+    __syncthreads();
+    if (p0 + threadIdx.x >= npix) continue;
+    float s0 = w[64], s1 = w[65];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint4 v = px[4 * threadIdx.x + (g ^ ((threadIdx.x >> 1) & 3))];
+      const __nv_bfloat162* vb = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(vb[e]);
+        const int c = g * 8 + 2 * e;
+        s0 = fmaf(w[c], f.x, s0); s1 = fmaf(w[32 + c], f.x, s1);
+        s0 = fmaf(w[c + 1], f.y, s0); s1 = fmaf(w[33 + c], f.y, s1);
+      }
+    }
+    out[p0 + threadIdx.x] = make_float2(scale * s0, scale * s1);
+  }
+}
+
 __global__ void __launch_bounds__(kHeadThreads) unet_head(const __nv_bfloat16* __restrict__ x, long long npix,
                                                           const float* __restrict__ Wb, float scale,
-                                                          float2* __restrict__ out, const float2* __restrict__ target,
+                                                          const float2* __restrict__ target,
                                                           float inv_count, float* __restrict__ loss,
                                                           float* __restrict__ gW, __nv_bfloat16* __restrict__ dx) {
   __shared__ float w[2 * 32 + 2];
   for (int i = threadIdx.x; i < 66; i += blockDim.x) w[i] = Wb[i];
   __syncthreads();
-  const bool train = target != nullptr;
   float gacc[66];
-  if (train) {
 #pragma unroll
-    for (int i = 0; i < 66; ++i) gacc[i] = 0.f;
-  }
+  for (int i = 0; i < 66; ++i) gacc[i] = 0.f;
   float lacc = 0.f;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
     float xv[32];
@@ -274,10 +306,6 @@ __global__ void __launch_bounds__(kHeadThreads) unet_head(const __nv_bfloat16* _
     float p0 = w[64], p1 = w[65];
 #pragma unroll
     for (int c = 0; c < 32; ++c) { p0 = fmaf(w[c], xv[c], p0); p1 = fmaf(w[32 + c], xv[c], p1); }
-    if (!train) {
-      out[p] = make_float2(scale * p0, scale * p1);
-      continue;
-    }
     const float2 t = target[p];
     const float e0 = p0 - t.x / scale, e1 = p1 - t.y / scale;
     lacc += e0 * e0 + e1 * e1;
@@ -298,7 +326,6 @@ __global__ void __launch_bounds__(kHeadThreads) unet_head(const __nv_bfloat16* _
 #pragma unroll
     for (int g = 0; g < 4; ++g) dp[g] = o[g];
   }
-  if (!train) return;
   // block reduction of the 66 gradient sums and the loss
   __shared__ float red[kHeadThreads / 32][67];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -365,6 +392,8 @@ inline int grid_for(long long work, int threads = 256) {
   const long long g = (work + threads - 1) / threads;
   return (int)std::max(1LL, std::min<long long>(g, (long long)sm_count() * 16));
 }
+// blocks of 256 along a row, one block row per row (up to the grid's limit)
+inline dim3 grid_rows(int per_row, int rows) { return dim3((per_row + 255) / 256, std::min(rows, 65535)); }
 
 }  // namespace
 
@@ -457,7 +486,7 @@ oh_status unet_forward(oh_unet* u, const uint8_t* rgbd, int n, int h, int w, flo
   const long long np0 = lvl_pix(n, h, w, 0);
   {
     KernelTimer kt(ctx, "unet_pack_input", st);
-    unet_pack_input<<<grid_for(np0), 256, 0, st>>>(rgbd, u->lut, np0, u->in0);
+    unet_pack_input<<<grid_for(4 * np0), 256, 0, st>>>(rgbd, u->lut, np0, u->in0);
     OH_LAUNCH_CHECK();
   }
   auto conv = [&](const Layer& L, const void* x, int x_cs, int hl, int wl, void* y, int y_cs) {
@@ -476,8 +505,8 @@ oh_status unet_forward(oh_unet* u, const uint8_t* rgbd, int n, int h, int w, flo
     OH_TRY(conv(u->layers[2 * l + 1], u->A[l], c, hl, wl, u->CAT[l], cat_cs(u, l)));
     if (l + 1 < kLevels) {
       KernelTimer kt(ctx, "unet_pool", st);
-      unet_pool<<<grid_for(lvl_pix(n, h, w, l + 1) * c / 8), 256, 0, st>>>(u->CAT[l], cat_cs(u, l), c, hl, wl, n,
-                                                                           u->P_[l + 1], c);
+      unet_pool<<<grid_rows(wl / 2 * c / 8, n * hl / 2), 256, 0, st>>>(u->CAT[l], cat_cs(u, l), c / 8, wl / 2, n * hl / 2,
+                                                                       u->P_[l + 1], c);
       OH_LAUNCH_CHECK();
       xin = u->P_[l + 1];
       xin_cs = c;
@@ -490,8 +519,8 @@ oh_status unet_forward(oh_unet* u, const uint8_t* rgbd, int n, int h, int w, flo
     const int hl = h >> l, wl = w >> l, c = u->chans[l], cb = u->chans[l + 1];
     {
       KernelTimer kt(ctx, "unet_up", st);
-      unet_up<<<grid_for(lvl_pix(n, h, w, l) * cb / 8), 256, 0, st>>>(below, below_cs, cb, hl / 2, wl / 2, n, u->CAT[l],
-                                                                      cat_cs(u, l), c);
+      unet_up<<<grid_rows(wl / 2 * cb / 8, n * hl / 2), 256, 0, st>>>(below, below_cs, cb / 8, wl / 2, n * hl / 2,
+                                                                      u->CAT[l], cat_cs(u, l), c);
       OH_LAUNCH_CHECK();
     }
     const Layer& La = u->layers[2 * kLevels + 2 * (kLevels - 2 - l)];
@@ -504,8 +533,7 @@ oh_status unet_forward(oh_unet* u, const uint8_t* rgbd, int n, int h, int w, flo
   if (out) {
     const Layer& H = u->layers.back();
     KernelTimer kt(ctx, "unet_head", st);
-    unet_head<<<grid_for(np0, kHeadThreads), kHeadThreads, 0, st>>>(u->D[0], np0, u->P + H.off_w, u->out_scale, out,
-                                                                    nullptr, 0.f, nullptr, nullptr, nullptr);
+    unet_head_out<<<grid_for(np0, kHeadThreads), kHeadThreads, 0, st>>>(u->D[0], np0, u->P + H.off_w, u->out_scale, out);
     OH_LAUNCH_CHECK();
   }
   return OH_OK;
@@ -520,9 +548,8 @@ oh_status unet_backward(oh_unet* u, const float2* target, int n, int h, int w, c
   const Layer& H = u->layers.back();
   {
     KernelTimer kt(ctx, "unet_head_loss", st);
-    unet_head<<<grid_for(np0, kHeadThreads), kHeadThreads, 0, st>>>(u->D[0], np0, u->P + H.off_w, u->out_scale,
-                                                                    nullptr, target, 1.f / (2.f * (float)np0), u->loss,
-                                                                    H.dwt, u->dZ1);
+    unet_head<<<grid_for(np0, kHeadThreads), kHeadThreads, 0, st>>>(u->D[0], np0, u->P + H.off_w, u->out_scale, target,
+                                                                    1.f / (2.f * (float)np0), u->loss, H.dwt, u->dZ1);
     OH_LAUNCH_CHECK();
   }
   auto wgrad = [&](const Layer& L, const void* x, int x_cs, const void* dz, int hl, int wl) -> oh_status {
