@@ -601,14 +601,9 @@ def _sec_pointcloud(ctx, dev, torch, st, timed, out, n, nx, ny, peaks=None):
     res = {"ms_per_hologram": ms, "holograms_per_s": 1000.0 / ms,
            "point_pixel_terms_per_s": n * nx * ny / (ms / 1000.0), "kernels_ms": kms,
            "rel_err_vs_fp64": acc["rel_l2"], "accuracy": acc, "dtype": "f32 (FP64-reduced phase tables)"}
-    t_direct = kms.get("pc_direct_f32")
-    if peaks and t_direct:
-        mufu = 3.0 * n * nx * ny          # per term: sqrt.approx, rcp.approx, sin.approx
-        res["roofline"] = {"bound": "mufu", "kernel": "pc_direct_f32", "unit": "MUFU results/s",
-                           "achieved": mufu / (t_direct * 1e-3), "peak": peaks["mufu_per_s"],
-                           "frac": mufu / (t_direct * 1e-3) / peaks["mufu_per_s"], "peak_source": "measured",
-                           "algorithmic_per_launch": mufu,
-                           "issue": compute_roofline("pc_direct_f32", t_direct, peaks)}
+    t_tc = kms.get("pc_tc_regions")
+    if peaks and t_tc:                    # operand builders: the issue slots bound it
+        res["roofline"] = compute_roofline("pc_tc_regions", t_tc, peaks)
     out["pointcloud_1024x1024_5000pts"] = res
     del f64
 

@@ -203,8 +203,8 @@ __device__ __forceinline__ void wrp_for_bins(const WRPGeom& g, const WrpBins& b,
 }
 
 // Bin counters and cursors are replicated kWrpRep times (replicas of one bin
-// a whole counter array apart): about 600 points share a plane-region
-// counter, and the replicas split that contention.  The replica of point k
+// a whole counter array apart): a hundred points and more share a counter, and
+// the replicas split that contention.  The replica of point k
 // is (k / 256) mod kWrpRep, so runs of consecutive points stay together in a
 // bin's list (the window kernels read the point records in list order, and
 // records of nearby points share cache lines).
