@@ -940,27 +940,28 @@ struct RowsPlan {
   RowsCfg c;
   int bn, smem;
 };
-RowsPlan rows_plan(const ConvArgs& a) {
+RowsPlan rows_plan(const ConvArgs& a, int sms) {
   RowsPlan best{};
-  double best_t = 0.0;
-  const double cchunks = a.cin / 32;
+  float best_t = 0.f;
+  const float cchunks = (float)(a.cin / 32);
   const int budget = 226 * 1024 - kRowsFixed;            // (1 KB for the biases)
   for (int bn : {32, 64, 96, 128, 192, 256}) {
     if (a.cout % bn) continue;
     const int step = 3 * bn * 64;                        // weights of one (dy, 32 channels)
-    const int gx = std::max(1, sm_count() / (a.cout / bn));
+    const int gx = std::max(1, sms / (a.cout / bn));
     for (int rows = 1; rows <= 16 && rows * bn <= 512; rows *= 2) {
-      const long long tiles = (long long)a.n * ((a.h + rows - 1) / rows) * a.tiles_x;
-      const double waves = (double)((tiles + gx - 1) / gx);
       const int ni = std::min(rows, kRowsIssuers), nbuf = 2 * rows * bn <= 512 ? 2 : 1;
       // as many steps in flight of both kinds as fit
       const int nb = std::min(kRowsB_Slots, std::max(3, budget / (rows * kRowsAStride + step)));
       const int na = std::min(kRowsA_Slots, (budget - nb * step) / kRowsAStride) / ni * ni;
       if (na < std::max(ni, 4)) continue;
-      const double mma = std::max({bn / 2.0, 32.0 + bn / 4.0, 120.0 / ni});
-      const double epi = (rows * (bn / 32) + 1) / 2 * 1000.0;
-      const double calc = 3.0 * cchunks * std::max({rows * 6.0 * mma, (rows * kRowsA + step) / 40.0, 2000.0 / nb, 2000.0 * rows / na});
-      const double t = waves * ((nbuf == 2 ? std::max(calc, epi) : calc + epi) + 300.0) + (nbuf == 2 ? epi : 0.0);
+      const uint32_t tiles = (uint32_t)a.n * a.tiles_x * ((uint32_t)(a.h + rows - 1) / rows);       // (< 2^31)
+      const float waves = (float)((tiles + gx - 1) / gx);
+      const float mma = std::max({bn / 2.f, 32.f + bn / 4.f, 120.f / ni});
+      const float epi = (rows * (bn / 32) + 1) / 2 * 1000.f;
+      const float calc = 3.f * cchunks * std::max({rows * 6.f * mma, (rows * kRowsA + step) / 40.f, 2000.f / nb,
+                                                   2000.f * rows / na});
+      const float t = waves * ((nbuf == 2 ? std::max(calc, epi) : calc + epi) + 300.f) + (nbuf == 2 ? epi : 0.f);
       if (best.bn == 0 || t < best_t) {
         best_t = t;
         best.bn = bn;
@@ -974,11 +975,11 @@ RowsPlan rows_plan(const ConvArgs& a) {
 
 template <int BN>
 oh_status launch_rows(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArgs& a, const RowsPlan& p,
-                      cudaStream_t st) {
+                      int sms, cudaStream_t st) {
   OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_rows<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
   const int ctiles = a.cout / BN;
   const long long tiles = (long long)a.n * ((a.h + p.c.rows - 1) / p.c.rows) * a.tiles_x;
-  const int gx = (int)std::min(tiles, (long long)std::max(1, sm_count() / ctiles));
+  const int gx = (int)std::min(tiles, (long long)std::max(1, sms / ctiles));
   conv_fwd_rows<BN><<<dim3(gx, ctiles), kRowsThreads, p.smem, st>>>(mX, mW, a, p.c);
   OH_LAUNCH_CHECK();
   return OH_OK;
@@ -1032,17 +1033,18 @@ oh_status conv_enqueue(oh_ctx* ctx, const ConvDesc& d, cudaStream_t st, const ch
   // 3x3 over whole 128-pixel rows
   const char* hv = std::getenv("OH_CONV_HALO");
   if (d.taps == 9 && a.by == 1 && a.bx == 128 && !(hv && std::atoi(hv) == 0)) {
-    const RowsPlan p = rows_plan(a);
+    const int sms = sm_count();
+    const RowsPlan p = rows_plan(a, sms);
     OH_TRY(tc::map_act4d(&mX, d.x, d.cin, d.x_cs, d.w, d.h, d.n, 136, 1));
     OH_TRY(tc::map_taps3d(&mW, d.w_mat, d.cin, d.cout, d.taps, p.bn, 3));
     KernelTimer kt(ctx, timer_name, st);
     switch (p.bn) {
-      case 32: return launch_rows<32>(mX, mW, a, p, st);
-      case 64: return launch_rows<64>(mX, mW, a, p, st);
-      case 96: return launch_rows<96>(mX, mW, a, p, st);
-      case 128: return launch_rows<128>(mX, mW, a, p, st);
-      case 192: return launch_rows<192>(mX, mW, a, p, st);
-      default: return launch_rows<256>(mX, mW, a, p, st);
+      case 32: return launch_rows<32>(mX, mW, a, p, sms, st);
+      case 64: return launch_rows<64>(mX, mW, a, p, sms, st);
+      case 96: return launch_rows<96>(mX, mW, a, p, sms, st);
+      case 128: return launch_rows<128>(mX, mW, a, p, sms, st);
+      case 192: return launch_rows<192>(mX, mW, a, p, sms, st);
+      default: return launch_rows<256>(mX, mW, a, p, sms, st);
     }
   }
   // output-channel tile: all of cout up to 256 (384 as two halves), else the
