@@ -110,9 +110,11 @@ __global__ void pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int f
                     turns * 0.5f * fmaxf(U, V) * fmaxf(U, V) * iz2 < 4.f && fminf(U, V) * fminf(U, V) * iz2 > 1e-25f && fabsf(p.w) < 1e30f &&
                     fabs(o.x) < 1e3 && fabs(o.y) < 1e3 && az < 1e3;
     if (fp64) {
-      // rank-six remainder; terms past p^2 q^2; the axis series' m^7 term
+      // rank-six remainder; terms past p^2 q^2; the axis series' m^7 term; the column
+      // factor (scaled by the row factor's maximum over whole regions) below 0.088
       const float c3 = chi * chi * chi, t = fmaxf(U, V) * iz, t3 = t * t * t;
-      ok = ok && c3 * c3 < 720.f * 1.2e-10f && kf * r0 * (pm * qm) * (pm * qm) * (pm + qm) < 1e-10f &&
+      const float qf = fminf((2.f * DY + (g.ny % kRows ? 3.f * V : -V)) * V * iz2, V * iz + V * V * iz2);
+      ok = ok && 0.25f * kf * r0 * pm * qf < 0.086f && c3 * c3 < 720.f * 1.2e-10f && kf * r0 * (pm * qm) * (pm * qm) * (pm + qm) < 1e-10f &&
            turns * t3 * t3 * t < 3e-11f;
     }
     o.fast = ok ? 1 : 0;
