@@ -19,7 +19,11 @@
 // core truncates each FP32 accumulation (a plain FP16 high/low split in one
 // accumulator lost 2e-5 over 700 points that way), so the products of the
 // multiples of 2^-8 have an accumulator of their own, in which sums up to 256
-// are exact, and the three products with a remainder, 2^-8 of that, another.
+// are exact, and the three products with a remainder, 2^-8 of that, another.  A
+// term adds at most 1.09 (sum over n of chi^n / n!, chi < 0.07, and the rounding),
+// so every 224 points the producers add both accumulators into the partial plane
+// in global memory (L2), which rounds to nearest: in one accumulator 32768
+// points in phase lost 4e-4, now 1.6e-6 (1024 x 1024, 5000 points: 727 -> 745 us).
 //
 // pc_tc_prep decides in FP64 per point whether the dropped terms stay below
 // 1e-6 rad at the worst corner of the plane; other points (near or strongly
@@ -29,9 +33,11 @@
 // 9 forms the per-region records of 32 points at a time (FP64 phases reduced to
 // 32-bit fractions of a turn), warps 0-7 build the operands of four points (K =
 // 32) per stage straight into shared memory in the 64-byte-swizzled layout a TMA
-// load would give, warp 8 issues tcgen05.mma, warps 4-7 read the accumulators.  Splits write partial planes that pc_tc_sum adds in order, so the
-// result does not depend on timing.  Waits are bounded: on timeout the CTA sets
-// the device error word and writes nothing.
+// load would give, warp 8 issues tcgen05.mma; warps 0-7 read the accumulators
+// between stages, while the tensor core waits.  Splits write partial planes that
+// pc_tc_sum adds in order, so the result does not depend on timing.  Waits are
+// bounded: on timeout the CTA sets the device error word and the outputs stay
+// unwritten.
 //
 // What bounds it: the operand producers (53 % of the issue slots) and shared
 // memory (63 %: their stores and the tensor core's operand reads).  16 producer
@@ -56,6 +62,7 @@ constexpr int kTile = 128 * kBK * 2;                   // 8 KB: 128 rows x 32 FP
 constexpr int kStageBytes = 4 * kTile;                 // Ahi, Alo, Bhi, Blo
 constexpr int kAccCols = 128, kTmemCols = 2 * kAccCols;   // exact products, products with remainders
 constexpr int kProducers = 8, kThreads = 32 * (kProducers + 2);
+constexpr int kGroup = 7 * (kBatch / kPts);            // stages (224 points) between additions to the partial plane
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // FP16 in, FP32 out
 
 // One point as a region sees it: phase in turns = frac(t0 + cy m) + rest(m) along
@@ -162,17 +169,6 @@ __global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ i
   if (threadIdx.x == 0) cnt->fast = before;
 }
 
-__device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const int* abort) {
-  const long long t0 = clock64();
-  while (!tc::mb_try(b, parity)) {
-    if (*((volatile const int*)abort) || clock64() - t0 > kWaitCycles) return false;
-  }
-  return true;
-}
-__device__ __forceinline__ void arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
-}
-
 // Byte offset of 16-byte chunk c of row r in a [128][32] FP16 tile with 64-byte swizzle.
 __device__ __forceinline__ int sw_off(int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); }
 
@@ -185,6 +181,28 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t* hi, uint32_t*
   const float2 f = __half22float2(h);
   *hi = h2u(h);
   *lo = h2u(__floats2half2_rn(a - f.x, b - f.y));
+}
+
+// w[k] of lane i of four <- w[i] of lane k
+__device__ __forceinline__ void quad_transpose(float4* w, int lane) {
+  auto swap = [&](float4& keep0, float4& keep1, bool up, int mask) {   // the upper lane sends keep0, the lower keep1
+    const float4 s = up ? keep0 : keep1;
+    const float4 r = make_float4(__shfl_xor_sync(0xffffffffu, s.x, mask), __shfl_xor_sync(0xffffffffu, s.y, mask),
+                                 __shfl_xor_sync(0xffffffffu, s.z, mask), __shfl_xor_sync(0xffffffffu, s.w, mask));
+    if (up) keep0 = r; else keep1 = r;
+  };
+  swap(w[0], w[1], lane & 1, 1);
+  swap(w[2], w[3], lane & 1, 1);
+  swap(w[0], w[2], lane & 2, 2);
+  swap(w[1], w[3], lane & 2, 2);
+}
+__device__ __forceinline__ void red_add4(float2* p, float4 v) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void put2(float2* p, float2 v, bool add) {
+  if (add) asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+  else *p = v;
 }
 
 // turns -> (cos, sin)
@@ -207,10 +225,11 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);
   uint64_t* full = bars;                  // [kStages], one arrival per producer warp
   uint64_t* empty = bars + kStages;       // [kStages], tcgen05.commit
-  uint64_t* done = bars + 2 * kStages;
-  uint64_t* rfull = done + 1;             // [2], the record warp's
-  uint64_t* rempty = done + 3;            // [2], one arrival per producer warp
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 5);
+  uint64_t* rfull = bars + 2 * kStages;   // [2], the record warp's
+  uint64_t* rempty = rfull + 2;           // [2], one arrival per producer warp
+  uint64_t* gdone = rfull + 4;            // a group's products are done (tcgen05.commit)
+  uint64_t* gfree = rfull + 5;            // a group's accumulators are read, one arrival per producer warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rfull + 6);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
   const int nbatch = (nfast + kBatch - 1) / kBatch;
   const int b0 = (int)((long long)blockIdx.y * nbatch / a.splits), b1 = (int)((long long)(blockIdx.y + 1) * nbatch / a.splits);
   const int first = b0 * kBatch, last = min(b1 * kBatch, nfast);
-  const int nst = (last - first + kPts - 1) / kPts;
+  const int nst = (last - first + kPts - 1) / kPts, ngroups = (nst + kGroup - 1) / kGroup;
   float2* part = a.part + (size_t)blockIdx.y * nx * ny;
   if (nfast == 0) return;                 // pc_tc_sum reads no partial plane then
   if (nst <= 0) {
@@ -234,8 +253,9 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { tc::mb_init(&full[s], kProducers); tc::mb_init(&empty[s], 1); }
-    tc::mb_init(done, 1);
     for (int s = 0; s < 2; ++s) { tc::mb_init(&rfull[s], 1); tc::mb_init(&rempty[s], kProducers); }
+    tc::mb_init(gdone, 1);
+    tc::mb_init(gfree, kProducers);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -253,16 +273,52 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
     const int par = rb & 1;
     const int offB0 = sw_off(2 * rb + par, j), offB1 = sw_off(2 * rb + 1 - par, j);
     constexpr int kPer = kBatch / kPts;                // stages per record batch
-    for (int it = 0; it < nst; ++it) {
-      const int s = it % kStages, batch = it / kPer, rs = batch & 1;
-      bool ok = true;
-      if (lane == 0) {
-        if (it % kPer == 0) ok = wait_live(&rfull[rs], (uint32_t)((batch >> 1) & 1), abort_flag);
-        ok = ok && wait_live(&empty[s], (uint32_t)(((it / kStages) & 1) ^ 1), abort_flag);
-        if (!ok) atomicExch(abort_flag, 1);
+    // group g's sums into the partial plane: TMEM lanes 32 (warp % 4) .. (region
+    // rows), 32 complex columns per warp / 4, turned so that four lanes write 64
+    // bytes of a row.  Every value has one writer, so the reductions (no wait for the
+    // old value) keep its order.
+    const int Yq = Y0 + 32 * (warp & 3) + (lane & ~3), Xw = X0 + 32 * (warp >> 2);
+    auto flush = [&](int g) -> bool {
+      if (!warp_wait(gdone, (uint32_t)(g & 1), abort_flag, lane)) return false;
+      tc::fence_after();
+      const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(64 * (warp >> 2));
+#pragma unroll 1
+      for (int c = 0; c < 32; c += 8) {
+        uint32_t v[32];                                  // exact products' sums, then the others'
+        tc::tmem_ld16x2(at + 2 * c, at + kAccCols + 2 * c, v);
+        float4 w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          auto sum = [&](int i) { return __uint_as_float(v[4 * q + i]) + __uint_as_float(v[16 + 4 * q + i]); };
+          w[q] = make_float4(sum(0), sum(1), sum(2), sum(3));
+        }
+        quad_transpose(w, lane);
+        const int X = Xw + c + 2 * (lane & 3);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (Yq + k >= ny || X >= nx) continue;
+          float2* dst = part + (size_t)(Yq + k) * nx + X;
+          if (nx % 2 == 0) {
+            if (g) red_add4(dst, w[k]);
+            else *reinterpret_cast<float4*>(dst) = w[k];
+          } else {
+            put2(dst, make_float2(w[k].x, w[k].y), g);
+            if (X + 1 < nx) put2(dst + 1, make_float2(w[k].z, w[k].w), g);
+          }
+        }
       }
-      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
-      __syncwarp();                       // the record warp's writes, seen by lane 0's wait
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) arrive(gfree);
+      return true;
+    };
+    int flushed = 0;
+    bool ok = true;
+    for (int it = 0; it < nst && ok; ++it) {
+      const int s = it % kStages, batch = it / kPer, rs = batch & 1;
+      if (it % kPer == 0) ok = warp_wait(&rfull[rs], (uint32_t)((batch >> 1) & 1), abort_flag, lane);
+      ok = ok && warp_wait(&empty[s], (uint32_t)(((it / kStages) & 1) ^ 1), abort_flag, lane);
+      if (!ok) break;
       const PcRec q = recs[rs][(it % kPer) * kPts + j];
       unsigned char* sAh = base + s * kStageBytes;
       unsigned char* sAl = sAh + kTile;
@@ -323,30 +379,38 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
         arrive(&full[s]);
         if (it % kPer == kPer - 1) arrive(&rempty[rs]);
       }
+      // a group is read out while its successor's first stages wait for the
+      // tensor core
+      const int next = kGroup * (flushed + 1);
+      if (it >= next && (it == next + 1 || it == nst - 1)) ok = flush(flushed++);
     }
+    while (ok && flushed < ngroups) ok = flush(flushed++);
   } else if (warp == kProducers) {
     if (lane == 0) {
       for (int it = 0; it < nst; ++it) {
         const int s = it % kStages;
-        if (!wait_live(&full[s], (uint32_t)((it / kStages) & 1), abort_flag)) {
+        bool ok = it % kGroup || it == 0 || wait_live(gfree, (uint32_t)((it / kGroup - 1) & 1), abort_flag);
+        ok = ok && wait_live(&full[s], (uint32_t)((it / kStages) & 1), abort_flag);
+        if (!ok) {
           atomicExch(abort_flag, 1);
           break;
         }
         tc::fence_after();
+        const uint32_t add = it % kGroup ? 1u : 0u;     // the group's first stage starts its accumulators
         unsigned char* st0 = base + s * kStageBytes;
         const uint64_t ah = tc::desc_sw64(su32(st0), 16, 512), al = tc::desc_sw64(su32(st0 + kTile), 16, 512);
         const uint64_t bh = tc::desc_sw64(su32(st0 + 2 * kTile), 16, 512), bl = tc::desc_sw64(su32(st0 + 3 * kTile), 16, 512);
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; ++kk) {
           const uint64_t adv = (uint64_t)((kk * 32) >> 4);
-          tc::umma_bf16(tmem, ah + adv, bh + adv, kIdesc, (it | kk) ? 1u : 0u);
-          tc::umma_bf16(tmem + kAccCols, ah + adv, bl + adv, kIdesc, (it | kk) ? 1u : 0u);
+          tc::umma_bf16(tmem, ah + adv, bh + adv, kIdesc, kk ? 1u : add);
+          tc::umma_bf16(tmem + kAccCols, ah + adv, bl + adv, kIdesc, kk ? 1u : add);
           tc::umma_bf16(tmem + kAccCols, al + adv, bh + adv, kIdesc, 1u);
           tc::umma_bf16(tmem + kAccCols, al + adv, bl + adv, kIdesc, 1u);
         }
         tc::umma_commit(&empty[s]);
+        if (it % kGroup == kGroup - 1 || it == nst - 1) tc::umma_commit(gdone);
       }
-      tc::umma_commit(done);              // arrives when every MMA issued above has completed
     }
   } else {
     // record warp: lane k forms point k of each batch
@@ -360,12 +424,7 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
     const int batches = b1 - b0;
     for (int b = 0; b < batches; ++b) {
       const int rs = b & 1;
-      bool ok = true;
-      if (lane == 0) {
-        ok = wait_live(&rempty[rs], (uint32_t)(((b >> 1) & 1) ^ 1), abort_flag);
-        if (!ok) atomicExch(abort_flag, 1);
-      }
-      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
+      if (!warp_wait(&rempty[rs], (uint32_t)(((b >> 1) & 1) ^ 1), abort_flag, lane)) break;
       const int k = first + b * kBatch + lane;
       PcRec r{};
       if (k < last) {
@@ -391,41 +450,19 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
       if (lane == 0) arrive(&rfull[rs]);
     }
   }
-  // epilogue: warps 4-7 own TMEM lanes 32 (warp - 4) .. + 31 = region rows
   __syncwarp();
-  const bool epi = warp >= 4 && warp < 8;
-  bool ok_done = true;
-  if (epi) ok_done = tc::mb_wait(done, 0, kWaitCycles);
-  tc::fence_after();
-  const bool good = __syncthreads_and(ok_done && !*((volatile int*)abort_flag));
-  if (good && epi) {
-    const int Y = Y0 + 32 * (warp - 4) + lane;
-#pragma unroll 1
-    for (int c = 0; c < 2 * kCols / 32; ++c) {
-      uint32_t v[32], lo[32];
-      const uint32_t at = tmem + ((uint32_t)(32 * (warp - 4)) << 16) + (uint32_t)(c * 32);
-      tc::tmem_ld32(at, v);
-      tc::tmem_ld32(at + kAccCols, lo);
-#pragma unroll
-      for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(lo[q]));
-      if (Y < ny) {
-        float2* dst = part + (size_t)Y * nx + X0 + 16 * c;
-        if (nx % 2 == 0) {
-#pragma unroll
-          for (int q = 0; q < 16; q += 2)
-            if (X0 + 16 * c + q < nx)
-              *reinterpret_cast<uint4*>(dst + q) = make_uint4(v[2 * q], v[2 * q + 1], v[2 * q + 2], v[2 * q + 3]);
-        } else {
-#pragma unroll
-          for (int q = 0; q < 16; ++q)
-            if (X0 + 16 * c + q < nx) dst[q] = make_float2(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
-        }
-      }
-    }
-  } else if (!good && threadIdx.x == 0) {
+  const bool good = __syncthreads_and(!*((volatile int*)abort_flag));
+  if (!good && threadIdx.x == 0) {
     atomicOr(a.err, 8);
     atomicOr(&a.cnt->aborted, 1);
-    tc::mb_wait(done, 0, kWaitCycles);    // the MMAs must have finished reading shared memory and TMEM
+  }
+  // after a timeout the issuer's products must have let go of shared memory and
+  // TMEM: one more commit tracks all of them
+  if (!good && threadIdx.x == 32 * kProducers) {
+    tc::mb_init(full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::umma_commit(full);
+    tc::mb_wait(full, 0, kWaitCycles);
   }
   tc::fence_before();
   __syncthreads();

@@ -2,6 +2,7 @@
 // what the FP32 (pc_tc.cu) and FP64 (pc_tc64.cu) forms share.
 #pragma once
 #include "context.h"
+#include "tc_common.cuh"
 
 namespace oh {
 
@@ -50,6 +51,28 @@ oh_status sort_points(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, bo
 // `slots` CTAs best: the fewest up to 8 that reach 95 %, `batches` record batches
 // each at least.
 int point_splits(int regions, int n, int slots, int batches);
+
+__device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const int* abort) {
+  const long long t0 = clock64();
+  while (!tc::mb_try(b, parity)) {
+    if (*((volatile const int*)abort) || clock64() - t0 > kWaitCycles) return false;
+  }
+  return true;
+}
+// the whole warp waits: lane 0 polls; false (and the abort flag) on timeout
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, int* abort, int lane) {
+  bool ok = true;
+  if (lane == 0) {
+    ok = wait_live(b, parity, abort);
+    if (!ok) atomicExch(abort, 1);
+  }
+  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  __syncwarp();
+  return ok;
+}
+__device__ __forceinline__ void arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::su32(b)) : "memory");
+}
 
 // 2^-(e+1) and its inverse, e the exponent of the largest amplitude (kept to
 // normal scales)

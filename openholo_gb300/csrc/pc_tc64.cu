@@ -70,33 +70,6 @@ struct Args {
   int* err;
 };
 
-__device__ __forceinline__ bool wait_live(uint64_t* b, uint32_t parity, const int* abort) {
-  const long long t0 = clock64();
-  while (!tc::mb_try(b, parity)) {
-    if (*((volatile const int*)abort) || clock64() - t0 > kWaitCycles) return false;
-  }
-  return true;
-}
-// the whole warp waits: lane 0 polls; false (and the abort flag) on timeout
-__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, int* abort, int lane) {
-  bool ok = true;
-  if (lane == 0) {
-    ok = wait_live(b, parity, abort);
-    if (!ok) atomicExch(abort, 1);
-  }
-  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-  __syncwarp();
-  return ok;
-}
-__device__ __forceinline__ void arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-
 // Byte offset of point j's 8 bytes (two terms' Re, Im) in K block blk of row r:
 // 64-byte swizzled rows of two blocks of 16 BF16.
 __device__ __forceinline__ int sw_off(int r, int blk, int j) {
@@ -199,17 +172,15 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(2 * c0);
 #pragma unroll 1
       for (int c = 0; c < 16; c += 4) {
-        uint32_t v[4][8];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tmem_ld8(at + k * kAccCols + 2 * c, v[k]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        uint32_t v[32];                                  // eight columns of each accumulator
+        tc::tmem_ld8x4(at + 2 * c, at + kAccCols + 2 * c, at + 2 * kAccCols + 2 * c, at + 3 * kAccCols + 2 * c, v);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           if (Y >= ny || X0 + c0 + c + i >= nx) continue;
           float4 o = g ? dst[c + i] : make_float4(0.f, 0.f, 0.f, 0.f);
           auto add = [&](int k, float h, float l) -> ff {
-            const ff s = ff_sum(__uint_as_float(v[0][k]), __uint_as_float(v[1][k]));
-            const float tail = __uint_as_float(v[2][k]) + __uint_as_float(v[3][k]);
+            const ff s = ff_sum(__uint_as_float(v[k]), __uint_as_float(v[8 + k]));
+            const float tail = __uint_as_float(v[16 + k]) + __uint_as_float(v[24 + k]);
             const ff t = ff_sum(h, s.h);
             return ff_quick(t.h, OH_FADD(OH_FADD(t.l, l), OH_FADD(s.l, tail)));
           };

@@ -1,7 +1,7 @@
 """The point-cloud sum where its tensor-core forms are weakest, against a sum in
 64 bits (r / lambda as z / lambda, reduced in extended precision, plus rho^2 / (r +
 z) / lambda): the corners of planes whose cross phase is as large as the form
-takes.
+takes, and sums that stay in phase over a whole chunk of points.
 
 Each tolerance is the form's own error, derived beside its test; none is larger
 than the error of the direct sum at the same sizes."""
@@ -72,3 +72,15 @@ def test_fp64_corners(ctx, nx, ny):
     pts = cloud(n, nx + ny, np.ones(n))
     rows = rows_of(ny)
     assert float((run(ctx, 1, pts, nx, ny)[rows] - reference(pts, nx, ny, rows)).abs().max()) <= n * 3e-10
+
+
+@pytest.mark.parametrize("nx,ny,n", [(1920, 1080, 32768), (256, 256, 5000), (1024, 1024, 20000)])
+def test_fp32_sums_in_phase(ctx, nx, ny, n):
+    """One point n times over, whole chunks of it in one block where the plane fills the
+    SMs.  One term is off by up to 2e-6 (operands 2^-21 each way, sine and cosine);
+    the sum is taken in n / 224 FP32 additions of 2^-25 each on average."""
+    pts = np.tile(cloud(1, 3, np.ones(1)), (n, 1))
+    rows = rows_of(ny)
+    rel, mx = off(run(ctx, 0, pts, nx, ny)[rows], reference(pts, nx, ny, rows))
+    tol = 2e-6 + (n / 224 + 8) * 2.0 ** -25
+    assert rel <= tol and mx <= 2 * tol
