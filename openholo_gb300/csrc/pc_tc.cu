@@ -25,6 +25,13 @@
 // in global memory (L2), which rounds to nearest: in one accumulator 32768
 // points in phase lost 4e-4, now 1.6e-6 (1024 x 1024, 5000 points: 727 -> 745 us).
 //
+// A point's operand error is 2^-22 of the scale, whatever its amplitude.  pc_tc_split
+// therefore cuts clouds of uneven amplitude into classes with scales S of their own,
+// until sum S^2 over the points is at most 8 times a lower bound of sum a^2: octaves
+// from the largest amplitude down, the last class whatever is left.  Amplitudes spread
+// evenly over 0..1 stay one class.  10000 points at 1 / 100 of one bright point:
+// 3.9e-5 with one scale, 1.5e-6 with two.
+//
 // pc_tc_prep decides in FP64 per point whether the dropped terms stay below
 // 1e-6 rad at the worst corner of the plane; other points (near or strongly
 // off-axis scenes) go to a list that the caller sums directly.
@@ -62,7 +69,8 @@ constexpr int kTile = 128 * kBK * 2;                   // 8 KB: 128 rows x 32 FP
 constexpr int kStageBytes = 4 * kTile;                 // Ahi, Alo, Bhi, Blo
 constexpr int kAccCols = 128, kTmemCols = 2 * kAccCols;   // exact products, products with remainders
 constexpr int kProducers = 8, kThreads = 32 * (kProducers + 2);
-constexpr int kGroup = 7 * (kBatch / kPts);            // stages (224 points) between additions to the partial plane
+constexpr int kGroup = 7;                              // batches (224 points) between additions to the partial plane
+constexpr int kPer = kBatch / kPts;                    // stages per batch
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // FP16 in, FP32 out
 
 // One point as a region sees it: phase in turns = frac(t0 + cy m) + rest(m) along
@@ -78,7 +86,7 @@ struct alignas(16) PcRec {
 struct PcTcArgs {
   PCGeom g;
   const PcPt* pts;
-  const int* list;                 // fast points, unless every point is fast
+  const int* list;                 // fast points by class, unless every point is fast and of one class
   Counts* cnt;
   int n, regions_x, splits;
   float2* part;                    // [splits][ny][nx]
@@ -88,9 +96,11 @@ struct PcTcArgs {
 // Per point: FP64 position, and whether the separable form holds over the whole
 // plane: every dropped term below 1e-6 rad at the plane's worst corner (see the
 // head of this file), fp64: near 1e-10 rad there (see pc_tc64.cu).
-__global__ void pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int fp64, PcPt* __restrict__ pts,
-                           Counts* __restrict__ cnt) {
-  unsigned amax = 0u;
+__global__ void __launch_bounds__(128) pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int fp64,
+                                                  PcPt* __restrict__ pts, Counts* __restrict__ cnt) {
+  __shared__ int hist[256];
+  for (int i = threadIdx.x; i < 256; i += 128) hist[i] = 0;
+  __syncthreads();
   int slow = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const float4 p = in[j];
@@ -125,48 +135,104 @@ __global__ void pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int f
            turns * t3 * t3 * t < 3e-11f;
     }
     o.fast = ok ? 1 : 0;
-    if (ok) amax = max(amax, __float_as_uint(fabsf(p.w)));
+    if (ok) atomicAdd(&hist[__float_as_uint(fabsf(p.w)) >> 23], 1);
     else ++slow;
     pts[j] = o;
   }
-  amax = __reduce_max_sync(0xffffffffu, amax);
   slow = __reduce_add_sync(0xffffffffu, slow);
-  if ((threadIdx.x & 31) == 0) {
-    if (amax) atomicMax(&cnt->amax, amax);
-    if (slow) atomicAdd(&cnt->slow, slow);
-  }
+  if ((threadIdx.x & 31) == 0 && slow) atomicAdd(&cnt->slow, slow);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 256; i += 128)
+    if (hist[i]) atomicAdd(&cnt->hist[i], hist[i]);
 }
 
-// One block: the fast points' indices and the slow points in input order.  With
-// no slow point the index list stays unwritten (and unread).
+// One block: the classes (see Counts and the head of this file), then the fast points'
+// indices by class and the slow points, both in input order.  With one class and no
+// slow point the index list stays unwritten (and unread).
 __global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ in, const PcPt* __restrict__ pts, int n,
                                                     int* __restrict__ list, float4* __restrict__ slow,
                                                     Counts* __restrict__ cnt) {
-  __shared__ int wsum[32];
-  if (cnt->slow == 0) {
-    if (threadIdx.x == 0) cnt->fast = n;
-    return;
+  __shared__ int hist[256], exps[kMaxCls], first[kMaxCls + 1], count[kMaxCls], next[kMaxCls + 1], wsum[32][kMaxCls + 1];
+  __shared__ int s_ncls;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 256) hist[threadIdx.x] = cnt->hist[threadIdx.x];
+  __syncthreads();
+  if (warp == 0) {
+    unsigned word[8];                                   // the exponents that occur
+#pragma unroll
+    for (int i = 0; i < 8; ++i) word[i] = __ballot_sync(0xffffffffu, hist[32 * i + lane] != 0);
+    if (lane == 0) {
+      auto each = [&](auto f) {                         // from the largest down, until f is false
+#pragma unroll
+        for (int i = 7; i >= 0; --i)
+          for (unsigned m = word[i]; m; m &= ~(0x80000000u >> __clz(m)))
+            if (!f(32 * i + 31 - __clz(m))) return;
+      };
+      int top = -1, rest = 0, c = 0, slot = 0;
+      float left = 0.f;                                 // of sum S^2, in units of 4^top
+      each([&](int e) {
+        if (top < 0) top = e;
+        rest += hist[e];
+        left += 8.f * (float)hist[e] * pow2f(2 * (e - top));
+        return true;
+      });
+      each([&](int e) {
+        const float S2 = 4.f * pow2f(2 * (e - top));
+        const bool all = S2 * (float)rest <= left || c == kMaxCls - 1;
+        exps[c] = e;
+        first[c] = slot;
+        count[c] = all ? rest : hist[e];
+        cnt->exp[c] = e;
+        cnt->batch[c] = slot / kBatch;
+        slot += all ? rest : (hist[e] + kBatch - 1) / kBatch * kBatch;
+        left -= S2 * (float)hist[e];
+        rest -= count[c];
+        ++c;
+        return !all;
+      });
+      s_ncls = c;
+      cnt->ncls = c;
+      cnt->batch[c] = (slot + kBatch - 1) / kBatch;
+      cnt->fast = slot;
+    }
   }
-  int before = 0;                                     // fast points of earlier rounds
+  __syncthreads();
+  const int ncls = s_ncls;
+  if (cnt->slow == 0 && ncls <= 1) return;
+  if (threadIdx.x <= kMaxCls) next[threadIdx.x] = threadIdx.x < ncls ? first[threadIdx.x] : 0;     // [kMaxCls]: slow points
+  for (int c = 0; c + 1 < ncls; ++c)
+    for (int i = first[c] + count[c] + threadIdx.x; i < first[c + 1]; i += 1024) list[i] = -1;
+  __syncthreads();
   for (int base = 0; base < n; base += 1024) {
     const int j = base + threadIdx.x;
-    const bool in_range = j < n;
-    const bool f = in_range && pts[j].fast;
-    const unsigned m = __ballot_sync(0xffffffffu, f);
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = __popc(m);
-    __syncthreads();
-    int pre = before, all = 0;
-    for (int w = 0; w < 32; ++w) {
-      if (w < (int)(threadIdx.x >> 5)) pre += wsum[w];
-      all += wsum[w];
+    int c = kMaxCls + 1;                                // none
+    if (j < n) {
+      c = kMaxCls;
+      if (pts[j].fast) {
+        const int e = (int)(__float_as_uint(fabsf(pts[j].a)) >> 23);
+        for (c = 0; c + 1 < ncls && exps[c + 1] >= e;) ++c;
+      }
     }
-    pre += __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
-    if (f) list[pre] = j;
-    else if (in_range) slow[j - pre] = in[j];
-    before += all;
+    const unsigned same = __match_any_sync(0xffffffffu, c);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (lane <= kMaxCls) wsum[warp][lane] = 0;
+    __syncwarp();
+    if (rank == 0 && c <= kMaxCls) wsum[warp][c] = __popc(same);
+    __syncthreads();
+    if (c <= kMaxCls) {
+      int at = next[c] + rank;
+      for (int w = 0; w < warp; ++w) at += wsum[w][c];
+      if (c < kMaxCls) list[at] = j;
+      else slow[at] = in[j];
+    }
+    __syncthreads();
+    if (threadIdx.x <= kMaxCls) {
+      int t = next[threadIdx.x];
+      for (int w = 0; w < 32; ++w) t += wsum[w][threadIdx.x];
+      next[threadIdx.x] = t;
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) cnt->fast = before;
 }
 
 // Byte offset of 16-byte chunk c of row r in a [128][32] FP16 tile with 64-byte swizzle.
@@ -220,6 +286,7 @@ __device__ __forceinline__ float cross_arg(float w) { return w * fmaf(w, fmaf(w,
 __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ PcRec recs[2][kBatch];
+  __shared__ int cls_batch[kMaxCls + 1], cls_e[kMaxCls];
   const uint32_t raw = su32(smem_dyn);
   unsigned char* base = smem_dyn + (((raw + 1023u) & ~1023u) - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);
@@ -236,11 +303,12 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
   const int X0 = (blockIdx.x % a.regions_x) * kCols, Y0 = (blockIdx.x / a.regions_x) * kRows;
   const int nx = a.g.nx, ny = a.g.ny;
   const int nfast = a.cnt->fast;
-  const bool identity = a.cnt->slow == 0;
+  const int ncls = a.cnt->ncls;
+  const bool identity = a.cnt->slow == 0 && ncls == 1;
   const int nbatch = (nfast + kBatch - 1) / kBatch;
   const int b0 = (int)((long long)blockIdx.y * nbatch / a.splits), b1 = (int)((long long)(blockIdx.y + 1) * nbatch / a.splits);
   const int first = b0 * kBatch, last = min(b1 * kBatch, nfast);
-  const int nst = (last - first + kPts - 1) / kPts, ngroups = (nst + kGroup - 1) / kGroup;
+  const int nst = (last - first + kPts - 1) / kPts;
   float2* part = a.part + (size_t)blockIdx.y * nx * ny;
   if (nfast == 0) return;                 // pc_tc_sum reads no partial plane then
   if (nst <= 0) {
@@ -259,6 +327,8 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x <= ncls) cls_batch[threadIdx.x] = a.cnt->batch[threadIdx.x];
+  if (threadIdx.x < ncls) cls_e[threadIdx.x] = class_exp(a.cnt->exp[threadIdx.x]);
   if (warp == 1) tc::tmem_alloc(tmem_slot, kTmemCols);
   tc::fence_before();
   __syncthreads();
@@ -272,13 +342,12 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
     // the two B rows of a column, in an order that spreads a quarter-warp over the banks
     const int par = rb & 1;
     const int offB0 = sw_off(2 * rb + par, j), offB1 = sw_off(2 * rb + 1 - par, j);
-    constexpr int kPer = kBatch / kPts;                // stages per record batch
     // group g's sums into the partial plane: TMEM lanes 32 (warp % 4) .. (region
     // rows), 32 complex columns per warp / 4, turned so that four lanes write 64
     // bytes of a row.  Every value has one writer, so the reductions (no wait for the
     // old value) keep its order.
     const int Yq = Y0 + 32 * (warp & 3) + (lane & ~3), Xw = X0 + 32 * (warp >> 2);
-    auto flush = [&](int g) -> bool {
+    auto flush = [&](int g, float rel) -> bool {         // rel: the group's scale over the first class's
       if (!warp_wait(gdone, (uint32_t)(g & 1), abort_flag, lane)) return false;
       tc::fence_after();
       const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(64 * (warp >> 2));
@@ -289,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
         float4 w[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          auto sum = [&](int i) { return __uint_as_float(v[4 * q + i]) + __uint_as_float(v[16 + 4 * q + i]); };
+          auto sum = [&](int i) { return rel * (__uint_as_float(v[4 * q + i]) + __uint_as_float(v[16 + 4 * q + i])); };
           w[q] = make_float4(sum(0), sum(1), sum(2), sum(3));
         }
         quad_transpose(w, lane);
@@ -312,7 +381,9 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
       if (lane == 0) arrive(gfree);
       return true;
     };
-    int flushed = 0;
+    Groups gr{cls_batch, ncls, b1, kGroup, 0, 0};       // the oldest group not read out
+    gr.start(b0);
+    int g = 0;
     bool ok = true;
     for (int it = 0; it < nst && ok; ++it) {
       const int s = it % kStages, batch = it / kPer, rs = batch & 1;
@@ -381,22 +452,35 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
       }
       // a group is read out while its successor's first stages wait for the
       // tensor core
-      const int next = kGroup * (flushed + 1);
-      if (it >= next && (it == next + 1 || it == nst - 1)) ok = flush(flushed++);
+      const int next = (gr.end - b0) * kPer;
+      if (it >= next && (it == next + 1 || it == nst - 1)) {
+        ok = flush(g++, pow2f(cls_e[gr.c] - cls_e[0]));
+        gr.start(gr.end);
+      }
     }
-    while (ok && flushed < ngroups) ok = flush(flushed++);
+    if (ok) flush(g, pow2f(cls_e[gr.c] - cls_e[0]));
   } else if (warp == kProducers) {
     if (lane == 0) {
+      Groups gr{cls_batch, ncls, b1, kGroup, 0, 0};
+      gr.start(b0);
+      int next = min(nst, (gr.end - b0) * kPer);
+      uint32_t add = 0u, gph = 0u;        // the group's first stage starts its accumulators
       for (int it = 0; it < nst; ++it) {
         const int s = it % kStages;
-        bool ok = it % kGroup || it == 0 || wait_live(gfree, (uint32_t)((it / kGroup - 1) & 1), abort_flag);
+        bool ok = true;
+        if (it == next) {
+          ok = wait_live(gfree, gph, abort_flag);
+          gph ^= 1u;
+          gr.start(gr.end);
+          next = min(nst, (gr.end - b0) * kPer);
+          add = 0u;
+        }
         ok = ok && wait_live(&full[s], (uint32_t)((it / kStages) & 1), abort_flag);
         if (!ok) {
           atomicExch(abort_flag, 1);
           break;
         }
         tc::fence_after();
-        const uint32_t add = it % kGroup ? 1u : 0u;     // the group's first stage starts its accumulators
         unsigned char* st0 = base + s * kStageBytes;
         const uint64_t ah = tc::desc_sw64(su32(st0), 16, 512), al = tc::desc_sw64(su32(st0 + kTile), 16, 512);
         const uint64_t bh = tc::desc_sw64(su32(st0 + 2 * kTile), 16, 512), bl = tc::desc_sw64(su32(st0 + 3 * kTile), 16, 512);
@@ -408,8 +492,9 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
           tc::umma_bf16(tmem + kAccCols, al + adv, bh + adv, kIdesc, 1u);
           tc::umma_bf16(tmem + kAccCols, al + adv, bl + adv, kIdesc, 1u);
         }
+        add = 1u;
         tc::umma_commit(&empty[s]);
-        if (it % kGroup == kGroup - 1 || it == nst - 1) tc::umma_commit(gdone);
+        if (it == next - 1) tc::umma_commit(gdone);
       }
     }
   } else {
@@ -418,8 +503,7 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
     const double Xc = ((double)(X0 + kCols / 2) + 0.5) * a.g.px - a.g.hlx;
     const double Yc = a.g.hly - ((double)(Y0 + kRows / 2) + 0.5) * a.g.py;
     const double ref = Xc * a.g.stx + Yc * a.g.sty;
-    float unscale;
-    const float scale = amp_scale(a.cnt->amax, &unscale);
+    int c = 0;
     auto frac32 = [](double t) { return (int)__double2ll_rn((t - rint(t)) * 4294967296.0); };
     const int batches = b1 - b0;
     for (int b = 0; b < batches; ++b) {
@@ -427,8 +511,10 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
       if (!warp_wait(&rempty[rs], (uint32_t)(((b >> 1) & 1) ^ 1), abort_flag, lane)) break;
       const int k = first + b * kBatch + lane;
       PcRec r{};
-      if (k < last) {
-        const PcPt p = a.pts[identity ? k : a.list[k]];
+      while (c + 1 < ncls && cls_batch[c + 1] <= b0 + b) ++c;
+      const int at = k < last ? identity ? k : a.list[k] : -1;
+      if (at >= 0) {
+        const PcPt p = a.pts[at];
         const double dx = Xc - p.x, dy = Yc - p.y;
         const double r2 = fma(dx, dx, fma(dy, dy, p.z * p.z));
         const double ri = rsqrt(r2), r0 = r2 * ri;
@@ -437,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
         r.cx = frac32((sx - a.g.stx) * a.g.px * il);
         r.cy = frac32((a.g.sty - sy) * a.g.py * il);
         const float rif = (float)ri, pxr = (float)a.g.px * rif, pyr = (float)a.g.py * rif;
-        r.amp = p.a * scale;
+        r.amp = p.a * pow2f(-cls_e[c]);
         r.c0 = (float)(r0 * il);
         r.ax = 2.f * (float)sx * pxr; r.bx = pxr * pxr;
         r.ay = -2.f * (float)sy * pyr; r.by = pyr * pyr;
@@ -479,8 +565,7 @@ __global__ void __launch_bounds__(256) pc_tc_sum(const float2* __restrict__ part
                                                  float2* __restrict__ field, float* __restrict__ fringe, int accumulate) {
   if (cnt->aborted) return;
   const bool none = cnt->fast == 0;
-  float unscale;
-  amp_scale(cnt->amax, &unscale);
+  const float unscale = pow2f(class_exp(cnt->exp[0]));
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     float2 v = make_float2(0.f, 0.f);
     if (!none)
@@ -498,18 +583,19 @@ namespace pctc {
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t sorted_bytes(int n) {
-  return 256 + align256((size_t)n * sizeof(PcPt)) + align256((size_t)n * sizeof(int)) + align256((size_t)n * sizeof(float4));
+  return align256(sizeof(Counts)) + align256((size_t)n * sizeof(PcPt)) +
+         align256(((size_t)n + kMaxCls * kBatch) * sizeof(int)) + align256((size_t)n * sizeof(float4));
 }
 
 oh_status sort_points(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, bool fp64, void* base, Sorted* out,
                       cudaStream_t st) {
   char* p = static_cast<char*>(base);
   out->cnt = (Counts*)p;
-  p += 256;
+  p += align256(sizeof(Counts));
   out->pts = (PcPt*)p;
   p += align256((size_t)n * sizeof(PcPt));
   out->list = (int*)p;
-  p += align256((size_t)n * sizeof(int));
+  p += align256(((size_t)n + kMaxCls * kBatch) * sizeof(int));
   out->slow = (float4*)p;
   OH_CUDA_TRY(cudaMemsetAsync(out->cnt, 0, sizeof(Counts), st));
   KernelTimer kt(ctx, "pc_tc_prep", st);

@@ -32,13 +32,23 @@ constexpr int kPts = 4;                                // points per operand sta
 constexpr int kBatch = 32;                             // points per record batch
 constexpr long long kWaitCycles = 2000000000LL;
 
+constexpr int kMaxCls = 12;
+
 struct PcPt { double x, y, z; float a; int fast; };
-struct Counts { int fast, slow; unsigned amax; int aborted; };
+// A chunk's points as pc_tc_split orders them.  The separable ones come in classes of
+// like amplitude, each with a scale of its own (operands are fixed point): class c
+// has the batches [batch[c], batch[c + 1]) and amplitudes below 2^(exp[c] - 126).
+struct Counts {
+  int fast;                        // list slots; every class but the last fills whole batches
+  int slow, aborted, ncls;
+  int batch[kMaxCls + 1], exp[kMaxCls];
+  int hist[256];                   // separable points by the exponent of their amplitude
+};
 
 // A chunk's points, sorted into separable and other ones (device memory).
 struct Sorted {
   PcPt* pts;
-  int* list;                       // separable points, unless every point is
+  int* list;                       // separable points (-1: none), unless all are in one class
   float4* slow;
   Counts* cnt;
 };
@@ -74,14 +84,22 @@ __device__ __forceinline__ void arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::su32(b)) : "memory");
 }
 
-// 2^-(e+1) and its inverse, e the exponent of the largest amplitude (kept to
-// normal scales)
-__device__ __forceinline__ float amp_scale(unsigned amax, float* inv) {
-  int e = (int)(amax >> 23) - 126;
-  e = amax == 0u ? 0 : max(-100, min(100, e));
-  *inv = __int_as_float((127 + e) << 23);
-  return __int_as_float((127 - e) << 23);
-}
+// A CTA's batches [b, b1) in groups: at most `most` batches of one class.
+struct Groups {
+  const int* batch;                // Counts::batch
+  int ncls, b1, most;
+  int c, end;                      // class and end of the current group
+  __device__ __forceinline__ void start(int b) {
+    while (c + 1 < ncls && batch[c + 1] <= b) ++c;
+    end = min(b1, b + most);
+    if (c + 1 < ncls) end = min(end, batch[c + 1]);
+  }
+};
+
+// Exponent of a class's scale: amplitudes times 2^-class_exp are at most one (kept to
+// normal scales).
+__device__ __forceinline__ int class_exp(int exp) { return max(-100, min(100, exp - 126)); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float(max(127 + e, 0) << 23); }
 
 }  // namespace pctc
 

@@ -20,7 +20,8 @@
 // within 24 bits of their common step and are exact, and one for the rest
 // (2^-25 and below).  Every 96 points the producers add the four into a
 // two-float partial plane in global memory (L2); pc_tc_sum64 adds the splits'
-// planes and converts.  Against a 64-bit sum with r / lambda to extended
+// planes and converts.  Steps are fixed relative to a class's scale (pc_tc_split): clouds of
+// uneven amplitude get a scale per class.  Against a 64-bit sum with r / lambda to extended
 // precision: 1.4e-12 (1024x1024, 5000 points; the direct kernel 8e-11).
 //
 // One CTA per region and split of the points, one per SM (TMEM full), 26 warps:
@@ -53,7 +54,7 @@ constexpr int kTile = 128 * 32 * 2;
 constexpr int kStages = 2, kStageBytes = 2 * kTiles * kTile;
 constexpr int kAccCols = 128, kTmemCols = 4 * kAccCols;
 constexpr int kAWarps = 16, kBWarps = 8, kThreads = 32 * (kAWarps + kBWarps + 2);
-constexpr int kFlush = 24;                             // stages (96 points) between additions to the partial plane
+constexpr int kGroup = 3;                              // batches (96 points) between additions to the partial plane
 constexpr uint32_t kIdesc = tc::idesc_bf16(128, 128, 0, 0);
 
 struct alignas(16) RecA { uint64_t t0, c1, c2, c3, c4; float c5, c6; ff a, b; float amp, qs; };
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
   __shared__ float4 tab[256];
   __shared__ RecA recA[2][kBatch];
   __shared__ RecB recB[2][kBatch];
+  __shared__ int cls_batch[kMaxCls + 1], cls_e[kMaxCls];
   const uint32_t raw = su32(smem_dyn);
   unsigned char* base = smem_dyn + (((raw + 1023u) & ~1023u) - raw);
   uint64_t* full = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);   // [2], one arrival per producer warp
@@ -120,11 +122,12 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
   const int X0 = (blockIdx.x % a.regions_x) * kCols, Y0 = (blockIdx.x / a.regions_x) * kRows;
   const int nx = a.g.nx, ny = a.g.ny;
   const int nfast = a.cnt->fast;
-  const bool identity = a.cnt->slow == 0;
+  const int ncls = a.cnt->ncls;
+  const bool identity = a.cnt->slow == 0 && ncls == 1;
   const int nbatch = (nfast + kBatch - 1) / kBatch;
   const int b0 = (int)((long long)blockIdx.y * nbatch / a.splits), b1 = (int)((long long)(blockIdx.y + 1) * nbatch / a.splits);
   const int first = b0 * kBatch, last = min(b1 * kBatch, nfast);
-  const int nst = (last - first + kPts - 1) / kPts, ngroups = (nst + kFlush - 1) / kFlush;
+  const int nst = (last - first + kPts - 1) / kPts;
   constexpr int kPer = kBatch / kPts;     // stages per record batch
   float4* part = a.part + (size_t)blockIdx.y * nx * ny;
   if (nfast == 0) return;                 // pc_tc_sum64 reads no partial plane then
@@ -149,6 +152,8 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   ff_directions(tab, threadIdx.x, kThreads);
+  if (threadIdx.x <= ncls) cls_batch[threadIdx.x] = a.cnt->batch[threadIdx.x];
+  if (threadIdx.x < ncls) cls_e[threadIdx.x] = class_exp(a.cnt->exp[threadIdx.x]);
   if (warp == 1) tc::tmem_alloc(tmem_slot, kTmemCols);
   tc::fence_before();
   __syncthreads();
@@ -165,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
     // group g's sums into the partial plane: TMEM lanes 32 (warp % 4) .. (region
     // rows), 16 complex columns per warp / 4
     const int Y = Y0 + 32 * (warp & 3) + lane, c0 = 16 * (warp >> 2);
-    auto flush = [&](int g) -> bool {
+    auto flush = [&](int g, float rel) -> bool {         // rel: the group's scale over the first class's
       if (!warp_wait(gdone, (uint32_t)(g & 1), abort_flag, lane)) return false;
       tc::fence_after();
       float4* dst = part + (size_t)Y * nx + X0 + c0;
@@ -181,8 +186,8 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
           auto add = [&](int k, float h, float l) -> ff {
             const ff s = ff_sum(__uint_as_float(v[k]), __uint_as_float(v[8 + k]));
             const float tail = __uint_as_float(v[16 + k]) + __uint_as_float(v[24 + k]);
-            const ff t = ff_sum(h, s.h);
-            return ff_quick(t.h, OH_FADD(OH_FADD(t.l, l), OH_FADD(s.l, tail)));
+            const ff t = ff_sum(h, OH_FMUL(rel, s.h));
+            return ff_quick(t.h, OH_FADD(OH_FADD(t.l, l), OH_FMUL(rel, OH_FADD(s.l, tail))));
           };
           const ff re = add(2 * i, o.x, o.y), im = add(2 * i + 1, o.z, o.w);
           dst[c + i] = make_float4(re.h, re.l, im.h, im.l);
@@ -193,7 +198,9 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       if (lane == 0) arrive(gfree);
       return true;
     };
-    int flushed = 0;
+    Groups gr{cls_batch, ncls, b1, kGroup, 0, 0};       // the oldest group not read out
+    gr.start(b0);
+    int g = 0;
     bool ok = true;
     for (int it = 0; it < nst && ok; ++it) {
       const int s = it & 1, batch = it / kPer, rs = batch & 1;
@@ -242,10 +249,13 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       }
       // a group is read out while its successor's first stages wait for the
       // tensor core
-      const int next = kFlush * (flushed + 1);
-      if (it >= next && (it == next + 1 || it == nst - 1)) ok = flush(flushed++);
+      const int next = (gr.end - b0) * kPer;
+      if (it >= next && (it == next + 1 || it == nst - 1)) {
+        ok = flush(g++, pow2f(cls_e[gr.c] - cls_e[0]));
+        gr.start(gr.end);
+      }
     }
-    while (ok && flushed < ngroups) ok = flush(flushed++);
+    if (ok) flush(g, pow2f(cls_e[gr.c] - cls_e[0]));
   } else if (warp < kAWarps + kBWarps) {
     // B: point slot j of column x; rows 2x (Re, -Im) and 2x + 1 (Im, Re)
     const int t = threadIdx.x - 32 * kAWarps, j = t & 3, x = t >> 2, m = x - kCols / 2;
@@ -307,9 +317,20 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
     }
   } else if (warp == kAWarps + kBWarps) {
     if (lane == 0) {
+      Groups gr{cls_batch, ncls, b1, kGroup, 0, 0};
+      gr.start(b0);
+      int next = min(nst, (gr.end - b0) * kPer);
+      uint32_t add = 0u, gph = 0u;        // the group's first stage starts its accumulators
       for (int it = 0; it < nst; ++it) {
-        const int s = it & 1, gi = it / kFlush;
-        bool ok = it % kFlush || it == 0 || wait_live(gfree, (uint32_t)((gi - 1) & 1), abort_flag);
+        const int s = it & 1;
+        bool ok = true;
+        if (it == next) {
+          ok = wait_live(gfree, gph, abort_flag);
+          gph ^= 1u;
+          gr.start(gr.end);
+          next = min(nst, (gr.end - b0) * kPer);
+          add = 0u;
+        }
         ok = ok && wait_live(&full[s], (uint32_t)((it >> 1) & 1), abort_flag);
         if (!ok) {
           atomicExch(abort_flag, 1);
@@ -317,7 +338,6 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
         }
         tc::fence_after();
         const uint32_t A = su32(base + s * kStageBytes), B = A + kTiles * kTile;
-        const uint32_t add = it % kFlush ? 1u : 0u;     // the group's first stage starts its accumulators
         const uint64_t dA = tc::desc_sw64(A, 16, 512), dB = tc::desc_sw64(B, 16, 512);
         // (unrolled: 28 products a stage, 64 clocks each, leave one thread no
         // time for address arithmetic)
@@ -328,8 +348,9 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
           tc::umma_bf16(tmem + op.acc * kAccCols, dA + (uint64_t)(op.at * (kTile >> 4) + op.ab * 2),
                         dB + (uint64_t)(op.bt * (kTile >> 4) + op.bb * 2), kIdesc, start ? add : 1u);
         }
+        add = 1u;
         tc::umma_commit(&empty[s]);
-        if (it % kFlush == kFlush - 1 || it == nst - 1) tc::umma_commit(gdone);
+        if (it == next - 1) tc::umma_commit(gdone);
       }
     }
   } else {
@@ -337,8 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
     const double Xc = ((double)(X0 + kCols / 2) + 0.5) * a.g.px - a.g.hlx;
     const double Yc = a.g.hly - ((double)(Y0 + kRows / 2) + 0.5) * a.g.py;
     const double ref = (Xc * a.g.stx + Yc * a.g.sty) * a.il;
-    float unscale;
-    const float scale = amp_scale(a.cnt->amax, &unscale);
+    int c = 0;
     auto fix64 = [](double t) { return (uint64_t)__double2ll_rn((t - rint(t)) * 9223372036854775808.0) << 1; };
     const int batches = b1 - b0;
     for (int b = 0; b < batches; ++b) {
@@ -348,8 +368,10 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
       RecA ra{};
       RecB rb{};
       ra.qs = 1.f;
-      if (k < last) {
-        const PcPt p = a.pts[identity ? k : a.list[k]];
+      while (c + 1 < ncls && cls_batch[c + 1] <= b0 + b) ++c;
+      const int at = k < last ? identity ? k : a.list[k] : -1;
+      if (at >= 0) {
+        const PcPt p = a.pts[at];
         const double dx = Xc - p.x, dy = Yc - p.y, az = fabs(p.z);
         const double rho2 = fma(dx, dx, dy * dy), r2 = fma(az, az, rho2);
         const double ri = rsqrt(r2), r0 = r2 * ri;
@@ -382,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) pc_tc64_regions(Args a) {
         const double qs = (double)(float)(1.01 * (fabs(ay) * (kRows / 2) + by * (kRows / 2) * (kRows / 2))), iqs = 1.0 / qs;
         ra.a = ff(ay * iqs); ra.b = ff(by * iqs);
         ra.qs = (float)qs;
-        ra.amp = p.a * scale;
+        ra.amp = p.a * pow2f(-cls_e[c]);
         rb.a = ff(2.0 * sx * tx); rb.b = ff(tx * tx);
         const double kr = 6.283185307179586476925286766559 * C;
         rb.kq = ff(-0.25 * kr * qs);
@@ -422,8 +444,7 @@ __global__ void __launch_bounds__(256) pc_tc_sum64(const float4* __restrict__ pa
                                                    double* __restrict__ fringe, int accumulate) {
   if (cnt->aborted) return;
   const bool none = cnt->fast == 0;
-  float unscale;
-  amp_scale(cnt->amax, &unscale);
+  const float unscale = pow2f(class_exp(cnt->exp[0]));
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     ff re{0.f, 0.f}, im{0.f, 0.f};
     if (!none)

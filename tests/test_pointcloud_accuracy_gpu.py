@@ -84,3 +84,25 @@ def test_fp32_sums_in_phase(ctx, nx, ny, n):
     rel, mx = off(run(ctx, 0, pts, nx, ny)[rows], reference(pts, nx, ny, rows))
     tol = 2e-6 + (n / 224 + 8) * 2.0 ** -25
     assert rel <= tol and mx <= 2 * tol
+
+
+def uneven(kind, n):
+    rng = np.random.default_rng(n)
+    if kind == "bright":
+        return np.where(np.arange(n) == n // 2, 1.0, 0.01)
+    if kind == "two_levels":
+        return np.where(np.arange(n) % 50 == 7, 1.0, 2e-3)
+    return np.exp(2.0 * rng.standard_normal(n))
+
+
+@pytest.mark.parametrize("kind,n,nx,ny", [("bright", 10001, 640, 480), ("bright", 2500, 300, 200),
+                                          ("two_levels", 6000, 300, 200), ("lognormal", 5000, 640, 480),
+                                          ("lognormal", 33000, 130, 129)])
+def test_uneven_amplitudes(ctx, kind, n, nx, ny):
+    """A point's operands are off by 2^-22 of its group's scale, and a group's scales add
+    up to at most sqrt(8) of the sum's L2 norm: 6e-7, with the rest below 2e-6.  FP64: 1e-11."""
+    pts = cloud(n, n, uneven(kind, n))
+    rows = rows_of(ny)
+    ref = reference(pts, nx, ny, rows)
+    assert off(run(ctx, 0, pts, nx, ny)[rows], ref)[0] <= 2e-6
+    assert off(run(ctx, 1, pts, nx, ny)[rows], ref)[0] <= 1e-11
