@@ -15,7 +15,9 @@
 // product C = A B^T with M = 128, N = 128 and K = 8 per point.
 //
 // Operands (amplitudes scaled by a power of two to at most one) are split into
-// a multiple of 2^-8 and an FP16 remainder (absolute error 2^-21).  The tensor
+// a multiple of 2^-8 and an FP16 remainder (absolute error 2^-21) and, where FINE asks
+// for it, the FP16 rest of that (2^-25; six products instead of four, sine and cosine
+// to 2^-23 instead of 2^-21: 1.2e-7 against 7.3e-7 of the L2 norm).  The tensor
 // core truncates each FP32 accumulation (a plain FP16 high/low split in one
 // accumulator lost 2e-5 over 700 points that way), so the products of the
 // multiples of 2^-8 have an accumulator of their own, in which sums up to 256
@@ -23,14 +25,14 @@
 // term adds at most 1.09 (sum over n of chi^n / n!, chi < 0.07, and the rounding),
 // so every 224 points the producers add both accumulators into the partial plane
 // in global memory (L2), which rounds to nearest: in one accumulator 32768
-// points in phase lost 4e-4, now 1.6e-6 (1024 x 1024, 5000 points: 727 -> 745 us).
+// points in phase lost 4e-4, now 1.4e-6 (1024 x 1024, 5000 points: 727 -> 745 us).
 //
 // A point's operand error is 2^-22 of the scale, whatever its amplitude.  pc_tc_split
 // therefore cuts clouds of uneven amplitude into classes with scales S of their own,
 // until sum S^2 over the points is at most 8 times a lower bound of sum a^2: octaves
 // from the largest amplitude down, the last class whatever is left.  Amplitudes spread
 // evenly over 0..1 stay one class.  10000 points at 1 / 100 of one bright point:
-// 3.9e-5 with one scale, 1.5e-6 with two.
+// 3.9e-5 with one scale, 7e-7 with two.
 //
 // pc_tc_prep decides in FP64 per point whether the dropped terms stay below
 // 1e-6 rad at the worst corner of the plane; other points (near or strongly
@@ -48,8 +50,9 @@
 //
 // What bounds it: the operand producers (53 % of the issue slots) and shared
 // memory (63 %: their stores and the tensor core's operand reads).  16 producer
-// warps in two groups were slower (0.79 against 0.73 ms: spills and spinning
-// waits).
+// warps in two groups were 8 % slower (spills and spinning waits).  1024 x 1024 x 5000
+// points: 790 us with two-part operands (5.74 ms directly), 988 with three; the phase
+// in whole numbers takes 45 us of it, in floats its square term left 1.3e-6.
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cmath>
@@ -66,21 +69,24 @@ using tc::su32;
 constexpr int kBK = 8 * kPts;                          // K per stage
 constexpr int kStages = 2;
 constexpr int kTile = 128 * kBK * 2;                   // 8 KB: 128 rows x 32 FP16
-constexpr int kStageBytes = 4 * kTile;                 // Ahi, Alo, Bhi, Blo
+template <bool FINE> constexpr int kParts = FINE ? 3 : 2;         // parts of an operand
+template <bool FINE> constexpr int kStageBytes = 2 * kParts<FINE> * kTile;         // A's parts, then B's
 constexpr int kAccCols = 128, kTmemCols = 2 * kAccCols;   // exact products, products with remainders
 constexpr int kProducers = 8, kThreads = 32 * (kProducers + 2);
 constexpr int kGroup = 7;                              // batches (224 points) between additions to the partial plane
 constexpr int kPer = kBatch / kPts;                    // stages per batch
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // FP16 in, FP32 out
 
-// One point as a region sees it: phase in turns = frac(t0 + cy m) + rest(m) along
-// the rows (m = row - 64), the same with cx along the columns (m = column - 32,
-// no t0).
+// One point as a region sees it: phase in turns = frac(t0 + m (cy + m c2y)) + m^2 qy +
+// rest(m) along the rows (m = row - 64), the same with cx, c2x, qx along the columns
+// (m = column - 32, no t0).
 struct alignas(16) PcRec {
   int t0, cx, cy;
   float amp;
   float c0, ax, bx, ay;            // r0 / lambda; p = m (ax + bx m), q = m (ay + by m)
-  float by, iqs, kq, pad;          // 1 / max |Q|; cross factor kq (rad)
+  float by, iqs, kq;               // 1 / max |Q|; cross factor kq (rad)
+  int c2x, c2y;
+  float qx, qy, pad;               // what c2x and c2y round off
 };
 
 struct PcTcArgs {
@@ -88,7 +94,7 @@ struct PcTcArgs {
   const PcPt* pts;
   const int* list;                 // fast points by class, unless every point is fast and of one class
   Counts* cnt;
-  int n, regions_x, splits;
+  int regions_x, splits;
   float2* part;                    // [splits][ny][nx]
   int* err;
 };
@@ -239,14 +245,22 @@ __global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ i
 __device__ __forceinline__ int sw_off(int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); }
 
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// Multiples of 2^-8 nearest (a, b), |a|, |b| <= 1 (adding 6 in FP16 rounds to
-// them), and FP16 remainders.
-__device__ __forceinline__ void split2(float a, float b, uint32_t* hi, uint32_t* lo) {
+// Parts of (a, b), |a|, |b| <= 1: the multiples of 2^-8 nearest them (adding 6 in FP16
+// rounds to them), FP16 remainders and, where wanted, FP16 rests of those.
+template <bool THIRD>
+__device__ __forceinline__ void split(float a, float b, uint32_t* hi, uint32_t* lo, uint32_t* rest) {
   const __half2 six = __floats2half2_rn(6.f, 6.f);
   const __half2 h = __hsub2(__hadd2(__floats2half2_rn(a, b), six), six);
   const float2 f = __half22float2(h);
+  a -= f.x;
+  b -= f.y;
+  const __half2 l = __floats2half2_rn(a, b);
   *hi = h2u(h);
-  *lo = h2u(__floats2half2_rn(a - f.x, b - f.y));
+  *lo = h2u(l);
+  if constexpr (THIRD) {
+    const float2 g = __half22float2(l);
+    *rest = h2u(__floats2half2_rn(a - g.x, b - g.y));
+  }
 }
 
 // w[k] of lane i of four <- w[i] of lane k
@@ -272,24 +286,39 @@ __device__ __forceinline__ void put2(float2* p, float2 v, bool add) {
 }
 
 // turns -> (cos, sin)
+template <bool FINE>
 __device__ __forceinline__ void cis(float t, float* c, float* s) {
-  t = 6.28318530717958647692f * (t - rintf(t));
-  *c = __cosf(t);
-  *s = __sinf(t);
+  t -= rintf(t);
+  if constexpr (FINE) {
+    sincospif(2.f * t, s, c);
+  } else {
+    t *= 6.28318530717958647692f;
+    *c = __cosf(t);
+    *s = __sinf(t);
+  }
 }
-__device__ __forceinline__ float axis_rest(float c0, float w, float bm2) {
-  // (r0 / lambda) (sqrt(1 + w) - 1) without its linear term
-  return c0 * fmaf(0.5f, bm2, w * w * fmaf(w, fmaf(w, -0.0390625f, 0.0625f), -0.125f));
+// Phase at offset m of one axis, (r0 / lambda) (sqrt(1 + w) - 1) and t0, without most of
+// its whole turns; *w = m (a + b m).  The terms in m and m^2 are whole numbers of 2^-32
+// turns (in floats the second, of up to two turns, was off by 1e-6 rad).
+__device__ __forceinline__ float axis_turns(int t0, int c1, int c2, float q, float c0, float a, float b, int m, float* w) {
+  const float mf = (float)m, m2 = mf * mf, bm = b * mf, abm = a + bm;
+  const unsigned um = (unsigned)m;
+  *w = mf * abm;
+  const float w2 = *w * *w;
+  // -w^2 / 8 without its term in m^2, then w^3 / 16 - 5 w^4 / 128
+  const float rest = fmaf(w2 * *w, fmaf(*w, -0.0390625f, 0.0625f), (-0.125f * m2 * mf) * b * (abm + a));
+  return (float)(int)((unsigned)t0 + um * ((unsigned)c1 + um * (unsigned)c2)) * 2.3283064365386963e-10f + fmaf(c0, rest, q * m2);
 }
 __device__ __forceinline__ float cross_arg(float w) { return w * fmaf(w, fmaf(w, 0.625f, -0.75f), 1.f); }
 
+template <bool FINE>
 __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ PcRec recs[2][kBatch];
   __shared__ int cls_batch[kMaxCls + 1], cls_e[kMaxCls];
   const uint32_t raw = su32(smem_dyn);
   unsigned char* base = smem_dyn + (((raw + 1023u) & ~1023u) - raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * kStageBytes<FINE>);
   uint64_t* full = bars;                  // [kStages], one arrival per producer warp
   uint64_t* empty = bars + kStages;       // [kStages], tcgen05.commit
   uint64_t* rfull = bars + 2 * kStages;   // [2], the record warp's
@@ -391,57 +420,51 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
       ok = ok && warp_wait(&empty[s], (uint32_t)(((it / kStages) & 1) ^ 1), abort_flag, lane);
       if (!ok) break;
       const PcRec q = recs[rs][(it % kPer) * kPts + j];
-      unsigned char* sAh = base + s * kStageBytes;
-      unsigned char* sAl = sAh + kTile;
-      unsigned char* sBh = sAh + 2 * kTile;
-      unsigned char* sBl = sAh + 3 * kTile;
+      unsigned char* sA = base + s * kStageBytes<FINE>;
+      unsigned char* sB = sA + kParts<FINE> * kTile;
+      auto put = [&](unsigned char* tile, int off, uint4 v) { *reinterpret_cast<uint4*>(tile + off) = v; };
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int m = rb - 64 + 64 * h;
-        const float mf = (float)m;
-        const float bm = q.by * mf, w = mf * (q.ay + bm);
-        float c, sn;
-        cis((float)(int)((unsigned)q.t0 + (unsigned)q.cy * (unsigned)m) * 2.3283064365386963e-10f + axis_rest(q.c0, w, bm * mf), &c, &sn);
+        float c, sn, w;
+        cis<FINE>(axis_turns(q.t0, q.cy, q.c2y, q.qy, q.c0, q.ay, q.by, rb - 64 + 64 * h, &w), &c, &sn);
         const float Qh = cross_arg(w) * q.iqs;
         float re = q.amp * c, im = q.amp * sn;
-        uint4 hi, lo;
-        split2(re, im, &hi.x, &lo.x);
+        uint4 hi, lo, rest = make_uint4(0u, 0u, 0u, 0u);
+        split<FINE>(re, im, &hi.x, &lo.x, &rest.x);
+        // (the other terms' rests meet columns below 0.07)
         re *= Qh; im *= Qh;
-        split2(re, im, &hi.y, &lo.y);
+        split<false>(re, im, &hi.y, &lo.y, nullptr);
         re *= Qh; im *= Qh;
-        split2(re, im, &hi.z, &lo.z);
+        split<false>(re, im, &hi.z, &lo.z, nullptr);
         re *= Qh; im *= Qh;
-        split2(re, im, &hi.w, &lo.w);
+        split<false>(re, im, &hi.w, &lo.w, nullptr);
         const int off = h ? offA1 : offA0;
-        *reinterpret_cast<uint4*>(sAh + off) = hi;
-        *reinterpret_cast<uint4*>(sAl + off) = lo;
+        put(sA, off, hi);
+        put(sA + kTile, off, lo);
+        if constexpr (FINE) put(sA + 2 * kTile, off, rest);
       }
       {
-        const int m = rb - 32;
-        const float mf = (float)m;
-        const float bm = q.bx * mf, w = mf * (q.ax + bm);
-        float c, sn;
-        cis((float)(int)((unsigned)q.cx * (unsigned)m) * 2.3283064365386963e-10f + axis_rest(q.c0, w, bm * mf), &c, &sn);
+        float c, sn, w;
+        cis<FINE>(axis_turns(0, q.cx, q.c2x, q.qx, q.c0, q.ax, q.bx, rb - 32, &w), &c, &sn);
         const float x = q.kq * cross_arg(w);
         const float x2 = 0.5f * x * x, x3 = x * x2 * 0.33333333333f;
         // R_n = (c + i s) (i x)^n / n!
-        uint4 hi, lo;
-        split2(c, sn, &hi.x, &lo.x);
-        split2(-x * sn, x * c, &hi.y, &lo.y);
-        split2(-x2 * c, -x2 * sn, &hi.z, &lo.z);
-        split2(x3 * sn, -x3 * c, &hi.w, &lo.w);
+        uint4 v[3];
+        split<FINE>(c, sn, &v[0].x, &v[1].x, &v[2].x);
+        split<FINE>(-x * sn, x * c, &v[0].y, &v[1].y, &v[2].y);
+        split<FINE>(-x2 * c, -x2 * sn, &v[0].z, &v[1].z, &v[2].z);
+        split<FINE>(x3 * sn, -x3 * c, &v[0].w, &v[1].w, &v[2].w);
         // row 2x takes (Re, -Im) of each term, row 2x + 1 (Im, Re)
         const uint32_t neg = 0x80000000u;
-        const uint4 h0 = make_uint4(hi.x ^ neg, hi.y ^ neg, hi.z ^ neg, hi.w ^ neg);
-        const uint4 l0 = make_uint4(lo.x ^ neg, lo.y ^ neg, lo.z ^ neg, lo.w ^ neg);
-        const uint4 h1 = make_uint4(__byte_perm(hi.x, 0, 0x1032), __byte_perm(hi.y, 0, 0x1032),
-                                    __byte_perm(hi.z, 0, 0x1032), __byte_perm(hi.w, 0, 0x1032));
-        const uint4 l1 = make_uint4(__byte_perm(lo.x, 0, 0x1032), __byte_perm(lo.y, 0, 0x1032),
-                                    __byte_perm(lo.z, 0, 0x1032), __byte_perm(lo.w, 0, 0x1032));
-        *reinterpret_cast<uint4*>(sBh + offB0) = par ? h1 : h0;
-        *reinterpret_cast<uint4*>(sBl + offB0) = par ? l1 : l0;
-        *reinterpret_cast<uint4*>(sBh + offB1) = par ? h0 : h1;
-        *reinterpret_cast<uint4*>(sBl + offB1) = par ? l0 : l1;
+#pragma unroll
+        for (int k = 0; k < kParts<FINE>; ++k) {
+          const uint4 u = v[k];
+          const uint4 r0 = make_uint4(u.x ^ neg, u.y ^ neg, u.z ^ neg, u.w ^ neg);
+          const uint4 r1 = make_uint4(__byte_perm(u.x, 0, 0x1032), __byte_perm(u.y, 0, 0x1032),
+                                      __byte_perm(u.z, 0, 0x1032), __byte_perm(u.w, 0, 0x1032));
+          put(sB + k * kTile, offB0, par ? r1 : r0);
+          put(sB + k * kTile, offB1, par ? r0 : r1);
+        }
       }
       // generic-proxy writes -> visible to the tensor core's async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -481,16 +504,22 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
           break;
         }
         tc::fence_after();
-        unsigned char* st0 = base + s * kStageBytes;
-        const uint64_t ah = tc::desc_sw64(su32(st0), 16, 512), al = tc::desc_sw64(su32(st0 + kTile), 16, 512);
-        const uint64_t bh = tc::desc_sw64(su32(st0 + 2 * kTile), 16, 512), bl = tc::desc_sw64(su32(st0 + 3 * kTile), 16, 512);
+        // part k of an operand kTile further on
+        const uint32_t st0 = su32(base + s * kStageBytes<FINE>);
+        const uint64_t da = tc::desc_sw64(st0, 16, 512), db = tc::desc_sw64(st0 + kParts<FINE> * kTile, 16, 512);
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; ++kk) {
-          const uint64_t adv = (uint64_t)((kk * 32) >> 4);
-          tc::umma_bf16(tmem, ah + adv, bh + adv, kIdesc, kk ? 1u : add);
-          tc::umma_bf16(tmem + kAccCols, ah + adv, bl + adv, kIdesc, kk ? 1u : add);
-          tc::umma_bf16(tmem + kAccCols, al + adv, bh + adv, kIdesc, 1u);
-          tc::umma_bf16(tmem + kAccCols, al + adv, bl + adv, kIdesc, 1u);
+          auto mma = [&](uint32_t acc, int i, int j, uint32_t on) {
+            tc::umma_bf16(acc, da + (uint64_t)((i * kTile + kk * 32) >> 4), db + (uint64_t)((j * kTile + kk * 32) >> 4), kIdesc, on);
+          };
+          mma(tmem, 0, 0, kk ? 1u : add);
+          mma(tmem + kAccCols, 0, 1, kk ? 1u : add);
+          mma(tmem + kAccCols, 1, 0, 1u);
+          mma(tmem + kAccCols, 1, 1, 1u);
+          if constexpr (FINE) {
+            mma(tmem + kAccCols, 0, 2, 1u);
+            mma(tmem + kAccCols, 2, 0, 1u);
+          }
         }
         add = 1u;
         tc::umma_commit(&empty[s]);
@@ -522,6 +551,14 @@ __global__ void __launch_bounds__(kThreads, 2) pc_tc_regions(PcTcArgs a) {
         r.t0 = frac32((r0 - ref) * il);
         r.cx = frac32((sx - a.g.stx) * a.g.px * il);
         r.cy = frac32((a.g.sty - sy) * a.g.py * il);
+        // (r0 / lambda) (1 - s^2) t^2 / 2 per squared pixel, t = pitch / r0
+        auto square = [&](double sn, double pitch, int* c2, float* q) {
+          const double t = pitch * ri, e = 2147483648.0 * (r0 * il) * fma(-sn, sn, 1.0) * t * t, n = rint(e);
+          *c2 = (int)n;
+          *q = (float)(e - n) * 2.3283064365386963e-10f;
+        };
+        square(sx, a.g.px, &r.c2x, &r.qx);
+        square(sy, a.g.py, &r.c2y, &r.qy);
         const float rif = (float)ri, pxr = (float)a.g.px * rif, pyr = (float)a.g.py * rif;
         r.amp = p.a * pow2f(-cls_e[c]);
         r.c0 = (float)(r0 * il);
@@ -622,8 +659,8 @@ int point_splits(int regions, int n, int slots, int batches) {
 bool pc_tc_wants(const PCGeom& g, int n, bool fp64) {
   // FP32: the direct kernels take about 0.24 us per point (a block's serial
   // chain) or 1.1e-6 us per term, whichever sum is due; below 60 us they beat the
-  // six launches and part-filled regions here (640x480 x 100 points: 57 us
-  // direct, 54 us here; 1024x1024 x 200: 247 and 78; 128x128 x 1000: 250 and 66).
+  // six launches and part-filled regions here (1024x1024 x 50 points: 78 us direct, 60
+  // us here; 1024x1024 x 200: 247 and 98; 128x128 x 1000: 250 and 84).
   // FP64: directly 3 to 7 us per point (a block's serial chain) or 73 ps per term
   // (the FP64 pipe); here 55 us at least (100x100 x 30 points: 90 us directly, 57
   // us here; 300x300 x 30: 262 and 61).
@@ -640,7 +677,7 @@ bool pc_tc_wants(const PCGeom& g, int n, bool fp64) {
 }
 
 oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, float2* field, float* fringe,
-                        bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st) {
+                        bool accumulate, bool fine, const float4** slow, const int** slow_n, cudaStream_t st) {
   const int rx = (g.nx + kCols - 1) / kCols, ry = (g.ny + kRows - 1) / kRows, regions = rx * ry;
   const int splits = point_splits(regions, n, 2 * sm_count(), 4);
   const size_t plane = (size_t)g.nx * g.ny, o_part = sorted_bytes(n);
@@ -649,14 +686,16 @@ oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, 
   float2* part = (float2*)((char*)ptr + o_part);
   Sorted s;
   OH_TRY(sort_points(ctx, g, pts, n, false, ptr, &s, st));
-  const int smem = kStages * kStageBytes + 1024 + 256;
-  OH_CUDA_TRY(cudaFuncSetAttribute(pc_tc_regions, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  PcTcArgs a{g, s.pts, s.list, s.cnt, n, rx, splits, part, ctx->dev_err};
-  {
+  PcTcArgs a{g, s.pts, s.list, s.cnt, rx, splits, part, ctx->dev_err};
+  auto launch = [&](auto kern, int stage_bytes) -> oh_status {
+    const int smem = kStages * stage_bytes + 1024 + 256;
+    OH_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     KernelTimer kt(ctx, "pc_tc_regions", st);
-    pc_tc_regions<<<dim3(regions, splits), kThreads, smem, st>>>(a);
+    kern<<<dim3(regions, splits), kThreads, smem, st>>>(a);
     OH_LAUNCH_CHECK();
-  }
+    return OH_OK;
+  };
+  OH_TRY(fine ? launch(pc_tc_regions<true>, kStageBytes<true>) : launch(pc_tc_regions<false>, kStageBytes<false>));
   KernelTimer kt(ctx, "pc_tc_sum", st);
   pc_tc_sum<<<(int)std::min<size_t>((plane + 255) / 256, (size_t)sm_count() * 16), 256, 0, st>>>(
       part, splits, plane, s.cnt, field, fringe, accumulate ? 1 : 0);

@@ -21,7 +21,7 @@ bool pc_tc_wants(const PCGeom& g, int n, bool fp64);
 // slow[0, *slow_n) (device) for the caller; the order within both groups is the
 // input's.  FP64: field double2, fringe double.
 oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, float2* field, float* fringe,
-                        bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st);
+                        bool accumulate, bool fine, const float4** slow, const int** slow_n, cudaStream_t st);
 oh_status pc_tc64_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, double2* field, double* fringe,
                           bool accumulate, const float4** slow, const int** slow_n, cudaStream_t st);
 

@@ -359,14 +359,20 @@ oh_status pointcloud_enqueue(oh_ctx* ctx, int prec, const oh_pc_params* p, const
   float* RY = B + (size_t)chunk * p->ny;
   float* E = RY + (size_t)chunk * p->ny;
   // The tensor-core form takes the points it can (1024x1024 x 5000 points: all
-  // of them, 5.74 -> 0.73 ms, 1.3e-6 -> 1.0e-6 off FP64); the direct kernels sum the others, or, in small
-  // sums, every point.
+  // of them, 5.74 -> 0.79 ms); the direct kernels sum the others, or, in small sums,
+  // every point.
   const bool tensor = pc_tc_wants(g, n, false);
+  // Error against 64 bits of the L2 norm, 1024x1024: the direct sum 3.2e-7 at 200
+  // points, 7.2e-7 at 1500, 8.4e-7 at 2000 and 1.3e-6 at 5000 (one FP32 addition after
+  // the other); the tensor-core form 7.3e-7 with two-part operands and 1.2e-7 with
+  // three-part ones at any count, 345 and 425 us at 2000 points.  So small clouds
+  // take three parts.
+  const bool fine = n < 2000;
   for (int j0 = 0; j0 < n; j0 += chunk) {
     const int cnt = std::min(chunk, n - j0);
     const float4* src = pts + j0;
     const int* n_dev = nullptr;
-    if (tensor) OH_TRY(pc_tc_enqueue(ctx, g, src, cnt, (float2*)field, (float*)fringe, j0 > 0, &src, &n_dev, st));
+    if (tensor) OH_TRY(pc_tc_enqueue(ctx, g, src, cnt, (float2*)field, (float*)fringe, j0 > 0, fine, &src, &n_dev, st));
     {
       KernelTimer kt(ctx, "pc_tables", st);
       pc_tables<<<std::max(1, std::min(cnt, oh::sm_count() * 8)), 256, 0, st>>>(g, src, cnt, n_dev, prm, A, RX, B, RY, E);

@@ -1,7 +1,8 @@
 """The point-cloud sum where its tensor-core forms are weakest, against a sum in
 64 bits (r / lambda as z / lambda, reduced in extended precision, plus rho^2 / (r +
 z) / lambda): the corners of planes whose cross phase is as large as the form
-takes, and sums that stay in phase over a whole chunk of points.
+takes, sums that stay in phase over a whole chunk of points, clouds of uneven
+amplitude, and small clouds, where the direct sum loses least.
 
 Each tolerance is the form's own error, derived beside its test; none is larger
 than the error of the direct sum at the same sizes."""
@@ -106,3 +107,14 @@ def test_uneven_amplitudes(ctx, kind, n, nx, ny):
     ref = reference(pts, nx, ny, rows)
     assert off(run(ctx, 0, pts, nx, ny)[rows], ref)[0] <= 2e-6
     assert off(run(ctx, 1, pts, nx, ny)[rows], ref)[0] <= 1e-11
+
+
+@pytest.mark.parametrize("n,nx,ny,pitch,scale", [(200, 300, 300, 8e-6, 1.0), (200, 300, 300, 2e-6, 1.0), (40, 1024, 700, 8e-6, 1.0),
+                                                 (1000, 257, 131, 8e-6, 1.0), (600, 300, 300, 8e-7, 0.1),
+                                                 (500, 640, 480, 2e-5, 10.0)])
+def test_fp32_small_clouds(ctx, n, nx, ny, pitch, scale):
+    """The direct FP32 sum is 3e-7 off for a few hundred points.  Three-part operands
+    (2^-25), phases of 2^-25 turns and a sine and cosine of 2^-23 leave 2e-7."""
+    pts = cloud(n, n + nx, None, scale)
+    rows = rows_of(ny)
+    assert off(run(ctx, 0, pts, nx, ny, pitch)[rows], reference(pts, nx, ny, rows, pitch))[0] <= 3e-7
