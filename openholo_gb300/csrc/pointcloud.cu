@@ -334,18 +334,32 @@ oh_status pointcloud_enqueue(oh_ctx* ctx, int prec, const oh_pc_params* p, const
     if (field) OH_CUDA_TRY(cudaMemsetAsync(field, 0, (size_t)p->nx * p->ny * (prec ? 16 : 8), st));
     return OH_OK;
   }
+  // The tensor-core form of one chunk, its refused points left in *src; without memory
+  // for its partial planes it is off and every point is left.
+  auto regions = [&](bool* tensor, auto enqueue, const float4** src, const int** n_dev) -> oh_status {
+    if (!*tensor) return OH_OK;
+    const oh_status s = enqueue(src, n_dev);
+    if (s != OH_ERR_ALLOC) return s;
+    *tensor = false;
+    set_error("");
+    return OH_OK;
+  };
   if (prec) {
     // the tensor-core form where it takes the points (1024x1024 x 5000 points: 382
-    // -> 3.8 ms), the direct kernel for the others and for small sums
-    const bool tensor = pc_tc_wants(g, n, true);
-    for (int j0 = 0; j0 < n; j0 += tensor ? kPcChunk : n) {
-      const int cnt = tensor ? std::min(kPcChunk, n - j0) : n;
+    // -> 3.9 ms), the direct kernel for the others and for small sums
+    bool tensor = pc_tc_wants(g, n, true);
+    for (int j0 = 0; j0 < n;) {
       const float4* src = pts + j0;
       const int* n_dev = nullptr;
-      if (tensor) OH_TRY(pc_tc64_enqueue(ctx, g, src, cnt, (double2*)field, (double*)fringe, j0 > 0, &src, &n_dev, st));
+      int cnt = std::min(kPcChunk, n - j0);
+      OH_TRY(regions(&tensor, [&](const float4** sl, const int** nd) {
+        return pc_tc64_enqueue(ctx, g, src, cnt, (double2*)field, (double*)fringe, j0 > 0, sl, nd, st);
+      }, &src, &n_dev));
+      if (!tensor) cnt = n - j0;
       KernelTimer kt(ctx, "pc_direct_f64", st);
-      pc_direct_f64<<<grid, kPcTX * kPcTY, 0, st>>>(g, src, cnt, n_dev, (double2*)field, (double*)fringe, tensor ? 1 : 0);
+      pc_direct_f64<<<grid, kPcTX * kPcTY, 0, st>>>(g, src, cnt, n_dev, (double2*)field, (double*)fringe, tensor || j0 > 0 ? 1 : 0);
       OH_LAUNCH_CHECK();
+      j0 += cnt;
     }
     return OH_OK;
   }
@@ -361,7 +375,7 @@ oh_status pointcloud_enqueue(oh_ctx* ctx, int prec, const oh_pc_params* p, const
   // The tensor-core form takes the points it can (1024x1024 x 5000 points: all
   // of them, 5.74 -> 0.79 ms); the direct kernels sum the others, or, in small sums,
   // every point.
-  const bool tensor = pc_tc_wants(g, n, false);
+  bool tensor = pc_tc_wants(g, n, false);
   // Error against 64 bits of the L2 norm, 1024x1024: the direct sum 3.2e-7 at 200
   // points, 7.2e-7 at 1500, 8.4e-7 at 2000 and 1.3e-6 at 5000 (one FP32 addition after
   // the other); the tensor-core form 7.3e-7 with two-part operands and 1.2e-7 with
@@ -372,7 +386,9 @@ oh_status pointcloud_enqueue(oh_ctx* ctx, int prec, const oh_pc_params* p, const
     const int cnt = std::min(chunk, n - j0);
     const float4* src = pts + j0;
     const int* n_dev = nullptr;
-    if (tensor) OH_TRY(pc_tc_enqueue(ctx, g, src, cnt, (float2*)field, (float*)fringe, j0 > 0, fine, &src, &n_dev, st));
+    OH_TRY(regions(&tensor, [&](const float4** sl, const int** nd) {
+      return pc_tc_enqueue(ctx, g, src, cnt, (float2*)field, (float*)fringe, j0 > 0, fine, sl, nd, st);
+    }, &src, &n_dev));
     {
       KernelTimer kt(ctx, "pc_tables", st);
       pc_tables<<<std::max(1, std::min(cnt, oh::sm_count() * 8)), 256, 0, st>>>(g, src, cnt, n_dev, prm, A, RX, B, RY, E);
