@@ -180,10 +180,11 @@ __global__ void __launch_bounds__(256) encode_map(int kind, int nx, int ny, cons
 template <typename R> __device__ __forceinline__ bool is_nan(R v) { return v != v; }
 
 // minimum and maximum of the block's values; a NaN among them makes both NaN
-// (the whole image was NaN when a transform along either axis met one)
+// (the whole image was NaN when a transform along either axis met one).  red: 2 values
+// per warp of shared memory.
+constexpr int kSsbThreads = 256, kSsbRed = 2 * kSsbThreads / 32;
 template <typename R>
-__device__ __forceinline__ void block_minmax(R mn, R mx, R* out) {
-  __shared__ R smn[32], smx[32];
+__device__ __forceinline__ void block_minmax(R mn, R mx, R* red, R* out) {
   auto lo = [](R a, R b) { return a < b || is_nan(a) ? a : b; };
   auto hi = [](R a, R b) { return a > b || is_nan(a) ? a : b; };
 #pragma unroll
@@ -191,11 +192,10 @@ __device__ __forceinline__ void block_minmax(R mn, R mx, R* out) {
     mn = lo(mn, __shfl_xor_sync(0xffffffffu, mn, o));
     mx = hi(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
-  const int nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) { smn[threadIdx.x >> 5] = mn; smx[threadIdx.x >> 5] = mx; }
+  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 4] = mn; red[(threadIdx.x >> 4) + 1] = mx; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int i = 1; i < nw; ++i) { mn = lo(mn, smn[i]); mx = hi(mx, smx[i]); }
+    for (int i = 2; i < kSsbRed; i += 2) { mn = lo(mn, red[i]); mx = hi(mx, red[i + 1]); }
     out[0] = mn;
     out[1] = mx;
   }
@@ -204,7 +204,7 @@ __device__ __forceinline__ void block_minmax(R mn, R mx, R* out) {
 // The masked axis has length n, the other length m: COLS ? strips of 1 << lw
 // columns : 1 << lw rows per block.
 template <typename R, bool COLS>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 3) ssb_lines(int kind, const typename cplx_of<R>::type* __restrict__ in,
+__global__ void __launch_bounds__(kSsbThreads, sizeof(R) == 8 ? 2 : 3) ssb_lines(int kind, const typename cplx_of<R>::type* __restrict__ in,
                                                  R* __restrict__ out, R* __restrict__ part, int n, int m, int lw,
                                                  FFTPlan pl, const void* __restrict__ tw_other) {
   typedef typename cplx_of<R>::type C;
@@ -261,20 +261,22 @@ __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 3) ssb_lines(int kin
     for (int l = 0; l < nl; ++l)
       for (int k = threadIdx.x; k < n; k += blockDim.x) emit(l, k);
   }
-  block_minmax(mn, mx, part + 2 * blockIdx.x);
+  // (in the lines' memory: the longest lines leave none beside them)
+  __syncthreads();
+  block_minmax(mn, mx, reinterpret_cast<R*>(smem_raw), part + 2 * blockIdx.x);
 }
 
 // out = (out - min) / (max - min), the extremes of np block partials
 template <typename R>
-__global__ void __launch_bounds__(256) ssb_finish(size_t n, const R* __restrict__ part, int np, const R* in, R* out) {
-  __shared__ R ext[2];
+__global__ void __launch_bounds__(kSsbThreads) ssb_finish(size_t n, const R* __restrict__ part, int np, const R* in, R* out) {
+  __shared__ R red[kSsbRed], ext[2];
   R mn = (R)INFINITY, mx = -(R)INFINITY;
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
     const R a = part[2 * i], b = part[2 * i + 1];
     mn = a < mn || is_nan(a) ? a : mn;
     mx = b > mx || is_nan(b) ? b : mx;
   }
-  block_minmax(mn, mx, ext);
+  block_minmax(mn, mx, red, ext);
   __syncthreads();
   const R lo = ext[0], rng = ext[1] - ext[0];
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -307,7 +309,7 @@ static oh_status run_ssb(oh_ctx* ctx, int kind, int nx, int ny, const void* fiel
   int lw = 0;
   while (lw < 3 && ((size_t)pl.lens * sizeof(C) << (lw + 1)) <= 48 * 1024 && (m >> (lw + 1)) >= 2 * oh::sm_count()) ++lw;
   const int blocks = (m + (1 << lw) - 1) >> lw;
-  const size_t smem = (size_t)pl.lens * sizeof(C) << lw;
+  const size_t smem = std::max((size_t)pl.lens * sizeof(C) << lw, kSsbRed * sizeof(R));
   const size_t total = (size_t)nx * ny;
   void* ptr;
   OH_TRY(scratch(ctx, "enc.red1", sizeof(R) * 2 * blocks, &ptr));
@@ -323,11 +325,11 @@ static oh_status run_ssb(oh_ctx* ctx, int kind, int nx, int ny, const void* fiel
   OH_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   {
     KernelTimer kt(ctx, "ssb_lines", st);
-    kern<<<blocks, 256, smem, st>>>(kind, (const C*)field, real, (R*)ptr, n, m, lw, pl, cols ? px.tw : py.tw);
+    kern<<<blocks, kSsbThreads, smem, st>>>(kind, (const C*)field, real, (R*)ptr, n, m, lw, pl, cols ? px.tw : py.tw);
     OH_LAUNCH_CHECK();
   }
   KernelTimer kt(ctx, "ssb_finish", st);
-  ssb_finish<R><<<(int)std::min<size_t>((total + 1023) / 1024, oh::sm_count() * 16), 256, 0, st>>>(total, (const R*)ptr, blocks, real, (R*)out);
+  ssb_finish<R><<<(int)std::min<size_t>((total + 1023) / 1024, oh::sm_count() * 16), kSsbThreads, 0, st>>>(total, (const R*)ptr, blocks, real, (R*)out);
   OH_LAUNCH_CHECK();
   return OH_OK;
 }
