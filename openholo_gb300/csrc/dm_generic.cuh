@@ -189,8 +189,9 @@ __device__ __forceinline__ double2 cis_turns(double t, const double2* tab) {
 template <typename R> constexpr int kDirs = sizeof(R) == 4 ? 0 : std::is_same<R, ff>::value ? 256 : 128;
 
 // Shared memory of the column pass after the lines: kept rows' positions,
-// active entries, and in FP64 the direction table and (evenly spaced layers)
-// the step factors.
+// active entries and their count, and in FP64 the direction table and (evenly
+// spaced layers) the step factors.  All that the kernel uses: columns near the limit
+// of a block's memory have no room for static variables beside it.
 template <typename R>
 inline size_t dm_col_gen_smem(int lens, int lwb, int G, int nrow, int n_entries, bool horner) {
   size_t o = (size_t)G * lens << lwb;
@@ -218,7 +219,6 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
   constexpr bool F64 = sizeof(R) == 8;
   constexpr bool KEEPG = KMAX <= 16;                    // g per sample in registers
   extern __shared__ unsigned char smem_raw[];
-  __shared__ int s_nact;
   const int W = 1 << lwb, Py = a.Py, pny = a.pny, lens = a.ply.lens, tid = threadIdx.x;
   const bool step = F64 && a.horner;
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
   C* dst = tab + kDirs<R>;
   uint16_t* pos = reinterpret_cast<uint16_t*>(dst + (step ? (size_t)nrow << lwb : 0));
   int16_t* list = reinterpret_cast<int16_t*>(pos + ((nrow + 7) & ~7));
+  int* s_nact = reinterpret_cast<int*>(list + ((a.n_entries + 1) & ~1));      // (not static: see dm_col_gen_smem)
   const int w = tid & (W - 1), p = (blockIdx.x << lwb) + w;
   const bool valid = p < a.Px;
   int kx = 0;
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
       if (act) list[n + __popc(m & ((1u << tid) - 1u))] = (int16_t)e;
       n += __popc(m);
     }
-    if (tid == 0) s_nact = n;
+    if (tid == 0) *s_nact = n;
   }
   if constexpr (std::is_same<R, ff>::value) {
     ff_directions(reinterpret_cast<float4*>(tab), tid, T);
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
     if constexpr (KEEPG) g[k] = tid + k * T < nk ? resid(k) : (R)0;
   }
   __syncthreads();
-  const int nact = s_nact;
+  const int nact = *s_nact;
   auto gof = [&](int k) -> R { if constexpr (KEEPG) return g[k]; else return resid(k); };
   // exp(i kz g) of sample k
   auto residual = [&](R kz, int k) -> C {
