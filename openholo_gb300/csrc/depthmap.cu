@@ -369,7 +369,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   size_t off = 0;
   auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
   size_t o_lut = carve(256 * sizeof(int16_t)), o_use = carve(nE * sizeof(int16_t)), o_kz = carve(nE * sizeof(R)),
-         o_cst = carve(nE * sizeof(C)), o_exc = carve(nE * a.Px * sizeof(C)), o_ey = carve(nE * a.Py * sizeof(C)),
+         o_exc = carve(nE * a.Px * sizeof(C)), o_ey = carve(nE * a.Py * sizeof(C)),
          o_eth = carve(a.ey_perm ? nE * a.Py * sizeof(R) : 0), o_lfx = carve(a.Px * sizeof(R)), o_lfy = carve(a.Py * sizeof(R)), o_lfyp = carve(a.Py * sizeof(R)),
          o_shy = carve(a.pny * sizeof(C)), o_shx = carve(a.pnx * sizeof(C)), o_any = carve(nU * sizeof(int)),
          o_dxh = carve(a.horner ? a.Px * sizeof(C) : 0), o_dyh = carve(a.horner ? a.Py * sizeof(C) : 0);
@@ -378,7 +378,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
     DMArgs<R> b = a;
     auto at = [](size_t o) { return reinterpret_cast<char*>(o); };
     b.lut = (int16_t*)at(o_lut); b.uslot_of_entry = (int16_t*)at(o_use); b.kzp = (R*)at(o_kz);
-    b.cst = (C*)at(o_cst); b.exc = (C*)at(o_exc); b.ey = (C*)at(o_ey); b.eth = (R*)at(o_eth);
+    b.exc = (C*)at(o_exc); b.ey = (C*)at(o_ey); b.eth = (R*)at(o_eth);
     b.lfx = (R*)at(o_lfx); b.lfy = (R*)at(o_lfy); b.lfyp = (R*)at(o_lfyp); b.shy = (C*)at(o_shy); b.shx = (C*)at(o_shx);
     b.slot_any = (int*)at(o_any);
     b.dxh = a.horner ? (C*)at(o_dxh) : nullptr;
@@ -397,7 +397,7 @@ static oh_status run_depthmap(oh_ctx* ctx, const oh_depthmap_params* p, const ui
   OH_TRY(scratch(ctx, "dm.tables", off, &ptr));
   char* base = (char*)ptr;
   a.lut = (int16_t*)(base + o_lut); a.uslot_of_entry = (int16_t*)(base + o_use); a.kzp = (R*)(base + o_kz);
-  a.cst = (C*)(base + o_cst); a.exc = (C*)(base + o_exc); a.ey = (C*)(base + o_ey);
+  a.exc = (C*)(base + o_exc); a.ey = (C*)(base + o_ey);
   a.eth = (R*)(base + o_eth);
   a.lfx = (R*)(base + o_lfx); a.lfy = (R*)(base + o_lfy); a.lfyp = (R*)(base + o_lfyp); a.shy = (C*)(base + o_shy); a.shx = (C*)(base + o_shx);
   a.slot_any = (int*)(base + o_any);

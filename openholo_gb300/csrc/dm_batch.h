@@ -43,7 +43,7 @@ template <typename R> struct FrameInfo {
 // Adds the base of a table region to the offsets FrameInfo::a holds.
 template <typename R> void relocate_tables(DMArgs<R>* a, char* base) {
   auto rel = [&](auto*& p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + reinterpret_cast<size_t>(p)); };
-  rel(a->lut); rel(a->uslot_of_entry); rel(a->kzp); rel(a->cst); rel(a->exc); rel(a->ey); rel(a->eth);
+  rel(a->lut); rel(a->uslot_of_entry); rel(a->kzp); rel(a->exc); rel(a->ey); rel(a->eth);
   rel(a->lfx); rel(a->lfy); rel(a->lfyp); rel(a->shy); rel(a->shx); rel(a->slot_any);
   if (a->dxh) rel(a->dxh);
   if (a->dyh) rel(a->dyh);

@@ -32,7 +32,7 @@ __device__ __forceinline__ double to_out(double v) { return v; }
 __device__ __forceinline__ double to_out(ff v) { return (double)v; }
 
 template <typename R>
-struct DMArgs {
+struct alignas(16) DMArgs {
   typedef typename cplx_of<R>::type C;
   typedef typename out_of<R>::type O;
   typedef typename cplx_of<O>::type OC;
@@ -50,8 +50,7 @@ struct DMArgs {
   int16_t* lut;          // 256
   int16_t* uslot_of_entry;
   R* kzp;                // k*z' per entry
-  C* cst;                // per-entry constant
-  C* exc;                // [entries][Px] cst*exp(i alpha fx^2)
+  C* exc;                // [entries][Px] entry constant * exp(i alpha fx^2)
   R* eth;                // [entries][Py] phase alpha fy^2 reduced to [-pi, pi], y storage order (fast passes)
   C* ey;                 // [entries][Py] exp(i alpha fy^2)
   R* lfx;                // [Px] (lambda fx)^2
@@ -113,7 +112,6 @@ __device__ __forceinline__ void dm_setup_body(const DMArgs<R>& a, const DMSetup&
   for (int e = tid; e < s.n_entries; e += nthr) {
     a.uslot_of_entry[e] = s.uslot_of_entry[e];
     a.kzp[e] = (R)(a.k * s.zp[e]);
-    a.cst[e] = mk((R)s.cre[e], (R)s.cim[e]);
   }
   for (int u = tid; u < s.n_uslots; u += nthr) a.slot_any[u] = 0;
   // reference frequency grid (HologramKernel.cu:85-86)

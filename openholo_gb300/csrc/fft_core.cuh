@@ -48,7 +48,8 @@ struct FFTPlan {
   const int* permp;       // perm in stored positions
 };
 
-// i / d for i < 2^18, d < 2^15 with m = ceil(2^32 / d) (0 stands for d = 1)
+// i / d with m = ceil(2^32 / d) (0 stands for d = 1), exact while i d <= 2^32: here i is at
+// most the elements of the lines that a block holds, below 2^15 like d
 __device__ __forceinline__ int fdiv(int i, uint32_t m) { return m ? (int)__umulhi((uint32_t)i, m) : i; }
 
 // stored position of line element p

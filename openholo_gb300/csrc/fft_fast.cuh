@@ -465,11 +465,6 @@ struct SchedImpl {
   __device__ __forceinline__ static void run(C* buf, int nl, int ls, int es, const C* tw, bool lf) {
     fstages<N, N, SGN, C, R0, Rest...>(buf, nl, ls, es, tw, lf);
   }
-  // all stages with a twiddle functor
-  template <int SGN, typename C, class TW>
-  __device__ __forceinline__ static void run_t(C* buf, int nl, int ls, int es, const TW& tw, bool lf) {
-    fstages_t<N, N, SGN, C, TW, R0, Rest...>(buf, nl, ls, es, tw, lf);
-  }
   // unnormalised inverse DFT of a line in this schedule's storage order,
   // output in natural order (the adjoint network)
   template <typename C, class TW>

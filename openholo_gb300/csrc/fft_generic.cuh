@@ -78,7 +78,9 @@ __device__ __forceinline__ ffc ldg_c(const ffc* p) {
 
 // Calls f(std::integral_constant<int, r>) for the straight-line radices and
 // f(std::integral_constant<int, 0>) for any other.
-// (18 and 30 occur in FP32's compile-time schedules only: WIDE takes them too.)
+// (18 and 30 occur in FP32's compile-time schedules only: WIDE takes them too.  The depth-map
+// passes do without it, as its registers would cost every other length; columns of
+// 4320 or 7680 that the fast pass refuses run those two stages through the loop.)
 template <bool WIDE, class F>
 __device__ __forceinline__ void with_radix(int r, F&& f) {
   switch (r) {

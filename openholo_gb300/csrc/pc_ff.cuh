@@ -1,5 +1,4 @@
-// The per-axis factors of the FP64 point-cloud sum in two-float arithmetic.  The
-// functions also run on the host.
+// The per-axis factors of the FP64 point-cloud sum in two-float arithmetic.
 #pragma once
 #include <cuda_bf16.h>
 #include "two_float.cuh"
@@ -19,7 +18,7 @@ struct AxisRec {
 
 // exp(2 pi i t / 2^64); extra: a further phase in turns, below 1e-6; tab: see
 // ff_rotate.
-OH_HD ffc ff_cis64(uint64_t t, float extra, const float4* tab) {
+OH_FF ffc ff_cis64(uint64_t t, float extra, const float4* tab) {
   const uint64_t r = t + (1ull << 55);
   const int idx = (int)(r >> 56);
   const int64_t f = (int64_t)(t - ((uint64_t)idx << 56));         // [-2^55, 2^55)
@@ -34,7 +33,7 @@ OH_HD ffc ff_cis64(uint64_t t, float extra, const float4* tab) {
   return ff_rotate({p, OH_FFMA(6.28318530717958647692f, extra, OH_FFMA(B, cb, q))}, tab[idx & 255]);
 }
 
-OH_HD ffc axis_cis(const AxisRec& r, int m, const float4* tab) {
+OH_FF ffc axis_cis(const AxisRec& r, int m, const float4* tab) {
   const uint64_t um = (uint64_t)(int64_t)m;
   const uint64_t t = r.t0 + um * (r.c1 + um * (r.c2 + um * (r.c3 + um * r.c4)));
   const float mf = (float)m, m2 = mf * mf;
@@ -42,7 +41,7 @@ OH_HD ffc axis_cis(const AxisRec& r, int m, const float4* tab) {
 }
 
 // w (1 - 3/4 w + 5/8 w^2 - 35/64 w^3) / Qs, w / Qs = m (a + b m)
-OH_HD ff axis_cross(const AxisRec& r, int m, float qs) {
+OH_FF ff axis_cross(const AxisRec& r, int m, float qs) {
   const float mf = (float)m, m2 = OH_FMUL(mf, mf);
   const float p1 = OH_FMUL(r.a.h, mf), p2 = OH_FMUL(r.b.h, m2);
   const float e1 = OH_FFMA(r.a.l, mf, OH_FFMA(r.a.h, mf, -p1)), e2 = OH_FFMA(r.b.l, m2, OH_FFMA(r.b.h, m2, -p2));
@@ -54,23 +53,15 @@ OH_HD ff axis_cross(const AxisRec& r, int m, float qs) {
 }
 
 // v rounded to BF16, as a float
-OH_HD float bf16_round(float v) {
-#if defined(__CUDA_ARCH__)
+OH_FF float bf16_round(float v) {
   return __bfloat162float(__float2bfloat16_rn(v));
-#else
-  uint32_t u;
-  std::memcpy(&u, &v, 4);
-  u = (u + 0x7fffu + ((u >> 16) & 1u)) & 0xffff0000u;
-  std::memcpy(&v, &u, 4);
-  return v;
-#endif
 }
 
 // v, |v| <= 1, as multiples of 2^-8 (unless !UNIT: |v| <= 2^-8), of 2^-16 and of
 // 2^-24, each at most 256 steps and so exact in BF16, then two BF16 rests (the
 // last below 2^-42): s[0] + ... + s[4].
 template <bool UNIT>
-OH_HD void ff_slices(ff v, float* s) {
+OH_FF void ff_slices(ff v, float* s) {
   float h = v.h;
   s[0] = 0.f;
   if (UNIT) { s[0] = OH_FSUB(OH_FADD(h, 49152.f), 49152.f); h = OH_FSUB(h, s[0]); }

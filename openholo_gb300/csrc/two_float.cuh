@@ -6,72 +6,62 @@
 // Results are not renormalised: l may reach a few units in h's last place (after
 // a cancellation of the h parts, any size); errors stay near 2^-47 of the
 // operands.  Everything is written with explicitly rounded operations: a
-// contraction to FMA would break the error terms.  The functions also run on
-// the host.
+// contraction to FMA would break the error terms.
 #pragma once
-#include <cmath>
 #include <cstdint>
-#include <cstring>
 #include "oh_common.cuh"
 
 namespace oh {
 
-#if defined(__CUDA_ARCH__)
 #define OH_FADD(a, b) __fadd_rn(a, b)
 #define OH_FSUB(a, b) __fsub_rn(a, b)
 #define OH_FMUL(a, b) __fmul_rn(a, b)
 #define OH_FFMA(a, b, c) __fmaf_rn(a, b, c)
-#else
-#define OH_FADD(a, b) ((float)((a) + (b)))
-#define OH_FSUB(a, b) ((float)((a) - (b)))
-#define OH_FMUL(a, b) ((float)((a) * (b)))
-#define OH_FFMA(a, b, c) std::fma((float)(a), (float)(b), (float)(c))
-#endif
-#define OH_HD __host__ __device__ __forceinline__
+#define OH_FF __device__ __forceinline__
 
 struct ff;
-OH_HD ff operator+(ff a, ff b);
-OH_HD ff operator*(ff a, ff b);
+OH_FF ff operator+(ff a, ff b);
+OH_FF ff operator*(ff a, ff b);
 struct ff {
   float h, l;
   ff() = default;
-  OH_HD ff(float h_, float l_) : h(h_), l(l_) {}
-  OH_HD explicit ff(double v) : h((float)v), l((float)(v - (double)(float)v)) {}
-  OH_HD explicit ff(float v) : h(v), l(0.f) {}
-  OH_HD explicit ff(int v) : ff((double)v) {}
-  friend OH_HD ff fma(ff a, ff b, ff c) { return a * b + c; }
-  OH_HD explicit operator double() const { return (double)h + (double)l; }
+  __host__ __device__ ff(float h_, float l_) : h(h_), l(l_) {}
+  __host__ __device__ explicit ff(double v) : h((float)v), l((float)(v - (double)(float)v)) {}
+  OH_FF explicit ff(float v) : h(v), l(0.f) {}
+  OH_FF explicit ff(int v) : ff((double)v) {}
+  friend OH_FF ff fma(ff a, ff b, ff c) { return a * b + c; }
+  OH_FF explicit operator double() const { return (double)h + (double)l; }
 };
 struct alignas(16) ffc { ff x, y; };
 template <> struct cplx_of<ff> { typedef ffc type; };
-OH_HD ffc mk(ff x, ff y) { ffc r; r.x = x; r.y = y; return r; }
+__host__ __device__ __forceinline__ ffc mk(ff x, ff y) { ffc r; r.x = x; r.y = y; return r; }
 
-OH_HD ff ff_quick(float a, float b) {            // |a| >= |b| or a = 0
+OH_FF ff ff_quick(float a, float b) {            // |a| >= |b| or a = 0
   const float s = OH_FADD(a, b);
   return {s, OH_FSUB(b, OH_FSUB(s, a))};
 }
-OH_HD ff ff_sum(float a, float b) {
+OH_FF ff ff_sum(float a, float b) {
   const float s = OH_FADD(a, b), t = OH_FSUB(s, a);
   return {s, OH_FADD(OH_FSUB(a, OH_FSUB(s, t)), OH_FSUB(b, t))};
 }
-OH_HD ff operator-(ff a) { return {-a.h, -a.l}; }
-OH_HD ff operator+(ff a, ff b) {
+OH_FF ff operator-(ff a) { return {-a.h, -a.l}; }
+OH_FF ff operator+(ff a, ff b) {
   const ff s = ff_sum(a.h, b.h);
   return {s.h, OH_FADD(s.l, OH_FADD(a.l, b.l))};
 }
-OH_HD ff operator-(ff a, ff b) { return a + (-b); }
-OH_HD ff operator*(ff a, ff b) {
+OH_FF ff operator-(ff a, ff b) { return a + (-b); }
+OH_FF ff operator*(ff a, ff b) {
   const float p = OH_FMUL(a.h, b.h);
   return {p, OH_FFMA(a.l, b.h, OH_FFMA(a.h, b.l, OH_FFMA(a.h, b.h, -p)))};
 }
-OH_HD ff ff_mulf(ff a, float b) {
+OH_FF ff ff_mulf(ff a, float b) {
   const float p = OH_FMUL(a.h, b);
   return {p, OH_FFMA(a.l, b, OH_FFMA(a.h, b, -p))};
 }
 
 // exp(i x) T for |x| <= pi / 256 (x.l any rounding error of it), T = (cos h, cos
 // l, sin h, sin l) of a direction.
-OH_HD ffc ff_rotate(ff x, float4 T) {
+OH_FF ffc ff_rotate(ff x, float4 T) {
   const float x2 = OH_FMUL(x.h, x.h);
   const float x2l = OH_FFMA(OH_FMUL(2.f, x.h), x.l, OH_FFMA(x.h, x.h, -x2));
   // sin x = x - x^3 (1 / 6 - x^2 / 120), cos x - 1 = -x^2 / 2 + x^4 (1 / 24 - x^2 / 720)
@@ -99,15 +89,10 @@ OH_HD ffc ff_rotate(ff x, float4 T) {
 }
 
 // exp(2 pi i t), |t| < 2^14; tab[i]: direction 2 pi i / 256 (see ff_rotate)
-OH_HD ffc ff_cis(ff t, const float4* tab) {
+OH_FF ffc ff_cis(ff t, const float4* tab) {
   const float big = 12582912.f;                  // 1.5 2^23: adding it rounds to an integer
   const float v = OH_FADD(OH_FMUL(t.h, 256.f), big);
-#if defined(__CUDA_ARCH__)
   const int idx = __float_as_int(v);
-#else
-  int idx;
-  std::memcpy(&idx, &v, 4);
-#endif
   const float r = OH_FSUB(t.h, OH_FMUL(OH_FSUB(v, big), 0.00390625f));     // exact
   const float c = 6.28318530717958647692f;                       // 2 pi = c + cl
   const float cl = (float)(6.28318530717958647692 - (double)6.28318530717958647692f);
