@@ -64,14 +64,15 @@ DMGenPlan dm_gen_plan(const DMArgs<R>& a, size_t smax) {
   return g;
 }
 
+// The same limit at every size: another thread may set it between here and the launch.
 template <typename K>
-static cudaError_t dm_gen_allow(K kern, size_t smem) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static cudaError_t dm_gen_allow(K kern, size_t static_bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(max_smem_per_block() - static_bytes));
 }
 
 template <typename R>
 cudaError_t dm_gen_row(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
-  cudaError_t e = dm_gen_allow(dm_row_gen<R>, g.smem_row);
+  cudaError_t e = dm_gen_allow(dm_row_gen<R>, 8192);         // (its layer tables, the two-float directions)
   if (e != cudaSuccess) return e;
   dm_row_gen<R><<<(a.pny + g.nr - 1) / g.nr, 256, g.smem_row, st>>>(a, g.nr, g.gr);
   return cudaGetLastError();
@@ -82,7 +83,7 @@ cudaError_t dm_gen_col(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) 
   typedef DMGenCfg<R> CF;
   const int blocks = (a.Px + (1 << g.lwb) - 1) >> g.lwb;
   auto launch = [&](auto kern, int threads) {
-    cudaError_t e = dm_gen_allow(kern, g.smem_col);
+    cudaError_t e = dm_gen_allow(kern, 0);
     if (e != cudaSuccess) return e;
     kern<<<blocks, threads, g.smem_col, st>>>(a, g.lwb, g.gc, g.row0, g.nrow);
     return cudaGetLastError();
@@ -92,7 +93,7 @@ cudaError_t dm_gen_col(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) 
 
 template <typename R>
 cudaError_t dm_gen_out(const DMArgs<R>& a, const DMGenPlan& g, cudaStream_t st) {
-  cudaError_t e = dm_gen_allow(dm_out_gen<R>, g.smem_out);
+  cudaError_t e = dm_gen_allow(dm_out_gen<R>, 0);
   if (e != cudaSuccess) return e;
   dm_out_gen<R><<<a.pny, 256, g.smem_out, st>>>(a);
   return cudaGetLastError();

@@ -322,7 +322,8 @@ static oh_status run_ssb(oh_ctx* ctx, int kind, int nx, int ny, const void* fiel
     real = (R*)tmp;
   }
   auto kern = cols ? ssb_lines<R, true> : ssb_lines<R, false>;
-  OH_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the same limit at every length: another thread may set it between here and the launch)
+  OH_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
   {
     KernelTimer kt(ctx, "ssb_lines", st);
     kern<<<blocks, kSsbThreads, smem, st>>>(kind, (const C*)field, real, (R*)ptr, n, m, lw, pl, cols ? px.tw : py.tw);

@@ -318,6 +318,7 @@ constexpr int kRowsLoaders = 4, kRowsIssuers = 4, kRowsEpiWarps = 8;
 constexpr int kRowsIssue0 = kRowsLoaders + 1, kRowsEpi0 = kRowsIssue0 + kRowsIssuers;       // first warp of each role
 constexpr int kRowsThreads = 32 * (kRowsEpi0 + kRowsEpiWarps);
 constexpr int kRowsA_Slots = 32, kRowsB_Slots = 16;     // at most
+constexpr int kRowsSmem = 226 * 1024;                   // at most (1 KB for the biases)
 constexpr int kRowsFixed = 1024 + kRowsEpiWarps * 2048 + (2 * kRowsA_Slots + 2 * kRowsB_Slots + 8) * 8 +
                            (kRowsA_Slots + kRowsB_Slots) * 4 + 64;
 
@@ -944,7 +945,7 @@ RowsPlan rows_plan(const ConvArgs& a, int sms) {
   RowsPlan best{};
   float best_t = 0.f;
   const float cchunks = (float)(a.cin / 32);
-  const int budget = 226 * 1024 - kRowsFixed;            // (1 KB for the biases)
+  const int budget = kRowsSmem - kRowsFixed;
   for (int bn : {32, 64, 96, 128, 192, 256}) {
     if (a.cout % bn) continue;
     const int step = 3 * bn * 64;                        // weights of one (dy, 32 channels)
@@ -976,7 +977,8 @@ RowsPlan rows_plan(const ConvArgs& a, int sms) {
 template <int BN>
 oh_status launch_rows(const CUtensorMap& mX, const CUtensorMap& mW, const ConvArgs& a, const RowsPlan& p,
                       int sms, cudaStream_t st) {
-  OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_rows<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+  // (the same limit whatever the plan: another thread may set it between here and the launch)
+  OH_CUDA_TRY(cudaFuncSetAttribute(conv_fwd_rows<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
   const int ctiles = a.cout / BN;
   const long long tiles = (long long)a.n * ((a.h + p.c.rows - 1) / p.c.rows) * a.tiles_x;
   const int gx = (int)std::min(tiles, (long long)std::max(1, sms / ctiles));
