@@ -97,7 +97,9 @@ OH_FF ffc ff_cis(ff t, const float4* tab) {
   const float c = 6.28318530717958647692f;                       // 2 pi = c + cl
   const float cl = (float)(6.28318530717958647692 - (double)6.28318530717958647692f);
   const float p = OH_FMUL(r, c);
-  return ff_rotate({p, OH_FFMA(t.l, c, OH_FFMA(r, cl, OH_FFMA(r, c, -p)))}, tab[idx & 255]);
+  // (t.l is a rounding error of t, not of what is left of it: joined to the high part first,
+  // as ff_rotate leaves out its products with x^2)
+  return ff_rotate(ff_quick(p, OH_FFMA(t.l, c, OH_FFMA(r, cl, OH_FFMA(r, c, -p)))), tab[idx & 255]);
 }
 
 // Fills tab[i] with direction 2 pi i / 256; thread tid of nthr.

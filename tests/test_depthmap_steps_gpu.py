@@ -1,13 +1,17 @@
-"""FP64 frames of many evenly spaced layers: the step from layer to layer against the
-transfer function of every layer.
+"""Two-float frames where errors could build up: many evenly spaced layers, by the step from
+layer to layer against the transfer function of every layer, and phases of several turns
+(of the pixels, of the transfer function at fine pitches) against the frame in 64 bits.
 
-Tolerance: a step rounds by 2^-46 in two floats, a random walk over the layers, and its
-factor is off by 1e-14, once per layer: 250 layers 2.7e-12."""
+Tolerances: a step rounds by 2^-46 in two floats, a random walk over the layers, and its
+factor is off by 1e-14, once per layer: 250 layers 2.7e-12.  Phases: 20 turns to 2^-47, and
+2 eps of the 1.5e4 radians that the 64-bit reference evaluates whole: 5e-12."""
 import numpy as np
 import pytest
 import torch
 
-from openholo_gb300 import _lib, depthmap
+from openholo_gb300 import _lib, depthmap, scenes
+from oracle import depthmap as odm
+from test_fft_generic_gpu import reference
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +28,19 @@ def test_many_layers(ctx, monkeypatch, nx, ny, layers, pad):
         out.append(depthmap.generate(ctx, p, img, dep, precision="fp64"))
     torch.cuda.synchronize()
     assert float((out[0] - out[1]).norm()) <= 2.7e-12 * float(out[1].norm())
+
+
+@pytest.mark.parametrize("pitch,near", [(8e-6, 0.3), (1.5e-6, 0.02)])
+def test_phases_of_several_turns(ctx, pitch, near):
+    nx, ny = 128, 96
+    kw = dict(pnx=nx, pny=ny, ppx=pitch, ppy=pitch, num_of_depth=6, pad=1, near=near, far=1.1 * near,
+              transform_viewing_window=0)
+    rng = np.random.default_rng(7)
+    img, dep = (rng.integers(1, 256, (ny, nx), dtype=np.uint8) for _ in range(2))
+    phase = scenes.seeded_phase(3, ny, nx).astype(np.float32)
+    ref, _ = reference(img, dep, odm.DMParams(**kw), phase)
+    p = depthmap.make_params(phase_mode=depthmap.OH_PHASE_ARRAY, **kw)
+    f = torch.empty((ny, nx), dtype=torch.complex128, device="cuda")
+    depthmap.generate(ctx, p, *(torch.from_numpy(v).cuda() for v in (img, dep, phase)), precision="fp64", field=f)
+    torch.cuda.synchronize()
+    assert np.linalg.norm(f.cpu().numpy() - ref) <= 5e-12 * np.linalg.norm(ref)
