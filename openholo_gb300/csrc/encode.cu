@@ -251,8 +251,11 @@ __global__ void __launch_bounds__(kSsbThreads, sizeof(R) == 8 ? 2 : 3) ssb_lines
     if (odd_o) { int o = l0 + l - ho; if (o < 0) o += m; v = cmul(v, two[o]); }
     const R r = v.x * scale;
     out[COLS ? (size_t)k * m + l0 + l : (size_t)(l0 + l) * n + k] = r;
-    mn = r < mn || is_nan(r) ? r : mn;
-    mx = r > mx || is_nan(r) ? r : mx;
+    // an infinity among one or two samples does not meet its opposite in the transform, as it
+    // does in longer lines (nor its imaginary part the real ones without a third line)
+    const R e = n < 3 ? r + (R)0 * (m < 3 ? r : v.x + v.y) : r;
+    mn = e < mn || is_nan(e) ? e : mn;
+    mx = e > mx || is_nan(e) ? e : mx;
   };
   if constexpr (COLS) {
     for (int idx = threadIdx.x; idx < n << lw; idx += blockDim.x)
