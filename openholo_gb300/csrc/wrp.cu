@@ -164,9 +164,9 @@ __device__ __forceinline__ void wrp_point(const WRPGeom& g, const double* xyz, i
 // Two binnings share one count / start / list layout: 64 x 64 tiles for the
 // direct tile kernels (bins [0, nd)) and, for points the tensor-core form
 // takes (series == 2 and use_tc), 128 x 128 regions (bins [nd, nd + regions)).
-// Windows of up to half a region bin by their centre: cells of step = 128 - 2 w
-// pixels, whose points' windows all lie inside the region that starts w before
-// the cell's first pixel, so a point has one bin; the regions overlap.  Wider
+// Windows of up to three quarters of a region bin by their centre: cells of step =
+// 128 - 2 w pixels, whose points' windows all lie inside the region that starts w
+// before the cell's first pixel, so a point has one bin; the regions overlap.  Wider
 // windows bin by every region of a partition of the plane that they touch.
 constexpr int kTcR = 128;
 
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256) wrp_tile_f32(WRPGeom g, const WrpPt* __re
 // region's complex64 sum, M = 128, N = 256, K = 4 per point.  BF16 high and
 // low parts, three products (Ahi Bhi + Ahi Blo + Alo Bhi), FP32 in TMEM.
 //
-// One CTA per region, 288 threads.  Warps 0-7 write the operands of 8 points
+// One CTA per region and part of its points, 288 threads.  Warps 0-7 write the operands of 8 points
 // (K = 32) per stage straight into shared memory, in the layout a TMA load
 // with 64-byte swizzle would give, then arrive on the stage's full barrier.  A
 // warp takes a pair of point slots, alternating between them over its lanes:
@@ -633,8 +633,13 @@ __global__ void __launch_bounds__(tcw::kThreads, 2) wrp_tc(WRPGeom g, const WrpP
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int region = blockIdx.x;
   const int X0 = (region % bins.regions_x) * bins.step - bins.off, Y0 = (region / bins.regions_x) * bins.step - bins.off;
-  const int b = start[region], e = start[region + 1];
+  int b = start[region], e = start[region + 1];
   if (b == e) return;                    // uniform: no window reaches this region
+  // this CTA's part of the region's points (whole stages, 64 points at least)
+  const int parts = max(1, min((int)gridDim.y, (e - b) / 64)), per = ((e - b + parts - 1) / parts + kPts - 1) & ~(kPts - 1);
+  b += (int)blockIdx.y * per;
+  if ((int)blockIdx.y >= parts || b >= e) return;
+  e = min(e, b + per);
   const int npts = e - b;
   const int nst = (npts + kPts - 1) / kPts;
 
@@ -904,7 +909,7 @@ oh_status oh_wrp_accumulate(oh_ctx* ctx, oh_precision prec, const oh_wrp_params*
   if (n_points == 0) return OH_OK;
   WRPGeom g{p->nx, p->ny, p->pitch, p->lambda, p->z_wrp, p->window};
   const int tiles_x = (p->nx + kWrpTile - 1) / kWrpTile, tiles_y = (p->ny + kWrpTile - 1) / kWrpTile;
-  const bool centred = p->window <= kTcR / 4;           // windows of at most half a region: one bin per point
+  const bool centred = p->window <= 3 * kTcR / 8;       // windows of at most 3/4 of a region: one bin per point
   const int step = centred ? kTcR - 2 * p->window : kTcR, off = centred ? 2 * p->window : 0;
   const int regions_x = (p->nx + off - 1) / step + 1, regions_y = (p->ny + off - 1) / step + 1;
   // bins a window touches per axis: direct tiles, tensor regions
@@ -954,7 +959,10 @@ oh_status oh_wrp_accumulate(oh_ctx* ctx, oh_precision prec, const oh_wrp_params*
     OH_LAUNCH_CHECK();
     if (use_tc) {
       KernelTimer kt2(ctx, "wrp_tc", st);
-      wrp_tc<<<nregions, tcw::kThreads, tcw::kSmemBytes, st>>>(g, pts, start + ntiles, list, bins,
+      // (a few times the CTAs that fit at once: one per region left half of the SMs idle on
+      // 700 x 500 pixels, or at 1920 x 1080 with windows wider than 3/4 of a region)
+      const int parts = std::max(1, std::min(16, (4 * oh::sm_count() + nregions - 1) / nregions));
+      wrp_tc<<<dim3(nregions, parts), tcw::kThreads, tcw::kSmemBytes, st>>>(g, pts, start + ntiles, list, bins,
                                                               (float2*)wrp, ctx->dev_err);
       OH_LAUNCH_CHECK();
     }
