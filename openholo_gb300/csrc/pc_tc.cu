@@ -73,6 +73,7 @@ template <bool FINE> constexpr int kParts = FINE ? 3 : 2;         // parts of an
 template <bool FINE> constexpr int kStageBytes = 2 * kParts<FINE> * kTile;         // A's parts, then B's
 constexpr int kAccCols = 128, kTmemCols = 2 * kAccCols;   // exact products, products with remainders
 constexpr int kProducers = 8, kThreads = 32 * (kProducers + 2);
+constexpr int kMinBatches = 2;                         // of a split (see point_splits)
 constexpr int kGroup = 7;                              // batches (224 points) between additions to the partial plane
 constexpr int kPer = kBatch / kPts;                    // stages per batch
 constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // FP16 in, FP32 out
@@ -99,9 +100,44 @@ struct PcTcArgs {
   int* err;
 };
 
-// Per point: FP64 position, and whether the separable form holds over the whole
+// FP64 position of a point, and whether the separable form holds over the whole
 // plane: every dropped term below 1e-6 rad at the plane's worst corner (see the
 // head of this file), fp64: near 1e-10 rad there (see pc_tc64.cu).
+__device__ __forceinline__ PcPt prep_point(const PCGeom& g, float4 p, int fp64) {
+  PcPt o;
+  o.x = (double)p.x * g.sx; o.y = (double)p.y * g.sy; o.z = (double)p.z * g.sz + g.off;
+  o.a = p.w;
+  const double az = fabs(o.z);
+  const float U = (float)(0.5 * kCols * g.px), V = (float)(0.5 * kRows * g.py), zf = (float)az, kf = (float)g.k;
+  // |p| r0^2 = |(dx + u)^2 - dx^2| over the plane's pixels: with D the farthest
+  // pixel, a region that ends at the edge gives 2 D U - U^2, one that runs past
+  // it 2 D U + U^2 at most
+  const float DX = (float)(g.hlx + fabs(o.x)), DY = (float)(g.hly + fabs(o.y));
+  const float eu = g.nx % kCols ? U : -U, ev = g.ny % kRows ? V : -V;
+  const float iz = 1.f / zf, iz2 = iz * iz;
+  const float pm = fminf((2.f * DX + eu) * U * iz2, U * iz + U * U * iz2);
+  const float qm = fminf((2.f * DY + ev) * V * iz2, V * iz + V * V * iz2);
+  const float r0 = sqrtf((DX + U) * (DX + U) + (DY + V) * (DY + V) + zf * zf);
+  const float chi = 0.25f * kf * r0 * pm * qm, m = fmaxf(pm, qm);
+  const float turns = kf * r0 * 0.15915494f;
+  // separable form: rank-four remainder, p^2 q^2 term, series ends (phase of
+  // one axis, P and Q), and the float part of the axis phases below 4 turns
+  bool ok = m < 0.01f && chi * chi * chi * chi < 24e-6f && 0.1f * kf * r0 * pm * pm * qm * qm < 2e-7f &&
+            0.0273f * m * m * m * m * m * turns < 3e-8f && chi * 0.55f * m * m * m < 2e-7f &&
+            turns * 0.5f * fmaxf(U, V) * fmaxf(U, V) * iz2 < 4.f && fminf(U, V) * fminf(U, V) * iz2 > 1e-25f && fabsf(p.w) < 1e30f &&
+            fabs(o.x) < 1e3 && fabs(o.y) < 1e3 && az < 1e3;
+  if (fp64) {
+    // rank-six remainder; terms past p^2 q^2; the axis series' m^7 term; the column
+    // factor (scaled by the row factor's maximum over whole regions) below 0.088
+    const float c3 = chi * chi * chi, t = fmaxf(U, V) * iz, t3 = t * t * t;
+    const float qf = fminf((2.f * DY + (g.ny % kRows ? 3.f * V : -V)) * V * iz2, V * iz + V * V * iz2);
+    ok = ok && 0.25f * kf * r0 * pm * qf < 0.086f && c3 * c3 < 720.f * 1.2e-10f && kf * r0 * (pm * qm) * (pm * qm) * (pm + qm) < 1e-10f &&
+         turns * t3 * t3 * t < 3e-11f;
+  }
+  o.fast = ok ? 1 : 0;
+  return o;
+}
+
 __global__ void __launch_bounds__(128) pc_tc_prep(PCGeom g, const float4* __restrict__ in, int n, int fp64,
                                                   PcPt* __restrict__ pts, Counts* __restrict__ cnt) {
   __shared__ int hist[256];
@@ -109,39 +145,8 @@ __global__ void __launch_bounds__(128) pc_tc_prep(PCGeom g, const float4* __rest
   __syncthreads();
   int slow = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const float4 p = in[j];
-    PcPt o;
-    o.x = (double)p.x * g.sx; o.y = (double)p.y * g.sy; o.z = (double)p.z * g.sz + g.off;
-    o.a = p.w;
-    const double az = fabs(o.z);
-    const float U = (float)(0.5 * kCols * g.px), V = (float)(0.5 * kRows * g.py), zf = (float)az, kf = (float)g.k;
-    // |p| r0^2 = |(dx + u)^2 - dx^2| over the plane's pixels: with D the farthest
-    // pixel, a region that ends at the edge gives 2 D U - U^2, one that runs past
-    // it 2 D U + U^2 at most
-    const float DX = (float)(g.hlx + fabs(o.x)), DY = (float)(g.hly + fabs(o.y));
-    const float eu = g.nx % kCols ? U : -U, ev = g.ny % kRows ? V : -V;
-    const float iz = 1.f / zf, iz2 = iz * iz;
-    const float pm = fminf((2.f * DX + eu) * U * iz2, U * iz + U * U * iz2);
-    const float qm = fminf((2.f * DY + ev) * V * iz2, V * iz + V * V * iz2);
-    const float r0 = sqrtf((DX + U) * (DX + U) + (DY + V) * (DY + V) + zf * zf);
-    const float chi = 0.25f * kf * r0 * pm * qm, m = fmaxf(pm, qm);
-    const float turns = kf * r0 * 0.15915494f;
-    // separable form: rank-four remainder, p^2 q^2 term, series ends (phase of
-    // one axis, P and Q), and the float part of the axis phases below 4 turns
-    bool ok = m < 0.01f && chi * chi * chi * chi < 24e-6f && 0.1f * kf * r0 * pm * pm * qm * qm < 2e-7f &&
-                    0.0273f * m * m * m * m * m * turns < 3e-8f && chi * 0.55f * m * m * m < 2e-7f &&
-                    turns * 0.5f * fmaxf(U, V) * fmaxf(U, V) * iz2 < 4.f && fminf(U, V) * fminf(U, V) * iz2 > 1e-25f && fabsf(p.w) < 1e30f &&
-                    fabs(o.x) < 1e3 && fabs(o.y) < 1e3 && az < 1e3;
-    if (fp64) {
-      // rank-six remainder; terms past p^2 q^2; the axis series' m^7 term; the column
-      // factor (scaled by the row factor's maximum over whole regions) below 0.088
-      const float c3 = chi * chi * chi, t = fmaxf(U, V) * iz, t3 = t * t * t;
-      const float qf = fminf((2.f * DY + (g.ny % kRows ? 3.f * V : -V)) * V * iz2, V * iz + V * V * iz2);
-      ok = ok && 0.25f * kf * r0 * pm * qf < 0.086f && c3 * c3 < 720.f * 1.2e-10f && kf * r0 * (pm * qm) * (pm * qm) * (pm + qm) < 1e-10f &&
-           turns * t3 * t3 * t < 3e-11f;
-    }
-    o.fast = ok ? 1 : 0;
-    if (ok) atomicAdd(&hist[__float_as_uint(fabsf(p.w)) >> 23], 1);
+    const PcPt o = prep_point(g, in[j], fp64);
+    if (o.fast) atomicAdd(&hist[__float_as_uint(fabsf(o.a)) >> 23], 1);
     else ++slow;
     pts[j] = o;
   }
@@ -154,15 +159,34 @@ __global__ void __launch_bounds__(128) pc_tc_prep(PCGeom g, const float4* __rest
 
 // One block: the classes (see Counts and the head of this file), then the fast points'
 // indices by class and the slow points, both in input order.  With one class and no
-// slow point the index list stays unwritten (and unread).
-__global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ in, const PcPt* __restrict__ pts, int n,
+// slow point the index list stays unwritten (and unread).  PREP (n <= 1024): forms the
+// points as well, two launches fewer: where every point is refused the form is all
+// overhead (147 -> 163 us at 300 points on 512 x 512).
+template <bool PREP>
+__global__ void __launch_bounds__(1024) pc_tc_split(PCGeom g, int fp64, const float4* __restrict__ in, PcPt* pts, int n,
                                                     int* __restrict__ list, float4* __restrict__ slow,
-                                                    Counts* __restrict__ cnt) {
+                                                    Counts* cnt) {
   __shared__ int hist[256], exps[kMaxCls], first[kMaxCls + 1], count[kMaxCls], next[kMaxCls + 1], wsum[32][kMaxCls + 1];
   __shared__ int s_ncls;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < 256) hist[threadIdx.x] = cnt->hist[threadIdx.x];
-  __syncthreads();
+  int nslow;
+  if constexpr (PREP) {
+    if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+    __syncthreads();
+    bool refused = false;
+    if (threadIdx.x < n) {
+      const PcPt o = prep_point(g, in[threadIdx.x], fp64);
+      if (o.fast) atomicAdd(&hist[__float_as_uint(fabsf(o.a)) >> 23], 1);
+      refused = !o.fast;
+      pts[threadIdx.x] = o;
+    }
+    nslow = __syncthreads_count(refused);
+    if (threadIdx.x == 0) { cnt->slow = nslow; cnt->aborted = 0; }
+  } else {
+    if (threadIdx.x < 256) hist[threadIdx.x] = cnt->hist[threadIdx.x];
+    nslow = cnt->slow;
+    __syncthreads();
+  }
   if (warp == 0) {
     unsigned word[8];                                   // the exponents that occur
 #pragma unroll
@@ -204,7 +228,11 @@ __global__ void __launch_bounds__(1024) pc_tc_split(const float4* __restrict__ i
   }
   __syncthreads();
   const int ncls = s_ncls;
-  if (cnt->slow == 0 && ncls <= 1) return;
+  if (nslow == 0 && ncls <= 1) return;
+  if (nslow == n) {                                     // (nothing to sort)
+    for (int j = threadIdx.x; j < n; j += 1024) slow[j] = in[j];
+    return;
+  }
   if (threadIdx.x <= kMaxCls) next[threadIdx.x] = threadIdx.x < ncls ? first[threadIdx.x] : 0;     // [kMaxCls]: slow points
   for (int c = 0; c + 1 < ncls; ++c)
     for (int i = first[c] + count[c] + threadIdx.x; i < first[c + 1]; i += 1024) list[i] = -1;
@@ -634,11 +662,16 @@ oh_status sort_points(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, bo
   out->list = (int*)p;
   p += align256(((size_t)n + kMaxCls * kBatch) * sizeof(int));
   out->slow = (float4*)p;
-  OH_CUDA_TRY(cudaMemsetAsync(out->cnt, 0, sizeof(Counts), st));
   KernelTimer kt(ctx, "pc_tc_prep", st);
+  if (n <= 1024) {
+    pc_tc_split<true><<<1, 1024, 0, st>>>(g, fp64 ? 1 : 0, pts, out->pts, n, out->list, out->slow, out->cnt);
+    OH_LAUNCH_CHECK();
+    return OH_OK;
+  }
+  OH_CUDA_TRY(cudaMemsetAsync(out->cnt, 0, sizeof(Counts), st));
   pc_tc_prep<<<std::min((n + 127) / 128, sm_count() * 8), 128, 0, st>>>(g, pts, n, fp64 ? 1 : 0, out->pts, out->cnt);
   OH_LAUNCH_CHECK();
-  pc_tc_split<<<1, 1024, 0, st>>>(pts, out->pts, n, out->list, out->slow, out->cnt);
+  pc_tc_split<false><<<1, 1024, 0, st>>>(g, 0, pts, out->pts, n, out->list, out->slow, out->cnt);
   OH_LAUNCH_CHECK();
   return OH_OK;
 }
@@ -659,27 +692,38 @@ int point_splits(int regions, int n, int slots, int batches) {
 bool pc_tc_wants(const PCGeom& g, int n, bool fp64) {
   // FP32: the direct kernels take about 0.24 us per point (a block's serial
   // chain) or 1.1e-6 us per term, whichever sum is due; below 60 us they beat the
-  // six launches and part-filled regions here (1024x1024 x 50 points: 78 us direct, 60
-  // us here; 1024x1024 x 200: 247 and 98; 128x128 x 1000: 250 and 84).
+  // launches and part-filled regions here (1024x1024 x 60 points: 87 us direct, 48
+  // here; x 120: 148 and 69; 128x128 x 500: 128 and 58).
   // FP64: directly 3 to 7 us per point (a block's serial chain) or 73 ps per term
   // (the FP64 pipe); here 55 us at least (100x100 x 30 points: 90 us directly, 57
   // us here; 300x300 x 30: 262 and 61).
   const double terms = (double)n * g.nx * g.ny;
-  if (fp64 ? 7.0 * n + 7.3e-5 * terms < 150.0 : 0.24 * n + 1.1e-6 * terms < 60.0) return false;
+  const double direct = fp64 ? 7.0 * n + 7.3e-5 * terms : 0.24 * n + 1.1e-6 * terms;
+  if (direct < (fp64 ? 150.0 : 60.0)) return false;
+  const long long regions = (long long)((g.nx + kCols - 1) / kCols) * ((g.ny + kRows - 1) / kRows);
+  if (regions >= (1 << 24)) return false;
+  if (!fp64 && n < 4096) {
+    // Small planes have few regions, and small clouds few points to split among more
+    // CTAs: 45 us, then 0.22 us for each point of a CTA alone on its SM (128x128 x 250
+    // points: 69 us directly, 110 here in one split).
+    const int splits = point_splits((int)regions, n, 2 * sm_count(), kMinBatches);
+    const double ctas = (double)regions * splits;
+    const double share = ctas > sm_count() ? 2.0 * std::ceil(ctas / (2.0 * sm_count())) : 1.0;
+    if (direct < 1.1 * (45.0 + 0.22 * share * n / splits)) return false;
+  }
   int dev = 0, major = 0, minor = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  const long long regions = (long long)((g.nx + kCols - 1) / kCols) * ((g.ny + kRows - 1) / kRows);
-  return major == 10 && minor == 3 && regions < (1 << 24);
+  return major == 10 && minor == 3;
 }
 
 oh_status pc_tc_enqueue(oh_ctx* ctx, const PCGeom& g, const float4* pts, int n, float2* field, float* fringe,
                         bool accumulate, bool fine, const float4** slow, const int** slow_n, cudaStream_t st) {
   const int rx = (g.nx + kCols - 1) / kCols, ry = (g.ny + kRows - 1) / kRows, regions = rx * ry;
-  const int splits = point_splits(regions, n, 2 * sm_count(), 4);
+  const int splits = point_splits(regions, n, 2 * sm_count(), kMinBatches);
   const size_t plane = (size_t)g.nx * g.ny, o_part = sorted_bytes(n);
   void* ptr;
   OH_TRY(scratch(ctx, "pc.tc", o_part + plane * splits * sizeof(float2), &ptr));
