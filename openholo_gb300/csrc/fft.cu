@@ -33,32 +33,35 @@ __device__ __forceinline__ void line_fft(C* buf, int nl, int ls, int es, const F
   }
 }
 
+// (FP32 schedules in 64 registers, four blocks per SM: in the 76 that they take without a
+// bound, 1920 x 1080 rows ran 35 us instead of 26; 7680 has shared memory for three.  The
+// plan's engine spills in 64: 1280-point rows 20 us instead of 12.)
 template <typename R, int SGN, int N>
-__global__ void __launch_bounds__(256, N > 0 ? 1 : sizeof(R) == 8 ? 2 : 3) fft_rows_kernel(const typename cplx_of<R>::type* __restrict__ in,
-                                                       typename cplx_of<R>::type* __restrict__ out,
-                                                       int nx, int ny, int rpb, int shift, R scale,
-                                                       FFTPlan pl) {
+__global__ void __launch_bounds__(sizeof(R) == 8 ? 512 : 256, sizeof(R) == 8 ? 1 : N > 4320 || N == 0 ? 3 : 4)
+fft_rows_kernel(const typename cplx_of<R>::type* __restrict__ in, typename cplx_of<R>::type* __restrict__ out,
+                int nx, int ny, int rpb, uint32_t mnx, int shift, R scale, FFTPlan pl) {
   typedef typename cplx_of<R>::type C;
   extern __shared__ unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int row0 = blockIdx.x * rpb;
   const int nrows = min(rpb, ny - row0);
-  const int ls = N > 0 ? nx : pl.lens;
-  const int hx = shift ? nx / 2 : 0;
-  for (int l = 0; l < nrows; ++l) {
-    const C* src = in + (size_t)(row0 + l) * nx;
-    for (int j = threadIdx.x; j < nx; j += blockDim.x) {
-      int i = j - hx; if (i < 0) i += nx;
-      buf[l * ls + line_at<N>(pl, j)] = src[i];
-    }
+  const int n = N > 0 ? N : nx, ls = N > 0 ? N : pl.lens;
+  const int hx = shift ? n / 2 : 0;
+  // (one loop over all rows, so that several loads are in flight on short rows too; mnx: see row_divider)
+  const C* src = in + (size_t)row0 * n;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < nrows * n; idx += blockDim.x) {
+    const int l = N > 0 ? idx / n : fdiv(idx, mnx), j = idx - l * n;
+    int i = j - hx; if (i < 0) i += n;
+    buf[l * ls + line_at<N>(pl, j)] = src[l * n + i];
   }
   line_fft<N, SGN>(buf, nrows, ls, 1, pl, -1);
-  for (int l = 0; l < nrows; ++l) {
-    C* dst = out + (size_t)(row0 + l) * nx;
-    for (int k = threadIdx.x; k < nx; k += blockDim.x) {
-      int m = k - hx; if (m < 0) m += nx;     // out[k] = A[(k - hx) mod nx]
-      dst[k] = cscale(buf[l * ls + line_out<N>(pl, m)], scale);
-    }
+  C* dst = out + (size_t)row0 * n;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < nrows * n; idx += blockDim.x) {
+    const int l = N > 0 ? idx / n : fdiv(idx, mnx), k = idx - l * n;
+    int m = k - hx; if (m < 0) m += n;     // out[k] = A[(k - hx) mod n]
+    dst[idx] = cscale(buf[l * ls + line_out<N>(pl, m)], scale);
   }
 }
 
@@ -66,10 +69,9 @@ __global__ void __launch_bounds__(256, N > 0 ? 1 : sizeof(R) == 8 ? 2 : 3) fft_r
 // unshifted transform FFT2(shift(in)) as cudaFFT leaves it in its input
 // buffer (HologramKernel.cu:207-210).
 template <typename R, int SGN, int N>
-__global__ void __launch_bounds__(512) fft_cols_kernel(typename cplx_of<R>::type* data,
-                                                       typename cplx_of<R>::type* aux,
-                                                       int nx, int ny, int lw, int shift, R scale,
-                                                       FFTPlan pl) {
+__global__ void __launch_bounds__(512, N > 4096 || sizeof(R) == 8 ? 1 : 2)
+fft_cols_kernel(typename cplx_of<R>::type* data, typename cplx_of<R>::type* aux, int nx, int ny, int lw, int shift,
+                R scale, FFTPlan pl) {
   typedef typename cplx_of<R>::type C;
   extern __shared__ unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
@@ -103,6 +105,23 @@ static int rows_per_block(int nx, int lens, size_t esz) {
   return rpb;
 }
 
+// Divider of nx (see fdiv): exact for a block's elements, of which there are at most 4096, or
+// nx in one row.
+static uint32_t row_divider(int nx) { return nx > 1 ? (uint32_t)(((1ull << 32) + nx - 1) / nx) : 0u; }
+
+// Threads per block of the plan's engine for lines of `elements` values in all: about a
+// butterfly each, more while the SMs still hold all blocks at once.  512 threads of 128
+// registers for every column strip left one block per SM (4096 x 512: 33 us, 26 in 64
+// registers; 2187 x 625, one column a block: 75, 29 with 64 threads), and 32 threads for
+// each of 25 blocks doubled the time of 100 x 100.
+template <typename R>
+static int line_threads(int elements, int blocks, int most = 512) {
+  int t = most;
+  while (t > 32 && elements < 10 * t) t /= 2;
+  while (t < most && 2 * t <= elements && blocks * 2LL * t <= (long long)sm_count() * (sizeof(R) == 8 ? 512 : 768)) t *= 2;
+  return t;
+}
+
 template <typename R>
 static oh_status launch_fft2d(oh_ctx* ctx, int nx, int ny, const void* in, void* out, void* aux,
                               int direction, int shift, int normalize, cudaStream_t st) {
@@ -129,7 +148,7 @@ static oh_status launch_fft2d(oh_ctx* ctx, int nx, int ny, const void* in, void*
       cudaError_t e = cudaFuncSetAttribute(fft_rows_kernel<R, SG, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)srow);
       if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(fft_rows)"); return; }
       KernelTimer kt(ctx, "fft_rows", st);
-      fft_rows_kernel<R, SG, NX><<<(ny + rpb - 1) / rpb, 256, srow, st>>>(cin, cout_, nx, ny, rpb, shift, (R)1, px);
+      fft_rows_kernel<R, SG, NX><<<(ny + rpb - 1) / rpb, NX > 0 ? 256 : line_threads<R>(rpb * nx, (ny + rpb - 1) / rpb, sizeof(R) == 8 ? 512 : 256), srow, st>>>(cin, cout_, nx, ny, rpb, row_divider(nx), shift, (R)1, px);
       note_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) rs = cuda_fail(e, "fft_rows launch");
     });
@@ -141,7 +160,7 @@ static oh_status launch_fft2d(oh_ctx* ctx, int nx, int ny, const void* in, void*
       cudaError_t e = cudaFuncSetAttribute(fft_cols_kernel<R, SG, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol);
       if (e != cudaSuccess) { rs = cuda_fail(e, "cudaFuncSetAttribute(fft_cols)"); return; }
       KernelTimer kt(ctx, "fft_cols", st);
-      fft_cols_kernel<R, SG, NY><<<nx / W, 512, scol, st>>>(cout_, static_cast<C*>(aux), nx, ny, log2_of(W), shift, scale, py);
+      fft_cols_kernel<R, SG, NY><<<nx / W, NY > 0 ? 512 : line_threads<R>(W * ny, nx / W), scol, st>>>(cout_, static_cast<C*>(aux), nx, ny, log2_of(W), shift, scale, py);
       note_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) rs = cuda_fail(e, "fft_cols launch");
     });
@@ -164,10 +183,10 @@ static oh_status launch_fft_rows(oh_ctx* ctx, int nx, int ny, const void* in, vo
   R scale = normalize ? (R)(1.0 / (double)nx) : (R)1;
   if (direction < 0) {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_rows_kernel<R, -1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)srow));
-    fft_rows_kernel<R, -1, 0><<<(ny + rpb - 1) / rpb, 256, srow, st>>>(static_cast<const C*>(in), static_cast<C*>(out), nx, ny, rpb, 0, scale, px);
+    fft_rows_kernel<R, -1, 0><<<(ny + rpb - 1) / rpb, line_threads<R>(rpb * nx, (ny + rpb - 1) / rpb, sizeof(R) == 8 ? 512 : 256), srow, st>>>(static_cast<const C*>(in), static_cast<C*>(out), nx, ny, rpb, row_divider(nx), 0, scale, px);
   } else {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_rows_kernel<R, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)srow));
-    fft_rows_kernel<R, 1, 0><<<(ny + rpb - 1) / rpb, 256, srow, st>>>(static_cast<const C*>(in), static_cast<C*>(out), nx, ny, rpb, 0, scale, px);
+    fft_rows_kernel<R, 1, 0><<<(ny + rpb - 1) / rpb, line_threads<R>(rpb * nx, (ny + rpb - 1) / rpb, sizeof(R) == 8 ? 512 : 256), srow, st>>>(static_cast<const C*>(in), static_cast<C*>(out), nx, ny, rpb, row_divider(nx), 0, scale, px);
   }
   OH_LAUNCH_CHECK();
   return OH_OK;
@@ -192,10 +211,10 @@ static oh_status launch_fft_cols(oh_ctx* ctx, int nx, int ny, void* data, int di
   const R scale = normalize ? (R)(1.0 / (double)ny) : (R)1;
   if (direction < 0) {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_cols_kernel<R, -1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol));
-    fft_cols_kernel<R, -1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
+    fft_cols_kernel<R, -1, 0><<<nx / W, line_threads<R>(W * ny, nx / W), scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
   } else {
     OH_CUDA_TRY(cudaFuncSetAttribute(fft_cols_kernel<R, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scol));
-    fft_cols_kernel<R, 1, 0><<<nx / W, 512, scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
+    fft_cols_kernel<R, 1, 0><<<nx / W, line_threads<R>(W * ny, nx / W), scol, st>>>(static_cast<C*>(data), nullptr, nx, ny, log2_of(W), 0, scale, py);
   }
   OH_LAUNCH_CHECK();
   return OH_OK;
