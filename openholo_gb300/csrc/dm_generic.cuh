@@ -382,8 +382,12 @@ __global__ void __launch_bounds__(T, MINB) dm_col_gen(DMArgs<R> a, int lwb, int 
           if (idx < nk) {
             const C h = cmul(cmul(ex, ldg_c(ey + (idx >> lwb))), residual(kz, k));
             const C x = line[(int)pos[idx >> lwb] << lwb];
-            acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
-            acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
+            if constexpr (F64) {
+              acc[k].x = fma(h.x, x.x, fma(-h.y, x.y, acc[k].x));
+              acc[k].y = fma(h.x, x.y, fma(h.y, x.x, acc[k].y));
+            } else {
+              acc[k] = cadd(acc[k], cmul(h, x));        // (one rounding of the sum per layer)
+            }
           }
         }
       }
